@@ -222,7 +222,7 @@ int32_t capture_pcg_graph(mycel_problem* p) {
       if (!p->prof64_ev[k][j]) cudaEventCreate(&p->prof64_ev[k][j]);
     cudaGraph_t graph;
     MYCEL_CUDA(c, cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-    for (int i = 0; i < kChunkIters; ++i) launch_pcg_iteration(p, c->profile && i == 0);
+    for (int i = 0; i < kChunkIters; ++i) launch_pcg_iteration(p, i, c->profile && i == 0);
     MYCEL_CUDA(c, cudaStreamEndCapture(s, &graph));
     MYCEL_CUDA(c, cudaGraphInstantiate(&p->pcg_graph[k], graph, 0));
     cudaGraphDestroy(graph);
@@ -238,7 +238,7 @@ void launch_pcg_chunk(mycel_problem* p, int gi) {
   cudaStream_t s = p->ctx->stream;
   if (p->pcg_graph_profiled) {
     cudaEventRecord(p->prof64_ev[gi][0], s);
-    launch_matvec64(p, p->d_p, p->d_ap, 1, &p->d_state->status);
+    launch_pcg_matvec(p, 0);
     cudaEventRecord(p->prof64_ev[gi][1], s);
   }
   cudaGraphLaunch(p->pcg_graph[gi], s);
@@ -259,6 +259,8 @@ int32_t pcg_solve_fp64(mycel_problem* p, const double* d_bv, const int32_t* d_nz
   if (p->n_active_fixed < 6) return set_error(c, MYCEL_E_UNDERCONSTRAINED, underconstrained_msg(p->n_active_fixed));
   int32_t st = ensure_pcg_workspace(p);
   if (st) return st;
+  if (!p->d_p2 && dalloc(p, &p->d_p2, p->g.nd))
+    return set_error(c, MYCEL_E_OOM, "out of device memory for the PCG workspace");
   // The kernels work on p->d_x / p->d_b; bind the caller's vectors.
   if (d_xv != p->d_x) MYCEL_CUDA(c, cudaMemcpyAsync(p->d_x, d_xv, sizeof(double) * p->g.nd, cudaMemcpyDeviceToDevice, s));
   double* saved_b = p->d_b;
@@ -289,7 +291,7 @@ int32_t pcg_solve_fp64(mycel_problem* p, const double* d_bv, const int32_t* d_nz
     return MYCEL_OK;
   }
   if (hs.nonzero_x) {
-    launch_matvec64(p, p->d_x, p->d_ap, 1, nullptr);
+    launch_matvec64(p, p->d_x, p->d_ap, 1);
     launch_pcg_init_r(p, 1);
     launch_pcg_dot_rr(p);
   } else {
@@ -322,7 +324,7 @@ int32_t pcg_solve_fp64(mycel_problem* p, const double* d_bv, const int32_t* d_nz
       launch_pcg_chunk(p, gi);
       MYCEL_CUDA(c, cudaGetLastError());
       launched += p->pcg_graph_chunk;
-      c->launches += 4 * p->pcg_graph_chunk - (p->pcg_graph_profiled ? 1 : 0);  // direct matvec counted itself
+      c->launches += 3 * p->pcg_graph_chunk - (p->pcg_graph_profiled ? 1 : 0);  // direct matvec counted itself
       MYCEL_CUDA(c, cudaMemcpyAsync(slot[gi], p->d_state, sizeof(PcgState), cudaMemcpyDeviceToHost, s));
       MYCEL_CUDA(c, cudaEventRecord(evs[gi], s));
       if (k == 0) continue;
@@ -658,7 +660,7 @@ extern "C" int32_t mycel_problem_destroy(mycel_problem* p) {
   mg_release(p);
   void* ptrs[] = {p->d_domain, p->d_nflags, p->d_fixed, p->d_err, p->d_active, p->d_e2a, p->d_F, p->d_b, p->d_fnz, p->d_bnz, p->d_rho_box,
                   p->d_case_F, p->d_case_b, p->d_case_nz,
-                  p->d_E, p->d_Ef, p->d_diag, p->d_invd, p->d_invdf, p->d_r, p->d_z, p->d_p, p->d_ap, p->d_x,
+                  p->d_E, p->d_Ef, p->d_diag, p->d_invd, p->d_invdf, p->d_r, p->d_z, p->d_p, p->d_p2, p->d_ap, p->d_x,
                   p->d_part, p->d_state, p->f_x, p->f_r, p->f_z, p->f_p0, p->f_p1, p->f_ap, p->d_r64, p->d_part2,
                   p->d_tmp0, p->d_tmp1, p->g_x, p->g_r, p->g_z, p->g_p0, p->g_p1, p->g_ap, p->g_invd};
   for (void* q : ptrs) dfree(p->ctx->stream, q);
@@ -843,7 +845,7 @@ extern "C" int32_t mycel_apply_k(mycel_problem* p, const double* x, double* y, i
     int32_t st = fast64_apply_k(p, p->d_tmp0, p->d_tmp1, projected);
     if (st) return st;
   } else {
-    launch_matvec64(p, p->d_tmp0, p->d_tmp1, projected, nullptr);
+    launch_matvec64(p, p->d_tmp0, p->d_tmp1, projected);
   }
   MYCEL_CUDA(p->ctx, cudaMemcpyAsync(y, p->d_tmp1, sizeof(double) * p->g.nd, cudaMemcpyDeviceToHost, s));
   MYCEL_CUDA(p->ctx, cudaStreamSynchronize(s));
@@ -1018,7 +1020,7 @@ extern "C" int32_t mycel_static_solve(mycel_problem* p, const mycel_static_optio
   launch_compliance(p, p->d_x, d_sc);
   launch_max_disp(p, p->d_x, d_sc + 1);
   if (reactions_out) {
-    launch_matvec64(p, p->d_x, p->d_ap, 0, nullptr);  // ApplyK(u) (StaticAnalysis.cs:103-110)
+    launch_matvec64(p, p->d_x, p->d_ap, 0);  // ApplyK(u) (StaticAnalysis.cs:103-110)
     launch_reactions(p, p->d_ap, p->d_tmp1, p->d_fixed, (int32_t)p->fixed_host.size());
     MYCEL_CUDA(c, cudaMemcpyAsync(reactions_out, p->d_tmp1, sizeof(double) * p->g.nd, cudaMemcpyDeviceToHost, s));
   }

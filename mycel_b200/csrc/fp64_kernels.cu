@@ -5,23 +5,23 @@
 //   k_matvec64      FemOperator.ApplyK/ApplyA (Fem/FemOperator.cs:196-294, MultiplyElementUnsafe :379-422).
 //                   Node-centric gather: one thread per node sums its <= 8 element contributions in the
 //                   8-colour order the reference scatters them, each contribution computed with the
-//                   reference's scale-then-dot order (ue = x*E; four lane chains; Vector256.Sum).
-//                   Threads are grouped by node parity class so every warp follows the same colour order and
-//                   reads the same KE rows (broadcast from the kernel parameter bank).
+//                   reference's scale-then-dot order (ue = x*E; four lane chains; Vector256.Sum). In the
+//                   PCG it also forms the direction (ProcessUpdatePChunk, Fem/PcgSolver.cs:529-553).
 //   k_diag          FemOperator.AssembleDiagonal (:143-172), same colour order; Jacobi inverse (JacobiPreconditioner.cs:25).
 //   k_dot_exact     PcgSolver DotParallel/ProcessDotChunk (Fem/PcgSolver.cs:385-450): one CTA per 8192-block,
 //                   producer warps stage products in shared memory, lanes 0-3 of warp 0 run the four
 //                   sequential lane chains, the last CTA adds the block partials in block order.
 //   k_xr_exact      ProcessUpdateXrNormChunk + ProcessApplyPrecDotChunk (:452-527) fused: two chain sets.
-//   k_update_p      ProcessUpdatePChunk (:529-553).
 //   k_filter_*      DensityFilter (Optimization/DensityFilter.cs:34-303) as a stencil in the reference's
 //                   neighbour order (jz, jy, jx ascending), weights (rmin - dist) * invHs_row.
 //   k_sens          SensitivityAnalysis (Optimization/SensitivityAnalysis.cs:98-144).
 //   k_oc            OcOptimizer.Update (Optimization/OcOptimizer.cs:12-175): one persistent cooperative kernel.
 #include <algorithm>
+#include <atomic>
 #include <mutex>
 #include <string>
 #include <cooperative_groups.h>
+#include <cuda_pipeline.h>
 #include <cuda_runtime.h>
 #include <math.h>
 #include <stdint.h>
@@ -32,17 +32,12 @@
 namespace mycel {
 
 constexpr int kBlock = 8192;  // PcgSolver.BlockSize
-constexpr int kChunk = 1024;  // products staged per shared-memory buffer
-constexpr int kDotThreads = 256;
 
 // ---------------------------------------------------------------------------------------------------------
 // helpers
 // ---------------------------------------------------------------------------------------------------------
-__device__ __forceinline__ double lane_sum(int mode, double a0, double a1, double a2, double a3) {
-  // Vector256<double>.Sum: Sum(lower) + Sum(upper) on .NET 8+ (mode 0); alternatives for the noise-floor study.
-  if (mode == 1) return (a0 + a2) + (a1 + a3);
-  if (mode == 2) return ((a0 + a1) + a2) + a3;
-  return (a0 + a1) + (a2 + a3);
+__device__ __forceinline__ double lane_sum(double a0, double a1, double a2, double a3) {
+  return (a0 + a1) + (a2 + a3);  // Vector256<double>.Sum: Sum(lower) + Sum(upper) on .NET 8+
 }
 
 // Math.Pow on the path (FemOperator.cs:100,133; SensitivityAnalysis.cs:93-95): the host C library's pow,
@@ -54,6 +49,17 @@ __device__ __forceinline__ int local_index(int ox, int oy, int oz) {
   // Hex8 local node order (Hex8Element.cs:8-16): (0,0,0),(1,0,0),(1,1,0),(0,1,0), then the same at z=1
   int base = oy ? (ox ? 2 : 3) : (ox ? 1 : 0);
   return base + 4 * oz;
+}
+
+// dynamic shared memory above 48 KB, allowed once per kernel and device
+template <auto K>
+static void allow_smem(int device, size_t bytes) {
+  static std::atomic<uint64_t> done[4];
+  if (device < 0 || device >= 256) device = 255;
+  const uint64_t bit = 1ull << (device & 63);
+  if (done[device >> 6].load(std::memory_order_acquire) & bit) return;
+  cudaFuncSetAttribute(K, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  done[device >> 6].fetch_or(bit, std::memory_order_release);
 }
 
 __device__ __forceinline__ double ld_volatile(const double* p) { return *(const volatile double*)p; }
@@ -215,211 +221,399 @@ void launch_diag(mycel_problem* p) {
 
 // ---------------------------------------------------------------------------------------------------------
 // y = K x (projected: y = x on constrained DOFs, ApplyA with xIsAlreadyProjected)
-// z-marching shared-memory tiles: a CTA owns 64 x 4 nodes and marches over ZSEG node planes; three planes of x
-// (one-node halo) and two element planes of E and the domain live in shared memory. Warp w handles the nodes
-// of one parity in x (i = i0 + 2 lane + (w & 1)) of row j0 + (w >> 1), so the colour order of the incident
-// elements, and the KE rows they read, are the same for the whole warp. The shared planes are stored
-// parity-split in x, so a warp's 8-byte loads hit consecutive words.
+// Bound by the FP64 pipe: 1,344 separately rounded operations per node (8 elements x (24 scalings + 3 rows of
+// 47), 24 adds). A CTA takes kMvNodes consecutive nodes of one node plane, in node order over rows (no lane is
+// lost to a tile edge), stages their neighbourhood in the planes k-1, k, k+1 in shared memory with 16-byte
+// asynchronous copies, all in flight at once, and each thread forms its node's eight contributions with
+// compile-time element positions, so that the KE entries are constant-bank operands and nothing but 24 shared
+// loads and the arithmetic is left per element; the contributions are kept and added in the colour order of the
+// node's parity (selects for x and y, a uniform branch for z). A lane chain is finished before the next is begun,
+// which keeps the live registers low.
+// FUSE: x = z + beta p_old (or z at a start), formed in shared memory; the owned nodes' values go to p_new, so the
+// iteration needs no pass of its own for p.
+// Against the z-marching 64 x 4 tiles this replaces (per-node runtime KE rows), p update included: 30x10x4 elements
+// 29.9 -> 6.7 us, 96x48x24 51.3 -> 20.6 us, 192x96x96 446 (without p) -> 256 us. What is left over the FP64 pipe's
+// 10 and 133 us are issue slots: a constant load for each KE entry and the selects of the colour order.
 // ---------------------------------------------------------------------------------------------------------
-constexpr int MX = 64, MY = 4;
-constexpr int MPX = MX + 2, MPY = MY + 2;   // node plane with halo
-constexpr int MEX = MX + 1, MEY = MY + 1;   // element plane
-constexpr int MPXH = (MPX + 1) / 2, MEXH = (MEX + 1) / 2;
+constexpr int kMvNodes = 128;
 
-__device__ __forceinline__ int psplit(int lx, int half) { return (lx & 1) * half + (lx >> 1); }
+// Staged ranges of a plane, in doubles: one contiguous range of the CTA's nodes and the rows before and after
+// (row pitch nx1), or, for rows longer than the CTA's span, three (one per node row). A range starts at the even
+// global index at or below its first entry (16-byte copies).
+struct MvStage {
+  int pitch;    // node positions between neighbouring rows
+  int nseg;     // ranges per plane
+  int seglen;   // doubles of a range
+  int segstep;  // doubles between ranges in shared memory (even)
+};
+__host__ __device__ inline MvStage mv_stage(int nx1) {
+  MvStage m;
+  const bool rows3 = nx1 > kMvNodes + 2;
+  m.pitch = rows3 ? kMvNodes + 2 : nx1;
+  m.nseg = rows3 ? 3 : 1;
+  m.seglen = 3 * (rows3 ? kMvNodes + 2 : kMvNodes + 2 + 2 * nx1);
+  m.segstep = (m.seglen + 3) & ~1;
+  return m;
+}
+inline size_t mv_smem(int nx1, bool fuse) {
+  const MvStage m = mv_stage(nx1);
+  return sizeof(double) * 3 * (size_t)m.nseg * m.segstep * (fuse ? 2 : 1);
+}
 
-__global__ void __launch_bounds__(256) k_matvec64(GridDims g, const __grid_constant__ KeD ke,
-                                                  const double* __restrict__ x, double* __restrict__ y,
-                                                  const double* __restrict__ E, const uint8_t* __restrict__ dom,
-                                                  const uint8_t* __restrict__ nf, int projected, int mode,
-                                                  const int* __restrict__ status, int zseg) {
-  __shared__ double xs[3][3][MPY][2 * MPXH];  // [slot][c][ly][parity-split lx]
-  __shared__ double es[2][MEY][2 * MEXH];
-  __shared__ uint8_t ds[2][MEY][2 * MEXH];
-  if (status && *status != PCG_RUNNING) return;
-  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-  const int px = w & 1, ty = w >> 1;
-  const int i0 = blockIdx.x * MX, j0 = blockIdx.y * MY, k0 = blockIdx.z * zseg;
-  const int k1 = min(k0 + zseg, g.nz1);
-  const int64_t sy = g.nx1, sz = (int64_t)g.nx1 * g.ny1;
-
-  auto load_plane = [&](int kk, int slot) {
-    for (int q = tid; q < MPY * MPX * 3; q += 256) {
-      int c = q % 3, rest = q / 3, lx = rest % MPX, ly = rest / MPX;
-      int i = i0 - 1 + lx, j = j0 - 1 + ly;
-      double v = 0.0;
-      if (kk >= 0 && kk < g.nz1 && i >= 0 && i < g.nx1 && j >= 0 && j < g.ny1) v = __ldg(x + 3 * (i + sy * j + sz * kk) + c);
-      xs[slot][c][ly][psplit(lx, MPXH)] = v;
-    }
+template <int FUSE>
+__global__ void __launch_bounds__(kMvNodes, 4) k_matvec64(GridDims g, const __grid_constant__ KeD ke,
+                                                          const double* __restrict__ x, const double* __restrict__ pold,
+                                                          double* __restrict__ pnew, double* __restrict__ y,
+                                                          const double* __restrict__ E, const uint8_t* __restrict__ dom,
+                                                          const uint8_t* __restrict__ nf, int projected,
+                                                          const PcgState* __restrict__ st, unsigned chunks) {
+  extern __shared__ __align__(16) double xs[];  // [plane k-1, k, k+1][range][position][component]; FUSE: then p_old's
+  const int tid = threadIdx.x;
+  const int k = (int)(blockIdx.x / chunks);
+  const int np = g.nx1 * g.ny1;  // nodes of a plane (all DOF indices fit in 31 bits)
+  const int n0 = (int)(blockIdx.x - (unsigned)k * chunks) * kMvNodes;
+  const MvStage m = mv_stage(g.nx1);
+  const int half = 3 * m.nseg * m.segstep;
+  const int status = st ? st->status : PCG_RUNNING;
+  const double beta = FUSE ? st->beta : 0.0;
+  const bool first = FUSE ? st->first != 0 : false;
+  const int64_t top = (g.nd + 1) & ~int64_t(1);  // vectors are allocated in multiples of 16 bytes
+  // first entry of range sgm of plane pl in the global vector (may lie before it)
+  auto range = [&](int pl, int sgm) -> int64_t {
+    return (int64_t)3 * np * (k - 1 + pl) + 3 * (n0 - 1 + (m.nseg == 3 ? (sgm - 1) * g.nx1 : -g.nx1));
   };
-  auto load_eplane = [&](int ke_, int slot) {
-    for (int q = tid; q < MEY * MEX; q += 256) {
-      int lx = q % MEX, ly = q / MEX;
-      int ie = i0 - 1 + lx, je = j0 - 1 + ly;
-      double v = 0.0;
-      uint8_t d = 0;
-      if (ke_ >= 0 && ke_ < g.nz && ie >= 0 && ie < g.nx && je >= 0 && je < g.ny) {
-        int64_t e = ie + (int64_t)g.nx * (je + (int64_t)g.ny * ke_);
-        d = __ldg(dom + e);
-        if (d) v = __ldg(E + e);
-      }
-      es[slot][ly][psplit(lx, MEXH)] = v;
-      ds[slot][ly][psplit(lx, MEXH)] = d;
+  int off[3][3];  // staged position of the CTA's first node in row dy of plane pl
+#pragma unroll
+  for (int pl = 0; pl < 3; ++pl)
+#pragma unroll
+    for (int dy = 0; dy < 3; ++dy) {
+      const int sgm = m.nseg == 3 ? dy : 0;
+      off[pl][dy] = (pl * m.nseg + sgm) * m.segstep + (int)(range(pl, sgm) & 1) + (m.nseg == 3 ? 0 : 3 * dy * m.pitch);
     }
-  };
-
-  load_plane(k0 - 1, (k0 + 2) % 3);
-  load_plane(k0, k0 % 3);
-  load_eplane(k0 - 1, (k0 + 1) & 1);
-  const int lxn = 1 + 2 * lane + px;  // plane-local x of this thread's node
-  const int i = i0 + lxn - 1, j = j0 + ty;
-  const bool mine = i < g.nx1 && j < g.ny1;
-  for (int k = k0; k < k1; ++k) {
-    load_plane(k + 1, (k + 1) % 3);
-    load_eplane(k, k & 1);
-    __syncthreads();
-    if (mine) {
-      double acc[3] = {0.0, 0.0, 0.0};
-#pragma unroll 1
-      for (int col = 0; col < 8; ++col) {
-        // node offset inside the element of colour col, and the element's local position
-        const int ox = (col & 1) ^ (i & 1), oy = ((col >> 1) & 1) ^ (j & 1), oz = ((col >> 2) & 1) ^ (k & 1);
-        const int sx = 1 - ox, sy_ = 1 - oy, sz_ = 1 - oz;  // element offset from (i-1, j-1, k-1)
-        const int lxe = lxn - 1 + sx, lye = ty + sy_;      // element plane coordinates
-        const int eslot = (k - 1 + sz_) & 1;
-        const uint8_t act = ds[eslot][lye][psplit(lxe, MEXH)];
-        if (!act) continue;  // outside the grid or inactive: no contribution
-        const double ee = es[eslot][lye][psplit(lxe, MEXH)];
-        double ue[24];
-#pragma unroll
-        for (int b = 0; b < 8; ++b) {
-          const int bx = (b == 1 || b == 2 || b == 5 || b == 6) ? 1 : 0;
-          const int by = (b == 2 || b == 3 || b == 6 || b == 7) ? 1 : 0;
-          const int bz = b >= 4 ? 1 : 0;
-          const int slot = (k - 1 + sz_ + bz + 3) % 3;
-          const int lx = lxn - 1 + sx + bx, ly = ty + sy_ + by;
-#pragma unroll
-          for (int c = 0; c < 3; ++c) ue[3 * b + c] = xs[slot][c][ly][psplit(lx, MPXH)] * ee;
-        }
-        const int a = (oy ? (ox ? 2 : 3) : (ox ? 1 : 0)) + 4 * oz;
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-          const double* row = ke.v + (3 * a + c) * 24;
-          double l[4];
-#pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            double s = row[q] * ue[q] + row[4 + q] * ue[4 + q];
-            s = s + row[8 + q] * ue[8 + q];
-            s = s + row[12 + q] * ue[12 + q];
-            s = s + row[16 + q] * ue[16 + q];
-            s = s + row[20 + q] * ue[20 + q];
-            l[q] = s;
-          }
-          acc[c] = acc[c] + lane_sum(mode, l[0], l[1], l[2], l[3]);
-        }
+  for (int pl = 0; pl < 3; ++pl) {
+    if (k - 1 + pl < 0 || k - 1 + pl >= g.nz1) continue;  // read by no contributing element
+    for (int sgm = 0; sgm < m.nseg; ++sgm) {
+      const int64_t f0 = range(pl, sgm), a0 = f0 & ~int64_t(1);
+      double* dst = xs + (pl * m.nseg + sgm) * m.segstep;
+      const int n2 = (int)((f0 - a0 + m.seglen + 1) >> 1);
+      for (int q = tid; q < n2; q += kMvNodes) {
+        const int64_t f = a0 + 2 * q;
+        if (f < 0 || f >= top) continue;
+        __pipeline_memcpy_async(dst + 2 * q, x + f, 16);
+        if (FUSE) __pipeline_memcpy_async(dst + half + 2 * q, pold + f, 16);
       }
-      const int64_t n = i + sy * j + sz * k;
-      const uint8_t f = projected ? nf[n] : 0;
-      const int cslot = k % 3;
+    }
+  }
+  __pipeline_commit();
+  const int nl = n0 + tid, n = nl < np ? nl : np - 1;
+  const int j = n / g.nx1, i = n - j * g.nx1;
+  const bool mine = nl < np;
+  // the node's elements (i-1+sx, j-1+sy, k-1+sz): E and whether they contribute
+  double ee[8];
+  unsigned act = 0;
 #pragma unroll
-      for (int c = 0; c < 3; ++c)
-        y[3 * n + c] = (f & (1 << c)) ? xs[cslot][c][ty + 1][psplit(lxn, MPXH)] : acc[c];
+  for (int v = 0; v < 8; ++v) {
+    const int ex = i - 1 + (v & 1), ey = j - 1 + ((v >> 1) & 1), ez = k - 1 + (v >> 2);
+    const bool in = mine && ex >= 0 && ex < g.nx && ey >= 0 && ey < g.ny && ez >= 0 && ez < g.nz;
+    const int64_t e = ex + (int64_t)g.nx * (ey + (int64_t)g.ny * ez);
+    if (in && dom[e]) act |= 1u << v;
+    ee[v] = in ? E[e] : 0.0;
+  }
+  __pipeline_wait_prior(0);
+  __syncthreads();
+  if (status != PCG_RUNNING) return;
+  if (FUSE && !first) {
+    double2 *z2 = reinterpret_cast<double2*>(xs), *q2 = reinterpret_cast<double2*>(xs + half);
+    for (int q = tid; q < half / 2; q += kMvNodes) {
+      const double2 zv = z2[q], pv = q2[q];
+      z2[q] = make_double2(zv.x + beta * pv.x, zv.y + beta * pv.y);
     }
     __syncthreads();
   }
+  double wl[4][3], wu[4][3];  // the elements below and above the node plane: [colour order][component]
+  const bool io = i & 1, jo = j & 1;
+  const double* xt = xs + 3 * (tid + 1);
+#pragma unroll 1  // half the code: the unrolled body waits for instructions (256 against 267 us on 192x96x96)
+  for (int sz = 0; sz < 2; ++sz) {
+    const double* kz = ke.v + (1 - sz) * (4 * 3 * 24);  // KE rows of the node's local position in these elements
+    const unsigned on4 = act >> (4 * sz);
+    double e4[4];
+    int o[2][3];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) e4[q] = sz ? ee[4 + q] : ee[q];
+#pragma unroll
+    for (int dy = 0; dy < 3; ++dy) {
+      o[0][dy] = sz ? off[1][dy] : off[0][dy];
+      o[1][dy] = sz ? off[2][dy] : off[1][dy];
+    }
+    double v[2][2][3];
+#pragma unroll
+    for (int sy = 0; sy < 2; ++sy)
+#pragma unroll
+      for (int sx = 0; sx < 2; ++sx) {
+        const int el = sx + 2 * sy;
+        const bool on = on4 >> el & 1;
+        if (!__any_sync(0xffffffffu, on)) {
+#pragma unroll
+          for (int c = 0; c < 3; ++c) v[sy][sx][c] = 0.0;
+          continue;
+        }
+        const int a = (1 - sy) ? ((1 - sx) ? 2 : 3) : ((1 - sx) ? 1 : 0);
+        double s01[3], s[3], s23[3];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+#pragma unroll
+          for (int t = 0; t < 6; ++t) {
+            const int col = q + 4 * t, b = col / 3, cb = col % 3;
+            const int bx = (b == 1 || b == 2 || b == 5 || b == 6) ? 1 : 0;
+            const int by = (b == 2 || b == 3 || b == 6 || b == 7) ? 1 : 0;
+            const int bz = b >= 4 ? 1 : 0;
+            const double ue = xt[o[bz][sy + by] + 3 * (sx - 1 + bx) + cb] * e4[el];
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+              const double pr = kz[(3 * a + c) * 24 + col] * ue;
+              s[c] = t == 0 ? pr : s[c] + pr;
+            }
+          }
+#pragma unroll
+          for (int c = 0; c < 3; ++c) {  // Vector256.Sum: (l0 + l1) + (l2 + l3)
+            if (q == 0) s01[c] = s[c];
+            else if (q == 1) s01[c] = s01[c] + s[c];
+            else if (q == 2) s23[c] = s[c];
+            else s23[c] = s23[c] + s[c];
+          }
+        }
+        // an element that does not contribute adds +0, which leaves the running sum (never -0) as it is
+#pragma unroll
+        for (int c = 0; c < 3; ++c) v[sy][sx][c] = on ? s01[c] + s23[c] : 0.0;
+      }
+    // colour order: even element row first (sy = 0 when j is odd), in it the even element first
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      const double a0 = jo ? v[0][0][c] : v[1][0][c], a1 = jo ? v[0][1][c] : v[1][1][c];
+      const double b0 = jo ? v[1][0][c] : v[0][0][c], b1 = jo ? v[1][1][c] : v[0][1][c];
+      const double t0 = io ? a0 : a1, t1 = io ? a1 : a0, t2 = io ? b0 : b1, t3 = io ? b1 : b0;
+      if (sz == 0) wl[0][c] = t0, wl[1][c] = t1, wl[2][c] = t2, wl[3][c] = t3;
+      else wu[0][c] = t0, wu[1][c] = t1, wu[2][c] = t2, wu[3][c] = t3;
+    }
+  }
+  if (!mine) return;
+  double acc[3] = {0.0, 0.0, 0.0};
+  if (k & 1) {  // the plane below has even elements
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+#pragma unroll
+      for (int q = 0; q < 8; ++q) acc[c] = acc[c] + (q < 4 ? wl : wu)[q & 3][c];
+  } else {
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+#pragma unroll
+      for (int q = 0; q < 8; ++q) acc[c] = acc[c] + (q < 4 ? wu : wl)[q & 3][c];
+  }
+  const int64_t nn = n + (int64_t)np * k;
+  const uint8_t f = projected ? nf[nn] : 0;
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    const double xv = xt[off[1][1] + c];
+    y[3 * nn + c] = (f & (1 << c)) ? xv : acc[c];
+    if (FUSE) pnew[3 * nn + c] = xv;
+  }
 }
 
-// z-segment length giving about 8 CTAs per SM (at least 2 planes per segment)
-inline int matvec64_zseg(const GridDims& g, int num_sms) {
-  int64_t txy = (int64_t)((g.nx1 + MX - 1) / MX) * ((g.ny1 + MY - 1) / MY);
-  int64_t segs = std::max<int64_t>(1, (8 * (int64_t)num_sms + txy - 1) / txy);
-  return (int)std::max<int64_t>(2, (g.nz1 + segs - 1) / segs);
-}
-
-void launch_matvec64(mycel_problem* p, const double* x, double* y, int projected, const int* d_status) {
+template <int FUSE>
+static void launch_mv(mycel_problem* p, const double* x, const double* pold, double* pnew, double* y, int projected,
+                      const PcgState* st) {
   const GridDims& g = p->g;
-  int zs = matvec64_zseg(g, p->ctx->num_sms);
-  dim3 grid((unsigned)((g.nx1 + MX - 1) / MX), (unsigned)((g.ny1 + MY - 1) / MY), (unsigned)((g.nz1 + zs - 1) / zs));
-  k_matvec64<<<grid, 256, 0, p->ctx->stream>>>(g, p->ke, x, y, p->d_E, p->d_domain, p->d_nflags, projected,
-                                               p->lane_mode, d_status, zs);
+  const unsigned chunks = (unsigned)(((int64_t)g.nx1 * g.ny1 + kMvNodes - 1) / kMvNodes);
+  allow_smem<k_matvec64<FUSE>>(p->ctx->device, std::max(mv_smem(kMvNodes + 2, FUSE != 0), mv_smem(kMvNodes + 3, FUSE != 0)));
+  k_matvec64<FUSE><<<chunks * (unsigned)g.nz1, kMvNodes, mv_smem(g.nx1, FUSE != 0), p->ctx->stream>>>(
+      g, p->ke, x, pold, pnew, y, p->d_E, p->d_domain, p->d_nflags, projected, st, chunks);
   p->ctx->launches++;
+}
+
+void launch_matvec64(mycel_problem* p, const double* x, double* y, int projected) {
+  launch_mv<0>(p, x, nullptr, nullptr, y, projected, nullptr);
+}
+
+void launch_pcg_matvec(mycel_problem* p, int it) {
+  launch_mv<1>(p, p->d_z, it & 1 ? p->d_p : p->d_p2, it & 1 ? p->d_p2 : p->d_p, p->d_ap, 1, p->d_state);
 }
 
 // ---------------------------------------------------------------------------------------------------------
 // exact block/lane reductions
 // ---------------------------------------------------------------------------------------------------------
-// Sequential 4-lane chain consumer: lanes 0..3 of the calling warp add buf[lane], buf[lane+4], ... in order.
-__device__ __forceinline__ double chain4(double acc, const double* buf, int m, int lane4) {
-  int q = lane4;
-  for (; q + 28 < m; q += 32) {
-    double v0 = buf[q], v1 = buf[q + 4], v2 = buf[q + 8], v3 = buf[q + 12];
-    double v4 = buf[q + 16], v5 = buf[q + 20], v6 = buf[q + 24], v7 = buf[q + 28];
-    acc = acc + v0; acc = acc + v1; acc = acc + v2; acc = acc + v3;
-    acc = acc + v4; acc = acc + v5; acc = acc + v6; acc = acc + v7;
+// One CTA per 8192-block: producer warps form the products chunk by chunk and stage them in shared memory, a row
+// per lane chain; lanes 0-3 of a warp run the sequential chains of a set.
+// What bounds it is the chain: 2,048 dependent additions of 8.1 cycles (8.5 us at 1.965 GHz). Everything else is
+// kept out of its way: a ring of kRing chunks is handed over by named barriers (no CTA-wide barrier stops a chain
+// for a producer's loads), the producers' accesses are contiguous over a warp (their traffic delays the chain's
+// loads: at a 32-byte stride the fused update's chain took 13.8 cycles an addition, now 11.7), and one group of
+// producers keeps ahead of the chain (two, or all chunks resident, were slower). 96x48x24 elements (44 blocks):
+// the direction's dot 22.0 -> 14.9 us, the fused update 30.8 -> 18.8 us; one block (30x10x4): 15.1 -> 9.3 and
+// 22.5 -> 10.8 us; 192x96x96 (666 blocks, bound by memory): 39 and 71 us.
+constexpr int kCh = 768;                         // elements per chunk
+constexpr int kRing = 4;                         // chunks in shared memory
+constexpr int kRow = kCh / 4 + 4;                // doubles per staged lane row (no bank conflicts)
+constexpr int kProd = kCh / 4;                   // producer threads, two pairs of elements each
+constexpr int chain_threads(int sets) { return 32 * sets + kProd; }
+static_assert(2 * kRing < 15 && kProd % 32 == 0 && kRow % 8 == 4, "barrier ids 1 .. 2 kRing, 15 hands a set over");
+
+template <int SETS>
+__device__ __forceinline__ void nb_sync(int id) {
+  asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(32 * SETS + kProd) : "memory");
+}
+template <int SETS>
+__device__ __forceinline__ void nb_arrive(int id) {
+  asm volatile("bar.arrive %0, %1;" ::"r"(id), "n"(32 * SETS + kProd) : "memory");
+}
+
+// acc + row[0] + row[1] + ... + row[m - 1], in that order (m <= kProd). A whole row is unrolled, so that the loads
+// run ahead of the additions (8.8 cycles an addition; loops over batches of 16 or 32 took 9.8 to 10.7).
+__device__ __forceinline__ double chain_row(double acc, const double* row, int m) {
+  const double2* r2 = reinterpret_cast<const double2*>(row);
+  if (m == kProd) {
+#pragma unroll
+    for (int q = 0; q < kProd / 2; ++q) {
+      const double2 v = r2[q];
+      acc = acc + v.x;
+      acc = acc + v.y;
+    }
+    return acc;
   }
-  for (; q < m; q += 4) acc = acc + buf[q];
+  int q = 0;
+  for (; q + 32 <= m; q += 32) {
+#pragma unroll
+    for (int k = 0; k < 16; ++k) {
+      const double2 v = r2[q / 2 + k];
+      acc = acc + v.x;
+      acc = acc + v.y;
+    }
+  }
+  for (; q < m; ++q) acc = acc + row[q];
   return acc;
 }
 
-// Last-CTA election for the final, block-ordered sum (returns true in exactly one CTA, for all its threads).
-__device__ __forceinline__ bool elect_last(unsigned int* counter) {
-  __shared__ bool last;
-  __threadfence();
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    unsigned int prev = atomicAdd(counter, 1u);
-    last = (prev == gridDim.x - 1);
+// The chains of one block over np pairs of elements (np even), SETS chain sets. A producer thread takes the pairs h
+// and h + kProd of a chunk (a warp's accesses are contiguous): load(q, h) fetches pair h as the thread's q-th,
+// store(q, h, put) gives its products to put(set, second, value). Pair h's entries belong to lanes 2 (h & 1) and
+// 2 (h & 1) + 1, column h >> 1. The caller has loaded the first chunk's pairs (first_pair) before it looks at the
+// solve's status. Returns lane l's chain of set w in lane l of warp w.
+template <int SETS>
+__device__ __forceinline__ int first_pair() {
+  return (int)threadIdx.x - 32 * SETS;
+}
+
+template <int SETS, class Load, class Store>
+__device__ __forceinline__ double block_chains(int np, double (*buf)[SETS][4][kRow], Load&& load, Store&& store) {
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int nch = (np + 2 * kProd - 1) / (2 * kProd);
+  double acc = 0.0;
+  if (tid >= 32 * SETS) {
+    const int pt = tid - 32 * SETS;
+    for (int t = 0; t < nch; ++t) {
+      if (t >= kRing) nb_sync<SETS>(1 + kRing + t % kRing);
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        const int c = pt + q * kProd, h = 2 * kProd * t + c;
+        if (h < np) store(q, h, [&](int set, int second, double v) { buf[t % kRing][set][2 * (c & 1) + second][c >> 1] = v; });
+      }
+      nb_arrive<SETS>(1 + t % kRing);
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        const int h = 2 * kProd * (t + 1) + pt + q * kProd;
+        if (h < np) load(q, h);
+      }
+    }
+  } else {
+    const int set = tid >> 5;
+    for (int t = 0; t < nch; ++t) {
+      nb_sync<SETS>(1 + t % kRing);
+      if (lane < 4)
+        acc = chain_row(acc, buf[t % kRing][set][lane], min(kProd, (np >> 1) - t * kProd));
+      __syncwarp();
+      if (t + kRing < nch) nb_arrive<SETS>(1 + kRing + t % kRing);
+    }
   }
-  __syncthreads();
-  if (last) __threadfence();
-  return last;
+  return acc;
+}
+
+// The block partials' final sums, by warp 0 of the last CTA to arrive: lane 0 publishes the CTA's partials (s1
+// only when SETS is 2) and counts it in; the last one's warp adds part[0], part[1], ... in block order (its lanes
+// load 32 partials at once, shuffles keep the order). True in the last CTA's warp 0, whose lanes all get the sums.
+// One block needs none of it.
+template <int SETS>
+__device__ __forceinline__ bool sum_blocks(double* part, unsigned* counter, double& s0, double& s1) {
+  const unsigned nb = gridDim.x, lane = threadIdx.x & 31;
+  if (nb == 1) {
+    s0 = 0.0 + s0;
+    s1 = 0.0 + s1;
+    return true;
+  }
+  unsigned prev = 0;
+  if (lane == 0) {
+    part[blockIdx.x] = s0;
+    if (SETS == 2) part[nb + blockIdx.x] = s1;
+    asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(prev) : "l"(counter) : "memory");
+  }
+  if (__shfl_sync(0xffffffffu, prev, 0) != nb - 1) return false;
+  __threadfence();
+  s0 = s1 = 0.0;
+  double v0 = lane < nb ? ld_volatile(part + lane) : 0.0;
+  double v1 = SETS == 2 && lane < nb ? ld_volatile(part + nb + lane) : 0.0;
+  for (unsigned base = 0; base < nb; base += 32) {
+    const unsigned nx = base + 32 + lane;  // the next 32 are on their way while these are added
+    const double w0 = nx < nb ? ld_volatile(part + nx) : 0.0;
+    const double w1 = SETS == 2 && nx < nb ? ld_volatile(part + nb + nx) : 0.0;
+    const unsigned cnt = min(32u, nb - base);
+#pragma unroll 8
+    for (unsigned q = 0; q < cnt; ++q) {
+      s0 = s0 + __shfl_sync(0xffffffffu, v0, q);
+      if (SETS == 2) s1 = s1 + __shfl_sync(0xffffffffu, v1, q);
+    }
+    v0 = w0;
+    v1 = w1;
+  }
+  return true;
 }
 
 // Phases of the single-chain dot kernel.
 enum DotPhase : int { PH_PAP = 0, PH_INIT_RR = 1 };
 
-__global__ void __launch_bounds__(kDotThreads) k_dot_exact(const double* __restrict__ a, const double* __restrict__ b,
-                                                           int64_t n, double* part, PcgState* st, int mode,
-                                                           int phase) {
-  if (st->status != PCG_RUNNING) return;
-  __shared__ double buf[2][kChunk];
+__global__ void __launch_bounds__(chain_threads(1), 4) k_dot_exact(const double* __restrict__ a, const double* __restrict__ b,
+                                                             int64_t n, double* part, PcgState* st, int phase) {
+  __shared__ __align__(16) double buf[kRing][1][4][kRow];
   const int64_t start = (int64_t)blockIdx.x * kBlock;
   const int cnt = (int)min((int64_t)kBlock, n - start);
   const int vc4 = cnt & ~3;
-  const int nch = (vc4 + kChunk - 1) / kChunk;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  double acc = 0.0;
-  for (int t = 0; t <= nch; ++t) {
-    if (warp > 0 && t < nch) {
-      const int base = t * kChunk;
-      double* dst = buf[t & 1];
-      for (int q = tid - 32; q < kChunk; q += kDotThreads - 32) {
-        int idx = base + q;
-        if (idx < vc4) dst[q] = a[start + idx] * b[start + idx];
-      }
-    }
-    if (warp == 0 && t > 0 && lane < 4) {
-      const int base = (t - 1) * kChunk;
-      acc = chain4(acc, buf[(t - 1) & 1], min(kChunk, vc4 - base), lane);
-    }
-    __syncthreads();
-  }
-  if (warp == 0) {
-    double l0 = __shfl_sync(0xffffffffu, acc, 0), l1 = __shfl_sync(0xffffffffu, acc, 1);
-    double l2 = __shfl_sync(0xffffffffu, acc, 2), l3 = __shfl_sync(0xffffffffu, acc, 3);
-    if (lane == 0) {
-      double s = lane_sum(mode, l0, l1, l2, l3);
-      for (int idx = vc4; idx < cnt; ++idx) s = s + a[start + idx] * b[start + idx];
-      part[blockIdx.x] = s;
-    }
-  }
-  if (!elect_last(&st->counter)) return;
-  if (tid != 0) return;
-  double sum = 0.0;
-  for (unsigned k = 0; k < gridDim.x; ++k) sum = sum + ld_volatile(part + k);
+  const int tid = threadIdx.x, lane = tid & 31;
+  const double2 *a2 = reinterpret_cast<const double2*>(a + start), *b2 = reinterpret_cast<const double2*>(b + start);
+  double2 av[2], bv[2];
+  double tv = 0.0;  // the block's last n mod 4 entries' products (lanes 0-2 of warp 0), added after the chains
+  if (tid < cnt - vc4) tv = a[start + vc4 + tid] * b[start + vc4 + tid];
+  const double rho0 = st->rho0, bnorm = st->bnorm, tol = st->tol;
+  const int iter = st->iter;
+  auto load = [&](int q, int h) {
+    av[q] = a2[h];
+    bv[q] = b2[h];
+  };
+  const int status = st->status, np = vc4 >> 1, h0 = first_pair<1>();
+  if (h0 >= 0 && h0 < np) load(0, h0);
+  if (h0 >= 0 && h0 + kProd < np) load(1, h0 + kProd);
+  if (status != PCG_RUNNING) return;
+  const double acc = block_chains<1>(np, buf, load, [&](int q, int, auto&& put) {
+    put(0, 0, av[q].x * bv[q].x);
+    put(0, 1, av[q].y * bv[q].y);
+  });
+  if (tid >= 32) return;
+  const double l0 = __shfl_sync(0xffffffffu, acc, 0), l1 = __shfl_sync(0xffffffffu, acc, 1);
+  const double l2 = __shfl_sync(0xffffffffu, acc, 2), l3 = __shfl_sync(0xffffffffu, acc, 3);
+  double sum = lane_sum(l0, l1, l2, l3), none = 0.0;
+  for (int q = 0; q < cnt - vc4; ++q) sum = sum + __shfl_sync(0xffffffffu, tv, q);
+  if (!sum_blocks<1>(part, &st->counter, sum, none) || lane != 0) return;
   st->counter = 0;
   if (phase == PH_PAP) {
-    st->iter += 1;
+    st->iter = iter + 1;
+    st->first = 0;
     double pap = sum;
     st->pap = pap;
     if (!(pap > 1e-30) || !isfinite(pap)) {
@@ -427,7 +621,7 @@ __global__ void __launch_bounds__(kDotThreads) k_dot_exact(const double* __restr
       st->status = PCG_BREAK_CURVATURE;
       return;
     }
-    double alpha = st->rho0 / pap;
+    double alpha = rho0 / pap;
     if (!isfinite(alpha) || alpha <= 0.0) {
       st->last_bad = alpha;
       st->status = PCG_BREAK_ALPHA;
@@ -436,118 +630,113 @@ __global__ void __launch_bounds__(kDotThreads) k_dot_exact(const double* __restr
     st->alpha = alpha;
   } else {  // PH_INIT_RR: rNormSq for a non-zero warm start (PcgSolver.cs:176-197)
     st->rn2 = sum;
-    double rel = sqrt(sum) / st->bnorm;
+    double rel = sqrt(sum) / bnorm;
     st->rel = rel;
     st->prev = rel;
-    if (rel <= st->tol) st->status = PCG_INIT_CONVERGED;
+    if (rel <= tol) st->status = PCG_INIT_CONVERGED;
   }
 }
 
-// Fused x/r update with ||r||^2 and z = r*invD with r.z. init=1: only the z part (rho0, p = z).
-__global__ void __launch_bounds__(kDotThreads) k_xr_exact(double* __restrict__ x, double* __restrict__ r,
-                                                          double* __restrict__ z, double* __restrict__ p,
-                                                          const double* __restrict__ ap,
-                                                          const double* __restrict__ invd, int64_t n, double* part,
-                                                          PcgState* st, int mode, int init) {
-  if (st->status != PCG_RUNNING) return;
-  __shared__ double bufA[2][kChunk];
-  __shared__ double bufB[2][kChunk];
-  const double alpha = st->alpha;
+// Fused x/r update with ||r||^2 and z = r*invD with r.z. INIT: only the z part (rho0; the first direction is z).
+template <int INIT>
+__global__ void __launch_bounds__(chain_threads(2), 3) k_xr_exact(double* __restrict__ x, double* __restrict__ r,
+                                                            double* __restrict__ z, const double* __restrict__ p,
+                                                            const double* __restrict__ ap,
+                                                            const double* __restrict__ invd, int64_t n, double* part,
+                                                            PcgState* st) {
+  extern __shared__ __align__(16) double xr_buf[];
+  auto buf = reinterpret_cast<double (*)[2][4][kRow]>(xr_buf);  // sets: r.r (not used at a start), r.z
+  __shared__ double rz_sum;
   const int64_t start = (int64_t)blockIdx.x * kBlock;
   const int cnt = (int)min((int64_t)kBlock, n - start);
   const int vc4 = cnt & ~3;
-  const int nch = (vc4 + kChunk - 1) / kChunk;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  double acc = 0.0;
-  for (int t = 0; t <= nch; ++t) {
-    if (warp > 0 && t < nch) {
-      const int base = t * kChunk;
-      double* da = bufA[t & 1];
-      double* db = bufB[t & 1];
-      for (int q = tid - 32; q < kChunk; q += kDotThreads - 32) {
-        int idx = base + q;
-        if (idx < vc4) {
-          int64_t j = start + idx;
-          double rv;
-          if (!init) {
-            double xv = x[j] + alpha * p[j];
-            rv = r[j] - alpha * ap[j];
-            x[j] = xv;
-            r[j] = rv;
-            da[q] = rv * rv;
-          } else {
-            rv = r[j];
-          }
-          double zv = rv * invd[j];
-          z[j] = zv;
-          if (init) p[j] = zv;
-          db[q] = rv * zv;
-        }
-      }
-    }
-    if (warp == 0 && t > 0 && lane < 8) {
-      const int base = (t - 1) * kChunk;
-      const int m = min(kChunk, vc4 - base);
-      if (lane < 4) {
-        if (!init) acc = chain4(acc, bufA[(t - 1) & 1], m, lane);
-      } else {
-        acc = chain4(acc, bufB[(t - 1) & 1], m, lane - 4);
-      }
-    }
-    __syncthreads();
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int status = st->status;
+  const double alpha = st->alpha;
+  double2 *x2 = reinterpret_cast<double2*>(x + start), *r2 = reinterpret_cast<double2*>(r + start),
+          *z2 = reinterpret_cast<double2*>(z + start);
+  const double2 *p2 = reinterpret_cast<const double2*>(p + start), *q2 = reinterpret_cast<const double2*>(ap + start),
+                *d2 = reinterpret_cast<const double2*>(invd + start);
+  double2 xv[2], rv[2], pv[2], qv[2], dv[2];
+  // the block's last n mod 4 entries, by lanes 0-2 of warp 0 (their terms are added after the chains)
+  const int64_t tj = start + vc4 + tid;
+  const bool tail = tid < cnt - vc4;
+  double tr = 0.0, tx = 0.0, tp = 0.0, tap = 0.0, td = 0.0;
+  if (tail) {
+    tr = r[tj];
+    td = invd[tj];
+    if (!INIT) tx = x[tj], tp = p[tj], tap = ap[tj];
   }
-  if (warp == 0) {
-    double a0 = __shfl_sync(0xffffffffu, acc, 0), a1 = __shfl_sync(0xffffffffu, acc, 1);
-    double a2 = __shfl_sync(0xffffffffu, acc, 2), a3 = __shfl_sync(0xffffffffu, acc, 3);
-    double b0 = __shfl_sync(0xffffffffu, acc, 4), b1 = __shfl_sync(0xffffffffu, acc, 5);
-    double b2 = __shfl_sync(0xffffffffu, acc, 6), b3 = __shfl_sync(0xffffffffu, acc, 7);
-    if (lane == 0) {
-      double sa = lane_sum(mode, a0, a1, a2, a3);
-      double sb = lane_sum(mode, b0, b1, b2, b3);
-      if (!init) {
-        for (int idx = vc4; idx < cnt; ++idx) {
-          int64_t j = start + idx;
-          double xi = x[j] + alpha * p[j];
-          double ri = r[j] - alpha * ap[j];
-          x[j] = xi;
-          r[j] = ri;
-          sa = sa + ri * ri;
-        }
-      }
-      for (int idx = vc4; idx < cnt; ++idx) {
-        int64_t j = start + idx;
-        double zi = r[j] * invd[j];
-        z[j] = zi;
-        if (init) p[j] = zi;
-        sb = sb + r[j] * zi;
-      }
-      part[blockIdx.x] = sa;
-      part[gridDim.x + blockIdx.x] = sb;
+  const double rho0 = st->rho0, bnorm = st->bnorm, tol = st->tol, prev = st->prev;
+  const int iter = st->iter, max_iter = st->max_iter, stag = st->stag;
+  auto load = [&](int q, int h) {
+    rv[q] = r2[h];
+    dv[q] = d2[h];
+    if (!INIT) {
+      qv[q] = q2[h];
+      pv[q] = p2[h];
+      xv[q] = x2[h];
     }
+  };
+  const int np = vc4 >> 1, h0 = first_pair<2>();
+  if (h0 >= 0 && h0 < np) load(0, h0);
+  if (h0 >= 0 && h0 + kProd < np) load(1, h0 + kProd);
+  if (status != PCG_RUNNING) return;
+  const double acc = block_chains<2>(np, buf, load, [&](int q, int h, auto&& put) {
+    double2 rn = rv[q];
+    if (!INIT) {
+      x2[h] = make_double2(xv[q].x + alpha * pv[q].x, xv[q].y + alpha * pv[q].y);
+      rn = make_double2(rv[q].x - alpha * qv[q].x, rv[q].y - alpha * qv[q].y);
+      r2[h] = rn;
+    }
+    const double2 zn = make_double2(rn.x * dv[q].x, rn.y * dv[q].y);
+    z2[h] = zn;
+    put(0, 0, rn.x * rn.x);
+    put(0, 1, rn.y * rn.y);
+    put(1, 0, rn.x * zn.x);
+    put(1, 1, rn.y * zn.y);
+  });
+  if (tid >= 64) return;
+  const double l0 = __shfl_sync(0xffffffffu, acc, 0), l1 = __shfl_sync(0xffffffffu, acc, 1);
+  const double l2 = __shfl_sync(0xffffffffu, acc, 2), l3 = __shfl_sync(0xffffffffu, acc, 3);
+  double rn2 = lane_sum(l0, l1, l2, l3);  // warp 0: r.r; warp 1: r.z, handed over
+  if (tid == 32) rz_sum = rn2;
+  asm volatile("bar.sync 15, 64;" ::: "memory");
+  if (tid >= 32) return;
+  double rho1 = rz_sum, trr = 0.0, trz = 0.0;
+  if (tail) {
+    if (!INIT) {
+      x[tj] = tx + alpha * tp;
+      tr = tr - alpha * tap;
+      r[tj] = tr;
+      trr = tr * tr;
+    }
+    const double tz = tr * td;
+    z[tj] = tz;
+    trz = tr * tz;
   }
-  if (!elect_last(&st->counter)) return;
-  if (tid != 0) return;
+  for (int q = 0; q < cnt - vc4; ++q) {
+    rn2 = rn2 + __shfl_sync(0xffffffffu, trr, q);
+    rho1 = rho1 + __shfl_sync(0xffffffffu, trz, q);
+  }
+  if (!sum_blocks<2>(part, &st->counter, rn2, rho1) || lane != 0) return;
   st->counter = 0;
-  const unsigned nb = gridDim.x;
-  if (init) {
-    double rho = 0.0;
-    for (unsigned k = 0; k < nb; ++k) rho = rho + ld_volatile(part + nb + k);
-    st->rho0 = rho;
-    if (st->max_iter <= 0) st->status = PCG_MAXITER;
+  if (INIT) {
+    st->rho0 = rho1;
+    st->first = 1;
+    if (max_iter <= 0) st->status = PCG_MAXITER;
     return;
   }
-  double rn2 = 0.0;
-  for (unsigned k = 0; k < nb; ++k) rn2 = rn2 + ld_volatile(part + k);
   st->rn2 = rn2;
-  double rel = sqrt(rn2) / st->bnorm;
+  double rel = sqrt(rn2) / bnorm;
   st->rel = rel;
-  if (rel <= st->tol) {
+  if (rel <= tol) {
     st->status = PCG_CONVERGED;
     return;
   }
-  if (fabs(rel - st->prev) < 1e-15 * rel) {
-    st->stag += 1;
-    if (st->stag > 50) {
+  if (fabs(rel - prev) < 1e-15 * rel) {
+    st->stag = stag + 1;
+    if (stag + 1 > 50) {
       st->status = PCG_STAGNATED;
       return;
     }
@@ -555,9 +744,7 @@ __global__ void __launch_bounds__(kDotThreads) k_xr_exact(double* __restrict__ x
     st->stag = 0;
   }
   st->prev = rel;
-  double rho1 = 0.0;
-  for (unsigned k = 0; k < nb; ++k) rho1 = rho1 + ld_volatile(part + nb + k);
-  double beta = rho1 / st->rho0;
+  double beta = rho1 / rho0;
   if (!isfinite(beta) || beta < 0.0) {
     st->last_bad = beta;
     st->status = PCG_BREAK_BETA;
@@ -565,14 +752,22 @@ __global__ void __launch_bounds__(kDotThreads) k_xr_exact(double* __restrict__ x
   }
   st->beta = beta;
   st->rho0 = rho1;
-  if (st->iter >= st->max_iter) st->status = PCG_MAXITER;
+  if (iter >= max_iter) st->status = PCG_MAXITER;
 }
 
-__global__ void k_update_p(double* __restrict__ p, const double* __restrict__ z, int64_t n, const PcgState* st) {
-  if (st->status != PCG_RUNNING) return;
-  const double beta = st->beta;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    p[i] = z[i] + beta * p[i];
+static void launch_dot(mycel_problem* p, const double* a, const double* b, int phase) {
+  k_dot_exact<<<(unsigned)num_blocks8192(p->g.nd), chain_threads(1), 0, p->ctx->stream>>>(a, b, p->g.nd, p->d_part,
+                                                                                          p->d_state, phase);
+  p->ctx->launches++;
+}
+
+template <int INIT>
+static void launch_xr(mycel_problem* p, const double* dir) {
+  constexpr size_t smem = sizeof(double) * kRing * 2 * 4 * kRow;
+  allow_smem<k_xr_exact<INIT>>(p->ctx->device, smem);
+  k_xr_exact<INIT><<<(unsigned)num_blocks8192(p->g.nd), chain_threads(2), smem, p->ctx->stream>>>(
+      p->d_x, p->d_r, p->d_z, dir, p->d_ap, p->d_invd, p->g.nd, p->d_part, p->d_state);
+  p->ctx->launches++;
 }
 
 // x projection (PcgSolver.cs:113-125) and "has non-zero x" flag
@@ -631,31 +826,18 @@ void launch_pcg_init_r(mycel_problem* p, int nonzero) {
 }
 
 void launch_pcg_dot_rr(mycel_problem* p) {
-  int64_t nb = num_blocks8192(p->g.nd);
-  k_dot_exact<<<(unsigned)nb, kDotThreads, 0, p->ctx->stream>>>(p->d_r, p->d_r, p->g.nd, p->d_part, p->d_state,
-                                                                p->lane_mode, PH_INIT_RR);
-  p->ctx->launches++;
+  launch_dot(p, p->d_r, p->d_r, PH_INIT_RR);
 }
 
-void launch_pcg_init_z(mycel_problem* p) {
-  int64_t nb = num_blocks8192(p->g.nd);
-  k_xr_exact<<<(unsigned)nb, kDotThreads, 0, p->ctx->stream>>>(p->d_x, p->d_r, p->d_z, p->d_p, p->d_ap, p->d_invd,
-                                                               p->g.nd, p->d_part, p->d_state, p->lane_mode, 1);
-  p->ctx->launches++;
-}
+void launch_pcg_init_z(mycel_problem* p) { launch_xr<1>(p, nullptr); }
 
-// One PCG iteration (PcgSolver.cs:235-357): Ap = A p; pAp, alpha; x, r, ||r||; z, rho1, beta; p = z + beta p.
-void launch_pcg_iteration(mycel_problem* p, bool skip_matvec) {
-  cudaStream_t s = p->ctx->stream;
-  int64_t nb = num_blocks8192(p->g.nd);
-  if (!skip_matvec) launch_matvec64(p, p->d_p, p->d_ap, 1, &p->d_state->status);
-  k_dot_exact<<<(unsigned)nb, kDotThreads, 0, s>>>(p->d_p, p->d_ap, p->g.nd, p->d_part, p->d_state, p->lane_mode,
-                                                   PH_PAP);
-  k_xr_exact<<<(unsigned)nb, kDotThreads, 0, s>>>(p->d_x, p->d_r, p->d_z, p->d_p, p->d_ap, p->d_invd, p->g.nd,
-                                                  p->d_part, p->d_state, p->lane_mode, 0);
-  k_update_p<<<(unsigned)std::min<int64_t>((p->g.nd + 255) / 256, 4096), 256, 0, s>>>(p->d_p, p->d_z, p->g.nd,
-                                                                                        p->d_state);
-  p->ctx->launches += 3;
+// PCG iteration `it` (PcgSolver.cs:235-357): p = z + beta p and Ap = A p (the direction alternates between two
+// buffers, d_p in even iterations); pAp, alpha; x, r, ||r||; z, rho1, beta.
+void launch_pcg_iteration(mycel_problem* p, int it, bool skip_matvec) {
+  const double* dir = it & 1 ? p->d_p2 : p->d_p;
+  if (!skip_matvec) launch_pcg_matvec(p, it);
+  launch_dot(p, dir, p->d_ap, PH_PAP);
+  launch_xr<0>(p, dir);
 }
 
 // ---------------------------------------------------------------------------------------------------------

@@ -79,7 +79,7 @@ struct PcgState {
   int max_iter;
   int stag;
   int nonzero_x;
-  int pad_;
+  int first;  // the next direction is z (a start)
   double tol, bnorm, bn2, rho0, rel, prev, alpha, beta, pap, rn2, last_bad;
   unsigned int counter;  // completion counter for the last-block pattern
   unsigned int counter2;
@@ -176,7 +176,7 @@ struct mycel_problem {
   double* d_invd = nullptr;       // [nd] Jacobi inverse diagonal
   float* d_invdf = nullptr;       // [n32] FP32 copy, padded layout
   // PCG workspace (FP64)
-  double *d_r = nullptr, *d_z = nullptr, *d_p = nullptr, *d_ap = nullptr, *d_x = nullptr;
+  double *d_r = nullptr, *d_z = nullptr, *d_p = nullptr, *d_p2 = nullptr, *d_ap = nullptr, *d_x = nullptr;
   double* d_part = nullptr;       // [2*nblocks] partial sums
   mycel::PcgState* d_state = nullptr;
   // mixed-form workspace
@@ -201,7 +201,6 @@ struct mycel_problem {
   // scratch for API calls
   double* d_tmp0 = nullptr;       // [nd]
   double* d_tmp1 = nullptr;       // [nd]
-  int lane_mode = 0;
   cudaGraphExec_t pcg_graph[2] = {nullptr, nullptr};
   int pcg_graph_chunk = 0;
   cudaEvent_t prof64_ev[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};
@@ -245,13 +244,14 @@ int64_t num_blocks8192(int64_t n);
 void launch_setup_nodes(mycel_problem* p, const int32_t* d_fixed, int32_t n_fixed, int32_t* d_count);
 void launch_update_E(mycel_problem* p, const double* d_rho_box, double penal);
 void launch_diag(mycel_problem* p);
-void launch_matvec64(mycel_problem* p, const double* x, double* y, int projected, const int* d_status);
+void launch_matvec64(mycel_problem* p, const double* x, double* y, int projected);
 void launch_project_x(mycel_problem* p, double* x, int* d_flag);
 void launch_pcg_bnorm(mycel_problem* p);
 void launch_pcg_init_r(mycel_problem* p, int nonzero);
 void launch_pcg_dot_rr(mycel_problem* p);
 void launch_pcg_init_z(mycel_problem* p);
-void launch_pcg_iteration(mycel_problem* p, bool skip_matvec = false);
+void launch_pcg_matvec(mycel_problem* p, int it);  // p = z + beta p, Ap = A p of iteration `it`
+void launch_pcg_iteration(mycel_problem* p, int it, bool skip_matvec = false);
 void launch_compliance(mycel_problem* p, const double* u, double* d_out);
 void launch_compliance(mycel_problem* p, const double* F, const int32_t* fnz, int32_t n_fnz, const double* u,
                        double* d_out);
