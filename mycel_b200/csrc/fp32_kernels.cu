@@ -15,6 +15,7 @@
 // Reductions use a fixed CTA decomposition and a fixed-order final sum, so results do not depend on timing.
 #include <cuda.h>
 #include <cudaTypedefs.h>
+#include <cuda_pipeline.h>
 #include <cuda_runtime.h>
 #include <math.h>
 #include <stdint.h>
@@ -30,6 +31,7 @@
 #include <mutex>
 #include <string>
 #include <tuple>
+#include <type_traits>
 
 #include "internal.h"
 
@@ -1970,33 +1972,55 @@ __device__ __forceinline__ int64_t mg_dof_node() { return blockIdx.x * (int64_t)
 __device__ __forceinline__ int mg_dof_comp() { return threadIdx.x >> 6; }
 static inline unsigned mg_dof_blocks(int64_t nn) { return (unsigned)((nn + 63) / 64); }
 
+// Neighbour nb of node n (nb = (dx+1) + 3 (dy+1) + 9 (dz+1), compile time): whether it lies in the grid, and its
+// node number. The tests of the six sides are made once per node.
+struct MgNode {
+  int n, nx1, sxy;
+  bool lo[3], hi[3];  // a neighbour below / above on axis x, y, z
+  __device__ __forceinline__ MgNode(const MgDims& d, int n_) : n(n_), nx1(d.nx + 1), sxy((d.nx + 1) * (d.ny + 1)) {
+    int i, j, k;
+    mg_ijk(n, nx1, d.ny + 1, &i, &j, &k);
+    lo[0] = i > 0; lo[1] = j > 0; lo[2] = k > 0;
+    hi[0] = i < d.nx; hi[1] = j < d.ny; hi[2] = k < d.nz;
+  }
+  __device__ __forceinline__ bool in(int nb) const {
+    const int dx = nb % 3 - 1, dy = (nb / 3) % 3 - 1, dz = nb / 9 - 1;
+    return (dx == 0 || (dx < 0 ? lo[0] : hi[0])) && (dy == 0 || (dy < 0 ? lo[1] : hi[1])) &&
+           (dz == 0 || (dz < 0 ? lo[2] : hi[2]));
+  }
+  __device__ __forceinline__ int at(int nb) const {
+    return n + (nb % 3 - 1) + nx1 * ((nb / 3) % 3 - 1) + sxy * (nb / 9 - 1);
+  }
+};
+
 // coarse-level product at node n by gather (ns: the stencil's row stride). mode 0: y = A x; 1: y = x + omega
-// invd (r - A x) (one Jacobi sweep); 2: y = r - A x on DOFs with a nonzero diagonal, 0 elsewhere
-__device__ __forceinline__ void mg_apply_node(const MgDims& d, int64_t ns, int64_t n, const float* __restrict__ S,
+// invd (r - A x) (one Jacobi sweep); 2: y = r - A x on DOFs with a nonzero diagonal, 0 elsewhere.
+// All 27 blocks without branches: a neighbour outside the grid has x taken as 0 and its block read at a valid node.
+// Later neighbours' blocks are n's own (row ci at entries 3 ci + cj), earlier ones the transposed blocks stored at
+// the neighbour (row ci at entries 3 cj + ci).
+__device__ __forceinline__ void mg_apply_node(const MgDims& d, int64_t ns, int n, const float* __restrict__ S,
                                               const float* __restrict__ x, const float* __restrict__ r,
                                               const float* __restrict__ invd, float* __restrict__ y, int mode,
                                               float omega) {
-  const int nx1 = d.nx + 1, ny1 = d.ny + 1;
-  int i, j, k;
-  mg_ijk(n, nx1, ny1, &i, &j, &k);
+  const MgNode g(d, n);
   float a0 = 0.f, a1 = 0.f, a2 = 0.f;
-  // all 27 blocks without branches: a neighbour outside the grid is read at a clamped (valid) node with x
-  // taken as 0. Later neighbours' blocks are n's own (row ci at entries 3 ci + cj), earlier ones the transposed
-  // blocks stored at the neighbour (row ci at entries 3 cj + ci).
 #pragma unroll
   for (int nb = 0; nb < 27; ++nb) {
-    const int ui = i + nb % 3 - 1, uj = j + (nb / 3) % 3 - 1, uk = k + nb / 9 - 1;
-    const int mi = min(max(ui, 0), d.nx), mj = min(max(uj, 0), d.ny), mk = min(max(uk, 0), d.nz);
-    const bool in = mi == ui && mj == uj && mk == uk;
-    const int64_t m = mi + (int64_t)nx1 * (mj + (int64_t)ny1 * mk);
-    const float x0 = in ? x[3 * m] : 0.f, x1 = in ? x[3 * m + 1] : 0.f, x2 = in ? x[3 * m + 2] : 0.f;
+    const int m = g.at(nb);
+    const bool in = g.in(nb);
+    float x0 = 0.f, x1 = 0.f, x2 = 0.f;
+    if (in) {
+      x0 = x[3 * m];
+      x1 = x[3 * m + 1];
+      x2 = x[3 * m + 2];
+    }
     if (nb >= 13) {
       const float* s = S + (int64_t)(nb - 13) * 9 * ns + n;
       a0 = fmaf(s[0], x0, fmaf(s[ns], x1, fmaf(s[2 * ns], x2, a0)));
       a1 = fmaf(s[3 * ns], x0, fmaf(s[4 * ns], x1, fmaf(s[5 * ns], x2, a1)));
       a2 = fmaf(s[6 * ns], x0, fmaf(s[7 * ns], x1, fmaf(s[8 * ns], x2, a2)));
     } else {
-      const float* s = S + (int64_t)(13 - nb) * 9 * ns + m;
+      const float* s = S + (int64_t)(13 - nb) * 9 * ns + max(m, 0);
       a0 = fmaf(s[0], x0, fmaf(s[3 * ns], x1, fmaf(s[6 * ns], x2, a0)));
       a1 = fmaf(s[ns], x0, fmaf(s[4 * ns], x1, fmaf(s[7 * ns], x2, a1)));
       a2 = fmaf(s[2 * ns], x0, fmaf(s[5 * ns], x1, fmaf(s[8 * ns], x2, a2)));
@@ -2005,7 +2029,7 @@ __device__ __forceinline__ void mg_apply_node(const MgDims& d, int64_t ns, int64
   const float acc[3] = {a0, a1, a2};
 #pragma unroll
   for (int cc = 0; cc < 3; ++cc) {
-    const int64_t q = 3 * n + cc;
+    const int q = 3 * n + cc;
     if (mode == 0) y[q] = acc[cc];
     else if (mode == 1) y[q] = fmaf(omega * invd[q], r[q] - acc[cc], x[q]);
     else y[q] = invd[q] != 0.0f ? r[q] - acc[cc] : 0.0f;
@@ -2013,30 +2037,33 @@ __device__ __forceinline__ void mg_apply_node(const MgDims& d, int64_t ns, int64
 }
 
 // the same for one row (DOF ci of node n): a third of the loads of a node
-__device__ __forceinline__ void mg_apply_row(const MgDims& d, int64_t ns, int64_t n, int ci,
+__device__ __forceinline__ void mg_apply_row(const MgDims& d, int64_t ns, int n, int ci,
                                              const float* __restrict__ S, const float* __restrict__ x,
                                              const float* __restrict__ r, const float* __restrict__ invd,
                                              float* __restrict__ y, int mode, float omega) {
-  const int nx1 = d.nx + 1, ny1 = d.ny + 1;
-  int i, j, k;
-  mg_ijk(n, nx1, ny1, &i, &j, &k);
+  const MgNode g(d, n);
+  const float* own = S + 3 * ci * ns + n;
+  const float* tr = S + ci * ns;
   float a = 0.f;
 #pragma unroll
   for (int nb = 0; nb < 27; ++nb) {
-    const int ui = i + nb % 3 - 1, uj = j + (nb / 3) % 3 - 1, uk = k + nb / 9 - 1;
-    const int mi = min(max(ui, 0), d.nx), mj = min(max(uj, 0), d.ny), mk = min(max(uk, 0), d.nz);
-    const bool in = mi == ui && mj == uj && mk == uk;
-    const int64_t m = mi + (int64_t)nx1 * (mj + (int64_t)ny1 * mk);
-    const float x0 = in ? x[3 * m] : 0.f, x1 = in ? x[3 * m + 1] : 0.f, x2 = in ? x[3 * m + 2] : 0.f;
+    const int m = g.at(nb);
+    const bool in = g.in(nb);
+    float x0 = 0.f, x1 = 0.f, x2 = 0.f;
+    if (in) {
+      x0 = x[3 * m];
+      x1 = x[3 * m + 1];
+      x2 = x[3 * m + 2];
+    }
     if (nb >= 13) {
-      const float* s = S + ((int64_t)(nb - 13) * 9 + 3 * ci) * ns + n;
+      const float* s = own + (int64_t)(nb - 13) * 9 * ns;
       a = fmaf(s[0], x0, fmaf(s[ns], x1, fmaf(s[2 * ns], x2, a)));
     } else {
-      const float* s = S + ((int64_t)(13 - nb) * 9 + ci) * ns + m;
+      const float* s = tr + (int64_t)(13 - nb) * 9 * ns + max(m, 0);
       a = fmaf(s[0], x0, fmaf(s[3 * ns], x1, fmaf(s[6 * ns], x2, a)));
     }
   }
-  const int64_t q = 3 * n + ci;
+  const int q = 3 * n + ci;
   if (mode == 0) y[q] = a;
   else if (mode == 1) y[q] = fmaf(omega * invd[q], r[q] - a, x[q]);
   else y[q] = invd[q] != 0.0f ? r[q] - a : 0.0f;
@@ -2202,44 +2229,40 @@ __global__ void k_mg_jacobi_fine(int64_t n, const float* __restrict__ r, const f
     x[q] = fmaf(omega * invd[q], r[q] - t[q], x[q]);
 }
 
-// restriction r_c = W^T res of a level's residual, component cc at coarse node n. PAD: the voxel grid in the
-// padded FP32 layout (row pitch pitch), res = r - t; otherwise box layout, res = t. Coarse DOFs with a zero
-// diagonal get 0.
-template <bool PAD>
-__device__ __forceinline__ void mg_restrict_comp(const MgDims& f, int pitch, const float* __restrict__ rf,
-                                                 const float* __restrict__ tf, const MgDims& c,
+// Restriction along one axis (n fine elements) to coarse node c: the fine nodes p - 1, p, p + 1 around its position
+// p carry the weights mg_pw gives them, 1 at p and 1/2 or 0 beside it (0 at an absent node, and next to an odd
+// count's last node, which coarsens alone); a node of weight 0 is read at p. Weights and offsets are formed once per
+// axis: clamps, tests and 64-bit indices per tap were 44 instructions of a serial thread each (a level of 44x28x15
+// nodes into the next: 10.5 -> 5.7 us; the voxel grid of 85x53x27 elements 11.3 -> 6.3 us, of 192x96x96 25 -> 20 us).
+struct MgAxis {
+  int o[3];  // fine coordinate x stride
+  float w[3];
+  __device__ __forceinline__ MgAxis(int c, int n, int stride) {
+    const int p = min(2 * c, n);
+    w[0] = c > 0 && 2 * c <= n ? 0.5f : 0.f;
+    w[1] = 1.f;
+    w[2] = 2 * c + 1 < n ? 0.5f : 0.f;
+    o[1] = p * stride;
+    o[0] = w[0] != 0.f ? o[1] - stride : o[1];
+    o[2] = w[2] != 0.f ? o[1] + stride : o[1];
+  }
+};
+
+// restriction r_c = W^T res of a level's residual, component cc at coarse node n (box layout)
+__device__ __forceinline__ void mg_restrict_comp(const MgDims& f, const float* __restrict__ tf, const MgDims& c,
                                                  const float* __restrict__ invdc, float* __restrict__ rc, int64_t n,
                                                  int cc, float* __restrict__ xc, float omega) {
-  const int cx1 = c.nx + 1, cy1 = c.ny + 1;
   int I, J, K;
-  mg_ijk(n, cx1, cy1, &I, &J, &K);
-  const int pi = min(2 * I, f.nx), pj = min(2 * J, f.ny), pk = min(2 * K, f.nz);
+  mg_ijk(n, c.nx + 1, c.ny + 1, &I, &J, &K);
+  const MgAxis ax(I, f.nx, 3), ay(J, f.ny, 3 * (f.nx + 1)), az(K, f.nz, 3 * (f.nx + 1) * (f.ny + 1));
   float a = 0.f;
-  // the 27 candidate fine nodes around the coarse node's position, without branches: a candidate outside the
-  // grid gets weight 0 and a clamped (valid) read
 #pragma unroll
-  for (int dk = -1; dk <= 1; ++dk) {
-    const int k0 = pk + dk, k = min(max(k0, 0), f.nz);
-    const float wz = (k0 == k) ? mg_pw(k, K, f.nz) : 0.f;
-#pragma unroll
-    for (int dj = -1; dj <= 1; ++dj) {
-      const int j0 = pj + dj, j = min(max(j0, 0), f.ny);
-      const float wy = (j0 == j) ? wz * mg_pw(j, J, f.ny) : 0.f;
-#pragma unroll
-      for (int di = -1; di <= 1; ++di) {
-        const int i0 = pi + di, i = min(max(i0, 0), f.nx);
-        const float w = (i0 == i) ? wy * mg_pw(i, I, f.nx) : 0.f;
-        const int64_t row = j + (int64_t)(f.ny + 1) * k;
-        const int64_t b = (PAD ? (int64_t)pitch * row + 3 * i : 3 * (i + (int64_t)(f.nx + 1) * row)) + cc;
-        a = fmaf(w, PAD ? rf[b] - tf[b] : tf[b], a);
-      }
-    }
-  }
+  for (int q = 0; q < 27; ++q)
+    a = fmaf(az.w[q / 9] * ay.w[q / 3 % 3] * ax.w[q % 3], tf[az.o[q / 9] + ay.o[q / 3 % 3] + ax.o[q % 3] + cc], a);
   const float d = invdc[3 * n + cc], rv = d != 0.f ? a : 0.f;
   rc[3 * n + cc] = rv;
   if (xc) xc[3 * n + cc] = omega * d * rv;  // the coarse level's first Jacobi sweep from x = 0
 }
-
 
 // prolongation x_f += W x_c, component cc at fine node n, on the finer level's free DOFs. PAD: the voxel grid
 // (padded FP32 layout, free = node flag bit clear); otherwise box layout, free = nonzero diagonal.
@@ -2286,37 +2309,23 @@ __device__ __forceinline__ void mg_restrict_node(const MgDims& f, int pitch, con
                                                  const float* __restrict__ tf, const MgDims& c,
                                                  const float* __restrict__ invdc, float* __restrict__ rc, int64_t n,
                                                  float* __restrict__ xc, float omega) {
-  const int cx1 = c.nx + 1, cy1 = c.ny + 1;
   int I, J, K;
-  mg_ijk(n, cx1, cy1, &I, &J, &K);
-  const int pi = min(2 * I, f.nx), pj = min(2 * J, f.ny), pk = min(2 * K, f.nz);
+  mg_ijk(n, c.nx + 1, c.ny + 1, &I, &J, &K);
+  const int rowp = PAD ? pitch : 3 * (f.nx + 1);
+  const MgAxis ax(I, f.nx, 3), ay(J, f.ny, rowp), az(K, f.nz, rowp * (f.ny + 1));
   float a0 = 0.f, a1 = 0.f, a2 = 0.f;
-  // the 27 candidate fine nodes around the coarse node's position, without branches: a candidate outside the
-  // grid gets weight 0 and a clamped (valid) read
 #pragma unroll
-  for (int dk = -1; dk <= 1; ++dk) {
-    const int k0 = pk + dk, k = min(max(k0, 0), f.nz);
-    const float wz = (k0 == k) ? mg_pw(k, K, f.nz) : 0.f;
-#pragma unroll
-    for (int dj = -1; dj <= 1; ++dj) {
-      const int j0 = pj + dj, j = min(max(j0, 0), f.ny);
-      const float wy = (j0 == j) ? wz * mg_pw(j, J, f.ny) : 0.f;
-#pragma unroll
-      for (int di = -1; di <= 1; ++di) {
-        const int i0 = pi + di, i = min(max(i0, 0), f.nx);
-        const float w = (i0 == i) ? wy * mg_pw(i, I, f.nx) : 0.f;
-        const int64_t row = j + (int64_t)(f.ny + 1) * k;
-        const int64_t b = PAD ? (int64_t)pitch * row + 3 * i : 3 * (i + (int64_t)(f.nx + 1) * row);
-        if (PAD) {
-          a0 = fmaf(w, rf[b] - tf[b], a0);
-          a1 = fmaf(w, rf[b + 1] - tf[b + 1], a1);
-          a2 = fmaf(w, rf[b + 2] - tf[b + 2], a2);
-        } else {
-          a0 = fmaf(w, tf[b], a0);
-          a1 = fmaf(w, tf[b + 1], a1);
-          a2 = fmaf(w, tf[b + 2], a2);
-        }
-      }
+  for (int q = 0; q < 27; ++q) {
+    const float w = az.w[q / 9] * ay.w[q / 3 % 3] * ax.w[q % 3];
+    const int b = az.o[q / 9] + ay.o[q / 3 % 3] + ax.o[q % 3];
+    if (PAD) {
+      a0 = fmaf(w, rf[b] - tf[b], a0);
+      a1 = fmaf(w, rf[b + 1] - tf[b + 1], a1);
+      a2 = fmaf(w, rf[b + 2] - tf[b + 2], a2);
+    } else {
+      a0 = fmaf(w, tf[b], a0);
+      a1 = fmaf(w, tf[b + 1], a1);
+      a2 = fmaf(w, tf[b + 2], a2);
     }
   }
   const float d0 = invdc[3 * n], d1 = invdc[3 * n + 1], d2 = invdc[3 * n + 2];
@@ -2344,48 +2353,68 @@ __global__ void k_mg_restrict(MgDims f, int pitch, const __grid_constant__ MgPtr
   mg_restrict_node<PAD>(f, pitch, rf.p[k], tf.p[k], c, invdc, rc.p[k], n, first_sweep ? xc.p[k] : nullptr, omega);
 }
 
-// prolongation x_f += W x_c at fine node n, on the finer level's free DOFs. PAD: the voxel grid (padded FP32
-// layout, free = node flag bit clear); otherwise box layout, free = nonzero diagonal.
+// prolongation x_f += W x_c on the finer level's free DOFs, for the pair of fine nodes (2 c, 2 c + 1) of a node row
+// that share their coarse columns, which are read once for both. PAD: the voxel grid (padded FP32 layout, free = node flag bit clear); otherwise box layout, free =
+// nonzero diagonal. Items of a level: (nx + 2) / 2 pairs a row. (192x96x96 elements: 32.7 us with a thread per node
+// and its eight coarse nodes one after another, 17.3 now; the small levels keep their 3.5 us.)
+__host__ __device__ __forceinline__ int64_t mg_pairs(const MgDims& d) {
+  return (int64_t)((d.nx + 2) >> 1) * (d.ny + 1) * (d.nz + 1);
+}
 template <bool PAD>
-__device__ __forceinline__ void mg_prolong_node(const MgDims& f, int pitch, const uint8_t* __restrict__ nf,
+__device__ __forceinline__ void mg_prolong_pair(const MgDims& f, int pitch, const uint8_t* __restrict__ nf,
                                                 const float* __restrict__ invdf, float* __restrict__ xf,
-                                                const MgDims& c, const float* __restrict__ xc, int64_t n) {
-  const int fx1 = f.nx + 1, fy1 = f.ny + 1;
-  int i, j, k;
-  mg_ijk(n, fx1, fy1, &i, &j, &k);
-  // per axis: two coarse nodes with their weights (the second with weight 0 unless the fine node lies midway)
-  int ci[2], cj[2], ck[2];
-  float wi[2], wj[2], wk[2];
-  auto axis = [](int f_, int n_, int nc_, int* cc, float* ww) {
+                                                const MgDims& c, const float* __restrict__ xc, int64_t item) {
+  int ci, j, k;
+  mg_ijk(item, (f.nx + 2) >> 1, f.ny + 1, &ci, &j, &k);
+  const int i = 2 * ci;
+  const bool odd = i < f.nx, last = i + 1 == f.nx;  // the second node exists; it is an odd count's last node
+  // coarse row of weight w0, and the next one of weight w1 (0: the fine node lies on a coarse one)
+  auto axis = [](int f_, int n_, int nc_, int* c_, float* w0, float* w1) {
     const bool mid = (f_ & 1) && f_ != n_;
-    cc[0] = ((f_ & 1) && f_ == n_) ? nc_ : (f_ >> 1);
-    cc[1] = min(cc[0] + 1, nc_);
-    ww[0] = mid ? 0.5f : 1.0f;
-    ww[1] = mid ? 0.5f : 0.0f;
+    *c_ = ((f_ & 1) && f_ == n_) ? nc_ : (f_ >> 1);
+    *w0 = mid ? 0.5f : 1.0f;
+    *w1 = mid ? 0.5f : 0.0f;
   };
-  axis(i, f.nx, c.nx, ci, wi);
-  axis(j, f.ny, c.ny, cj, wj);
-  axis(k, f.nz, c.nz, ck, wk);
-  const int cx1 = c.nx + 1, cy1 = c.ny + 1;
-  float a0 = 0.f, a1 = 0.f, a2 = 0.f;
+  int cj, ck;
+  float wj[2], wk[2];
+  axis(j, f.ny, c.ny, &cj, &wj[0], &wj[1]);
+  axis(k, f.nz, c.nz, &ck, &wk[0], &wk[1]);
+  const int row = 3 * (c.nx + 1), plane = row * (c.ny + 1);
+  const float* base = xc + 3 * ci + row * cj + plane * ck;
+  const int64_t n = i + (int64_t)(f.nx + 1) * (j + (int64_t)(f.ny + 1) * k);
+  const int64_t b = PAD ? (int64_t)pitch * (j + (int64_t)(f.ny + 1) * k) + 3 * i : 3 * n;
+  // every load first (an absent coarse row is read at its neighbour, an absent column or node at the first)
+  const int oy = wj[1] != 0.f ? row : 0, oz = wk[1] != 0.f ? plane : 0, ox = odd ? 3 : 0;
+  float v[4][6], x[6], d[6];
+  uint8_t fl[2];
 #pragma unroll
-  for (int qz = 0; qz < 2; ++qz)
+  for (int q = 0; q < 4; ++q)
 #pragma unroll
-    for (int qy = 0; qy < 2; ++qy)
-#pragma unroll
-      for (int qx = 0; qx < 2; ++qx) {
-        const float w = wi[qx] * wj[qy] * wk[qz];
-        const int64_t m = ci[qx] + (int64_t)cx1 * (cj[qy] + (int64_t)cy1 * ck[qz]);
-        a0 = fmaf(w, xc[3 * m], a0);
-        a1 = fmaf(w, xc[3 * m + 1], a1);
-        a2 = fmaf(w, xc[3 * m + 2], a2);
-      }
-  const float acc[3] = {a0, a1, a2};
-  const int64_t b = PAD ? (int64_t)pitch * (j + (int64_t)fy1 * k) + 3 * i : 3 * n;
+    for (int cc = 0; cc < 3; ++cc) {
+      v[q][cc] = base[(q & 1 ? oy : 0) + (q >> 1 ? oz : 0) + cc];
+      v[q][3 + cc] = base[(q & 1 ? oy : 0) + (q >> 1 ? oz : 0) + ox + cc];
+    }
 #pragma unroll
   for (int cc = 0; cc < 3; ++cc) {
-    const bool fr = PAD ? !(nf[n] & (1 << cc)) : (invdf[3 * n + cc] != 0.0f);
-    if (fr) xf[b + cc] += acc[cc];
+    x[cc] = xf[b + cc];
+    x[3 + cc] = xf[b + ox + cc];
+    if (!PAD) d[cc] = invdf[3 * n + cc], d[3 + cc] = invdf[3 * n + ox + cc];
+  }
+  if (PAD) fl[0] = nf[n], fl[1] = nf[n + (odd ? 1 : 0)];
+  float e[3] = {0.f, 0.f, 0.f}, o[3] = {0.f, 0.f, 0.f};  // the even and the odd node's sums
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const float w = wj[q & 1] * wk[q >> 1];  // x weight 1 (even node, or the last of an odd count) or 1/2
+#pragma unroll
+    for (int cc = 0; cc < 3; ++cc) {
+      e[cc] = fmaf(w, v[q][cc], e[cc]);
+      o[cc] = last ? fmaf(w, v[q][3 + cc], o[cc]) : fmaf(0.5f * w, v[q][3 + cc], fmaf(0.5f * w, v[q][cc], o[cc]));
+    }
+  }
+#pragma unroll
+  for (int q = 0; q < 6; ++q) {
+    const bool fr = PAD ? !(fl[q / 3] & (1 << q % 3)) : d[q] != 0.0f;
+    if (fr && (q < 3 || odd)) xf[b + q] = x[q] + (q < 3 ? e[q] : o[q - 3]);
   }
 }
 
@@ -2396,8 +2425,8 @@ __global__ void k_mg_prolong(MgDims f, int pitch, const uint8_t* __restrict__ nf
   int64_t n;
   int k;
   mg_item_case<MULTI>(blockIdx.x * (int64_t)blockDim.x + threadIdx.x, ncase, &n, &k);
-  if (n >= mg_nn(f) || !mg_running(st ? st + k : nullptr)) return;
-  mg_prolong_node<PAD>(f, pitch, nf, invdf, xf.p[k], c, xc.p[k], n);
+  if (n >= mg_pairs(f) || !mg_running(st ? st + k : nullptr)) return;
+  mg_prolong_pair<PAD>(f, pitch, nf, invdf, xf.p[k], c, xc.p[k], n);
 }
 
 
@@ -2477,10 +2506,11 @@ __global__ void __launch_bounds__(1024) k_mg_coarse_setup(MgDims d, const float*
 
 // The coarse levels from T down to the coarsest and back in one launch of one thread-block cluster: levels
 // this small cost more in separate launches than in work. The cluster's CTAs are co-scheduled, so a cluster
-// barrier separates the phases; all vectors stay in global memory (L2).
-constexpr int kMgTailCtas = 8, kMgTailThreads = 512;
-// levels of at most this many nodes go to the cluster kernel (on the bridge: 12x6x6 and below). Measured on
-// the bridge: 2 nodes per cluster thread (8,192, from 24x12x12 down) 45.2 SIMP iter/s, 2,048 47.7, 256 47.2.
+// barrier separates the phases.
+// Sixteen CTAs (the opt-in size): a level of up to about 1,700 nodes fits in their shared memory with its stencil,
+// and the copies at the start take half as long as with eight (16.8 against 20.9 us for 480 + 105 + 24 nodes).
+constexpr int kMgTailCtas = 16, kMgTailThreads = 512;
+// levels of at most this many nodes go to the cluster kernel, as far as they fit (mg_tail_plan)
 constexpr int64_t kMgTailMaxNodes = 2048;
 
 struct MgTailLevel {
@@ -2489,19 +2519,24 @@ struct MgTailLevel {
   const float* S;
   const float* invd;
   float *xa, *xb, *r, *t;  // case 0's vectors; case k's at + k * 3 nn
+  // the level in the shared-memory form (mg_tail_smem): padded node grid's row and plane strides and size (nodes),
+  // rows (DOFs) and rows per CTA, and the shared-memory offsets (4-byte words) of the CTA's stencil rows (-1: read
+  // from global memory), x, t (4 psize a case), 1/diag (all rows), r (the CTA's rows, a case) and the nodes'
+  // coordinates
+  int psy, psz, psize, rows, rpc;
+  int oS, ox, ot, oi, orr, oc;
 };
 struct MgTail {
   int T, L, sweeps, nc;
   const double* ainv;
+  int group;     // load cases the shared-memory form takes at once (0: it does not fit, vectors stay in global memory)
+  int ocr, ocx;  // shared-memory offsets of the coarsest level's r and x (nc a case)
+  int smem;      // its bytes
   MgTailLevel lv[kMgMaxLevels];
 };
 
-// phase barrier of the tail kernel: the cluster's barrier, or the CTA's when it runs as one CTA
-__device__ __forceinline__ void mg_cluster_sync(bool one_cta) {
-  if (one_cta) {
-    __syncthreads();
-    return;
-  }
+// phase barrier of the tail kernel
+__device__ __forceinline__ void mg_cluster_sync() {
   asm volatile("barrier.cluster.arrive.release;\n" ::: "memory");
   asm volatile("barrier.cluster.wait.acquire;\n" ::: "memory");
 }
@@ -2509,10 +2544,11 @@ __device__ __forceinline__ void mg_cluster_sync(bool one_cta) {
 // Levels T .. L-1 of the V-cycle for ncase load cases: from r of level T (restricted by the caller) to the
 // smoothed correction of level T, left in its xa. Work items are numbered with the case fastest; a case whose
 // state is not running is skipped, and the kernel returns at once (every thread alike) when none is.
-// Body for the threads gt (of gs) of the cluster (or the single CTA when one_cta) that runs this V-cycle's tail.
+// Body for the threads gt (of gs) of the cluster that runs this V-cycle's tail, with the vectors in global memory: used
+// where the levels do not fit in shared memory (mg_tail_plan) and for several sweeps.
 template <bool MULTI>
 __device__ __forceinline__ void mg_tail_body(const MgTail& tl, const float* __restrict__ om, const MixState* st,
-                                             int ncase, int64_t gt, int64_t gs, bool one_cta) {
+                                             int ncase, int64_t gt, int64_t gs) {
   bool any = false;
   for (int k = 0; k < ncase; ++k) any = any || mg_running(st ? st + k : nullptr);
   if (!any) return;
@@ -2547,13 +2583,13 @@ __device__ __forceinline__ void mg_tail_body(const MgTail& tl, const float* __re
     float *x = v.xa, *o = v.xb;  // x = omega invd r, written with r by the restriction into this level
     for (int k = 1; k < tl.sweeps; ++k) {
       apply(v, x, o, 1, w);
-      mg_cluster_sync(one_cta);
+      mg_cluster_sync();
       float* tmp = x;
       x = o;
       o = tmp;
     }
     apply(v, x, v.t, 2, 0.0f);
-    mg_cluster_sync(one_cta);
+    mg_cluster_sync();
     const bool smoothed = l + 1 < tl.L - 1;  // the coarsest level is solved, not smoothed
     const float wc = smoothed ? om[l + 1] : 0.0f;
     for (int64_t q = gt; q < cnd * ncase; q += gs) {
@@ -2561,10 +2597,10 @@ __device__ __forceinline__ void mg_tail_body(const MgTail& tl, const float* __re
       int k;
       mg_item_case<MULTI>(q, ncase, &it, &k);
       if (live(k))
-        mg_restrict_comp<false>(v.d, 0, nullptr, v.t + k * nd, cv.d, cv.invd, cv.r + k * cnd, it / 3, (int)(it % 3),
+        mg_restrict_comp(v.d, v.t + k * nd, cv.d, cv.invd, cv.r + k * cnd, it / 3, (int)(it % 3),
                                 smoothed ? cv.xa + k * cnd : nullptr, wc);
     }
-    mg_cluster_sync(one_cta);
+    mg_cluster_sync();
     xc[l] = x;
   }
   {  // coarsest level: x = A^-1 r, one warp per (row, case)
@@ -2583,7 +2619,7 @@ __device__ __forceinline__ void mg_tail_body(const MgTail& tl, const float* __re
       for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
       if (lane == 0) v.xa[k * nd + row] = (float)acc;
     }
-    mg_cluster_sync(one_cta);
+    mg_cluster_sync();
     xc[tl.L - 1] = v.xa;
   }
   for (int l = tl.L - 2; l >= tl.T; --l) {
@@ -2600,10 +2636,10 @@ __device__ __forceinline__ void mg_tail_body(const MgTail& tl, const float* __re
         mg_prolong_comp<false>(v.d, 0, nullptr, v.invd, x + k * nd, tl.lv[l + 1].d, xc[l + 1] + k * cnd, it / 3,
                                (int)(it % 3));
     }
-    mg_cluster_sync(one_cta);
+    mg_cluster_sync();
     for (int k = 0; k < tl.sweeps; ++k) {
       apply(v, x, o, 1, w);
-      mg_cluster_sync(one_cta);
+      mg_cluster_sync();
       float* tmp = x;
       x = o;
       o = tmp;
@@ -2622,11 +2658,334 @@ __device__ __forceinline__ void mg_tail_body(const MgTail& tl, const float* __re
   }
 }
 
+// The same phases (one sweep) with the levels in shared memory. What bounds the small levels is latency, not work:
+// in mg_tail_body ten phases of 162 loads from L2 with their index arithmetic (about 1,000 instructions a row, one
+// at a time) behind ten cluster barriers, 42 to 67 us a V-cycle. Here a CTA keeps its rows of every level's stencil
+// (copied once at the start), the whole of every level's x and t (four floats a node, padded by a zero node on each
+// side, so that a neighbour is a constant step away and needs no test), 1/diag and the nodes' coordinates, and a row
+// is 129 instructions. Only the products and the coarsest solve are split over the cluster: a thread per row writes
+// its result to all eight CTAs' copies, and one cluster barrier follows; restriction and prolongation are done by
+// every CTA for itself. Each row's chain of products, each restriction and prolongation sum and the coarsest rows are
+// formed in the order of mg_tail_body, so the results are its bits (an absent neighbour's zero product leaves a sum
+// as it is). 480 + 105 + 24 nodes: 42 -> 16.8 us; four cases on 1,683 nodes and below: 125 -> 21 us and the four
+// launches of the finest level; eight problems' clusters side by side: 67 -> 21 us.
+constexpr int kTailEnt = 84;  // words of a staged stencil row: 81 entries, and no bank conflicts of 16-byte loads
+
+__device__ __forceinline__ void mg_cluster_arrive() { asm volatile("barrier.cluster.arrive.release;\n" ::: "memory"); }
+__device__ __forceinline__ void mg_cluster_wait() { asm volatile("barrier.cluster.wait.acquire;\n" ::: "memory"); }
+// v to the same shared-memory word of every CTA of the cluster
+__device__ __forceinline__ void mg_put_all(float* p, float v) {
+  const uint32_t a = smem_u32(p);
+#pragma unroll
+  for (int r = 0; r < kMgTailCtas; ++r) {
+    uint32_t ra;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(a), "r"(r));
+    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(ra), "f"(v) : "memory");
+  }
+}
+
+__device__ __forceinline__ void mg_tail_smem(const MgTail& tl, const float* __restrict__ om, const MixState* st,
+                                             int ncase, int rank, float* sm) {
+  const int tid = threadIdx.x, nth = blockDim.x, warp = tid >> 5, lane = tid & 31, nwarp = nth >> 5;
+  unsigned live = 0;
+  for (int k = 0; k < ncase; ++k) live |= mg_running(st ? st + k : nullptr) ? 1u << k : 0u;
+  if (!live) return;  // the same for every CTA of the cluster
+  mg_cluster_arrive();  // remote stores wait until every CTA has started
+  int* smi = reinterpret_cast<int*>(sm);
+  const int T = tl.T, L = tl.L, nc = tl.nc;
+  // What comes from global memory is copied asynchronously, all of it on its way at once (a load and a store a
+  // time were 8 us of latency). First the CTA's stencil rows: a warp takes 9 entries of 32 rows, its entries
+  // compile-time constants.
+  for (int l = T; l < L - 1; ++l) {
+    const MgTailLevel& v = tl.lv[l];
+    const int lo = rank * v.rpc, nr = max(0, min(v.rpc, v.rows - lo)), nch = (nr + 31) >> 5;
+    if (v.oS < 0) continue;
+    const int64_t ns = mg_ns(v.d);
+    const int nx1 = v.d.nx + 1, sxy = nx1 * (v.d.ny + 1);
+    for (int q = warp; q < nch * 9; q += nwarp) {
+      const int blk = q / nch, lr = 32 * (q - nch * blk) + lane;
+      if (lr >= nr) continue;
+      const int row = lo + lr, n = row / 3, ci = row - 3 * n;
+      float* dst = sm + v.oS + lr * kTailEnt;
+      auto entries = [&](auto B) {
+        constexpr int kBlk = decltype(B)::value;
+#pragma unroll
+        for (int nb = 3 * kBlk; nb < 3 * kBlk + 3; ++nb) {
+          // own blocks at the node, an earlier neighbour's transposed ones at the neighbour (before the first node:
+          // no such neighbour, zero)
+          const int m = nb >= 13 ? n : n + (nb % 3 - 1) + nx1 * ((nb / 3) % 3 - 1) + sxy * (nb / 9 - 1);
+          const float* src = v.S + ((nb >= 13 ? (nb - 13) * 9 + 3 * ci : (13 - nb) * 9 + ci) * ns + m);
+          const int64_t step = nb >= 13 ? ns : 3 * ns;
+#pragma unroll
+          for (int cj = 0; cj < 3; ++cj)
+            if (m >= 0) __pipeline_memcpy_async(dst + 3 * nb + cj, src + cj * step, 4);
+            else dst[3 * nb + cj] = 0.f;
+        }
+      };
+      switch (blk) {  // the same for the warp
+        case 0: entries(std::integral_constant<int, 0>()); break;
+        case 1: entries(std::integral_constant<int, 1>()); break;
+        case 2: entries(std::integral_constant<int, 2>()); break;
+        case 3: entries(std::integral_constant<int, 3>()); break;
+        case 4: entries(std::integral_constant<int, 4>()); break;
+        case 5: entries(std::integral_constant<int, 5>()); break;
+        case 6: entries(std::integral_constant<int, 6>()); break;
+        case 7: entries(std::integral_constant<int, 7>()); break;
+        default: entries(std::integral_constant<int, 8>()); break;
+      }
+    }
+  }
+  for (int l = T; l < L; ++l) {  // 1/diag; coordinates i | j << 10 | k << 20; zeros (the padding stays zero)
+    const MgTailLevel& v = tl.lv[l];
+    for (int q = tid; q < v.rows; q += nth) __pipeline_memcpy_async(sm + v.oi + q, v.invd + q, 4);
+    const int nx1 = v.d.nx + 1, ny1 = v.d.ny + 1;
+    for (int n = tid; n < (int)v.nn; n += nth) {
+      int i, j, k;
+      mg_ijk(n, nx1, ny1, &i, &j, &k);
+      smi[v.oc + n] = i | j << 10 | k << 20;
+    }
+    if (l == L - 1) break;
+    for (int q = tid; q < v.psize * tl.group; q += nth) {
+      reinterpret_cast<float4*>(sm + v.ox)[q] = make_float4(0.f, 0.f, 0.f, 0.f);
+      reinterpret_cast<float4*>(sm + v.ot)[q] = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+  }
+  bool started = false;
+  for (int c0 = 0; c0 < ncase; c0 += tl.group) {
+    const int g = min(tl.group, ncase - c0);
+    if (!(live >> c0 & ((1u << g) - 1))) continue;
+    // item of a loop over `items` items x cases -> item, case (items x cases is far below 2^20)
+    auto split = [&](int it, int items, int* c) {
+      *c = g == 1 ? 0 : __float2int_rz(((float)it + 0.5f) * (1.0f / (float)items));
+      return it - *c * items;
+    };
+    auto pad = [&](const MgTailLevel& v, int n) {  // padded position of a node
+      const int q = smi[v.oc + n];
+      return ((q & 1023) + 1) + v.psy * ((q >> 10 & 1023) + 1) + v.psz * ((q >> 20) + 1);
+    };
+    __syncthreads();  // coordinates and zeros; an earlier group is done with its vectors
+    {  // level T: x = omega invd r (written with r by the restriction into it) and the CTA's rows of r
+      const MgTailLevel& v = tl.lv[T];
+      const int lo = rank * v.rpc, nr = max(0, min(v.rpc, v.rows - lo));
+      if (T < L - 1) {
+        for (int it = tid; it < v.rows * g; it += nth) {
+          int c;
+          const int row = split(it, v.rows, &c), n = row / 3;
+          __pipeline_memcpy_async(sm + v.ox + 4 * (c * v.psize + pad(v, n)) + row - 3 * n,
+                                  v.xa + ((int64_t)(c0 + c) * v.rows + row), 4);
+        }
+        for (int it = tid; it < nr * g; it += nth) {
+          int c;
+          const int lr = split(it, nr, &c);
+          __pipeline_memcpy_async(sm + v.orr + c * v.rpc + lr, v.r + ((int64_t)(c0 + c) * v.rows + lo + lr), 4);
+        }
+      } else {
+        for (int it = tid; it < nc * g; it += nth) __pipeline_memcpy_async(sm + tl.ocr + it, v.r + ((int64_t)c0 * nc + it), 4);
+      }
+    }
+    __pipeline_commit();
+    __pipeline_wait_prior(0);
+    __syncthreads();
+    if (!started) mg_cluster_wait();
+    started = true;
+    // rows of A x on level l, x in shared memory; the result handed to put(case, row, its word, value)
+    auto apply = [&](const MgTailLevel& v, int mode, float w, auto&& put) {
+      const int lo = rank * v.rpc, nr = max(0, min(v.rpc, v.rows - lo));
+      const int sy = 4 * v.psy, sz = 4 * v.psz;
+      for (int it = tid; it < nr * g; it += nth) {
+        int c;
+        const int lr = split(it, nr, &c), row = lo + lr, n = row / 3, ci = row - 3 * n;
+        const int at = 4 * (c * v.psize + pad(v, n));
+        const float* x = sm + v.ox + at;
+        float a = 0.f;
+        if (v.oS >= 0) {
+          const float4* s4 = reinterpret_cast<const float4*>(sm + v.oS + lr * kTailEnt);
+          float s[kTailEnt];
+#pragma unroll
+          for (int q = 0; q < kTailEnt / 4; ++q) {
+            const float4 t = s4[q];
+            s[4 * q] = t.x; s[4 * q + 1] = t.y; s[4 * q + 2] = t.z; s[4 * q + 3] = t.w;
+          }
+#pragma unroll
+          for (int nb = 0; nb < 27; ++nb) {
+            const float4 xm = *reinterpret_cast<const float4*>(x + 4 * (nb % 3 - 1) + sy * ((nb / 3) % 3 - 1) + sz * (nb / 9 - 1));
+            a = fmaf(s[3 * nb], xm.x, fmaf(s[3 * nb + 1], xm.y, fmaf(s[3 * nb + 2], xm.z, a)));
+          }
+        } else {
+          const int64_t ns = mg_ns(v.d);
+          const MgNode gn(v.d, n);
+#pragma unroll
+          for (int nb = 0; nb < 27; ++nb) {
+            const float4 xm = *reinterpret_cast<const float4*>(x + 4 * (nb % 3 - 1) + sy * ((nb / 3) % 3 - 1) + sz * (nb / 9 - 1));
+            const float* q = nb >= 13 ? v.S + ((int64_t)(nb - 13) * 9 + 3 * ci) * ns + n
+                                      : v.S + ((int64_t)(13 - nb) * 9 + ci) * ns + max(gn.at(nb), 0);
+            const int64_t step = nb >= 13 ? ns : 3 * ns;
+            a = fmaf(q[0], xm.x, fmaf(q[step], xm.y, fmaf(q[2 * step], xm.z, a)));
+          }
+        }
+        const float id = sm[v.oi + row], rv = sm[v.orr + c * v.rpc + lr];
+        put(c, row, at + ci, mode == 1 ? fmaf(w * id, rv - a, x[ci]) : (id != 0.0f ? rv - a : 0.0f));
+      }
+    };
+    for (int l = T; l < L - 1; ++l) {
+      const MgTailLevel& v = tl.lv[l];
+      const MgTailLevel& cv = tl.lv[l + 1];
+      apply(v, 2, 0.0f, [&](int, int, int at, float val) { mg_put_all(sm + v.ot + at, val); });
+      mg_cluster_arrive();
+      mg_cluster_wait();
+      const bool smoothed = l + 1 < L - 1;
+      const float wc = smoothed ? om[l + 1] : 0.0f;
+      const int clo = rank * cv.rpc;
+      for (int it = tid; it < cv.rows * g; it += nth) {  // restriction, every CTA for itself
+        int c;
+        const int row = split(it, cv.rows, &c), n = row / 3, ci = row - 3 * n, q = smi[cv.oc + n];
+        const int I = q & 1023, J = q >> 10 & 1023, K = q >> 20;
+        const MgAxis ax(I, v.d.nx, 4), ay(J, v.d.ny, 4 * v.psy), az(K, v.d.nz, 4 * v.psz);
+        const float* t = sm + v.ot + 4 * (c * v.psize + 1 + v.psy + v.psz) + ci;
+        float a = 0.f;
+#pragma unroll
+        for (int u = 0; u < 27; ++u)
+          a = fmaf(az.w[u / 9] * ay.w[u / 3 % 3] * ax.w[u % 3], t[az.o[u / 9] + ay.o[u / 3 % 3] + ax.o[u % 3]], a);
+        const float d = sm[cv.oi + row], rv = d != 0.f ? a : 0.f;
+        if (smoothed) {
+          if (row >= clo && row < clo + cv.rpc) sm[cv.orr + c * cv.rpc + row - clo] = rv;
+          sm[cv.ox + 4 * (c * cv.psize + (I + 1) + cv.psy * (J + 1) + cv.psz * (K + 1)) + ci] = wc * d * rv;
+        } else {
+          sm[tl.ocr + c * nc + row] = rv;
+        }
+      }
+      __syncthreads();
+    }
+    for (int it = rank * nwarp + warp; it < nc * g; it += kMgTailCtas * nwarp) {  // coarsest: x = A^-1 r, a warp a row
+      int c;
+      const int row = split(it, nc, &c);
+      const float* r = sm + tl.ocr + c * nc;
+      double acc = 0.0;
+      for (int col = lane; col < nc; col += 32) acc = fma(tl.ainv[(int64_t)row * nc + col], (double)r[col], acc);
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+      if (lane < kMgTailCtas) {
+        uint32_t ra;
+        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(smem_u32(sm + tl.ocx + c * nc + row)), "r"(lane));
+        asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(ra), "f"((float)acc) : "memory");
+      }
+    }
+    mg_cluster_arrive();
+    mg_cluster_wait();
+    for (int l = L - 2; l >= T; --l) {
+      const MgTailLevel& v = tl.lv[l];
+      const MgTailLevel& cv = tl.lv[l + 1];
+      // the coarse x: three floats a node on the coarsest level, else padded (a smoothed level's is where t was)
+      const bool coarsest = l + 1 == L - 1;
+      const int cs = coarsest ? 3 : 4, csy = coarsest ? cs * (cv.d.nx + 1) : cs * cv.psy,
+                csz = coarsest ? csy * (cv.d.ny + 1) : cs * cv.psz;
+      for (int it = tid; it < (int)v.nn * g; it += nth) {  // prolongation, every CTA for itself
+        int c;
+        const int n = split(it, (int)v.nn, &c), q = smi[v.oc + n], i = q & 1023, j = q >> 10 & 1023, k = q >> 20;
+        // per axis: two coarse nodes and their weights (an absent second one has weight 0 and is not read)
+        int o[3][2];
+        float w[3][2];
+        auto axis = [&](int a, int f_, int n_, int nc_, int stride) {
+          const bool mid = (f_ & 1) && f_ != n_;
+          const int c_ = ((f_ & 1) && f_ == n_) ? nc_ : (f_ >> 1);
+          o[a][0] = c_ * stride;
+          o[a][1] = mid ? o[a][0] + stride : o[a][0];
+          w[a][0] = mid ? 0.5f : 1.0f;
+          w[a][1] = mid ? 0.5f : 0.0f;
+        };
+        axis(0, i, v.d.nx, cv.d.nx, cs);
+        axis(1, j, v.d.ny, cv.d.ny, csy);
+        axis(2, k, v.d.nz, cv.d.nz, csz);
+        const float* xc = coarsest ? sm + tl.ocx + c * nc : sm + cv.ot + 4 * (c * cv.psize + 1 + cv.psy + cv.psz);
+        float a[3] = {0.f, 0.f, 0.f};
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+          const float wt = w[0][u & 1] * w[1][u >> 1 & 1] * w[2][u >> 2];
+          const float* p = xc + o[0][u & 1] + o[1][u >> 1 & 1] + o[2][u >> 2];
+#pragma unroll
+          for (int ci = 0; ci < 3; ++ci) a[ci] = fmaf(wt, p[ci], a[ci]);
+        }
+        float* x = sm + v.ox + 4 * (c * v.psize + (i + 1) + v.psy * (j + 1) + v.psz * (k + 1));
+#pragma unroll
+        for (int ci = 0; ci < 3; ++ci)
+          if (sm[v.oi + 3 * n + ci] != 0.0f) x[ci] += a[ci];
+      }
+      __syncthreads();
+      if (l > T) {  // the smoothed x goes where t was
+        apply(v, 1, om[l], [&](int, int, int at, float val) { mg_put_all(sm + v.ot + at, val); });
+        mg_cluster_arrive();
+        mg_cluster_wait();
+      } else {
+        apply(v, 1, om[l], [&](int c, int row, int, float val) {
+          if (live >> (c0 + c) & 1) v.xa[(int64_t)(c0 + c) * v.rows + row] = val;
+        });
+      }
+    }
+    if (T == L - 1 && rank == 0)
+      for (int it = tid; it < nc * g; it += nth)
+        if (live >> (c0 + it / nc) & 1) tl.lv[T].xa[(int64_t)c0 * nc + it] = sm[tl.ocx + it];
+  }
+}
+
 template <bool MULTI>
 __global__ void __launch_bounds__(kMgTailThreads)
     k_mg_tail(const __grid_constant__ MgTail tl, const float* __restrict__ om, const MixState* st, int ncase) {
-  mg_tail_body<MULTI>(tl, om, st, ncase, blockIdx.x * (int64_t)blockDim.x + threadIdx.x,
-                      (int64_t)gridDim.x * blockDim.x, gridDim.x == 1);
+  extern __shared__ __align__(16) float tail_smem[];
+  if (tl.group) mg_tail_smem(tl, om, st, ncase, (int)blockIdx.x, tail_smem);
+  else
+    mg_tail_body<MULTI>(tl, om, st, ncase, blockIdx.x * (int64_t)blockDim.x + threadIdx.x,
+                        (int64_t)gridDim.x * blockDim.x);
+}
+
+// Shared-memory layout of mg_tail_smem for the levels from T and up to ncase load cases: every level's stencil rows
+// resident if that leaves room for a case, else the finest level's read from global memory; as many cases at once
+// as fit. group 0: not even one does (or several sweeps are asked for), the vectors stay in global memory.
+constexpr int kMgTailSmemMax = 220 * 1024;
+static bool mg_tail_layout(MgTail& tl, int g, bool resident) {
+  int64_t o = 0;
+  auto take = [&](int64_t n) {
+    const int64_t at = o;
+    o += (n + 3) & ~int64_t(3);
+    return (int)std::min<int64_t>(at, INT_MAX / 2);
+  };
+  for (int l = tl.T; l < tl.L; ++l) {
+    MgTailLevel& v = tl.lv[l];
+    v.rows = (int)(3 * v.nn);
+    v.rpc = (v.rows + kMgTailCtas - 1) / kMgTailCtas;
+    v.oc = take(v.nn);
+    v.oi = take(v.rows);
+    if (l == tl.L - 1) break;
+    v.psy = v.d.nx + 3;
+    v.psz = v.psy * (v.d.ny + 3);
+    v.psize = v.psz * (v.d.nz + 3);
+    v.ox = take((int64_t)g * 4 * v.psize);
+    v.ot = take((int64_t)g * 4 * v.psize);
+    v.orr = take((int64_t)g * v.rpc);
+    v.oS = resident || l > tl.T ? take((int64_t)kTailEnt * v.rpc) : -1;
+  }
+  tl.ocr = take((int64_t)g * tl.nc);
+  tl.ocx = take((int64_t)g * tl.nc);
+  tl.group = g;
+  tl.smem = (int)std::min<int64_t>(o * (int64_t)sizeof(float), INT_MAX);
+  return o * (int64_t)sizeof(float) <= kMgTailSmemMax;
+}
+// The tail of ncase load cases: from the first level of at most kMgTailMaxNodes nodes whose cases all fit with its
+// stencil (a level that took its cases in several passes, or its stencil from L2, is cheaper as separate kernels:
+// 125 us against about 50 for four cases on 1,683 nodes); none fits or several sweeps: from the first level of at
+// most kMgTailMaxNodes nodes, as few cases at a time as must be.
+static void mg_tail_plan(MgTail& tl, int ncase) {
+  const int T0 = tl.T, gmax = std::min(ncase, kMgMaxCases);
+  if (tl.sweeps == 1) {
+    for (tl.T = T0; tl.T < tl.L; ++tl.T)
+      if (mg_tail_layout(tl, gmax, true)) return;
+    tl.T = T0;
+    for (int resident = 1; resident >= 0; --resident)
+      for (int g = gmax; g >= 1; --g)
+        if (mg_tail_layout(tl, g, resident != 0)) return;
+  }
+  tl.T = T0;
+  tl.group = 0;
+  tl.smem = 0;
 }
 
 // Outer step, part 1. mode 0: x += alpha p, r -= alpha q (FP64, padded layout), ||r|| against the stop and
@@ -3040,8 +3399,8 @@ struct MgHier {
   float* f_t = nullptr;  // FP32 outer form: A x of the voxel level's smoothing (padded FP32 layout)
   float* eig[kMgMaxLevels] = {};  // last eigenvector estimate of D^-1 A per smoothed level (warm start)
   bool eig_valid = false;
-  int T = 1;             // first level handled by the cluster kernel k_mg_tail
-  MgTail tail{};
+  MgTail tails[2] = {};  // the cluster kernel's levels (from its T): of a single solve, of load cases together
+  const MgTail& tail(int nc) const { return tails[nc > 1 ? 1 : 0]; }
   bool prefers_f64 = false;  // an FP32 outer solve of this problem stalled: later ones start in FP64
   int ncap = 1;          // load cases the level vectors have room for (case k at + k * nd)
   // load cases solved together (mg_solve_cases): per case the FP32 work vectors x, r, z, p0, p1, ap, t of the
@@ -3115,6 +3474,8 @@ void mg_release(mycel_problem* p) {
   p->mg = nullptr;
 }
 
+static const void* mg_tail_pk_kernel(bool multi);  // the packed launches' cluster kernel
+
 static int32_t mg_ensure(mycel_problem* p, bool* available) {
   static std::once_flag smem_once;
   static cudaError_t smem_err = cudaSuccess;
@@ -3124,6 +3485,14 @@ static int32_t mg_ensure(mycel_problem* p, bool* available) {
       smem_err = cudaFuncSetAttribute(k_mg_apply_nodes_tma, cudaFuncAttributeMaxDynamicSharedMemorySize, kS1Smem);
     if (smem_err == cudaSuccess)  // four CTAs of 54 KB per SM
       smem_err = cudaFuncSetAttribute(k_mg_apply_nodes_tma, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+    for (const void* k : {(const void*)k_mg_tail<false>, (const void*)k_mg_tail<true>, mg_tail_pk_kernel(false),
+                          mg_tail_pk_kernel(true)})
+      if (smem_err == cudaSuccess)
+        smem_err = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kMgTailSmemMax);
+    if (kMgTailCtas > 8)
+      for (const void* k : {(const void*)k_mg_tail<false>, (const void*)k_mg_tail<true>, mg_tail_pk_kernel(false),
+                            mg_tail_pk_kernel(true)})
+        if (smem_err == cudaSuccess) smem_err = cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
   });
   if (smem_err != cudaSuccess)
     return set_error(p->ctx, MYCEL_E_DEVICE, std::string("multigrid shared memory: ") + cudaGetErrorString(smem_err));
@@ -3219,6 +3588,7 @@ static int32_t mg_ensure(mycel_problem* p, bool* available) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(kMgTailCtas);
     cfg.blockDim = dim3(kMgTailThreads);
+    cfg.dynamicSmemBytes = kMgTailSmemMax;
     cudaLaunchAttribute at{};
     at.id = cudaLaunchAttributeClusterDimension;
     at.val.clusterDim.x = kMgTailCtas;
@@ -3235,23 +3605,26 @@ static int32_t mg_ensure(mycel_problem* p, bool* available) {
     }
   }
   // levels T .. L-1 in one cluster launch: T is the first coarse level of at most kMgTailMaxNodes nodes
-  mg->T = L - 1;
+  MgTail tl{};
+  tl.T = L - 1;
   for (int l = 1; l < L; ++l)
     if (mg->lv[l].nn <= kMgTailMaxNodes) {
-      mg->T = l;
+      tl.T = l;
       break;
     }
-  mg->tail.T = mg->T;
-  mg->tail.L = L;
-  mg->tail.sweeps = mg->sweeps;
-  mg->tail.nc = (int)nc;
-  mg->tail.ainv = mg->ainv;
+  tl.L = L;
+  tl.sweeps = mg->sweeps;
+  tl.nc = (int)nc;
+  tl.ainv = mg->ainv;
   for (int l = 1; l < L; ++l) {
     const MgLevel& v = mg->lv[l];
-    mg->tail.lv[l] = {v.d, v.nn, v.S, v.invd, v.xa, v.xb, v.r, v.t};
+    tl.lv[l] = {v.d, v.nn, v.S, v.invd, v.xa, v.xb, v.r, v.t};
   }
+  mg->tails[0] = mg->tails[1] = tl;
+  mg_tail_plan(mg->tails[0], 1);
+  mg_tail_plan(mg->tails[1], mg->ncap);
   // launches per outer iteration: matvec, k_mg_enter*, the V-cycle (as issued by mg_vcycle), k_mg_exit*
-  const int sw = mg->sweeps, T = mg->T;
+  const int sw = mg->sweeps, T = mg->tails[0].T;
   const int cycle = 4 * (sw - 1) + 2 + (T - 1) * (1 + sw) + 1 + (T - 1) * (1 + sw) + 1 + 1;
   mg->per_iter = 3 + cycle;
   p->mg = mg;
@@ -3266,23 +3639,22 @@ static unsigned mg_blocks(int64_t n) { return (unsigned)((n + 255) / 256); }
 // the bridge: level 2, 31k nodes, 9.6 vs 14.5 us; level 1, 233k nodes, 43 vs 51 us)
 // the small levels' kernel: one 8-CTA cluster with cluster barriers between phases (a single CTA with CTA
 // barriers was measured slower: 51.9 against 56.6 SIMP iter/s on the bridge)
-static int mg_tail_ctas() { return kMgTailCtas; }
-
 static void launch_mg_tail(cudaStream_t s, MgHier* mg, const float* om, const MixState* st, int nc) {
-  const int ctas = mg_tail_ctas();
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(ctas);
+  cfg.gridDim = dim3(kMgTailCtas);
   cfg.blockDim = dim3(kMgTailThreads);
+  const MgTail& tl = mg->tail(nc);
+  cfg.dynamicSmemBytes = (size_t)tl.smem;
   cfg.stream = s;
   cudaLaunchAttribute at{};
   at.id = cudaLaunchAttributeClusterDimension;
-  at.val.clusterDim.x = ctas;
+  at.val.clusterDim.x = kMgTailCtas;
   at.val.clusterDim.y = 1;
   at.val.clusterDim.z = 1;
   cfg.attrs = &at;
-  cfg.numAttrs = ctas > 1 ? 1 : 0;
-  if (nc == 1) cudaLaunchKernelEx(&cfg, k_mg_tail<false>, mg->tail, om, st, nc);
-  else cudaLaunchKernelEx(&cfg, k_mg_tail<true>, mg->tail, om, st, nc);
+  cfg.numAttrs = 1;
+  if (nc == 1) cudaLaunchKernelEx(&cfg, k_mg_tail<false>, tl, om, st, nc);
+  else cudaLaunchKernelEx(&cfg, k_mg_tail<true>, tl, om, st, nc);
 }
 
 // case k's vector of a level whose case vectors follow one another (base + k * nd)
@@ -3394,7 +3766,7 @@ static int mg_vcycle(mycel_problem* p, cudaStream_t s, const MgRun& R) {
   const GridDims& g = p->g;
   const float* om = mg->sc->omega;  // device: damping of level l at om + l
   const int sb = stream_blocks(p);
-  const int nc = R.n;
+  const int nc = R.n, T = mg->tail(nc).T;
   MixState* st = R.st;
   auto cst = [&](int k) { return st ? st + k : nullptr; };
   int nl = 0;
@@ -3416,7 +3788,7 @@ static int mg_vcycle(mycel_problem* p, cudaStream_t s, const MgRun& R) {
                                                                om + 1, nc);
   nl++;
   float* xc[kMgMaxLevels] = {};
-  for (int l = 1; l < mg->T; ++l) {
+  for (int l = 1; l < T; ++l) {
     MgLevel& v = lv[l];
     float *x = v.xa, *o = v.xb;
     const MgPtrs r = lv_ptrs(v.r, v.nd, nc);
@@ -3437,13 +3809,13 @@ static int mg_vcycle(mycel_problem* p, cudaStream_t s, const MgRun& R) {
     nl += 1 + mg->sweeps;
   }
   launch_mg_tail(s, mg, om, st, nc);
-  xc[mg->T] = lv[mg->T].xa;
+  xc[T] = lv[T].xa;
   nl++;
-  for (int l = mg->T - 1; l >= 1; --l) {
+  for (int l = T - 1; l >= 1; --l) {
     MgLevel& v = lv[l];
     float* x = xc[l];
     float* o = x == v.xa ? v.xb : v.xa;
-    (nc == 1 ? k_mg_prolong<false, false> : k_mg_prolong<false, true>)<<<mg_blocks(v.nn * nc), 256, 0, s>>>(v.d, 0, nullptr, v.invd, lv_ptrs(x, v.nd, nc), lv[l + 1].d,
+    (nc == 1 ? k_mg_prolong<false, false> : k_mg_prolong<false, true>)<<<mg_blocks(mg_pairs(v.d) * nc), 256, 0, s>>>(v.d, 0, nullptr, v.invd, lv_ptrs(x, v.nd, nc), lv[l + 1].d,
                                                               lv_ptrs(xc[l + 1], lv[l + 1].nd, nc), st, nc);
     const MgPtrs r = lv_ptrs(v.r, v.nd, nc);
     for (int k = 0; k < mg->sweeps; ++k) {
@@ -3453,7 +3825,7 @@ static int mg_vcycle(mycel_problem* p, cudaStream_t s, const MgRun& R) {
     xc[l] = x;
     nl += 1 + mg->sweeps;
   }
-  (nc == 1 ? k_mg_prolong<true, false> : k_mg_prolong<true, true>)<<<mg_blocks(lv[0].nn * nc), 256, 0, s>>>(lv[0].d, g.rp, p->d_nflags, nullptr, mg_ptrs(R.xf, nc),
+  (nc == 1 ? k_mg_prolong<true, false> : k_mg_prolong<true, true>)<<<mg_blocks(mg_pairs(lv[0].d) * nc), 256, 0, s>>>(lv[0].d, g.rp, p->d_nflags, nullptr, mg_ptrs(R.xf, nc),
                                                               lv[1].d, lv_ptrs(xc[1], lv[1].nd, nc), st, nc);
   nl++;
   for (int q = 1; q < mg->sweeps; ++q)
@@ -3597,7 +3969,7 @@ static int32_t capture_inner_graph(mycel_problem* p, const InnerForm& F, int chu
       } else {
         launch_inner_mv(p, F, s, pprev, pcur);
       }
-      if (mg) mg->l1_timing = (c->profile && t == 0 && mg->T > 1) ? mg->l1ev[k] : nullptr;
+      if (mg) mg->l1_timing = (c->profile && t == 0 && mg->tails[0].T > 1) ? mg->l1ev[k] : nullptr;
       launch_inner_xr(p, F, s, pcur, 0);
       if (mg) mg->l1_timing = nullptr;
     }
@@ -3733,7 +4105,7 @@ static int32_t refined_loop(mycel_problem* p, const InnerForm& F, const double* 
           c->prof_nodes[F.prof_slot] += p->g.nn;
           c->prof_elems[F.prof_slot] += p->n_active;
         }
-        if (F.mg && p->mg->T > 1 &&
+        if (F.mg && p->mg->tails[0].T > 1 &&
             cudaEventElapsedTime(&ms_, p->mg->l1ev[pi][0], p->mg->l1ev[pi][1]) == cudaSuccess) {
           c->prof_ms[3] += ms_;
           c->prof_n[3] += 1;
@@ -4077,7 +4449,7 @@ int32_t kernel_bench(mycel_problem* p, int which, int reps, double* avg_us) {
   if (which == 3) {
     bool avail = false;
     if ((st = mg_ensure(p, &avail))) return st;
-    if (!avail || p->mg->T <= 1) return set_error(c, MYCEL_E_ARG, "kernel_bench: no multigrid level 1 on the whole GPU");
+    if (!avail || p->mg->tails[0].T <= 1) return set_error(c, MYCEL_E_ARG, "kernel_bench: no multigrid level 1 on the whole GPU");
     mg = p->mg;
     if (mg->setup_version != p->e_version) {
       mg_setup(p);
@@ -4611,8 +4983,8 @@ __global__ void k_mg_prolong_pk(const PkProlong* __restrict__ tab,
     int64_t q;
     int k;
     mg_item_case<MULTI>((int64_t)(code & kPkLbMask) * blockDim.x + threadIdx.x, a.ncase, &q, &k);
-    if (q >= mg_nn(a.f) || !mg_running(a.st ? a.st + k : nullptr)) continue;
-    mg_prolong_node<PAD>(a.f, a.pitch, a.nf, a.invdf, a.xf.p[k], a.c, a.xc.p[k], q);
+    if (q >= mg_pairs(a.f) || !mg_running(a.st ? a.st + k : nullptr)) continue;
+    mg_prolong_pair<PAD>(a.f, a.pitch, a.nf, a.invdf, a.xf.p[k], a.c, a.xc.p[k], q);
   }
 }
 
@@ -4625,9 +4997,15 @@ struct PkTail {  // the cluster kernel of a problem's V-cycle (all its cases); o
 
 template <bool MULTI>
 __global__ void __launch_bounds__(kMgTailThreads) k_mg_tail_pk(const PkTail* __restrict__ tab) {
+  extern __shared__ __align__(16) float tail_smem[];
   const PkTail& t = tab[blockIdx.x / kMgTailCtas];
-  mg_tail_body<MULTI>(t.tl, t.om, t.st, t.ncase, (int64_t)(blockIdx.x % kMgTailCtas) * blockDim.x + threadIdx.x,
-                      (int64_t)kMgTailCtas * blockDim.x, false);
+  if (t.tl.group) mg_tail_smem(t.tl, t.om, t.st, t.ncase, (int)(blockIdx.x % kMgTailCtas), tail_smem);
+  else
+    mg_tail_body<MULTI>(t.tl, t.om, t.st, t.ncase, (int64_t)(blockIdx.x % kMgTailCtas) * blockDim.x + threadIdx.x,
+                      (int64_t)kMgTailCtas * blockDim.x);
+}
+static const void* mg_tail_pk_kernel(bool multi) {
+  return multi ? (const void*)k_mg_tail_pk<true> : (const void*)k_mg_tail_pk<false>;
 }
 
 // state ops of the right-hand sides (a kernel parameter, so the host may rewrite its copy at once): -1 none,
@@ -4687,6 +5065,7 @@ struct PkLaunch {
   int n;
   unsigned blocks;  // work items when every entry runs (its launches alone's CTAs)
   unsigned grid;    // persistent CTAs of the launch
+  size_t smem = 0;  // cluster kernel: the largest shared memory of its entries
 };
 
 // A right-hand side of a packed solve: its voxel-level FP32 vectors, state, RHS and solution.
@@ -4880,6 +5259,7 @@ static void pk_issue(const PackPlan& P, const PkLaunch& L, cudaStream_t s, int s
       cudaLaunchConfig_t cfg = {};
       cfg.gridDim = dim3((unsigned)(kMgTailCtas * L.n));
       cfg.blockDim = dim3(kMgTailThreads);
+      cfg.dynamicSmemBytes = L.smem;
       cfg.stream = s;
       cudaLaunchAttribute at{};
       at.id = cudaLaunchAttributeClusterDimension;
@@ -5039,7 +5419,7 @@ static int32_t pk_build(mycel_ctx* c, PackWork* w, std::vector<PkUnit>& units, c
     return r;
   };
   int maxT = 1;
-  for (const Prob& q : probs) maxT = std::max(maxT, q.p->mg->T);
+  for (const Prob& q : probs) maxT = std::max(maxT, q.p->mg->tail(q.nc).T);
   std::vector<std::vector<float*>> xc(probs.size(), std::vector<float*>(kMgMaxLevels, nullptr));
   fine_mv();
   for (int multi = 0; multi < 2; ++multi) {  // voxel grid -> level 1, with level 1's first sweep
@@ -5078,7 +5458,7 @@ static int32_t pk_build(mycel_ctx* c, PackWork* w, std::vector<PkUnit>& units, c
         for (size_t qi = 0; qi < probs.size(); ++qi) {
           const Prob& q = probs[qi];
           MgHier* mg = q.p->mg;
-          if (l >= mg->T || (q.nc > 1) != (multi == 1)) continue;
+          if (l >= mg->tail(q.nc).T || (q.nc > 1) != (multi == 1)) continue;
           const MgLevel& v = mg->lv[l];
           const bool is_node = !(v.nn * q.nc <= kMgDofMaxNodes);
           if (is_node != (node == 1)) continue;
@@ -5108,7 +5488,7 @@ static int32_t pk_build(mycel_ctx* c, PackWork* w, std::vector<PkUnit>& units, c
       for (size_t qi = 0; qi < probs.size(); ++qi) {
         const Prob& q = probs[qi];
         MgHier* mg = q.p->mg;
-        if (l >= mg->T || (q.nc > 1) != (multi == 1)) continue;
+        if (l >= mg->tail(q.nc).T || (q.nc > 1) != (multi == 1)) continue;
         const MgLevel& v = mg->lv[l];
         const MgLevel& cv = mg->lv[l + 1];
         PkRestrict a{};
@@ -5141,16 +5521,19 @@ static int32_t pk_build(mycel_ctx* c, PackWork* w, std::vector<PkUnit>& units, c
       if ((q.nc > 1) != (multi == 1)) continue;
       MgHier* mg = q.p->mg;
       PkTail t{};
-      t.tl = mg->tail;
+      t.tl = mg->tail(q.nc);
       t.om = mg->sc->omega;
       t.st = q.st;
       t.ncase = q.nc;
       e.push_back(t);
       nb.push_back(kMgTailCtas);
       es.push_back({const_cast<MixState*>(q.st), q.nc});
-      xc[qi][mg->T] = mg->lv[mg->T].xa;
+      xc[qi][t.tl.T] = mg->lv[t.tl.T].xa;
     }
+    size_t smem = 0;
+    for (const PkTail& t : e) smem = std::max(smem, (size_t)t.tl.smem);
     B.add(P.vcycle, PK_TAIL, false, multi == 1, 0, e, nb, es);
+    if (!e.empty()) P.vcycle.back().smem = smem;
   }
   for (int l = maxT - 1; l >= 1; --l) {
     for (int multi = 0; multi < 2; ++multi) {  // level l + 1 -> l, into xa (the downward sweep's vector)
@@ -5160,7 +5543,7 @@ static int32_t pk_build(mycel_ctx* c, PackWork* w, std::vector<PkUnit>& units, c
       for (size_t qi = 0; qi < probs.size(); ++qi) {
         const Prob& q = probs[qi];
         MgHier* mg = q.p->mg;
-        if (l >= mg->T || (q.nc > 1) != (multi == 1)) continue;
+        if (l >= mg->tail(q.nc).T || (q.nc > 1) != (multi == 1)) continue;
         const MgLevel& v = mg->lv[l];
         PkProlong a{};
         a.f = v.d;
@@ -5173,14 +5556,14 @@ static int32_t pk_build(mycel_ctx* c, PackWork* w, std::vector<PkUnit>& units, c
         a.st = q.st;
         a.ncase = q.nc;
         e.push_back(a);
-        nb.push_back(mg_blocks(v.nn * q.nc));
+        nb.push_back(mg_blocks(mg_pairs(v.d) * q.nc));
         es.push_back({const_cast<MixState*>(q.st), q.nc});
       }
       B.add(P.vcycle, PK_PROLONG, false, multi == 1, 0, e, nb, es);
     }
     applies(l, false);
     for (size_t qi = 0; qi < probs.size(); ++qi)
-      if (l < probs[qi].p->mg->T) xc[qi][l] = probs[qi].p->mg->lv[l].xb;  // one sweep: xa -> xb
+      if (l < probs[qi].p->mg->tail(probs[qi].nc).T) xc[qi][l] = probs[qi].p->mg->lv[l].xb;  // one sweep: xa -> xb
   }
   for (int multi = 0; multi < 2; ++multi) {  // level 1 -> voxel grid, into each unit's z
     std::vector<PkProlong> e;
@@ -5201,7 +5584,7 @@ static int32_t pk_build(mycel_ctx* c, PackWork* w, std::vector<PkUnit>& units, c
       a.st = q.st;
       a.ncase = q.nc;
       e.push_back(a);
-      nb.push_back(mg_blocks(mg->lv[0].nn * q.nc));
+      nb.push_back(mg_blocks(mg_pairs(mg->lv[0].d) * q.nc));
       es.push_back({const_cast<MixState*>(q.st), q.nc});
     }
     B.add(P.vcycle, PK_PROLONG, true, multi == 1, 0, e, nb, es);
