@@ -1331,33 +1331,46 @@ __global__ void k_pow(int64_t n, const double* __restrict__ x, const double* __r
 // ---------------------------------------------------------------------------------------------------------
 // OC update: persistent cooperative kernel with a bounded grid barrier
 // ---------------------------------------------------------------------------------------------------------
-// Every wait gives up after OcArgs::max_polls polls of __nanosleep(64) (about 1 s by default, longer for large
-// n, see launch_oc) and sets the error flag, so a grid that cannot meet ends with MYCEL_E_TIMEOUT on the host.
-__device__ bool grid_sync_bounded(unsigned int* bar, int* err, long long max_polls, unsigned int extra) {
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    volatile unsigned int* vgen = bar + 1;
-    unsigned int gen = *vgen;
-    __threadfence();
-    unsigned int arrived = atomicAdd(bar, 1u);
-    if (arrived == gridDim.x - 1 + extra) {
-      bar[0] = 0;
-      __threadfence();
-      atomicAdd(bar + 1, 1u);
-    } else {
-      long long spins = 0;
-      while (*vgen == gen) {
-        if (++spins > max_polls || *(volatile int*)err) {
-          atomicExch(err, 1);
-          break;
-        }
-        __nanosleep(64);
+// The barrier counts arrivals without end (launch_oc clears the word): its k-th use waits for k * gridDim.x of
+// them, so a waiter sees the last arrival itself and no second word is needed. Only thread 0's own stores (and what
+// it has observed of its CTA's by __syncthreads) are released: the callers publish partial sums only.
+// Every wait gives up after OcArgs::max_polls polls (about 1 s by default, longer for large n, see launch_oc; all
+// but the first 64 sleep 64 ns) and sets the error flag, so a grid that cannot meet ends with MYCEL_E_TIMEOUT.
+struct GridBar {
+  unsigned int* bar;  // bar[0]: arrivals
+  int* err;
+  long long max_polls;
+  unsigned int extra;  // arrivals waited for beyond the grid (0; 1 only to test the time-out path)
+  unsigned int target = 0;
+};
+__device__ __forceinline__ unsigned int ld_acquire(const unsigned int* p) {
+  unsigned int v;
+  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+// arrival and wait by one thread of the CTA; false once any CTA has given up
+__device__ __forceinline__ bool grid_meet(GridBar& g) {
+  unsigned int old;
+  asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(old) : "l"(g.bar) : "memory");
+  const unsigned int want = g.target + g.extra;
+  if (old + 1 != want) {
+    long long polls = 0;
+    while (ld_acquire(g.bar) < want) {
+      if (++polls > g.max_polls || ((polls & 15) == 0 && *(volatile int*)g.err)) {
+        atomicExch(g.err, 1);
+        return false;
       }
+      if (polls > 64) __nanosleep(64);
     }
-    __threadfence();
   }
+  return *(volatile int*)g.err == 0;
+}
+__device__ bool grid_sync_bounded(GridBar& g) {
+  g.target += gridDim.x;
+  bool ok = true;
   __syncthreads();
-  return *(volatile int*)err == 0;
+  if (threadIdx.x == 0) ok = grid_meet(g);
+  return __syncthreads_and(ok ? 1 : 0) != 0;
 }
 
 __device__ __forceinline__ double clampd(double v, double lo, double hi) {
@@ -1385,17 +1398,27 @@ __device__ __forceinline__ double oc_new_rho(double r, double dc, double si, boo
   return clampd(r * sqrt(b), lo, hi);
 }
 
-__device__ double block_sum(double v, double* sh) {
-  for (int o = 16; o > 0; o >>= 1) v = v + __shfl_down_sync(0xffffffffu, v, o);
-  int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+// CTA sums of two values (lanes by a fixed shuffle tree, then the warps in order): bits as of one sum after the
+// other. Thread 0 has the first, thread 1 the second.
+__device__ __forceinline__ double block_sum2(double v0, double v1, double* sh) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    v0 = v0 + __shfl_down_sync(0xffffffffu, v0, o);
+    v1 = v1 + __shfl_down_sync(0xffffffffu, v1, o);
+  }
+  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
   __syncthreads();
-  if (l == 0) sh[w] = v;
+  if (l == 0) {
+    sh[w] = v0;
+    sh[8 + w] = v1;
+  }
   __syncthreads();
   double t = 0.0;
-  if (threadIdx.x == 0) {
-    for (int k = 0; k < (int)(blockDim.x >> 5); ++k) t = t + sh[k];
+  if (threadIdx.x < 2) {
+#pragma unroll
+    for (int k = 0; k < 8; ++k) t = t + sh[8 * threadIdx.x + k];
   }
-  return t;  // valid in thread 0
+  return t;
 }
 
 struct OcArgs {
@@ -1417,37 +1440,274 @@ struct OcArgs {
 };
 // scratch layout (grid = gridDim.x): [0, 4 grid) two alternating pairs of per-block partial sums (value, sum of
 // magnitudes) of the volume trials; [4 grid, 7 grid) per-block max change, volume and grey sums;
-// [7 grid, 7 grid + 4) two alternating broadcast cells of sequential sums; then the barrier words.
+// [7 grid, 7 grid + 4) two alternating broadcast cells of sequential sums; the barrier words (4 doubles); then
+// [7 grid + 8, 11 grid + 8) the chunks of a sequential sum: totals, binades, steps from an even and an odd sum.
 
-// Grid-wide deterministic sums of two per-thread values; every block gets the same totals (thread 0 valid).
-__device__ void grid_total2(double m0, double m1, const OcArgs& a, int slot, double* sh, bool* ok, double* t0,
-                            double* t1) {
-  double b0 = block_sum(m0, sh);
-  double b1 = block_sum(m1, sh);
+// Grid-wide deterministic sums of two per-thread values; every thread of every block gets the same totals.
+// Latency is all there is to it: both values go through one reduction, one warp carries the partials to and from
+// memory, and its loads of the other blocks' partials are issued together. Lane l takes blocks l, l + 32, ... in
+// order, then a fixed shuffle tree (the same order in every block, so every block gets the same bits).
+__device__ __forceinline__ bool grid_total2(double m0, double m1, const OcArgs& a, GridBar& g, int slot, double* sh,
+                                            double* t0, double* t1) {
+  const double b = block_sum2(m0, m1, sh);
   double* part = a.scratch + (size_t)slot * 2 * gridDim.x;
-  if (threadIdx.x == 0) {
-    part[blockIdx.x] = b0;
-    part[gridDim.x + blockIdx.x] = b1;
-  }
-  if (!grid_sync_bounded(a.bar, a.err, a.max_polls, a.extra)) {
-    *ok = false;
-    return;
-  }
-  // warp 0 adds the block partials: lane l takes blocks l, l + 32, ... in order, then a fixed shuffle tree
-  // (the same order in every block, so every block gets the same bits)
-  double s0 = 0.0, s1 = 0.0;
+  const unsigned n = gridDim.x;
+  g.target += n;
+  bool ok = true;
   if (threadIdx.x < 32) {
-    for (unsigned k = threadIdx.x; k < gridDim.x; k += 32) {
-      s0 = s0 + ld_volatile(part + k);
-      s1 = s1 + ld_volatile(part + gridDim.x + k);
+    if (threadIdx.x < 2) part[threadIdx.x * n + blockIdx.x] = b;
+    __syncwarp();
+    if (threadIdx.x == 0) ok = grid_meet(g);
+    __syncwarp();
+    double s0 = 0.0, s1 = 0.0;
+    for (unsigned k0 = threadIdx.x; k0 < n; k0 += 32 * 10) {
+      double p0[10], p1[10];
+#pragma unroll
+      for (int j = 0; j < 10; ++j) {
+        const unsigned k = k0 + 32 * j;
+        p0[j] = k < n ? ld_volatile(part + k) : 0.0;
+        p1[j] = k < n ? ld_volatile(part + n + k) : 0.0;
+      }
+#pragma unroll
+      for (int j = 0; j < 10; ++j)
+        if (k0 + 32 * j < n) {
+          s0 = s0 + p0[j];
+          s1 = s1 + p1[j];
+        }
     }
+#pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
       s0 = s0 + __shfl_xor_sync(0xffffffffu, s0, o);
       s1 = s1 + __shfl_xor_sync(0xffffffffu, s1, o);
     }
+    if (threadIdx.x == 0) {
+      sh[16] = s0;
+      sh[17] = s1;
+    }
   }
-  *t0 = s0;
-  *t1 = s1;
+  ok = __syncthreads_and(ok ? 1 : 0) != 0;
+  *t0 = sh[16];
+  *t1 = sh[17];
+  return ok;
+}
+
+// ---- sums in element order, in parallel ------------------------------------------------------------------
+// The reference adds n terms one after the other. While the running sum stays in one binade [2^e, 2^(e+1)) it is
+// an integer M of units u = 2^(e-52), and adding a term t >= 0 rounds to M + round(t / u): the integer nearest to
+// t / u, whatever M is, except that a tie goes to the even sum and so depends on M's last bit. A run of terms is
+// therefore a pair of integers, the increments from an even and from an odd M; pairs compose (associatively), so
+// threads, warps and blocks can each take a run and the sum comes out with the bits of the sequential one. What a
+// run may not do is leave the binade: then (and for terms that are negative or not finite) its terms are added one
+// by one. The binade a chunk of terms begins in is guessed from an ordinary parallel sum of the chunks before it;
+// the guess is checked against the sum itself, so a wrong one costs time only. With n terms of like size the sum
+// crosses about log2 n binades, most of them in the first chunk.
+struct SumStep {
+  long long even, odd;  // increments (units of the binade) from an even and from an odd sum; kStepOut: leaves it
+};
+constexpr long long kStepOut = 1ll << 54;
+__device__ __forceinline__ SumStep step_then(SumStep f, SumStep g) {
+  SumStep r;
+  r.even = min(f.even + ((f.even & 1) ? g.odd : g.even), kStepOut);
+  r.odd = min(f.odd + ((f.odd & 1) ? g.even : g.odd), kStepOut);
+  return r;
+}
+__device__ __forceinline__ SumStep step_of(double t, double inv_u) {
+  const double q = t * inv_u;  // a power of two: exact (or far below one half)
+  SumStep r;
+  if (t >= 0.0 && q < 0x1p53) {
+    const long long k = __double2ll_rn(q);  // nearest, ties to even: the increment of an even sum
+    r.even = k;
+    r.odd = fabs(q - (double)k) == 0.5 ? (long long)(q + q) - k : k;  // a tie: the other neighbour
+  } else {
+    r.even = r.odd = kStepOut;
+  }
+  return r;
+}
+__device__ __forceinline__ SumStep warp_steps(SumStep v) {  // lane 0: the lanes' steps in lane order
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    SumStep w;
+    w.even = __shfl_down_sync(0xffffffffu, v.even, o);
+    w.odd = __shfl_down_sync(0xffffffffu, v.odd, o);
+    v = step_then(v, w);
+  }
+  return v;
+}
+// biased exponent of a sum that can take steps, or 0 (zero, negative, not finite, or so large or small that the
+// units or their reciprocal leave the normal range)
+__device__ __forceinline__ int sum_binade(double acc) {
+  const int hi = (int)((unsigned long long)__double_as_longlong(acc) >> 52);
+  return hi >= 100 && hi <= 1900 ? hi : 0;
+}
+__device__ __forceinline__ double binade_inv_u(int b) { return __longlong_as_double((long long)(2098 - b) << 52); }
+// acc after a run's step taken in binade b; false (acc unchanged) if the sum is not in b or the run leaves it
+__device__ __forceinline__ bool take_step(double& acc, int b, long long even, long long odd) {
+  const long long bits = __double_as_longlong(acc);
+  if (b == 0 || (int)((unsigned long long)bits >> 52) != b) return false;
+  const long long m = (bits & 0xfffffffffffffll) | (1ll << 52);
+  const long long m2 = m + ((m & 1) ? odd : even);
+  if (m2 >= (1ll << 53)) return false;
+  acc = __longlong_as_double(((long long)b << 52) | (m2 & 0xfffffffffffffll));
+  return true;
+}
+
+enum OcSum : int { OC_SUM_S, OC_SUM_VOLUME, OC_SUM_PHYS, OC_SUM_GREY };
+__device__ __forceinline__ double oc_seq_term(const OcArgs& a, const OcParams& prm, int kind, double lam, int64_t i) {
+  const int64_t e = a.idx ? (int64_t)a.idx[i] : i;
+  if (kind == OC_SUM_PHYS) return a.rho_phys[e];
+  if (kind == OC_SUM_GREY) {
+    const double rb = a.rho_grey[e];
+    return rb * (1.0 - rb);
+  }
+  const double si = a.s[e];
+  if (kind == OC_SUM_S) return si;
+  return si * ((a.pas && a.pas[e]) ? 1.0 : oc_new_rho(a.rho[e], a.dc[e], si, false, lam, prm.move, prm.rho_min));
+}
+
+constexpr int kSeqTile = 1024, kSeqPiece = 128;  // terms of a CTA's tile; of a warp's piece of it
+struct SeqSmem {
+  double term[kSeqTile];
+  SumStep piece[8];
+  SumStep chunk[256];
+  int binade[256];
+  double acc;
+  int next;
+};
+// acc + terms [i0, i1) in order, by one CTA (acc in sm.acc): a tile of terms at a time, each warp the step of one
+// piece in the sum's present binade; thread 0 takes the steps in order and adds the terms of a piece that leaves
+// the binade one by one, after which the pieces behind it are stepped again in the new one.
+__device__ __forceinline__ void seq_range(const OcArgs& a, const OcParams& prm, int kind, double lam, int64_t i0,
+                                          int64_t i1, SeqSmem& sm) {
+  const int tid = threadIdx.x, w = tid >> 5, l = tid & 31;
+  for (int64_t base = i0; base < i1; base += kSeqTile) {
+    const int cnt = (int)min((int64_t)kSeqTile, i1 - base);
+    const int np = (cnt + kSeqPiece - 1) / kSeqPiece;
+    for (int k = tid; k < np * kSeqPiece; k += 256)
+      sm.term[k] = k < cnt ? oc_seq_term(a, prm, kind, lam, base + k) : 0.0;  // a running sum + 0 is itself
+    __syncthreads();
+    for (int lo = 0; lo < np;) {
+      const int b = sum_binade(sm.acc);
+      if (b && w >= lo && w < np) {
+        const double iu = binade_inv_u(b);
+        const double* t = sm.term + w * kSeqPiece + 4 * l;
+        SumStep v = step_then(step_then(step_of(t[0], iu), step_of(t[1], iu)),
+                              step_then(step_of(t[2], iu), step_of(t[3], iu)));
+        v = warp_steps(v);
+        if (l == 0) sm.piece[w] = v;
+      }
+      __syncthreads();
+      if (tid == 0) {
+        double acc = sm.acc;
+        int k = lo;
+        while (k < np && take_step(acc, b, sm.piece[k].even, sm.piece[k].odd)) ++k;
+        if (k < np) {
+          const double* t = sm.term + k * kSeqPiece;
+#pragma unroll 16
+          for (int j = 0; j < kSeqPiece; ++j) acc = acc + t[j];
+          ++k;
+        }
+        sm.acc = acc;
+        sm.next = k;
+      }
+      __syncthreads();
+      lo = sm.next;
+    }
+  }
+}
+
+// Sum of a kind of term over i = 0 .. n-1 in that order (the reference's sequential loops); every thread gets it.
+// Short sums: block 0 alone. Else the blocks take one chunk each: a plain sum (for the guess of the binade the
+// next chunks begin in), then the chunk's step in the guessed binade; block 0 takes the steps in order and walks
+// through the chunks whose step does not hold.
+__device__ __noinline__ double sequential_sum(const OcArgs& a, const OcParams& prm, int kind, double lam, int cell,
+                                              GridBar& g, double* sh, SeqSmem& sm, bool* ok) {
+  const int tid = threadIdx.x;
+  const unsigned nb = gridDim.x;
+  double* c = a.scratch + (size_t)7 * nb + 2 * cell;
+  double* tot = a.scratch + (size_t)7 * nb + 8;
+  long long* bin = (long long*)(tot + nb);
+  long long* even = (long long*)(tot + 2 * (size_t)nb);
+  long long* odd = (long long*)(tot + 3 * (size_t)nb);
+  const bool split = a.n > 2 * kSeqTile;
+  const int64_t len = max((int64_t)256, (a.n + nb - 1) / nb);
+  const int nchunk = (int)((a.n + len - 1) / len);
+  *ok = true;
+  if (split) {
+    const int64_t i0 = min(a.n, (int64_t)blockIdx.x * len), i1 = min(a.n, i0 + len);
+    double v = 0.0;
+    for (int64_t i = i0 + tid; i < i1; i += 256) v = v + oc_seq_term(a, prm, kind, lam, i);
+    const double bs = block_sum2(v, 0.0, sh);
+    if (tid == 0) tot[blockIdx.x] = bs;
+    if (!grid_sync_bounded(g)) {
+      *ok = false;
+      return 0.0;
+    }
+    double before = 0.0;
+    for (unsigned k = tid; k < blockIdx.x; k += 256) before = before + ld_volatile(tot + k);
+    before = block_sum2(before, 0.0, sh);
+    if (tid == 0) sm.acc = before;
+    __syncthreads();
+    const int b = sum_binade(sm.acc);
+    const double iu = binade_inv_u(b);
+    // thread t: a run of consecutive terms, so that lanes and warps compose in term order
+    const int64_t run = (i1 - i0 + 255) / 256;
+    const int64_t r0 = min(i1, i0 + tid * run), r1 = min(i1, r0 + run);
+    SumStep st{0, 0};
+    if (b)
+      for (int64_t i = r0; i < r1; ++i) st = step_then(st, step_of(oc_seq_term(a, prm, kind, lam, i), iu));
+    st = warp_steps(st);
+    if ((tid & 31) == 0) sm.piece[tid >> 5] = st;
+    __syncthreads();
+    if (tid == 0) {
+      st = sm.piece[0];
+      for (int k = 1; k < 8; ++k) st = step_then(st, sm.piece[k]);
+      bin[blockIdx.x] = b;
+      even[blockIdx.x] = st.even;
+      odd[blockIdx.x] = st.odd;
+    }
+    if (!grid_sync_bounded(g)) {
+      *ok = false;
+      return 0.0;
+    }
+  }
+  if (blockIdx.x == 0) {
+    if (tid == 0) sm.acc = 0.0;
+    __syncthreads();
+    if (!split) {
+      seq_range(a, prm, kind, lam, 0, a.n, sm);
+    } else {
+      for (int k0 = 0; k0 < nchunk;) {
+        const int k = k0 + tid, kn = min(256, nchunk - k0);
+        if (tid < kn) {
+          sm.binade[tid] = (int)*(volatile long long*)(bin + k);
+          sm.chunk[tid].even = *(volatile long long*)(even + k);
+          sm.chunk[tid].odd = *(volatile long long*)(odd + k);
+        }
+        __syncthreads();
+        if (tid == 0) {
+          double acc = sm.acc;
+          int j = 0;
+          while (j < kn && take_step(acc, sm.binade[j], sm.chunk[j].even, sm.chunk[j].odd)) ++j;
+          sm.acc = acc;
+          sm.next = j;
+        }
+        __syncthreads();
+        const int j = sm.next;
+        k0 += j;
+        __syncthreads();  // sm.next is read before seq_range writes it
+        if (j < kn) {
+          seq_range(a, prm, kind, lam, k0 * len, min(a.n, (k0 + 1) * len), sm);
+          ++k0;
+        }
+      }
+    }
+    if (tid == 0) *(volatile double*)c = sm.acc;
+  }
+  if (!grid_sync_bounded(g)) {
+    *ok = false;
+    return 0.0;
+  }
+  return ld_volatile(c);
 }
 
 // A volume V(lambda) of the bisection: the grid's tree sum, with an error bound against any other order of the
@@ -1457,88 +1717,74 @@ struct OcVol {
   bool exact;
 };
 
-__global__ void __launch_bounds__(256) k_oc(OcArgs a, OcParams prm) {
+// What bounds it: a trial's terms are one divide and one square root per element, a few microseconds at most; below
+// about a million elements the trials (30 to 50 a call) are bound by the latency of the grid's sum and barrier. So a
+// thread keeps its elements in registers when 8 per thread hold them, and the sum and the barrier are one step
+// (grid_total2).
+// Measured on B200, a whole call: 221,184 elements deciding on sums in element order 5.81 ms -> 0.56 ms (those sums
+// were added by one warp, 13 ns a term); 121,635 elements on the grid's sums 227 us -> 152 us.
+__global__ void __launch_bounds__(256) k_oc(const __grid_constant__ OcArgs a, const __grid_constant__ OcParams prm) {
   __shared__ double sh[32];
-  __shared__ double bc[4];
+  __shared__ SeqSmem sm;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   const int64_t t0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   bool ok = true;
   int slot = 0, cell = 0;
+  GridBar gb{a.bar, a.err, a.max_polls, a.extra};
   auto element = [&](int64_t i) -> int64_t { return a.idx ? (int64_t)a.idx[i] : i; };
-  auto term = [&](int64_t e, double lam) -> double {
-    const double si = a.s[e];
-    return si * ((a.pas && a.pas[e]) ? 1.0 : oc_new_rho(a.rho[e], a.dc[e], si, false, lam, prm.move, prm.rho_min));
-  };
-  // Sum of f(i) over i = 0 .. n-1 in that order (the reference's sequential loops), by warp 0 of block 0: its
-  // lanes evaluate 32 consecutive terms, then every lane adds them one by one in index order. The other blocks
-  // wait at the grid barrier; the result is broadcast through a scratch cell.
-  auto sequential_sum = [&](auto f) -> double {
-    double* c = a.scratch + (size_t)7 * gridDim.x + 2 * cell;
+  auto seq = [&](int kind, double lam) -> double {
     cell ^= 1;
-    if (blockIdx.x == 0 && threadIdx.x < 32) {
-      double acc = 0.0;
-      for (int64_t base = 0; base < a.n; base += 32) {
-        const int64_t i = base + threadIdx.x;
-        const double t = i < a.n ? f(i) : 0.0;
-        const int cnt = (int)min((int64_t)32, a.n - base);
-        for (int k = 0; k < cnt; ++k) acc = acc + __shfl_sync(0xffffffffu, t, k);
-      }
-      if (threadIdx.x == 0) *(volatile double*)c = acc;
-    }
-    if (!grid_sync_bounded(a.bar, a.err, a.max_polls, a.extra)) {
-      ok = false;
-      return 0.0;
-    }
-    return ld_volatile(c);
+    return sequential_sum(a, prm, kind, lam, cell, gb, sh, sm, &ok);
   };
   // tree depth of a grid total: the per-thread chain, the warp and block steps, the lane-strided block partials
   const double depth = (double)((a.n + stride - 1) / stride) + 5.0 + 8.0 + (double)((gridDim.x + 31) / 32) + 5.0;
+  // the thread's elements t0, t0 + stride, ... summed in that order; the loads of 8 of them are issued before
+  // their terms are added, so the index -> data load chains overlap; with at most 8 they are loaded once
+  constexpr int kB = 8;
+  double si[kB], rr[kB], dd[kB];
+  unsigned pp = 0;
+  auto load = [&](int64_t base) {
+    pp = 0;
+#pragma unroll
+    for (int k = 0; k < kB; ++k) {
+      const int64_t i = base + k * stride;
+      const int64_t e = i < a.n ? element(i) : 0;
+      if (i < a.n && a.pas && a.pas[e]) pp |= 1u << k;
+      si[k] = i < a.n ? a.s[e] : 0.0;
+      rr[k] = i < a.n ? a.rho[e] : 0.0;
+      dd[k] = i < a.n ? a.dc[e] : 0.0;
+    }
+  };
+  const bool held = a.n <= kB * stride;
+  if (held) load(t0);
   auto volume = [&](double lam) -> OcVol {
-    // the thread's elements t0, t0 + stride, ... summed in that order; the loads of 8 of them are issued before
-    // their terms are added, so the index -> data load chains overlap
-    constexpr int kB = 8;
     double v = 0.0, va = 0.0;
     for (int64_t base = t0; base < a.n; base += kB * stride) {
-      double si[kB], rr[kB], dd[kB];
-      bool pp[kB];
-#pragma unroll
-      for (int k = 0; k < kB; ++k) {
-        const int64_t i = base + k * stride;
-        const int64_t e = i < a.n ? element(i) : 0;
-        pp[k] = i < a.n && a.pas && a.pas[e];
-        si[k] = i < a.n ? a.s[e] : 0.0;
-        rr[k] = i < a.n ? a.rho[e] : 0.0;
-        dd[k] = i < a.n ? a.dc[e] : 0.0;
-      }
+      if (!held) load(base);
 #pragma unroll
       for (int k = 0; k < kB; ++k)
         if (base + k * stride < a.n) {
-          const double t = si[k] * (pp[k] ? 1.0 : oc_new_rho(rr[k], dd[k], si[k], false, lam, prm.move, prm.rho_min));
+          const double t =
+              si[k] * (((pp >> k) & 1) ? 1.0 : oc_new_rho(rr[k], dd[k], si[k], false, lam, prm.move, prm.rho_min));
           v = v + t;
           va = va + fabs(t);
         }
     }
     double tv = 0.0, ta = 0.0;
-    grid_total2(v, va, a, slot, sh, &ok, &tv, &ta);
+    if (!grid_total2(v, va, a, gb, slot, sh, &tv, &ta)) ok = false;
     slot ^= 1;
-    if (threadIdx.x == 0) {
-      bc[0] = tv;
-      bc[1] = ta;
-    }
-    __syncthreads();
     OcVol r;
-    r.v = bc[0];
+    r.v = tv;
     // |tree - exact| <= gamma_depth sum|t| and |sequential - exact| <= gamma_(n-1) sum|t|, gamma_k = k u / (1 - k u);
     // doubled for the rounding of the computed sum of magnitudes and of the bound itself
-    r.bound = 2.0 * ((double)a.n + depth) * 0x1p-53 * bc[1] * 1.0000001;
+    r.bound = 2.0 * ((double)a.n + depth) * 0x1p-53 * ta * 1.0000001;
     r.exact = false;
-    __syncthreads();
     return r;
   };
   // the volume at lam in the reference's order, when a decision needs it
   auto make_exact = [&](OcVol& x, double lam) {
     if (x.exact) return;
-    x.v = sequential_sum([&](int64_t i) { return term(element(i), lam); });
+    x.v = seq(OC_SUM_VOLUME, lam);
     x.bound = 0.0;
     x.exact = true;
   };
@@ -1547,17 +1793,13 @@ __global__ void __launch_bounds__(256) k_oc(OcArgs a, OcParams prm) {
   if (prm.total_s >= 0.0) {
     ts = prm.total_s;
   } else if (prm.exact) {
-    ts = sequential_sum([&](int64_t i) { return a.s[element(i)]; });
+    ts = seq(OC_SUM_S, 0.0);
   } else {
     double sv = 0.0;
     for (int64_t i = t0; i < a.n; i += stride) sv = sv + a.s[element(i)];
     double t1 = 0.0;
-    grid_total2(sv, 0.0, a, slot, sh, &ok, &ts, &t1);
+    if (!grid_total2(sv, 0.0, a, gb, slot, sh, &ts, &t1)) ok = false;
     slot ^= 1;
-    if (threadIdx.x == 0) bc[0] = ts;
-    __syncthreads();
-    ts = bc[0];
-    __syncthreads();
   }
   if (!ok) return;
   const double tv = prm.f * ts;
@@ -1655,22 +1897,16 @@ __global__ void __launch_bounds__(256) k_oc(OcArgs a, OcParams prm) {
       if (sh[k] > mc) mc = sh[k];
   }
   double* part = a.scratch + (size_t)4 * gridDim.x;
-  double bvs = block_sum(vs, sh);
-  double bgs = block_sum(gs, sh);
-  if (threadIdx.x == 0) {
-    part[blockIdx.x] = mc;
-    part[gridDim.x + blockIdx.x] = bvs;
-    part[2 * gridDim.x + blockIdx.x] = bgs;
-  }
-  if (!grid_sync_bounded(a.bar, a.err, a.max_polls, a.extra)) return;
+  const double bsum = block_sum2(vs, gs, sh);
+  if (threadIdx.x == 0) part[blockIdx.x] = mc;
+  if (threadIdx.x < 2) part[(1 + threadIdx.x) * gridDim.x + blockIdx.x] = bsum;
+  if (!grid_sync_bounded(gb)) return;
   // exact mode: the volume and grey sums in the reference's element order (:328-335)
   double svol = 0.0, sgrey = 0.0;
   if (prm.exact && a.rho_phys) {
-    svol = sequential_sum([&](int64_t i) { return a.rho_phys[element(i)]; });
-    sgrey = sequential_sum([&](int64_t i) {
-      const double rb = a.rho_grey[element(i)];
-      return rb * (1.0 - rb);
-    });
+    svol = seq(OC_SUM_PHYS, 0.0);
+    if (!ok) return;
+    sgrey = seq(OC_SUM_GREY, 0.0);
     if (!ok) return;
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -1708,7 +1944,8 @@ int launch_oc(mycel_ctx* ctx, int64_t n, const int32_t* d_index, const double* r
   unsigned int* bar = (unsigned int*)(d_scratch + 7 * (size_t)grid + 4);
   int* err = (int*)(bar + 4);
   if (cudaMemsetAsync(bar, 0, 8 * sizeof(unsigned int), ctx->stream) != cudaSuccess) return MYCEL_E_DEVICE;
-  // each wait: about 1 s of polling, plus room for the sequential sums of the exact mode (about 20 ns per term)
+  // each wait: about 1 s of polling, plus room for the sequential sums of the exact mode (at worst, when no step of
+  // one holds, block 0 adds all terms one by one at about 10 ns each)
   long long polls = ctx->oc_wait_polls > 0 ? ctx->oc_wait_polls : (1ll << 24) + 4 * (long long)n;
   OcArgs a{n, d_index, rho, dc, s, passive, rho_new, rho_phys_for_metrics,
            rho_tilde_for_grey ? rho_tilde_for_grey : rho_phys_for_metrics, d_scratch, bar, err, d_out,
@@ -1730,9 +1967,9 @@ int launch_oc(mycel_ctx* ctx, int64_t n, const int32_t* d_index, const double* r
 // in the file-scope array below, which every GPU that loads the library holds until the process exits.
 // ---------------------------------------------------------------------------------------------------------
 constexpr int kOcNoAllocMaxBlocks = 1024;                                // persistent OC blocks it can serve
-constexpr int kOcNoAllocScratch = 8 * kOcNoAllocMaxBlocks + 8;           // partials + barrier words + error flag
+constexpr int kOcNoAllocScratch = 12 * kOcNoAllocMaxBlocks + 8;          // partials, barrier words, chunk steps
 constexpr int kOcNoAllocOut = (int)((sizeof(OcOut) + sizeof(double) - 1) / sizeof(double));
-static __device__ __align__(256) double g_oc_noalloc[kOcNoAllocScratch + kOcNoAllocOut];  // 65.7 KB
+static __device__ __align__(256) double g_oc_noalloc[kOcNoAllocScratch + kOcNoAllocOut];  // 98.4 KB
 
 namespace {
 std::mutex g_oc_noalloc_mu;

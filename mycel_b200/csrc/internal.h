@@ -299,8 +299,8 @@ void launch_heaviside(mycel_ctx* ctx, int64_t n, const int32_t* idx, const doubl
                       double* out, double beta, double eta, int mode);
 // Blocks of the persistent OC kernel per SM on the current device (occupancy, clamped to [1, 2]).
 int oc_blocks_per_sm(int* out);
-// Scratch the OC kernel needs for a grid of `grid` blocks: partial sums, broadcast cells, barrier words.
-inline size_t oc_scratch_doubles(int grid) { return (size_t)7 * grid + 4 + 4; }
+// Scratch the OC kernel needs for a grid of `grid` blocks: partial sums, broadcast cells, barrier words, chunk steps.
+inline size_t oc_scratch_doubles(int grid) { return (size_t)11 * grid + 8; }
 int launch_oc(mycel_ctx* ctx, int64_t n, const int32_t* d_index /*box index of element i or null*/,
               const double* rho, const double* dc, const double* s, const uint8_t* passive, double* rho_new,
               const double* rho_phys_for_metrics, const double* rho_tilde_for_grey, const OcParams& prm,
