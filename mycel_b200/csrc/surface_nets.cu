@@ -5,14 +5,16 @@
 //   k_sn_pad       the 1-voxel zero-padded copy of the density and its threshold mask (:48-78)
 //   k_sn_detect    counts face saddles and corner kisses of the current mask (a pass that finds none changes
 //                  nothing, so the common case skips the next kernel)
+//   k_sn_bits      the threshold mask as bit rows, for k_sn_compose
 //   k_sn_compose   MakeWellComposed (:352-435): the reference resolves saddles and kisses in one sequential
 //                  lexicographic sweep per pass, each resolution changing the voxels the later checks read.
 //                  A check at (px, py, pz) touches only the voxels (px..px+1, py..py+1, pz..pz+1), so two
-//                  checks interact only if their positions differ by at most 1 per axis; with
-//                  t = px + 2 py + 4 pz every such earlier position has a smaller t and no two positions of
-//                  the same t interact. Running the checks wavefront by wavefront in t therefore gives the
-//                  sequential result exactly. One thread-block cluster runs all wavefronts of all passes,
-//                  with a cluster barrier between wavefronts (its CTAs are co-scheduled).
+//                  checks interact only if their positions differ by at most 1 per axis. In the skewed
+//                  coordinates x' = px + py + 2 pz, y' = py + pz, z' = pz the later of two such positions is
+//                  nowhere smaller, so boxes of x' y' z' can run in waves X + Y + Z, and the positions of a box in
+//                  wavefronts t = x' + y' + z', with the sequential result exactly. Only boxes, waves and
+//                  wavefronts that hold something to resolve are run. One thread-block cluster runs all passes,
+//                  with a cluster barrier between waves (its CTAs are co-scheduled).
 //   k_sn_cells     one vertex per dual cell with mixed corners (:89-179), the reference's float arithmetic
 //                  with every operation rounded (no contraction)
 //   k_sn_scan_*    deterministic exclusive prefix sums (vertex numbers in cell order; quad slots in edge order)
@@ -42,53 +44,6 @@ struct SnGrid {
   int nx, ny, nz;
   int64_t sy, sz;  // padded strides
 };
-
-__device__ __forceinline__ bool sn_saddle(uint8_t* s, float* rho, float thr, int64_t i00, int64_t i10, int64_t i01,
-                                          int64_t i11) {
-  const bool s00 = s[i00], s10 = s[i10], s01 = s[i01], s11 = s[i11];
-  if (!(s00 == s11 && s10 == s01 && s00 != s10)) return false;
-  const int64_t a = s00 ? i10 : i00, b = s00 ? i01 : i11;  // the two empty voxels of the diagonal pair
-  const int64_t pick = rho[a] >= rho[b] ? a : b;
-  s[pick] = 1;
-  if (rho[pick] < thr) rho[pick] = thr;
-  return true;
-}
-
-__device__ __forceinline__ bool sn_kiss(uint8_t* s, float* rho, float thr, int64_t dA, int64_t dB, int64_t a1,
-                                        int64_t a2, int64_t a3, int64_t b1, int64_t b2, int64_t b3) {
-  if (!(s[dA] && s[dB])) return false;
-  const bool linked = (s[a1] && (s[b1] || s[b2])) || (s[a2] && (s[b1] || s[b3])) || (s[a3] && (s[b2] || s[b3]));
-  if (linked) return false;
-  s[a1] = 1;
-  s[b1] = 1;
-  if (rho[a1] < thr) rho[a1] = thr;
-  if (rho[b1] < thr) rho[b1] = thr;
-  return true;
-}
-
-// the three face checks at (x, y, z), in the reference's order (XY, XZ, YZ); returns the resolutions made
-__device__ __forceinline__ int sn_faces(const SnGrid& g, uint8_t* s, float* rho, float thr, int64_t x, int64_t y,
-                                        int64_t z) {
-  const int64_t b = x + y * g.sy + z * g.sz;
-  int n = 0;
-  if (x < g.nx && y < g.ny && sn_saddle(s, rho, thr, b, b + 1, b + g.sy, b + g.sy + 1)) n++;
-  if (x < g.nx && z < g.nz && sn_saddle(s, rho, thr, b, b + 1, b + g.sz, b + g.sz + 1)) n++;
-  if (y < g.ny && z < g.nz && sn_saddle(s, rho, thr, b, b + g.sy, b + g.sz, b + g.sz + g.sy)) n++;
-  return n;
-}
-
-// the corner-kiss check of the 2x2x2 cube at (x, y, z): the first of its four diagonals that needs it
-__device__ __forceinline__ int sn_cube(const SnGrid& g, uint8_t* s, float* rho, float thr, int64_t x, int64_t y,
-                                       int64_t z) {
-  const int64_t c000 = x + y * g.sy + z * g.sz, c100 = c000 + 1, c010 = c000 + g.sy, c110 = c010 + 1;
-  const int64_t c001 = c000 + g.sz, c101 = c001 + 1, c011 = c001 + g.sy, c111 = c011 + 1;
-  return (sn_kiss(s, rho, thr, c000, c111, c100, c010, c001, c110, c101, c011) ||
-          sn_kiss(s, rho, thr, c100, c011, c000, c110, c101, c010, c001, c111) ||
-          sn_kiss(s, rho, thr, c010, c101, c000, c110, c011, c100, c001, c111) ||
-          sn_kiss(s, rho, thr, c001, c110, c000, c101, c011, c100, c010, c111))
-             ? 1
-             : 0;
-}
 
 __global__ void k_sn_pad(SnGrid g, const float* __restrict__ in, float thr, float* __restrict__ rho,
                          uint8_t* __restrict__ s) {
@@ -133,44 +88,280 @@ __global__ void k_sn_detect(SnGrid g, const uint8_t* __restrict__ s, unsigned lo
   if ((threadIdx.x & 31) == 0 && c) atomicAdd(count, c);
 }
 
+// mask row (y, z) of the padded grid as words of 32 voxels, lowest x in the lowest bit; one warp per word
+__global__ void k_sn_bits(SnGrid g, int words, const uint8_t* __restrict__ s, uint32_t* __restrict__ bits) {
+  const int64_t nw = (int64_t)words * (g.ny + 2) * (g.nz + 2);
+  const int lane = threadIdx.x & 31;
+  for (int64_t w = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; w < nw;
+       w += ((int64_t)gridDim.x * blockDim.x) >> 5) {
+    const int64_t row = w / words;
+    const int64_t x = (w % words) * 32 + lane;
+    const uint32_t m = __ballot_sync(0xffffffffu, x < g.sy && s[row * g.sy + x]);
+    if (lane == 0) bits[w] = m;
+  }
+}
+
 constexpr int kSnCtas = 8, kSnThreads = 1024;
+constexpr int kSnGroup = 256, kSnGroups = kSnThreads / kSnGroup;  // threads of a box; boxes of a CTA at a time
+constexpr int kBx = 32, kBy = 16, kBz = 16;                       // a box's extent in x', y', z'
+constexpr int kRowsY = kBy + 2, kRowsZ = kBz + 1;                 // mask rows it reads
+
+// k_sn_compose's view of the grid: boxes (X, Y, Z) with Y = Z + K (y = y' - z' lies in [1, ny]), their flags and
+// those of the waves
+struct SnBoxes {
+  int nX, nK, nZ, waves, words;
+  uint32_t* bits;
+  uint8_t* box[2];   // per box: holds a position to check (one set for the faces, one for the corner kisses)
+  uint8_t* wave[2];  // per wave: has such a box
+  int64_t nbox;
+};
+inline SnBoxes sn_boxes(const SnGrid& g) {
+  SnBoxes b{};
+  b.nX = (g.nx + g.ny + 2 * g.nz) / kBx + 1;
+  b.nK = (g.ny + kBy - 1) / kBy + 1;
+  b.nZ = g.nz / kBz + 1;
+  b.waves = b.nX + (b.nK + b.nZ - 1) + b.nZ;
+  b.words = (g.nx + 2 + 31) / 32;
+  b.nbox = (int64_t)b.nX * b.nK * b.nZ;
+  return b;
+}
 
 __device__ __forceinline__ void sn_cluster_sync() {
   asm volatile("barrier.cluster.arrive.release;\n" ::: "memory");
   asm volatile("barrier.cluster.wait.acquire;\n" ::: "memory");
 }
+__device__ __forceinline__ void sn_group_sync(int group) {
+  asm volatile("bar.sync %0, %1;\n" ::"r"(group + 1), "n"(kSnGroup) : "memory");
+}
+
+// voxels x0 .. x0 + 63 of mask row (y, z), 0 outside the padded grid
+__device__ __forceinline__ uint64_t sn_row(const SnGrid& g, const SnBoxes& b, int x0, int y, int z) {
+  if (y < 0 || y > g.ny + 1 || z < 0 || z > g.nz + 1) return 0;
+  const uint32_t* r = b.bits + ((int64_t)z * (g.ny + 2) + y) * b.words;
+  const int w = x0 >> 5, sh = x0 & 31;
+  const uint32_t a0 = w >= 0 && w < b.words ? r[w] : 0u;
+  const uint32_t a1 = w + 1 >= 0 && w + 1 < b.words ? r[w + 1] : 0u;
+  const uint32_t a2 = w + 2 >= 0 && w + 2 < b.words ? r[w + 2] : 0u;
+  return (uint64_t)__funnelshift_r(a0, a1, sh) | ((uint64_t)__funnelshift_r(a1, a2, sh) << 32);
+}
+
+// bits i of a row of positions (x + i, y, z) in [0, 32): which lie in [1, hi]
+__device__ __forceinline__ uint32_t sn_range(int x, int hi) {
+  const int lo = max(0, 1 - x), up = min(31, hi - x);
+  return lo > up ? 0u : (0xffffffffu >> (31 - (up - lo))) << lo;
+}
+__device__ __forceinline__ uint32_t sn_saddles(uint64_t r, uint64_t q) {  // the 2x2 faces of rows r and q
+  const uint32_t a = (uint32_t)r, b = (uint32_t)(r >> 1), c = (uint32_t)q, d = (uint32_t)(q >> 1);
+  return ~(a ^ d) & ~(b ^ c) & (a ^ b);
+}
+__device__ __forceinline__ uint32_t sn_kisses(uint32_t dA, uint32_t dB, uint32_t a1, uint32_t a2, uint32_t a3,
+                                              uint32_t b1, uint32_t b2, uint32_t b3) {
+  return dA & dB & ~((a1 & (b1 | b2)) | (a2 & (b1 | b3)) | (a3 & (b2 | b3)));
+}
+// the positions (x + i, y, z) with something to resolve; r00, r10, r01, r11: rows (y, z), (y + 1, z), (y, z + 1),
+// (y + 1, z + 1) from voxel x on
+__device__ __forceinline__ uint32_t sn_candidates(const SnGrid& g, bool kiss, int x, int y, int z, uint64_t r00,
+                                                  uint64_t r10, uint64_t r01, uint64_t r11) {
+  if (y < 1 || y > g.ny || z < 1 || z > g.nz) return 0;
+  if (!kiss) {
+    uint32_t m = 0;
+    const uint32_t inner = sn_range(x, g.nx - 1);
+    if (y < g.ny) m |= sn_saddles(r00, r10) & inner;
+    if (z < g.nz) m |= sn_saddles(r00, r01) & inner;
+    if (y < g.ny && z < g.nz) {
+      const uint32_t a = (uint32_t)r00, b = (uint32_t)r10, c = (uint32_t)r01, d = (uint32_t)r11;
+      m |= ~(a ^ d) & ~(b ^ c) & (a ^ b) & sn_range(x, g.nx);
+    }
+    return m;
+  }
+  if (y >= g.ny || z >= g.nz) return 0;
+  const uint32_t c000 = (uint32_t)r00, c100 = (uint32_t)(r00 >> 1), c010 = (uint32_t)r10, c110 = (uint32_t)(r10 >> 1);
+  const uint32_t c001 = (uint32_t)r01, c101 = (uint32_t)(r01 >> 1), c011 = (uint32_t)r11, c111 = (uint32_t)(r11 >> 1);
+  return (sn_kisses(c000, c111, c100, c010, c001, c110, c101, c011) |
+          sn_kisses(c100, c011, c000, c110, c101, c010, c001, c111) |
+          sn_kisses(c010, c101, c000, c110, c011, c100, c001, c111) |
+          sn_kisses(c001, c110, c000, c101, c011, c100, c010, c111)) &
+         sn_range(x, g.nx - 1);
+}
+
+// marks the box of position (x, y, z) and its wave, if that comes after wave w: the flags of the waves up to the
+// running one stay as they are, so every thread of the cluster finds the same waves to run
+__device__ __forceinline__ void sn_mark(const SnBoxes& b, int set, int w, int x, int y, int z) {
+  const int X = (x + y + 2 * z) / kBx, Y = (y + z) / kBy, Z = z / kBz;
+  if (X + Y + Z <= w) return;
+  b.box[set][((int64_t)Z * b.nK + (Y - Z)) * b.nX + X] = 1;
+  b.wave[set][X + Y + Z] = 1;
+}
+
+// A position's voxels: corner k = (k & 1, k >> 1 & 1, k >> 2) of its 2x2x2 cube, bits in the group's rows
+struct SnCorner {
+  uint32_t (*rows)[2];  // the group's mask rows, two words each
+  int row;              // the position's row
+  int bit;              // its bit there
+  __device__ __forceinline__ int at_row(int k) const { return row + ((k >> 1) & 1) + (k >> 2) * (kRowsY + 1); }
+  __device__ __forceinline__ int at_bit(int k) const { return bit + (k & 1) + ((k >> 1) & 1) + (k >> 2) * 2; }
+  __device__ __forceinline__ bool get(int k) const {
+    const int c = at_bit(k);
+    return (((const volatile uint32_t*)rows[at_row(k)])[c >> 5] >> (c & 31)) & 1;
+  }
+  __device__ __forceinline__ void put(int k) const {
+    const int c = at_bit(k);
+    atomicOr(&rows[at_row(k)][c >> 5], 1u << (c & 31));
+  }
+};
+
+// makes corner k of the position (x, y, z) solid, in every copy of the mask, and marks the later boxes with
+// positions that check it (a position interacts with none of another box of its own wave)
+__device__ __forceinline__ void sn_fill(const SnGrid& g, const SnBoxes& b, bool kiss, int w, const SnCorner& c,
+                                        uint8_t* s, float* rho, float thr, int x, int y, int z, int k) {
+  const int vx = x + (k & 1), vy = y + ((k >> 1) & 1), vz = z + (k >> 2);
+  const int64_t v = vx + vy * g.sy + vz * g.sz;
+  c.put(k);
+  atomicOr(b.bits + ((int64_t)vz * (g.ny + 2) + vy) * b.words + (vx >> 5), 1u << (vx & 31));
+  s[v] = 1;
+  if (rho[v] < thr) rho[v] = thr;
+  const int hi = kiss ? 1 : 0;  // cubes start one voxel before the end
+  for (int d = 0; d < 8; ++d) {
+    const int px = vx - (d & 1), py = vy - ((d >> 1) & 1), pz = vz - (d >> 2);
+    if (px >= 1 && px <= g.nx - hi && py >= 1 && py <= g.ny - hi && pz >= 1 && pz <= g.nz - hi)
+      sn_mark(b, kiss, w, px, py, pz);
+  }
+}
+
+// the three face checks at (x, y, z), in the reference's order (XY, XZ, YZ), or the cube's first corner kiss that
+// needs it; returns the resolutions made
+__device__ __forceinline__ int sn_resolve(const SnGrid& g, const SnBoxes& b, bool kiss, int w, const SnCorner& c,
+                                          uint8_t* s, float* rho, float thr, int x, int y, int z) {
+  if (!kiss) {
+    int n = 0;
+    auto face = [&](int k10, int k01) {
+      const bool s00 = c.get(0), s10 = c.get(k10), s01 = c.get(k01), s11 = c.get(k10 | k01);
+      if (!(s00 == s11 && s10 == s01 && s00 != s10)) return;
+      const int ka = s00 ? k10 : 0, kb = s00 ? k01 : k10 | k01;  // the two empty voxels of the diagonal pair
+      auto at = [&](int k) { return rho[(x + (k & 1)) + (y + ((k >> 1) & 1)) * g.sy + (z + (k >> 2)) * g.sz]; };
+      sn_fill(g, b, kiss, w, c, s, rho, thr, x, y, z, at(ka) >= at(kb) ? ka : kb);
+      ++n;
+    };
+    if (x < g.nx && y < g.ny) face(1, 2);
+    if (x < g.nx && z < g.nz) face(1, 4);
+    if (y < g.ny && z < g.nz) face(2, 4);
+    return n;
+  }
+  auto diagonal = [&](int dA, int dB, int a1, int a2, int a3, int b1, int b2, int b3) {
+    if (!(c.get(dA) && c.get(dB))) return false;
+    if ((c.get(a1) && (c.get(b1) || c.get(b2))) || (c.get(a2) && (c.get(b1) || c.get(b3))) ||
+        (c.get(a3) && (c.get(b2) || c.get(b3))))
+      return false;
+    sn_fill(g, b, kiss, w, c, s, rho, thr, x, y, z, a1);
+    sn_fill(g, b, kiss, w, c, s, rho, thr, x, y, z, b1);
+    return true;
+  };
+  return (diagonal(0, 7, 1, 2, 4, 3, 5, 6) || diagonal(1, 6, 0, 3, 5, 2, 4, 7) || diagonal(2, 5, 0, 3, 6, 1, 4, 7) ||
+          diagonal(4, 3, 0, 5, 6, 1, 2, 7))
+             ? 1
+             : 0;
+}
+
+// one box: thread (ty, tz) of the group has the 32 positions of row (y', z') and runs those with something to
+// resolve when their wavefront comes; empty wavefronts are skipped
+__device__ __forceinline__ int sn_box(const SnGrid& g, const SnBoxes& b, bool kiss, uint32_t (*rows)[2], int* red,
+                                      uint8_t* s, float* rho, float thr, int X, int Y, int Z, int tid, int group) {
+  const int X0 = X * kBx, Y0 = Y * kBy, Z0 = Z * kBz;
+  // row (y, z) starts at voxel X0 - y - 2 z, the place of its first position
+  for (int q = tid; q < kRowsY * kRowsZ; q += kSnGroup) {
+    const int z = Z0 + q / kRowsY, y = Y0 + q % kRowsY - z;
+    const uint64_t r = sn_row(g, b, X0 - y - 2 * z, y, z);
+    rows[q][0] = (uint32_t)r;
+    rows[q][1] = (uint32_t)(r >> 32);
+  }
+  sn_group_sync(group);
+  const int ty = tid % kBy, tz = tid / kBy;
+  const int z = Z0 + tz, y = Y0 + ty - z, x0 = X0 - y - 2 * z;
+  const int row = tz * kRowsY + ty;
+  auto word = [&](int q) {
+    const volatile uint32_t* p = rows[q];
+    return (uint64_t)p[0] | ((uint64_t)p[1] << 32);
+  };
+  constexpr int kNone = 1 << 20;
+  int done = -1, n = 0;
+  for (;;) {
+    uint32_t m = sn_candidates(g, kiss, x0, y, z, word(row), word(row + 1) >> 1, word(row + kRowsY + 1) >> 2,
+                               word(row + kRowsY + 2) >> 3);
+    const int first = done + 1 - ty - tz;  // positions before it have had their turn
+    if (first > 31) m = 0;
+    else if (first > 0) m &= 0xffffffffu << first;
+    const int mine = m ? __ffs(m) - 1 + ty + tz : kNone;
+    const int wm = __reduce_min_sync(0xffffffffu, mine);
+    if ((tid & 31) == 0) red[tid >> 5] = wm;
+    sn_group_sync(group);
+    int t = ((volatile int*)red)[0];
+#pragma unroll
+    for (int k = 1; k < kSnGroup / 32; ++k) t = min(t, ((volatile int*)red)[k]);
+    if (t == kNone) break;
+    if (mine == t) {
+      const int i = t - ty - tz;
+      const SnCorner c{rows, row, i};
+      n += sn_resolve(g, b, kiss, X + Y + Z, c, s, rho, thr, x0 + i, y, z);
+    }
+    done = t;
+    sn_group_sync(group);
+  }
+  sn_group_sync(group);  // the rows and red are the next box's
+  return n;
+}
 
 // MakeWellComposed: passes until one changes nothing (at most 8). flags[k] collects "pass k changed"
-// (zeroed by the caller); out[0] = passes run, out[1] = resolutions made.
+// (zeroed by the caller); out[0] = passes run, out[1] = resolutions made. box and wave flags start at zero.
+// What bounds it: latency, that of the ordered steps. Wavefronts t = x + 2y + 4z over the whole grid (768 of them
+// for 192x96x96, in each sweep of each pass, 2.2 us for a barrier of the cluster and byte loads from L2) were run
+// whether or not they had anything to resolve; here a sweep looks at all rows at once (32 positions a thread, as
+// words), then runs only the waves of boxes that need it, a box in shared memory.
+// Measured on B200, 192x96x96: a smooth density field (one graded surface) 10.3 ms -> 0.12 ms; the whole extraction of
+// random fields with 28 thousand / 510 thousand resolutions in 8 passes 47 -> 12 ms / 80 -> 49 ms.
 __global__ void __cluster_dims__(kSnCtas, 1, 1) __launch_bounds__(kSnThreads)
-    k_sn_compose(SnGrid g, uint8_t* s, float* rho, float thr, int* flags, long long* out) {
+    k_sn_compose(SnGrid g, SnBoxes b, uint8_t* s, float* rho, float thr, int* flags, long long* out) {
+  __shared__ uint32_t rows[kSnGroups][kRowsY * kRowsZ][2];
+  __shared__ int red[kSnGroups][kSnGroup / 32];
   __shared__ int cta_changes;
   const int64_t gt = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, gs = (int64_t)gridDim.x * blockDim.x;
-  const int64_t pairs = (int64_t)g.ny * g.nz;
+  const int group = threadIdx.x / kSnGroup, tid = threadIdx.x % kSnGroup;
+  const int ngroups = (int)gridDim.x * kSnGroups, pairs = b.nK * b.nZ;
   long long mine = 0;
   int pass = 0;
   for (; pass < 8; ++pass) {
     if (threadIdx.x == 0) cta_changes = 0;
     __syncthreads();
     int local = 0;
-    // face checks at x in [1, nx], y in [1, ny], z in [1, nz], wavefront t = x + 2y + 4z
-    for (int64_t t = 7; t <= (int64_t)g.nx + 2 * g.ny + 4 * g.nz; ++t) {
-      for (int64_t q = gt; q < pairs; q += gs) {
-        const int64_t y = 1 + q % g.ny, z = 1 + q / g.ny, x = t - 2 * y - 4 * z;
-        if (x >= 1 && x <= g.nx) local += sn_faces(g, s, rho, thr, x, y, z);
+    // face checks at x in [1, nx], y in [1, ny], z in [1, nz], then corner-kiss checks one short of that
+    for (int set = 0; set < 2; ++set) {
+      const bool kiss = set == 1;
+      if (kiss && !(g.nx > 1 && g.ny > 1 && g.nz > 1)) continue;
+      const int64_t items = (int64_t)b.words * g.ny * g.nz;
+      for (int64_t q = gt; q < items; q += gs) {
+        const int x = 1 + 32 * (int)(q % b.words);
+        const int64_t r = q / b.words;
+        const int y = 1 + (int)(r % g.ny), z = 1 + (int)(r / g.ny);
+        const uint32_t m = sn_candidates(g, kiss, x, y, z, sn_row(g, b, x, y, z), sn_row(g, b, x, y + 1, z),
+                                         sn_row(g, b, x, y, z + 1), sn_row(g, b, x, y + 1, z + 1));
+        if (m) {  // the word lies in at most two boxes
+          sn_mark(b, set, -1, x + __ffs(m) - 1, y, z);
+          sn_mark(b, set, -1, x + 31 - __clz(m), y, z);
+        }
       }
       sn_cluster_sync();
-    }
-    // corner-kiss checks at x in [1, nx-1], y in [1, ny-1], z in [1, nz-1]
-    if (g.nx > 1 && g.ny > 1 && g.nz > 1) {
-      const int64_t kp = (int64_t)(g.ny - 1) * (g.nz - 1);
-      for (int64_t t = 7; t <= (int64_t)(g.nx - 1) + 2 * (g.ny - 1) + 4 * (g.nz - 1); ++t) {
-        for (int64_t q = gt; q < kp; q += gs) {
-          const int64_t y = 1 + q % (g.ny - 1), z = 1 + q / (g.ny - 1), x = t - 2 * y - 4 * z;
-          if (x >= 1 && x <= g.nx - 1) local += sn_cube(g, s, rho, thr, x, y, z);
+      for (int w = 0; w < b.waves; ++w) {
+        if (!((volatile uint8_t*)b.wave[set])[w]) continue;  // the same for all threads, see sn_mark
+        for (int p = (int)blockIdx.x * kSnGroups + group; p < pairs; p += ngroups) {
+          const int Z = p / b.nK, Y = Z + p % b.nK, X = w - Y - Z;
+          if (X < 0 || X >= b.nX) continue;
+          if (!((volatile uint8_t*)b.box[set])[(int64_t)p * b.nX + X]) continue;
+          local += sn_box(g, b, kiss, rows[group], red[group], s, rho, thr, X, Y, Z, tid, group);
         }
         sn_cluster_sync();
       }
+      // this sweep's flags are done with; the next sweep that sets them comes after a cluster barrier
+      for (int64_t q = gt; q < b.nbox; q += gs) b.box[set][q] = 0;
+      for (int64_t q = gt; q < b.waves; q += gs) b.wave[set][q] = 0;
     }
     mine += local;
     if (local) atomicAdd(&cta_changes, local);
@@ -577,8 +768,19 @@ int32_t surface_nets_core(mycel_ctx* ctx, int32_t nx, int32_t ny, int32_t nz, fl
       cudaGetLastError();
       return set_error(ctx, MYCEL_E_DEVICE, "iso-surface: the well-composedness cluster kernel cannot be scheduled");
     }
-    k_sn_compose<<<kSnCtas, kSnThreads, 0, s>>>(g, d_s, d_rho, threshold, d_flags, d_scal + 1);
-    ctx->launches++;
+    SnBoxes b = sn_boxes(g);
+    const size_t nbits = sizeof(uint32_t) * b.words * (ny + 2) * (nz + 2), nflag = (size_t)b.nbox + b.waves;
+    b.bits = (uint32_t*)alloc(nbits);
+    uint8_t* marks = (uint8_t*)alloc(2 * nflag);
+    if (oom) return set_error(ctx, MYCEL_E_OOM, "out of device memory for the iso-surface");
+    for (int k = 0; k < 2; ++k) {
+      b.box[k] = marks + k * nflag;
+      b.wave[k] = b.box[k] + b.nbox;
+    }
+    MYCEL_CUDA(ctx, cudaMemsetAsync(marks, 0, 2 * nflag, s));
+    k_sn_bits<<<sn_grid_blocks((int64_t)(nbits / sizeof(uint32_t)) * 32, nsm), 256, 0, s>>>(g, b.words, d_s, b.bits);
+    k_sn_compose<<<kSnCtas, kSnThreads, 0, s>>>(g, b, d_s, d_rho, threshold, d_flags, d_scal + 1);
+    ctx->launches += 2;
     MYCEL_CUDA(ctx, cudaGetLastError());
   }
   k_sn_cells<<<sn_grid_blocks(C, nsm), 256, 0, s>>>(g, d_rho, d_s, threshold, h, origin[0], origin[1], origin[2],
