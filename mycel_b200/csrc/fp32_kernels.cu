@@ -55,23 +55,6 @@ struct MixState {
 constexpr int kT = 256;
 constexpr double kFlushFactor = 1e-1;
 
-// the last of nblk CTAs to arrive (a launch's CTAs, or those of one problem of a packed launch)
-__device__ __forceinline__ bool elect_last_n(unsigned int* counter, unsigned nblk) {
-  __shared__ bool last;
-  __threadfence();
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    unsigned int prev = atomicAdd(counter, 1u);
-    last = (prev == nblk - 1);
-  }
-  __syncthreads();
-  if (last) __threadfence();
-  return last;
-}
-__device__ __forceinline__ bool elect_last32(unsigned int* counter) {
-  return elect_last_n(counter, gridDim.x * gridDim.y);
-}
-
 // deterministic block sum of a double (result valid in linear thread 0); works for 1-D and 2-D blocks
 __device__ __forceinline__ double bsum(double v, double* sh) {
   const int tid = threadIdx.y * blockDim.x + threadIdx.x;
@@ -95,6 +78,89 @@ __device__ __forceinline__ double warp_sum_parts(const double* part, unsigned n)
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
   return s;
+}
+
+// Sums of N per-thread values over nblk CTAs (a launch's, or those of one problem of a packed launch; bid: this
+// one), at most 8 warps each: the orders of bsum and, by the last CTA to arrive, of warp_sum_parts over
+// part[k nblk .. (k + 1) nblk). True in thread 0 of that CTA, which gets the totals in v; the counter is left
+// at zero.
+// Every step of an inner solve ends in one of these, and with a few CTAs a step is all latency: the N values share
+// each step, warp 0 alone carries the partials to memory and back (its lane 0 counts the CTA in with a release of
+// just those stores; everything else a step writes is for later launches), and the partials of the other CTAs are
+// read several at a time. With CTA-wide fences, one sum after the other and one load at a time, the FP64 product's
+// sum at 58 thousand nodes took 1.1 us longer (12.5 us against 11.4 us with the product), the three sums of an outer
+// multigrid step at 123 thousand nodes (96 CTAs) most of the 5 us that step has lost since.
+template <int N>
+__device__ __forceinline__ bool grid_sums(double (&v)[N], double* part, unsigned bid, unsigned nblk,
+                                          unsigned int* counter) {
+  __shared__ double red[N][8];
+  const int tid = threadIdx.y * blockDim.x + threadIdx.x;
+  const int nw = (blockDim.x * blockDim.y) >> 5;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+    for (int k = 0; k < N; ++k) v[k] += __shfl_down_sync(0xffffffffu, v[k], o);
+  __syncthreads();  // red may still be read by warp 0 in a call before this one
+  if ((tid & 31) == 0)
+#pragma unroll
+    for (int k = 0; k < N; ++k) red[k][tid >> 5] = v[k];
+  __syncthreads();
+  if (tid >= 32) return false;
+  if (tid < N) {
+    double w[8], t = 0.0;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) w[k] = k < nw ? red[tid][k] : 0.0;
+#pragma unroll
+    for (int k = 0; k < 8; ++k)
+      if (k < nw) t += w[k];
+    part[(size_t)tid * nblk + bid] = t;
+  }
+  __syncwarp();
+  unsigned int before = 0;
+  if (tid == 0)
+    asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(before) : "l"(counter) : "memory");
+  before = __shfl_sync(0xffffffffu, before, 0);
+  if (before != nblk - 1) return false;
+  constexpr int B = N == 1 ? 16 : N == 2 ? 8 : 6;
+#pragma unroll
+  for (int k = 0; k < N; ++k) v[k] = 0.0;
+  for (unsigned q = tid; q < nblk; q += 32 * B) {
+    double w[N][B];
+#pragma unroll
+    for (int j = 0; j < B; ++j)
+#pragma unroll
+      for (int k = 0; k < N; ++k)
+        w[k][j] = q + 32 * j < nblk ? *(const volatile double*)(part + (size_t)k * nblk + q + 32 * j) : 0.0;
+#pragma unroll
+    for (int j = 0; j < B; ++j)
+      if (q + 32 * j < nblk)
+#pragma unroll
+        for (int k = 0; k < N; ++k) v[k] += w[k][j];
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+    for (int k = 0; k < N; ++k) v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
+  if (tid != 0) return false;
+  *counter = 0;
+  return true;
+}
+
+// p.Ap partials of a matvec launch: CTA sum, fixed-order sum of the CTA partials by the last CTA, alpha.
+// A launch whose bounded waits gave up has set *err; its last CTA then ends the inner solve as a breakdown.
+__device__ __forceinline__ void mv32_finish(double pap, MixState* st, double* part, const int* err, unsigned nblk,
+                                            unsigned bid) {
+  const double rho0 = st->rho0;
+  double v[1] = {pap};
+  if (!grid_sums<1>(v, part, bid, nblk, &st->counter)) return;
+  const double s = v[0];
+  st->first = 0;
+  st->pap = s;
+  if ((err && *(volatile const int*)err) || !(s > 0.0) || !isfinite(s)) {
+    st->status = MIX_BREAKDOWN;
+    return;
+  }
+  st->alpha = rho0 / s;
 }
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -153,11 +219,10 @@ __global__ void __launch_bounds__(TX * TY, 3) k_mv32(GridDims g, const __grid_co
                                                      double* part, int zseg) {
   __shared__ float4 xs[NSLOT][PY][PX];  // node planes, one float4 per node (w unused)
   __shared__ float es[NESLOT][EY][EX];
-  __shared__ double sh[32];
   if (MODE == 1 && st->status != MIX_RUNNING) return;
   const float beta = MODE == 1 ? (float)st->beta : 0.0f;
   const bool first = MODE == 1 ? (st->first != 0) : true;
-  const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * TX + tx;
+  const int tx = threadIdx.x, ty = threadIdx.y;
   const int i0 = blockIdx.x * TX, j0 = blockIdx.y * TY, k0 = blockIdx.z * zseg;
   const int k1 = min(k0 + zseg, g.nz1);
   const int64_t sy = g.nx1, sz = (int64_t)g.nx1 * g.ny1;
@@ -350,30 +415,9 @@ __global__ void __launch_bounds__(TX * TY, 3) k_mv32(GridDims g, const __grid_co
     }
     __syncthreads();
   }
-  if (MODE != 1) return;
-  double b = bsum(pap, sh);
-  const unsigned nblk = gridDim.x * gridDim.y * gridDim.z;
-  const unsigned bid = (blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
-  if (tid == 0) part[bid] = b;
-  // last-CTA election over the 3-D grid
-  __shared__ bool last;
-  __threadfence();
-  __syncthreads();
-  if (tid == 0) last = (atomicAdd(&st->counter, 1u) == nblk - 1);
-  __syncthreads();
-  if (!last) return;
-  __threadfence();
-  if (tid >= 32) return;
-  double s = warp_sum_parts(part, nblk);
-  if (tid != 0) return;
-  st->counter = 0;
-  st->first = 0;
-  st->pap = s;
-  if (!(s > 0.0) || !isfinite(s)) {
-    st->status = MIX_BREAKDOWN;
-    return;
-  }
-  st->alpha = st->rho0 / s;
+  if (MODE == 1)
+    mv32_finish(pap, st, part, nullptr, gridDim.x * gridDim.y * gridDim.z,
+                (blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x);
 }
 
 // z-segment length: enough segments that the grid holds about 8 CTAs per SM (the kernel is latency-bound
@@ -480,32 +524,6 @@ __device__ __forceinline__ void hex_apply2(const HexOpF& op, float2 E, float2 (&
   }
 }
 
-// p.Ap partials of a matvec launch: CTA sum, fixed-order sum of the CTA partials by the last CTA, alpha.
-// A launch whose bounded waits gave up has set *err; its last CTA then ends the inner solve as a breakdown.
-__device__ __forceinline__ void mv32_finish(double pap, double* sh, MixState* st, double* part, int tid,
-                                            const int* err, unsigned nblk, unsigned bid) {
-  const double b = bsum(pap, sh);
-  if (tid == 0) part[bid] = b;
-  __shared__ bool last;
-  __threadfence();
-  __syncthreads();
-  if (tid == 0) last = (atomicAdd(&st->counter, 1u) == nblk - 1);
-  __syncthreads();
-  if (!last) return;
-  __threadfence();
-  if (tid >= 32) return;
-  const double s = warp_sum_parts(part, nblk);
-  if (tid != 0) return;
-  st->counter = 0;
-  st->first = 0;
-  st->pap = s;
-  if ((err && *(const volatile int*)err) || !(s > 0.0) || !isfinite(s)) {
-    st->status = MIX_BREAKDOWN;
-    return;
-  }
-  st->alpha = st->rho0 / s;
-}
-
 // TMA (cp.async.bulk.tensor) node-plane loads: the FP32 vectors are 3-D tensors [nz1][ny1][rp] floats; a copy
 // brings a [FPY][FBW] box whose x start is rounded down to 16 bytes, and zero-fills what lies outside the grid.
 constexpr int FNST = 4;                                     // node-plane stages in flight
@@ -550,7 +568,6 @@ __device__ __forceinline__ int mv32f_body(const GridDims& g, const A& a, int zse
   // [FNST] stages of x (MODE 0) or z (MODE 1), then MODE 1: [FNST] stages of p_{t-1}; then y-exchange
   float* yb = reinterpret_cast<float*>(fac_smem + (size_t)FNST * kFacStagePitch * (MODE == 1 ? 2 : 1));
   __shared__ __align__(8) unsigned long long full[FNST];
-  __shared__ double sh[32];
   if (st && st->status != MIX_RUNNING) return 0;  // MODE 0 gets a state only inside the multigrid cycle
   const float beta = MODE == 1 ? (float)st->beta : 0.0f;
   const bool two = MODE == 1 && st->first == 0;  // p_t = z + beta p_{t-1} (else p_t = z)
@@ -713,7 +730,7 @@ __device__ __forceinline__ int mv32f_body(const GridDims& g, const A& a, int zse
   if (all_ok && tid == 0)
     for (int q = 0; q < FNST; ++q) asm volatile("mbarrier.inval.shared::cta.b64 [%0];\n" ::"r"(smem_u32(&full[q])) : "memory");
   if (!ok && a.err) atomicExch(a.err, 1);
-  if (MODE == 1) mv32_finish(pap, sh, a.st, a.part, tid, a.err, nblk, bid);
+  if (MODE == 1) mv32_finish(pap, a.st, a.part, a.err, nblk, bid);
   return all_ok ? 1 : -1;
 }
 
@@ -843,10 +860,9 @@ __global__ void __launch_bounds__(FX * FY, 2) k_mv64f(GridDims g, const __grid_c
   extern __shared__ __align__(128) unsigned char fac_smem[];
   double* yb = reinterpret_cast<double*>(fac_smem + (size_t)FNST * kFac64StagePitch * (MODE == 1 ? 2 : 1));
   __shared__ __align__(8) unsigned long long full[FNST];
-  __shared__ double sh[32];
-  if (MODE == 1 && st->status != MIX_RUNNING) return;
   const double beta = MODE == 1 ? st->beta : 0.0;
   const bool two = MODE == 1 && st->first == 0;
+  if (MODE == 1 && st->status != MIX_RUNNING) return;
   const int l = threadIdx.x, w = threadIdx.y, tid = w * FX + l;
   const int i0 = blockIdx.x * FOX, j0 = blockIdx.y * FOY, k0 = blockIdx.z * zseg;
   const int k1 = min(k0 + zseg, g.nz1);
@@ -974,7 +990,7 @@ __global__ void __launch_bounds__(FX * FY, 2) k_mv64f(GridDims g, const __grid_c
   }
   if (!ok && err) atomicExch(err, 1);
   if (MODE == 1)
-    mv32_finish(pap, sh, st, part, tid, err, gridDim.x * gridDim.y * gridDim.z,
+    mv32_finish(pap, st, part, err, gridDim.x * gridDim.y * gridDim.z,
                 (blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x);
 }
 
@@ -1082,7 +1098,6 @@ __global__ void __launch_bounds__(TC_THREADS) k_mv32tc(GridDims g, const __grid_
   __shared__ float dsm[CX * CY][25];              // scaled MMA outputs per element
   __shared__ __align__(8) unsigned long long mbar;
   __shared__ uint32_t tmem_base_sh;
-  __shared__ double sh[32];
   __shared__ int fail_sh;
   if (MODE == 1 && st->status != MIX_RUNNING) return;
   const float beta = MODE == 1 ? (float)st->beta : 0.0f;
@@ -1264,33 +1279,9 @@ __global__ void __launch_bounds__(TC_THREADS) k_mv32tc(GridDims g, const __grid_
                  : "memory");
   }
   if (!ok && tid == 0 && err) atomicExch(err, 1);
-  if (MODE != 1) return;
-  double bsum_v = bsum(pap, sh);
-  const unsigned nblk = gridDim.x * gridDim.y * gridDim.z;
-  const unsigned bid = (blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
-  if (tid == 0) part[bid] = bsum_v;
-  __shared__ bool last;
-  __threadfence();
-  __syncthreads();
-  if (tid == 0) last = (atomicAdd(&st->counter, 1u) == nblk - 1);
-  __syncthreads();
-  if (!last) return;
-  __threadfence();
-  if (tid >= 32) return;
-  double s = warp_sum_parts(part, nblk);
-  if (tid != 0) return;
-  st->counter = 0;
-  st->first = 0;
-  st->pap = s;
-  if (fail_sh || (err && *(volatile int*)err)) {
-    st->status = MIX_BREAKDOWN;
-    return;
-  }
-  if (!(s > 0.0) || !isfinite(s)) {
-    st->status = MIX_BREAKDOWN;
-    return;
-  }
-  st->alpha = st->rho0 / s;
+  if (MODE == 1)
+    mv32_finish(fail_sh ? __longlong_as_double(0x7ff8000000000000ll) : pap, st, part, err,
+                gridDim.x * gridDim.y * gridDim.z, (blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x);
 }
 
 static int tc_zseg(const GridDims& g, int num_sms) {
@@ -1502,19 +1493,10 @@ static int32_t resolve_mv32(mycel_problem* p) {
 
 // End of a vector step: CTA sums of r.r and r.z, fixed-order sums by the last CTA, and the inner PCG's scalar
 // logic (recursive residual, replacement and stop triggers, beta).
-__device__ __forceinline__ void xr_tail(double rr, double rz, MixState* st, double* part, int mode, double* sh) {
-  double brr = bsum(rr, sh);
-  double brz = bsum(rz, sh);
-  if (threadIdx.x == 0) {
-    part[blockIdx.x] = brr;
-    part[gridDim.x + blockIdx.x] = brz;
-  }
-  if (!elect_last32(&st->counter)) return;
-  if (threadIdx.x >= 32) return;
-  double srr = warp_sum_parts(part, gridDim.x);
-  double srz = warp_sum_parts(part + gridDim.x, gridDim.x);
-  if (threadIdx.x != 0) return;
-  st->counter = 0;
+__device__ __forceinline__ void xr_tail(double rr, double rz, MixState* st, double* part, int mode) {
+  double v[2] = {rr, rz};
+  if (!grid_sums<2>(v, part, blockIdx.x, gridDim.x, &st->counter)) return;
+  const double srr = v[0], srz = v[1];
   const double rn = sqrt(srr);
   st->rn = rn;
   if (mode == 2) {  // start of a solve
@@ -1552,37 +1534,57 @@ __device__ __forceinline__ void xr_tail(double rr, double rz, MixState* st, doub
   if (st->iter >= st->max_iter) st->status = MIX_MAXITER;
 }
 
-// FP64 vectors of the fast FP64 form (padded layout, n even): the same step as k_xr32
+// FP64 vectors of the fast FP64 form (padded layout, n even): the same step as k_xr32. Latency bounds it up to a
+// few hundred thousand nodes (a thread takes 8 pairs, whatever the size, up to 8 CTAs an SM): the loads of 4 pairs
+// go out together, the first before the state is looked at. 58 thousand nodes: 11.5 us -> 8.1 us.
 __global__ void __launch_bounds__(kT) k_xr64(int64_t n, double* __restrict__ x, double* __restrict__ r,
                                              double* __restrict__ z, const double* __restrict__ p,
                                              const double* __restrict__ ap, const double* __restrict__ invd,
                                              MixState* st, double* part, int mode) {
-  __shared__ double sh[32];
-  if (mode == 0 && st->status != MIX_RUNNING) return;
-  const double alpha = mode ? 0.0 : st->alpha;
+  constexpr int U = 4;
   double rr = 0.0, rz = 0.0;
   const int64_t n2 = n >> 1;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n2; i += stride) {
-    double2 rv = reinterpret_cast<const double2*>(r)[i];
-    const double2 iv = reinterpret_cast<const double2*>(invd)[i];
-    if (mode == 0) {
-      double2 xv = reinterpret_cast<const double2*>(x)[i];
-      const double2 pv = reinterpret_cast<const double2*>(p)[i];
-      const double2 av = reinterpret_cast<const double2*>(ap)[i];
-      xv.x = fma(alpha, pv.x, xv.x);
-      xv.y = fma(alpha, pv.y, xv.y);
-      rv.x = fma(-alpha, av.x, rv.x);
-      rv.y = fma(-alpha, av.y, rv.y);
-      reinterpret_cast<double2*>(x)[i] = xv;
-      reinterpret_cast<double2*>(r)[i] = rv;
+  const int64_t t0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  double2 rv[U], iv[U], xv[U], pv[U], av[U];
+  auto load = [&](int64_t base) {
+#pragma unroll
+    for (int k = 0; k < U; ++k) {
+      const int64_t i = base + k * stride;
+      if (i >= n2) continue;
+      rv[k] = reinterpret_cast<const double2*>(r)[i];
+      iv[k] = reinterpret_cast<const double2*>(invd)[i];
+      if (mode == 0) {
+        xv[k] = reinterpret_cast<const double2*>(x)[i];
+        pv[k] = reinterpret_cast<const double2*>(p)[i];
+        av[k] = reinterpret_cast<const double2*>(ap)[i];
+      }
     }
-    const double2 zv = make_double2(rv.x * iv.x, rv.y * iv.y);
-    reinterpret_cast<double2*>(z)[i] = zv;
-    rr += rv.x * rv.x + rv.y * rv.y;
-    rz += rv.x * zv.x + rv.y * zv.y;
+  };
+  load(t0);
+  if (mode == 0 && st->status != MIX_RUNNING) return;
+  const double alpha = mode ? 0.0 : st->alpha;
+  for (int64_t base = t0; base < n2; base += U * stride) {
+    if (base != t0) load(base);
+#pragma unroll
+    for (int k = 0; k < U; ++k) {
+      const int64_t i = base + k * stride;
+      if (i >= n2) continue;
+      if (mode == 0) {
+        xv[k].x = fma(alpha, pv[k].x, xv[k].x);
+        xv[k].y = fma(alpha, pv[k].y, xv[k].y);
+        rv[k].x = fma(-alpha, av[k].x, rv[k].x);
+        rv[k].y = fma(-alpha, av[k].y, rv[k].y);
+        reinterpret_cast<double2*>(x)[i] = xv[k];
+        reinterpret_cast<double2*>(r)[i] = rv[k];
+      }
+      const double2 zv = make_double2(rv[k].x * iv[k].x, rv[k].y * iv[k].y);
+      reinterpret_cast<double2*>(z)[i] = zv;
+      rr += rv[k].x * rv[k].x + rv[k].y * rv[k].y;
+      rz += rv[k].x * zv.x + rv[k].y * zv.y;
+    }
   }
-  xr_tail(rr, rz, st, part, mode, sh);
+  xr_tail(rr, rz, st, part, mode);
 }
 
 // x += alpha p, r -= alpha Ap, z = r invD; partials of r.r and r.z (FP64). mode 0: CG step; 1: residual
@@ -1591,7 +1593,6 @@ __global__ void __launch_bounds__(kT) k_xr32(int64_t n, float* __restrict__ x, f
                                              float* __restrict__ z, const float* __restrict__ p,
                                              const float* __restrict__ ap, const float* __restrict__ invd,
                                              MixState* st, double* part, int mode) {
-  __shared__ double sh[32];
   if (mode == 0 && st->status != MIX_RUNNING) return;
   const float alpha = mode ? 0.f : (float)st->alpha;
   double rr = 0.0, rz = 0.0;
@@ -1630,7 +1631,7 @@ __global__ void __launch_bounds__(kT) k_xr32(int64_t n, float* __restrict__ x, f
       rz += (double)rv * zv;
     }
   }
-  xr_tail(rr, rz, st, part, mode, sh);
+  xr_tail(rr, rz, st, part, mode);
 }
 
 // Conversions between box-ordered FP64 DOF vectors and the padded FP32 / FP64 layouts walk node rows: row
@@ -2988,69 +2989,101 @@ static void mg_tail_plan(MgTail& tl, int ncase) {
   tl.smem = 0;
 }
 
-// Outer step, part 1. mode 0: x += alpha p, r -= alpha q (FP64, padded layout), ||r|| against the stop and
-// replacement thresholds. All modes: the voxel level's FP32 residual rf = r and its first Jacobi sweep
-// xf = omega invd rf (padded FP32 layout).
-__global__ void __launch_bounds__(kT) k_mg_enter(GridDims g, double* __restrict__ x, double* __restrict__ r,
-                                                 const double* __restrict__ p, const double* __restrict__ q,
-                                                 const float* __restrict__ invdf, float* __restrict__ rf,
-                                                 float* __restrict__ xf, const float* __restrict__ om, MixState* st,
-                                                 double* part, int mode) {
-  __shared__ double sh[32];
-  if (!mg_running(st)) return;
-  const double alpha = st->alpha;
-  const float omega = *om;
-  const int rl = 3 * g.nx1;
-  const int64_t total = (int64_t)g.ny1 * g.nz1 * rl;
-  double rr = 0.0;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t row = i / rl;
-    const int t = (int)(i - row * rl);
-    const int64_t a = (int64_t)g.rp64 * row + t, b = (int64_t)g.rp * row + t;
-    double rv = r[a];
-    if (mode == 0) {
-      x[a] = fma(alpha, p[a], x[a]);
-      rv = fma(-alpha, q[a], rv);
-      r[a] = rv;
-      rr += rv * rv;
-    }
-    const float rfv = (float)rv;
-    rf[b] = rfv;
-    xf[b] = omega * invdf[b] * rfv;
-  }
-  if (mode != 0) return;
-  const double br = bsum(rr, sh);
-  if (threadIdx.x == 0) part[blockIdx.x] = br;
-  if (!elect_last32(&st->counter)) return;
-  if (threadIdx.x >= 32) return;
-  const double s = warp_sum_parts(part, gridDim.x);
-  if (threadIdx.x != 0) return;
-  st->counter = 0;
-  const double rn = sqrt(s);
+// End of an outer step's first part: ||r|| against the stop and replacement thresholds.
+__device__ __forceinline__ void mg_enter_tail(double rr, MixState* st, double* part, unsigned bx, unsigned nb) {
+  double v[1] = {rr};
+  if (!grid_sums<1>(v, part, bx, nb, &st->counter)) return;
+  const double rn = sqrt(v[0]);
   st->rn = rn;
   st->iter += 1;
   if (rn <= st->target || rn <= st->flush_at) st->status = MIX_FLUSH;
   else if (st->iter >= st->max_iter) st->status = MIX_MAXITER;
 }
 
-// End of an outer step (CTA partials of (z, r), (z, A p), (r, r) in b1..b3, valid in thread 0): fixed-order
-// sums by the last CTA. mode 0: beta = -alpha (z, A p) / rho, rho = (z, r). mode 1 (after a true-residual
-// replacement, direction kept): the same beta, new replacement threshold. mode 2 (start): rho, next direction
-// p = z.
-__device__ __forceinline__ void mg_exit_tail(double b1, double b2, double b3, MixState* st, double* part, int mode,
-                                             unsigned bx, unsigned nb) {
-  if (threadIdx.x == 0) {
-    part[bx] = b1;
-    part[nb + bx] = b2;
-    part[2 * nb + bx] = b3;
+// Outer step, part 1. mode 0: x += alpha p, r -= alpha q (FP64, padded layout), ||r|| against the stop and
+// replacement thresholds. All modes: the voxel level's FP32 residual rf = r and its first Jacobi sweep
+// xf = omega invd rf (padded FP32 layout).
+// The thread's DOFs i, i + stride, ... of the box order as places of the padded rows: one division, then steps.
+struct RowWalk {
+  int rl, dt, t;
+  int64_t dr, row, left;
+  __device__ __forceinline__ RowWalk(const GridDims& g, int64_t total) : rl(3 * g.nx1) {
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, stride = (int64_t)gridDim.x * blockDim.x;
+    left = i < total ? (total - i + stride - 1) / stride : 0;
+    row = i / rl;
+    t = (int)(i - row * rl);
+    dr = stride / rl;
+    dt = (int)(stride - dr * rl);
   }
-  if (!elect_last_n(&st->counter, nb)) return;
-  if (threadIdx.x >= 32) return;
-  const double szr = warp_sum_parts(part, nb);
-  const double szq = warp_sum_parts(part + nb, nb);
-  const double srr = warp_sum_parts(part + 2 * nb, nb);
-  if (threadIdx.x != 0) return;
-  st->counter = 0;
+  __device__ __forceinline__ void next() {
+    t += dt;
+    row += dr;
+    if (t >= rl) {
+      t -= rl;
+      ++row;
+    }
+  }
+};
+
+// The FP64 outer steps walk single DOFs (the padded FP32 and FP64 rows have different pitches) and are bound by
+// latency: 16 DOFs a thread up to 8 CTAs an SM. The loads of U = 8 go out together, without a division each; of
+// U = 2 where CTAs fill the chip (outer_wide).
+// 110x22x22: k_mg_enter 14.5 us -> 8.3 us, k_mg_exit 15.0 us -> 7.2 us.
+template <int U>
+__global__ void __launch_bounds__(kT) k_mg_enter(GridDims g, double* __restrict__ x, double* __restrict__ r,
+                                                 const double* __restrict__ p, const double* __restrict__ q,
+                                                 const float* __restrict__ invdf, float* __restrict__ rf,
+                                                 float* __restrict__ xf, const float* __restrict__ om, MixState* st,
+                                                 double* part, int mode) {
+  if (!mg_running(st)) return;
+  const double alpha = st->alpha;
+  const float omega = *om;
+  double rr = 0.0;
+  RowWalk w(g, (int64_t)g.ny1 * g.nz1 * 3 * g.nx1);
+  for (; w.left > 0; w.left -= U) {
+    int64_t a[U], b[U];
+    double rv[U], xv[U], pv[U], qv[U];
+    float iv[U];
+#pragma unroll
+    for (int k = 0; k < U; ++k) {
+      if (k >= w.left) continue;
+      a[k] = (int64_t)g.rp64 * w.row + w.t;
+      b[k] = (int64_t)g.rp * w.row + w.t;
+      rv[k] = r[a[k]];
+      iv[k] = invdf[b[k]];
+      if (mode == 0) {
+        xv[k] = x[a[k]];
+        pv[k] = p[a[k]];
+        qv[k] = q[a[k]];
+      }
+      w.next();
+    }
+#pragma unroll
+    for (int k = 0; k < U; ++k) {
+      if (k >= w.left) continue;
+      if (mode == 0) {
+        x[a[k]] = fma(alpha, pv[k], xv[k]);
+        rv[k] = fma(-alpha, qv[k], rv[k]);
+        r[a[k]] = rv[k];
+        rr += rv[k] * rv[k];
+      }
+      const float rfv = (float)rv[k];
+      rf[b[k]] = rfv;
+      xf[b[k]] = omega * iv[k] * rfv;
+    }
+  }
+  if (mode != 0) return;
+  mg_enter_tail(rr, st, part, blockIdx.x, gridDim.x);
+}
+
+// End of an outer step (per-thread sums of (z, r), (z, A p), (r, r)). mode 0: beta = -alpha (z, A p) / rho,
+// rho = (z, r). mode 1 (after a true-residual replacement, direction kept): the same beta, new replacement
+// threshold. mode 2 (start): rho, next direction p = z.
+__device__ __forceinline__ void mg_exit_tail(double zr, double zq, double rr, MixState* st, double* part, int mode,
+                                             unsigned bx, unsigned nb) {
+  double v[3] = {zr, zq, rr};
+  if (!grid_sums<3>(v, part, bx, nb, &st->counter)) return;
+  const double szr = v[0], szq = v[1], srr = v[2];
   st->pmode = 0;  // the next step follows a matvec
   if (!(szr > 0.0) || !isfinite(szr)) {  // (z, r) > 0 for an SPD preconditioner and r != 0
     st->status = MIX_BREAKDOWN;
@@ -3080,125 +3113,169 @@ __device__ __forceinline__ void mg_exit_tail(double b1, double b2, double b3, Mi
 
 // Outer step, part 2: the voxel level's last Jacobi sweep written as the FP64 preconditioned residual
 // z = xf + omega invd (rf - tf) (tf = A xf), then (z, r), (z, A p) and (r, r) (mg_exit_tail).
+template <int U>
 __global__ void __launch_bounds__(kT) k_mg_exit(GridDims g, const float* __restrict__ rf, const float* __restrict__ tf,
                                                 const float* __restrict__ xf, const float* __restrict__ invdf,
                                                 const double* __restrict__ r, const double* __restrict__ q,
                                                 double* __restrict__ z, const float* __restrict__ om, MixState* st,
                                                 double* part, int mode) {
-  __shared__ double sh[32];
   if (!mg_running(st)) return;
   const float omega = *om;
-  const int rl = 3 * g.nx1;
-  const int64_t total = (int64_t)g.ny1 * g.nz1 * rl;
   double zr = 0.0, zq = 0.0, rr = 0.0;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t row = i / rl;
-    const int t = (int)(i - row * rl);
-    const int64_t a = (int64_t)g.rp64 * row + t, b = (int64_t)g.rp * row + t;
-    const double zv = (double)fmaf(omega * invdf[b], rf[b] - tf[b], xf[b]);
-    const double rv = r[a];
-    z[a] = zv;
-    zr += zv * rv;
-    zq += zv * q[a];
-    rr += rv * rv;
+  RowWalk w(g, (int64_t)g.ny1 * g.nz1 * 3 * g.nx1);
+  for (; w.left > 0; w.left -= U) {
+    int64_t a[U];
+    double rv[U], qv[U];
+    float iv[U], rfv[U], tv[U], xv[U];
+#pragma unroll
+    for (int k = 0; k < U; ++k) {
+      if (k >= w.left) continue;
+      a[k] = (int64_t)g.rp64 * w.row + w.t;
+      const int64_t b = (int64_t)g.rp * w.row + w.t;
+      iv[k] = invdf[b];
+      rfv[k] = rf[b];
+      tv[k] = tf[b];
+      xv[k] = xf[b];
+      rv[k] = r[a[k]];
+      qv[k] = q[a[k]];
+      w.next();
+    }
+#pragma unroll
+    for (int k = 0; k < U; ++k) {
+      if (k >= w.left) continue;
+      const double zv = (double)fmaf(omega * iv[k], rfv[k] - tv[k], xv[k]);
+      z[a[k]] = zv;
+      zr += zv * rv[k];
+      zq += zv * qv[k];
+      rr += rv[k] * rv[k];
+    }
   }
-  const double b1 = bsum(zr, sh);
-  const double b2 = bsum(zq, sh);
-  const double b3 = bsum(rr, sh);
-  mg_exit_tail(b1, b2, b3, st, part, mode, blockIdx.x, gridDim.x);
+  mg_exit_tail(zr, zq, rr, st, part, mode, blockIdx.x, gridDim.x);
 }
 
 // The same two parts for the FP32 outer iteration (mixed multigrid form): all vectors in the padded FP32 layout,
 // the voxel level's residual is the outer residual r itself and its smoothed correction is built in place in z
 // (a mapped matvec input). Dots accumulate in FP64.
 // body for CTA bx of nb (a launch, or one unit's share of a packed launch)
+// U float4 of each vector are loaded together. U = 1 where CTAs fill the chip (8 an SM: memory bounds the step and
+// more registers a thread would halve the CTAs in flight); U = 4 below, where a thread's four or five steps were
+// four or five latencies. The line lies where the CTAs reach 3 per SM, what U = 4 leaves resident. Measured with
+// the sums: 85x53x27 (96 CTAs) enter 8.0 us -> 6.2 us, exit 10.9 us -> 5.8 us; 192x96x96 (1,184 CTAs) 32.3 us ->
+// 30.9 us, 29.4 us -> 25.0 us.
+template <int U>
 __device__ __forceinline__ void mg_enter32_body(int64_t n, float* __restrict__ x, float* __restrict__ r,
                                                 const float* __restrict__ p, const float* __restrict__ q,
                                                 const float* __restrict__ invd, float* __restrict__ xf,
                                                 const float* __restrict__ om, MixState* st, double* part, int mode,
                                                 unsigned bx, unsigned nb) {
-  __shared__ double sh[32];
+  double rr = 0.0;
+  const int64_t n4 = n >> 2;  // n is a multiple of 4 (row pitch)
+  const int64_t t0 = bx * (int64_t)blockDim.x + threadIdx.x, stride = (int64_t)nb * blockDim.x;
+  float4 rv[U], iv[U], xv[U], pv[U], qv[U];
+  auto load = [&](int64_t base) {
+#pragma unroll
+    for (int k = 0; k < U; ++k) {
+      const int64_t i = base + k * stride;
+      if (i >= n4) continue;
+      rv[k] = reinterpret_cast<const float4*>(r)[i];
+      iv[k] = reinterpret_cast<const float4*>(invd)[i];
+      if (mode == 0) {
+        xv[k] = reinterpret_cast<const float4*>(x)[i];
+        pv[k] = reinterpret_cast<const float4*>(p)[i];
+        qv[k] = reinterpret_cast<const float4*>(q)[i];
+      }
+    }
+  };
+  load(t0);  // before the state is looked at
   if (!mg_running(st)) return;
   const float alpha = (float)st->alpha;
   const float omega = *om;
-  double rr = 0.0;
-  const int64_t n4 = n >> 2;  // n is a multiple of 4 (row pitch)
-  for (int64_t i = bx * (int64_t)blockDim.x + threadIdx.x; i < n4; i += (int64_t)nb * blockDim.x) {
-    float4 rv = reinterpret_cast<const float4*>(r)[i];
-    const float4 iv = reinterpret_cast<const float4*>(invd)[i];
-    if (mode == 0) {
-      float4 xv = reinterpret_cast<const float4*>(x)[i];
-      const float4 pv = reinterpret_cast<const float4*>(p)[i];
-      const float4 qv = reinterpret_cast<const float4*>(q)[i];
-      xv.x = fmaf(alpha, pv.x, xv.x); xv.y = fmaf(alpha, pv.y, xv.y);
-      xv.z = fmaf(alpha, pv.z, xv.z); xv.w = fmaf(alpha, pv.w, xv.w);
-      rv.x = fmaf(-alpha, qv.x, rv.x); rv.y = fmaf(-alpha, qv.y, rv.y);
-      rv.z = fmaf(-alpha, qv.z, rv.z); rv.w = fmaf(-alpha, qv.w, rv.w);
-      reinterpret_cast<float4*>(x)[i] = xv;
-      reinterpret_cast<float4*>(r)[i] = rv;
-      rr += (double)rv.x * rv.x + (double)rv.y * rv.y + (double)rv.z * rv.z + (double)rv.w * rv.w;
+  for (int64_t base = t0; base < n4; base += U * stride) {
+    if (base != t0) load(base);
+#pragma unroll
+    for (int k = 0; k < U; ++k) {
+      const int64_t i = base + k * stride;
+      if (i >= n4) continue;
+      float4 rk = rv[k];
+      if (mode == 0) {
+        float4 xk = xv[k];
+        xk.x = fmaf(alpha, pv[k].x, xk.x); xk.y = fmaf(alpha, pv[k].y, xk.y);
+        xk.z = fmaf(alpha, pv[k].z, xk.z); xk.w = fmaf(alpha, pv[k].w, xk.w);
+        rk.x = fmaf(-alpha, qv[k].x, rk.x); rk.y = fmaf(-alpha, qv[k].y, rk.y);
+        rk.z = fmaf(-alpha, qv[k].z, rk.z); rk.w = fmaf(-alpha, qv[k].w, rk.w);
+        reinterpret_cast<float4*>(x)[i] = xk;
+        reinterpret_cast<float4*>(r)[i] = rk;
+        rr += (double)rk.x * rk.x + (double)rk.y * rk.y + (double)rk.z * rk.z + (double)rk.w * rk.w;
+      }
+      reinterpret_cast<float4*>(xf)[i] = make_float4(omega * iv[k].x * rk.x, omega * iv[k].y * rk.y,
+                                                     omega * iv[k].z * rk.z, omega * iv[k].w * rk.w);
     }
-    reinterpret_cast<float4*>(xf)[i] =
-        make_float4(omega * iv.x * rv.x, omega * iv.y * rv.y, omega * iv.z * rv.z, omega * iv.w * rv.w);
   }
   if (mode != 0) return;
-  const double br = bsum(rr, sh);
-  if (threadIdx.x == 0) part[bx] = br;
-  if (!elect_last_n(&st->counter, nb)) return;
-  if (threadIdx.x >= 32) return;
-  const double s = warp_sum_parts(part, nb);
-  if (threadIdx.x != 0) return;
-  st->counter = 0;
-  const double rn = sqrt(s);
-  st->rn = rn;
-  st->iter += 1;
-  if (rn <= st->target || rn <= st->flush_at) st->status = MIX_FLUSH;
-  else if (st->iter >= st->max_iter) st->status = MIX_MAXITER;
+  mg_enter_tail(rr, st, part, bx, nb);
 }
 
+template <int U>
 __global__ void __launch_bounds__(kT) k_mg_enter32(int64_t n, float* __restrict__ x, float* __restrict__ r,
                                                    const float* __restrict__ p, const float* __restrict__ q,
                                                    const float* __restrict__ invd, float* __restrict__ xf,
                                                    const float* __restrict__ om, MixState* st, double* part, int mode) {
-  mg_enter32_body(n, x, r, p, q, invd, xf, om, st, part, mode, blockIdx.x, gridDim.x);
+  mg_enter32_body<U>(n, x, r, p, q, invd, xf, om, st, part, mode, blockIdx.x, gridDim.x);
 }
 
+template <int U>
 __device__ __forceinline__ void mg_exit32_body(int64_t n, const float* __restrict__ r, const float* __restrict__ tf,
                                                float* __restrict__ z, const float* __restrict__ invd,
                                                const float* __restrict__ q, const float* __restrict__ om,
                                                MixState* st, double* part, int mode, unsigned bx, unsigned nb) {
-  __shared__ double sh[32];
-  if (!mg_running(st)) return;
-  const float omega = *om;
   double zr = 0.0, zq = 0.0, rr = 0.0;
   const int64_t n4 = n >> 2;
-  for (int64_t i = bx * (int64_t)blockDim.x + threadIdx.x; i < n4; i += (int64_t)nb * blockDim.x) {
-    const float4 rv = reinterpret_cast<const float4*>(r)[i];
-    const float4 tv = reinterpret_cast<const float4*>(tf)[i];
-    const float4 iv = reinterpret_cast<const float4*>(invd)[i];
-    const float4 qv = reinterpret_cast<const float4*>(q)[i];
-    float4 zv = reinterpret_cast<const float4*>(z)[i];
-    zv.x = fmaf(omega * iv.x, rv.x - tv.x, zv.x);
-    zv.y = fmaf(omega * iv.y, rv.y - tv.y, zv.y);
-    zv.z = fmaf(omega * iv.z, rv.z - tv.z, zv.z);
-    zv.w = fmaf(omega * iv.w, rv.w - tv.w, zv.w);
-    reinterpret_cast<float4*>(z)[i] = zv;
-    zr += (double)zv.x * rv.x + (double)zv.y * rv.y + (double)zv.z * rv.z + (double)zv.w * rv.w;
-    zq += (double)zv.x * qv.x + (double)zv.y * qv.y + (double)zv.z * qv.z + (double)zv.w * qv.w;
-    rr += (double)rv.x * rv.x + (double)rv.y * rv.y + (double)rv.z * rv.z + (double)rv.w * rv.w;
+  const int64_t t0 = bx * (int64_t)blockDim.x + threadIdx.x, stride = (int64_t)nb * blockDim.x;
+  float4 rv[U], tv[U], iv[U], qv[U], z0[U];
+  auto load = [&](int64_t base) {
+#pragma unroll
+    for (int k = 0; k < U; ++k) {
+      const int64_t i = base + k * stride;
+      if (i >= n4) continue;
+      rv[k] = reinterpret_cast<const float4*>(r)[i];
+      tv[k] = reinterpret_cast<const float4*>(tf)[i];
+      iv[k] = reinterpret_cast<const float4*>(invd)[i];
+      qv[k] = reinterpret_cast<const float4*>(q)[i];
+      z0[k] = reinterpret_cast<const float4*>(z)[i];
+    }
+  };
+  load(t0);
+  if (!mg_running(st)) return;
+  const float omega = *om;
+  for (int64_t base = t0; base < n4; base += U * stride) {
+    if (base != t0) load(base);
+#pragma unroll
+    for (int k = 0; k < U; ++k) {
+      const int64_t i = base + k * stride;
+      if (i >= n4) continue;
+      float4 zv = z0[k];
+      zv.x = fmaf(omega * iv[k].x, rv[k].x - tv[k].x, zv.x);
+      zv.y = fmaf(omega * iv[k].y, rv[k].y - tv[k].y, zv.y);
+      zv.z = fmaf(omega * iv[k].z, rv[k].z - tv[k].z, zv.z);
+      zv.w = fmaf(omega * iv[k].w, rv[k].w - tv[k].w, zv.w);
+      reinterpret_cast<float4*>(z)[i] = zv;
+      zr += (double)zv.x * rv[k].x + (double)zv.y * rv[k].y + (double)zv.z * rv[k].z + (double)zv.w * rv[k].w;
+      zq += (double)zv.x * qv[k].x + (double)zv.y * qv[k].y + (double)zv.z * qv[k].z + (double)zv.w * qv[k].w;
+      rr += (double)rv[k].x * rv[k].x + (double)rv[k].y * rv[k].y + (double)rv[k].z * rv[k].z +
+            (double)rv[k].w * rv[k].w;
+    }
   }
-  const double b1 = bsum(zr, sh);
-  const double b2 = bsum(zq, sh);
-  const double b3 = bsum(rr, sh);
-  mg_exit_tail(b1, b2, b3, st, part, mode, bx, nb);
+  mg_exit_tail(zr, zq, rr, st, part, mode, bx, nb);
 }
 
+template <int U>
 __global__ void __launch_bounds__(kT) k_mg_exit32(int64_t n, const float* __restrict__ r, const float* __restrict__ tf,
                                                   float* __restrict__ z, const float* __restrict__ invd,
                                                   const float* __restrict__ q, const float* __restrict__ om,
                                                   MixState* st, double* part, int mode) {
-  mg_exit32_body(n, r, tf, z, invd, q, om, st, part, mode, blockIdx.x, gridDim.x);
+  mg_exit32_body<U>(n, r, tf, z, invd, q, om, st, part, mode, blockIdx.x, gridDim.x);
 }
+static bool outer_wide(const mycel_problem* p, int sb) { return sb <= 3 * p->ctx->num_sms; }
 
 // Power iteration for lambda_max(D^-1 A) of a level: a fixed pseudo-random start on DOFs with a nonzero
 // inverse diagonal, then y = A x, x = D^-1 y / ||D^-1 y||; after the last product lambda ~ ||D^-1 A x||.
@@ -3225,20 +3302,14 @@ struct MgScratch {
 // ||D^-1 y|| by fixed-order sums into sc->norm; with `omega_out` also that level's damping
 __global__ void __launch_bounds__(kT) k_mg_pow_norm(int64_t n, const float* __restrict__ y, const float* __restrict__ invd,
                                                     double* part, MgScratch* sc, float* omega_out) {
-  __shared__ double sh[32];
   double s = 0.0;
   for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < n; q += (int64_t)gridDim.x * blockDim.x) {
     const double v = (double)invd[q] * y[q];
     s += v * v;
   }
-  const double b = bsum(s, sh);
-  if (threadIdx.x == 0) part[blockIdx.x] = b;
-  if (!elect_last32(&sc->counter)) return;
-  if (threadIdx.x >= 32) return;
-  const double t = warp_sum_parts(part, gridDim.x);
-  if (threadIdx.x != 0) return;
-  sc->counter = 0;
-  const float nrm = (float)sqrt(t);
+  double v[1] = {s};
+  if (!grid_sums<1>(v, part, blockIdx.x, gridDim.x, &sc->counter)) return;
+  const float nrm = (float)sqrt(v[0]);
   sc->norm = nrm;
   if (omega_out) *omega_out = (nrm > 0.0f && isfinite(nrm)) ? kMgOmegaScale / nrm : 0.5f;
 }
@@ -3854,22 +3925,23 @@ static int launch_mg_step(mycel_problem* p, cudaStream_t s, const void* pcur, in
   MgRun R;
   R.st = st;
   if (f64) {
-    k_mg_enter<<<sb, kT, 0, s>>>(p->g, p->g_x, p->g_r, (const double*)pcur, p->g_ap, p->d_invdf, p->f_r, p->f_p0, om,
-                                 st, p->d_part2, mode);
+    (outer_wide(p, sb) ? k_mg_enter<8> : k_mg_enter<2>)<<<sb, kT, 0, s>>>(
+        p->g, p->g_x, p->g_r, (const double*)pcur, p->g_ap, p->d_invdf, p->f_r, p->f_p0, om, st, p->d_part2, mode);
     R.rf[0] = p->f_r;
     R.xf[0] = p->f_p0;
     R.tf[0] = p->f_ap;
     nl += 1 + mg_vcycle(p, s, R);
-    k_mg_exit<<<sb, kT, 0, s>>>(p->g, p->f_r, p->f_ap, p->f_p0, p->d_invdf, p->g_r, p->g_ap, p->g_z, om, st,
-                                p->d_part2, mode);
+    (outer_wide(p, sb) ? k_mg_exit<8> : k_mg_exit<2>)<<<sb, kT, 0, s>>>(
+        p->g, p->f_r, p->f_ap, p->f_p0, p->d_invdf, p->g_r, p->g_ap, p->g_z, om, st, p->d_part2, mode);
   } else {
-    k_mg_enter32<<<sb, kT, 0, s>>>(p->g.n32, p->f_x, p->f_r, (const float*)pcur, p->f_ap, p->d_invdf, p->f_z, om, st,
-                                   p->d_part2, mode);
+    (outer_wide(p, sb) ? k_mg_enter32<4> : k_mg_enter32<1>)<<<sb, kT, 0, s>>>(
+        p->g.n32, p->f_x, p->f_r, (const float*)pcur, p->f_ap, p->d_invdf, p->f_z, om, st, p->d_part2, mode);
     R.rf[0] = p->f_r;
     R.xf[0] = p->f_z;
     R.tf[0] = mg->f_t;
     nl += 1 + mg_vcycle(p, s, R);
-    k_mg_exit32<<<sb, kT, 0, s>>>(p->g.n32, p->f_r, mg->f_t, p->f_z, p->d_invdf, p->f_ap, om, st, p->d_part2, mode);
+    (outer_wide(p, sb) ? k_mg_exit32<4> : k_mg_exit32<1>)<<<sb, kT, 0, s>>>(
+        p->g.n32, p->f_r, mg->f_t, p->f_z, p->d_invdf, p->f_ap, om, st, p->d_part2, mode);
   }
   return nl + 1;
 }
@@ -4376,8 +4448,9 @@ static int launch_mg_step_cases(mycel_problem* p, cudaStream_t s, int n, const i
   int nl = 0;
   for (int k = 0; k < n; ++k) {
     float* pcur = cwv(mg, k, 3 + pcur_sel[k]);
-    k_mg_enter32<<<sb, kT, 0, s>>>(p->g.n32, cwv(mg, k, 0), cwv(mg, k, 1), pcur, cwv(mg, k, 5), p->d_invdf,
-                                   cwv(mg, k, 2), om, R.st + k, p->d_part2, mode);
+    (outer_wide(p, sb) ? k_mg_enter32<4> : k_mg_enter32<1>)<<<sb, kT, 0, s>>>(
+        p->g.n32, cwv(mg, k, 0), cwv(mg, k, 1), pcur, cwv(mg, k, 5), p->d_invdf, cwv(mg, k, 2), om, R.st + k,
+        p->d_part2, mode);
     R.rf[k] = cwv(mg, k, 1);
     R.xf[k] = cwv(mg, k, 2);
     R.tf[k] = cwv(mg, k, 6);
@@ -4385,8 +4458,9 @@ static int launch_mg_step_cases(mycel_problem* p, cudaStream_t s, int n, const i
   }
   nl += mg_vcycle(p, s, R);
   for (int k = 0; k < n; ++k) {
-    k_mg_exit32<<<sb, kT, 0, s>>>(p->g.n32, cwv(mg, k, 1), cwv(mg, k, 6), cwv(mg, k, 2), p->d_invdf, cwv(mg, k, 5), om,
-                                  R.st + k, p->d_part2, mode);
+    (outer_wide(p, sb) ? k_mg_exit32<4> : k_mg_exit32<1>)<<<sb, kT, 0, s>>>(
+        p->g.n32, cwv(mg, k, 1), cwv(mg, k, 6), cwv(mg, k, 2), p->d_invdf, cwv(mg, k, 5), om, R.st + k, p->d_part2,
+        mode);
     nl++;
   }
   return nl;
@@ -4867,7 +4941,7 @@ struct PkVec {  // k_mg_enter32 / k_mg_exit32 of a right-hand side
   unsigned nb;
 };
 
-__global__ void __launch_bounds__(kT) k_mg_enter32_pk(const PkVec* __restrict__ tab, const unsigned* __restrict__ items,
+__global__ void __launch_bounds__(kT, 2) k_mg_enter32_pk(const PkVec* __restrict__ tab, const unsigned* __restrict__ items,
                                                       const unsigned* __restrict__ count, int mode) {
   const unsigned cnt = *count;
   for (unsigned w = blockIdx.x; w < cnt; w += gridDim.x) {
@@ -4875,11 +4949,11 @@ __global__ void __launch_bounds__(kT) k_mg_enter32_pk(const PkVec* __restrict__ 
     const unsigned code = items[w];
     const PkVec& a = tab[code >> kPkLbBits];
     const int md = mode >= 0 ? mode : *(const volatile int*)&a.st->pmode;
-    mg_enter32_body(a.n, a.x, a.r, a.p, a.q, a.invd, a.z, a.om, a.st, a.part, md, code & kPkLbMask, a.nb);
+    mg_enter32_body<4>(a.n, a.x, a.r, a.p, a.q, a.invd, a.z, a.om, a.st, a.part, md, code & kPkLbMask, a.nb);
   }
 }
 
-__global__ void __launch_bounds__(kT) k_mg_exit32_pk(const PkVec* __restrict__ tab, const unsigned* __restrict__ items,
+__global__ void __launch_bounds__(kT, 2) k_mg_exit32_pk(const PkVec* __restrict__ tab, const unsigned* __restrict__ items,
                                                      const unsigned* __restrict__ count, int mode) {
   const unsigned cnt = *count;
   for (unsigned w = blockIdx.x; w < cnt; w += gridDim.x) {
@@ -4887,7 +4961,7 @@ __global__ void __launch_bounds__(kT) k_mg_exit32_pk(const PkVec* __restrict__ t
     const unsigned code = items[w];
     const PkVec& a = tab[code >> kPkLbBits];
     const int md = mode >= 0 ? mode : *(const volatile int*)&a.st->pmode;
-    mg_exit32_body(a.n, a.r, a.t, a.z, a.invd, a.q, a.om, a.st, a.part, md, code & kPkLbMask, a.nb);
+    mg_exit32_body<4>(a.n, a.r, a.t, a.z, a.invd, a.q, a.om, a.st, a.part, md, code & kPkLbMask, a.nb);
   }
 }
 
