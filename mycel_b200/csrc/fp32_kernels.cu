@@ -2088,7 +2088,86 @@ __global__ void __launch_bounds__(256) k_mg_apply_nodes(MgDims d, const float* _
   mg_apply_node(d, mg_ns(d), n, S, x.p[c], r.p[c], invd, y.p[c], mode, mode == 1 ? *om : 0.0f);
 }
 
+// One row per thread for the 64 (node, case) items from t0 on, by a CTA of kMgDofThreads: the fmaf chain of
+// mg_apply_row. Latency bounds these levels (a few CTAs an SM at most): with its loads in the chain's order a thread
+// held a few of its 162 in flight. Here all 81 of its stencil entries are loaded at once, coalesced, into registers,
+// and x, which the 64 items share, comes through shared memory as 9 runs of consecutive nodes per case (cp.async,
+// zero outside the array). Every load of the row is then one latency, and half of them are left.
+// B200, us: 2,816 nodes (44 CTAs) 6.4 -> 4.0, 18,490 (289) 6.9 -> 5.2. The registers leave 3 CTAs an SM: a second,
+// nearly empty wave costs more than it gives (30,625 nodes, 479 CTAs: 8.4 against 7.7; 11,781 nodes x 4 cases, 737
+// CTAs: 12.5 against 9.8), so levels of more CTAs than that keep mg_apply_row (MgLevel::max_shared).
+constexpr int kRowStage = 2464;  // floats: 27 ncase (63 / ncase + 4), at most 8 cases
 template <bool MULTI>
+__device__ __forceinline__ void mg_apply_rows(const MgDims& d, int64_t t0, int ncase, const float* __restrict__ S,
+                                              const MgPtrs& x, const MgPtrs& r, const float* __restrict__ invd,
+                                              const MgPtrs& y, int mode, const float* __restrict__ om,
+                                              const MixState* st, float* xs) {
+  const int64_t nn = mg_nn(d), ns = mg_ns(d);
+  const int nx1 = d.nx + 1, sxy = nx1 * (d.ny + 1);
+  int64_t n, lo;
+  int c, c0;
+  mg_item_case<MULTI>(t0 + (threadIdx.x & 63), ncase, &n, &c);
+  mg_item_case<MULTI>(t0, ncase, &lo, &c0);
+  const int ci = threadIdx.x >> 6;
+  const bool valid = n < nn;
+  const int R3 = MULTI ? 3 * (63 / ncase + 4) : 198;  // floats of a run: the items' nodes and one on either side
+  const int64_t n3 = 3 * nn;
+  auto stage = [&](const float* src, int run, int row, int o) {
+    const int64_t q = 3 * (lo - 1 + nx1 * (run % 3 - 1) + sxy * (run / 3 - 1)) + o;
+    const bool in = q >= 0 && q < n3;
+    __pipeline_memcpy_async(xs + row * R3 + o, src + (in ? q : 0), 4, in ? 0 : 4);
+  };
+  if (MULTI) {
+    for (int row = threadIdx.x >> 5; row < 9 * ncase; row += kMgDofThreads / 32)
+      for (int o = threadIdx.x & 31; o < R3; o += 32) stage(x.p[row / 9], row % 9, row, o);
+  } else {
+#pragma unroll
+    for (int k = 0; k < (9 * 198 + kMgDofThreads - 1) / kMgDofThreads; ++k) {
+      const int e = threadIdx.x + k * kMgDofThreads;
+      if (e < 9 * 198) stage(x.p[0], e / 198, e / 198, e % 198);
+    }
+  }
+  __pipeline_commit();
+  float sv[27][3];
+  float rq = 0.f, iq = 0.f;
+  const MgNode g(d, (int)n);
+  const int64_t q = 3 * n + ci;
+  if (valid) {
+    const float* own = S + 3 * ci * ns + n;
+    const float* tr = S + ci * ns;
+#pragma unroll
+    for (int nb = 0; nb < 27; ++nb) {
+      const float* s = nb >= 13 ? own + (int64_t)(nb - 13) * 9 * ns : tr + (int64_t)(13 - nb) * 9 * ns + max(g.at(nb), 0);
+#pragma unroll
+      for (int k = 0; k < 3; ++k) sv[nb][k] = s[(nb >= 13 ? k : 3 * k) * ns];
+    }
+    if (mode != 0) {
+      rq = r.p[c][q];
+      iq = invd[q];
+    }
+  }
+  const float omega = mode == 1 ? *om : 0.0f;
+  const bool run = valid && mg_running(st ? st + c : nullptr);
+  __pipeline_wait_prior(0);
+  __syncthreads();
+  if (!run) return;
+  float a = 0.f;
+  const float* xc = xs + c * 9 * R3 + 3 * (int)(n - lo);
+#pragma unroll
+  for (int nb = 0; nb < 27; ++nb) {
+    const float* xp = xc + (nb / 3) * R3 + 3 * (nb % 3);
+    const bool in = g.in(nb);
+    const float x0 = in ? xp[0] : 0.f, x1 = in ? xp[1] : 0.f, x2 = in ? xp[2] : 0.f;
+    a = fmaf(sv[nb][0], x0, fmaf(sv[nb][1], x1, fmaf(sv[nb][2], x2, a)));
+  }
+  float* yo = y.p[c] + q;
+  if (mode == 0) *yo = a;
+  else if (mode == 1) *yo = fmaf(omega * iq, rq - a, xc[4 * R3 + 3 + ci]);
+  else *yo = iq != 0.0f ? rq - a : 0.0f;
+}
+
+// SHARED: the CTA's items together (mg_apply_rows), else each row for itself
+template <bool MULTI, bool SHARED>
 __global__ void __launch_bounds__(kMgDofThreads) k_mg_apply(MgDims d, const float* __restrict__ S,
                                                             const __grid_constant__ MgPtrs x,
                                                             const __grid_constant__ MgPtrs r,
@@ -2096,12 +2175,17 @@ __global__ void __launch_bounds__(kMgDofThreads) k_mg_apply(MgDims d, const floa
                                                             const __grid_constant__ MgPtrs y, int mode,
                                                             const float* __restrict__ om, const MixState* st,
                                                             int ncase) {
-  const int64_t nn = mg_nn(d);
-  int64_t n;  // (node, case) pair, the case fastest
-  int c;
-  mg_item_case<MULTI>(mg_dof_node(), ncase, &n, &c);
-  if (n >= nn || !mg_running(st ? st + c : nullptr)) return;
-  mg_apply_row(d, mg_ns(d), n, mg_dof_comp(), S, x.p[c], r.p[c], invd, y.p[c], mode, mode == 1 ? *om : 0.0f);
+  if constexpr (SHARED) {
+    __shared__ float xs[kRowStage];
+    mg_apply_rows<MULTI>(d, (int64_t)blockIdx.x * 64, ncase, S, x, r, invd, y, mode, om, st, xs);
+  } else {
+    const int64_t nn = mg_nn(d);
+    int64_t n;  // (node, case) pair, the case fastest
+    int c;
+    mg_item_case<MULTI>(mg_dof_node(), ncase, &n, &c);
+    if (n >= nn || !mg_running(st ? st + c : nullptr)) return;
+    mg_apply_row(d, mg_ns(d), n, mg_dof_comp(), S, x.p[c], r.p[c], invd, y.p[c], mode, mode == 1 ? *om : 0.0f);
+  }
 }
 
 // Coarse-level product of a large level (one case) with the stencil streamed into shared memory by TMA: the
@@ -3437,6 +3521,7 @@ struct MgLevel {
   int64_t nn = 0, nd = 0;
   float *S = nullptr, *invd = nullptr, *xa = nullptr, *xb = nullptr, *r = nullptr, *t = nullptr;
   bool staged = false;  // products of one case by k_mg_apply_nodes_tma through tm_s
+  int64_t max_shared = 0;  // products of up to this many nodes x cases by CTAs that share x (mg_apply_rows)
   int* err = nullptr;   // the problem's bounded-wait error word
   CUtensorMap tm_s{};   // the stencil as a 2-D tensor [126 rows][ns nodes], boxes of [9][kS1Box]
 };
@@ -3601,6 +3686,7 @@ static int32_t mg_ensure(mycel_problem* p, bool* available) {
     v.S = (float*)alloc(sizeof(float) * 9 * kMgHalf * mg_ns(v.d));  // zeroed: the row padding stays 0
     v.invd = (float*)alloc(sizeof(float) * v.nd);
     v.err = p->d_err;
+    v.max_shared = (int64_t)3 * p->ctx->num_sms * 64;
     if (v.S && v.nn > kMgDofMaxNodes) {  // the levels whose products run a thread per node
       const PFN_cuTensorMapEncodeTiled encode = tensor_map_encoder();
       cuuint64_t dims[2] = {(cuuint64_t)mg_ns(v.d), (cuuint64_t)(9 * kMgHalf)};
@@ -3738,8 +3824,9 @@ static MgPtrs lv_ptrs(float* base, int64_t nd, int n) {
 static void launch_mg_apply(cudaStream_t s, const MgLevel& v, const MgPtrs& x, const MgPtrs& r, const float* invd,
                             const MgPtrs& y, int mode, const float* om, const MixState* st, int nc) {
   if (v.nn * nc <= kMgDofMaxNodes)
-    (nc == 1 ? k_mg_apply<false> : k_mg_apply<true>)<<<mg_dof_blocks(v.nn * nc), kMgDofThreads, 0, s>>>(
-        v.d, v.S, x, r, invd, y, mode, om, st, nc);
+    (v.nn * nc <= v.max_shared ? (nc == 1 ? k_mg_apply<false, true> : k_mg_apply<true, true>)
+                               : (nc == 1 ? k_mg_apply<false, false> : k_mg_apply<true, false>))
+        <<<mg_dof_blocks(v.nn * nc), kMgDofThreads, 0, s>>>(v.d, v.S, x, r, invd, y, mode, om, st, nc);
   else if (nc == 1 && v.staged)
     k_mg_apply_nodes_tma<<<(unsigned)((v.nn + kS1Nodes - 1) / kS1Nodes), 256, kS1Smem, s>>>(
         v.d, v.tm_s, x.p[0], r.p[0], invd, y.p[0], mode, om, st, v.err);
@@ -4996,17 +5083,14 @@ template <bool MULTI>
 __global__ void __launch_bounds__(kMgDofThreads) k_mg_apply_pk(const PkApply* __restrict__ tab,
                                                                const unsigned* __restrict__ items,
                                                                const unsigned* __restrict__ count, int mode) {
+  __shared__ float xs[kRowStage];
   const unsigned cnt = *count;
   for (unsigned w = blockIdx.x; w < cnt; w += gridDim.x) {
     const unsigned code = items[w];
     const PkApply& a = tab[code >> kPkLbBits];
-    const int64_t nn = mg_nn(a.d);
-    int64_t q;
-    int c;
-    mg_item_case<MULTI>((int64_t)(code & kPkLbMask) * 64 + (threadIdx.x & 63), a.ncase, &q, &c);
-    if (q >= nn || !mg_running(a.st ? a.st + c : nullptr)) continue;
-    mg_apply_row(a.d, mg_ns(a.d), q, (int)(threadIdx.x >> 6), a.S, a.x.p[c], a.r.p[c], a.invd, a.y.p[c], mode,
-                 mode == 1 ? *a.om : 0.0f);
+    mg_apply_rows<MULTI>(a.d, (int64_t)(code & kPkLbMask) * 64, a.ncase, a.S, a.x, a.r, a.invd, a.y, mode, a.om, a.st,
+                         xs);
+    __syncthreads();  // xs is the next item's
   }
 }
 
