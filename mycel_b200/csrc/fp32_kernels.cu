@@ -1739,6 +1739,32 @@ constexpr int kMgMaxCases = 8;
 struct MgPtrs {
   float* p[kMgMaxCases];
 };
+
+// The factorised product of several load cases in one launch: case blockIdx.z / tiles_z, each with the tiles and the
+// partial sums of k_mv32f. On a small grid one case leaves SMs idle and a launch is mostly latency (64x32x40: 135 CTAs
+// for 296 places).
+// Four cases there: 4 x 6.2 -> 14.8 us, with the sums 4 x 9.7 -> 21.2 us; their outer steps, also together, 4 x 5.8 ->
+// 7.8 us and 4 x 5.3 -> 6.6 us.
+template <int MODE>
+struct CasesMv {
+  CUtensorMap tm_a[kMgMaxCases], tm_b[MODE == 1 ? kMgMaxCases : 1];
+  float *pnew[kMgMaxCases], *y[kMgMaxCases];
+  MixState* st;  // one per case, or null
+  double* part;  // pitch doubles per case
+  int pitch, tiles_z;
+};
+template <int MODE>
+__global__ void __launch_bounds__(FX * FY, 2) k_mv32f_cases(GridDims g, const __grid_constant__ HexOpF op,
+                                                            const __grid_constant__ CasesMv<MODE> v,
+                                                            const float* __restrict__ E,
+                                                            const uint8_t* __restrict__ nf, int zseg, int* err) {
+  const int c = blockIdx.z / v.tiles_z, bz = blockIdx.z % v.tiles_z;
+  const MvArgs a{&op, &v.tm_a[c], &v.tm_b[MODE == 1 ? c : 0], v.pnew[c], v.y[c], E, nf,
+                 v.st ? v.st + c : nullptr, v.part + (size_t)c * v.pitch, err, 1};
+  mv32f_body<MODE>(g, a, zseg, blockIdx.x, blockIdx.y, bz, gridDim.x * gridDim.y * v.tiles_z,
+                   (bz * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x);
+}
+
 // (item, case) from a thread number with the case fastest; one case: the number itself (no division). The
 // kernels are instantiated for one case (MULTI false: the single solve's code, compile-time case 0) and for
 // several.
@@ -3423,6 +3449,10 @@ static int32_t ensure_mixed(mycel_problem* p) {
   std::call_once(smem_once, [] {
     cudaError_t a = cudaFuncSetAttribute(k_mv32f<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fac_smem_bytes(0));
     cudaError_t b = cudaFuncSetAttribute(k_mv32f<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fac_smem_bytes(1));
+    if (a == cudaSuccess)
+      a = cudaFuncSetAttribute(k_mv32f_cases<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fac_smem_bytes(0));
+    if (b == cudaSuccess)
+      b = cudaFuncSetAttribute(k_mv32f_cases<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fac_smem_bytes(1));
     smem_err = a != cudaSuccess ? a : b;
   });
   if (smem_err != cudaSuccess)
@@ -3835,10 +3865,52 @@ static void launch_mg_apply(cudaStream_t s, const MgLevel& v, const MgPtrs& x, c
         v.d, v.S, x, r, invd, y, mode, om, st, nc);
 }
 
+// Per case the input (MODE 0: x; 1: z, with the old direction), pnew and y of launch_mv32_variant, which runs them one
+// by one where the product is not the factorised one or the cases' partial sums do not fit side by side (pitch 0).
+// Returns the kernels launched.
+template <int MODE>
+static int launch_mv32_cases(mycel_problem* p, cudaStream_t s, int n, float* const* in, float* const* pold,
+                             float* const* pnew, float* const* y, MixState* st, int pitch) {
+  if (n > 1 && pitch > 0 && p->mv32 != MYCEL_MV32_TENSOR && p->mv32 != MYCEL_MV32_DENSE) {
+    const int zs = fac_zseg(p->g, mv32f_resident_per_sm() * p->ctx->num_sms);
+    dim3 grid = fac_grid(p->g, zs);
+    CasesMv<MODE> v{};
+    bool mapped = true;
+    for (int k = 0; k < n && mapped; ++k) {
+      const CUtensorMap* ta = tmap_of(p, in[k]);
+      const CUtensorMap* tb = MODE == 1 ? tmap_of(p, pold[k]) : ta;
+      mapped = ta && tb;
+      if (!mapped) break;
+      v.tm_a[k] = *ta;
+      if (MODE == 1) {
+        v.tm_b[k] = *tb;
+        v.pnew[k] = pnew[k];
+      }
+      v.y[k] = y[k];
+    }
+    if (mapped) {
+      v.st = st;
+      v.part = p->d_part2;
+      v.pitch = pitch;
+      v.tiles_z = (int)grid.z;
+      grid.z *= (unsigned)n;
+      k_mv32f_cases<MODE><<<grid, dim3(FX, FY), fac_smem_bytes(MODE), s>>>(p->g, p->hexop, v, p->d_Ef, p->d_nflags, zs,
+                                                                           p->d_err);
+      return 1;
+    }
+  }
+  for (int k = 0; k < n; ++k)
+    launch_mv32_variant<MODE>(p, s, MODE == 0 ? in[k] : nullptr, MODE == 1 ? in[k] : nullptr,
+                              MODE == 1 ? pold[k] : nullptr, MODE == 1 ? pnew[k] : nullptr, y[k], 1,
+                              st ? st + k : nullptr, p->d_part2);
+  return n;
+}
+
 // The load cases one V-cycle advances: their states (one per case, contiguous) and their voxel-level vectors
 // (padded FP32 layout): residual rf, first sweep / correction xf (a mapped matvec input) and tf = A xf.
 struct MgRun {
   int n = 1;
+  int pitch = 0;  // of the cases' partial sums in d_part2, see cases_pitch
   MixState* st = nullptr;
   float* rf[kMgMaxCases] = {};
   float* xf[kMgMaxCases] = {};
@@ -3937,8 +4009,7 @@ static int mg_vcycle(mycel_problem* p, cudaStream_t s, const MgRun& R) {
       k_mg_jacobi_fine<<<sb, kT, 0, s>>>(g.n32, R.rf[k], R.tf[k], p->d_invdf, R.xf[k], om, cst(k));
       nl += 2;
     }
-  for (int k = 0; k < nc; ++k) fine_mv(k);
-  nl += nc;
+  nl += launch_mv32_cases<0>(p, s, nc, R.xf, nullptr, nullptr, R.tf, st, R.pitch);
   // restriction to level 1, with level 1's first sweep (unless level 1 is the coarsest)
   (nc == 1 ? k_mg_restrict<true, false> : k_mg_restrict<true, true>)<<<mg_blocks(lv[1].nn * nc), 256, 0, s>>>(lv[0].d, g.rp, mg_ptrs(R.rf, nc), mg_ptrs(R.tf, nc),
                                                                lv[1].d, lv[1].invd, lv_ptrs(lv[1].r, lv[1].nd, nc), st,
@@ -3992,8 +4063,7 @@ static int mg_vcycle(mycel_problem* p, cudaStream_t s, const MgRun& R) {
       k_mg_jacobi_fine<<<sb, kT, 0, s>>>(g.n32, R.rf[k], R.tf[k], p->d_invdf, R.xf[k], om, cst(k));
       nl += 2;
     }
-  for (int k = 0; k < nc; ++k) fine_mv(k);
-  return nl + nc;
+  return nl + launch_mv32_cases<0>(p, s, nc, R.xf, nullptr, nullptr, R.tf, st, R.pitch);
 }
 
 // The outer step after the matvec (mode 0), or the preconditioned residual after a start (2) or a true-residual
@@ -4523,33 +4593,76 @@ static int32_t mg_ensure_cases(mycel_problem* p, int n) {
 // vector q of case k: 0 x, 1 r, 2 z, 3 p0, 4 p1, 5 ap, 6 t
 static float* cwv(MgHier* mg, int k, int q) { return mg->cw.v[k][q]; }
 
-// One outer step of every case (mode 0: after the matvec; 1: after a replacement; 2: start): k_mg_enter32 per
-// case, one V-cycle for all, k_mg_exit32 per case. Returns the kernels launched.
+// Doubles of d_part2 per case for the sums of n cases side by side (its last 128 hold other scalars), 0 if they do
+// not fit
+static int cases_pitch(mycel_problem* p, int n) {
+  const dim3 t = fac_grid(p->g, fac_zseg(p->g, mv32f_resident_per_sm() * p->ctx->num_sms));
+  const int64_t pitch = std::max<int64_t>((int64_t)t.x * t.y * t.z, 3 * (int64_t)stream_blocks(p));
+  return pitch * n + 128 <= p->n_part2 ? (int)pitch : 0;
+}
+
+// One outer step of every case (mode 0: after the matvec; 1: after a replacement; 2: start): the first parts, one
+// V-cycle, the second parts, each for all cases in one launch. Returns the kernels launched.
+struct CasesVec {
+  float *x[kMgMaxCases], *r[kMgMaxCases], *z[kMgMaxCases], *p[kMgMaxCases], *q[kMgMaxCases], *t[kMgMaxCases];
+};
+template <int U>
+__global__ void __launch_bounds__(kT) k_mg_enter32_cases(int64_t n, const __grid_constant__ CasesVec v,
+                                                         const float* __restrict__ invd, const float* __restrict__ om,
+                                                         MixState* st, double* part, int pitch, int mode) {
+  const int c = blockIdx.y;
+  mg_enter32_body<U>(n, v.x[c], v.r[c], v.p[c], v.q[c], invd, v.z[c], om, st + c, part + (size_t)c * pitch, mode,
+                     blockIdx.x, gridDim.x);
+}
+template <int U>
+__global__ void __launch_bounds__(kT) k_mg_exit32_cases(int64_t n, const __grid_constant__ CasesVec v,
+                                                        const float* __restrict__ invd, const float* __restrict__ om,
+                                                        MixState* st, double* part, int pitch, int mode) {
+  const int c = blockIdx.y;
+  mg_exit32_body<U>(n, v.r[c], v.t[c], v.z[c], invd, v.q[c], om, st + c, part + (size_t)c * pitch, mode, blockIdx.x,
+                    gridDim.x);
+}
+
 static int launch_mg_step_cases(mycel_problem* p, cudaStream_t s, int n, const int* pcur_sel, int mode) {
   MgHier* mg = p->mg;
-  const int sb = stream_blocks(p);
+  const int sb = stream_blocks(p), pitch = cases_pitch(p, n);
   const float* om = mg->sc->omega;
   MgRun R;
   R.n = n;
+  R.pitch = pitch;
   R.st = mg->cw.st;
+  CasesVec v{};
+  for (int k = 0; k < n; ++k) {
+    v.x[k] = cwv(mg, k, 0);
+    v.r[k] = R.rf[k] = cwv(mg, k, 1);
+    v.z[k] = R.xf[k] = cwv(mg, k, 2);
+    v.p[k] = cwv(mg, k, 3 + pcur_sel[k]);
+    v.q[k] = cwv(mg, k, 5);
+    v.t[k] = R.tf[k] = cwv(mg, k, 6);
+  }
   int nl = 0;
-  for (int k = 0; k < n; ++k) {
-    float* pcur = cwv(mg, k, 3 + pcur_sel[k]);
-    (outer_wide(p, sb) ? k_mg_enter32<4> : k_mg_enter32<1>)<<<sb, kT, 0, s>>>(
-        p->g.n32, cwv(mg, k, 0), cwv(mg, k, 1), pcur, cwv(mg, k, 5), p->d_invdf, cwv(mg, k, 2), om, R.st + k,
-        p->d_part2, mode);
-    R.rf[k] = cwv(mg, k, 1);
-    R.xf[k] = cwv(mg, k, 2);
-    R.tf[k] = cwv(mg, k, 6);
-    nl++;
-  }
+  // the cases of [k, k + m): all at once, or one by one where their sums do not fit side by side
+  const int m = pitch ? n : 1;
+  const bool wide = outer_wide(p, sb * m);
+  auto from = [&](int k) {
+    CasesVec w{};
+    for (int j = 0; j < m; ++j) {
+      w.x[j] = v.x[k + j];
+      w.r[j] = v.r[k + j];
+      w.z[j] = v.z[k + j];
+      w.p[j] = v.p[k + j];
+      w.q[j] = v.q[k + j];
+      w.t[j] = v.t[k + j];
+    }
+    return w;
+  };
+  for (int k = 0; k < n; k += m, ++nl)
+    (wide ? k_mg_enter32_cases<4> : k_mg_enter32_cases<1>)<<<dim3(sb, m), kT, 0, s>>>(
+        p->g.n32, from(k), p->d_invdf, om, R.st + k, p->d_part2, pitch, mode);
   nl += mg_vcycle(p, s, R);
-  for (int k = 0; k < n; ++k) {
-    (outer_wide(p, sb) ? k_mg_exit32<4> : k_mg_exit32<1>)<<<sb, kT, 0, s>>>(
-        p->g.n32, cwv(mg, k, 1), cwv(mg, k, 6), cwv(mg, k, 2), p->d_invdf, cwv(mg, k, 5), om, R.st + k, p->d_part2,
-        mode);
-    nl++;
-  }
+  for (int k = 0; k < n; k += m, ++nl)
+    (wide ? k_mg_exit32_cases<4> : k_mg_exit32_cases<1>)<<<dim3(sb, m), kT, 0, s>>>(
+        p->g.n32, from(k), p->d_invdf, om, R.st + k, p->d_part2, pitch, mode);
   return nl;
 }
 
@@ -4571,13 +4684,15 @@ static int32_t capture_cases_graph(mycel_problem* p, int n) {
     int nl = 0;
     for (int t = 0; t < 2; ++t) {
       int sel[kMgMaxCases];
+      float *z[kMgMaxCases], *pcur[kMgMaxCases], *pprev[kMgMaxCases], *ap[kMgMaxCases];
       for (int k = 0; k < n; ++k) {
-        float* pcur = cwv(mg, k, (t & 1) ? 4 : 3);
-        float* pprev = cwv(mg, k, (t & 1) ? 3 : 4);
-        launch_mv32_variant<1>(p, s, nullptr, cwv(mg, k, 2), pprev, pcur, cwv(mg, k, 5), 1, cw.st + k, p->d_part2);
+        z[k] = cwv(mg, k, 2);
+        pcur[k] = cwv(mg, k, (t & 1) ? 4 : 3);
+        pprev[k] = cwv(mg, k, (t & 1) ? 3 : 4);
+        ap[k] = cwv(mg, k, 5);
         sel[k] = t & 1;
-        nl++;
       }
+      nl += launch_mv32_cases<1>(p, s, n, z, pprev, pcur, ap, cw.st, cases_pitch(p, n));
       nl += launch_mg_step_cases(p, s, n, sel, 0);
     }
     cw.per_chunk = nl;
