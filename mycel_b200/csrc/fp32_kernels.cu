@@ -458,16 +458,31 @@ __device__ __forceinline__ float2 f2mul(float2 a, float2 b) { return __fmul2_rn(
 __device__ __forceinline__ float2 f2fma(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
 
 // 8-point Walsh-Hadamard butterflies over the index bits (x, y, z): afterwards v[p] = sum_a s_p(a) v_a,
-// s_p(a) the product over the axes odd in p of (2 a_axis - 1).
-__device__ __forceinline__ void wht8x2(float2 (&v)[8]) {
+// s_p(a) the product over the axes odd in p of (2 a_axis - 1). The x and y butterflies of an element's two node
+// planes (4 nodes each) do not involve the other plane, so a plane shared by two elements is taken once
+// (wht4*) and each element then takes the z butterflies of its two planes (wht_z*): 16 instead of 24 operations
+// a component, the same ones in the same order.
+__device__ __forceinline__ void wht4x2(float2 (&v)[4]) {
 #pragma unroll
-  for (int bit = 1; bit < 8; bit <<= 1)
+  for (int bit = 1; bit < 4; bit <<= 1)
 #pragma unroll
-    for (int a = 0; a < 8; ++a)
+    for (int a = 0; a < 4; ++a)
       if (!(a & bit)) {
         const float2 lo = v[a], hi = v[a | bit];
         v[a] = f2add(hi, lo);
         v[a | bit] = f2sub(hi, lo);
+      }
+}
+template <class T>
+__device__ __forceinline__ void wht4s(T (&v)[4]) {
+#pragma unroll
+  for (int bit = 1; bit < 4; bit <<= 1)
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+      if (!(a & bit)) {
+        const T lo = v[a], hi = v[a | bit];
+        v[a] = hi + lo;
+        v[a | bit] = hi - lo;
       }
 }
 
@@ -484,13 +499,20 @@ __device__ __forceinline__ void iwht8x2(float2 (&v)[8]) {
       }
 }
 
-// y = E KE(h) u for two elements at once (lanes .x, .y); u[c][a]: component c at local node
-// a = x | y << 1 | z << 2 (bit order, not the reference's local numbering). The outputs of component c are
-// handed to sink(c, y_c[8]) as soon as they are formed, which keeps few of them live.
+// y = E KE(h) u for two elements at once (lanes .x, .y); lo[c], hi[c]: wht4 of component c on the element's lower
+// and upper node plane (local node a = x | y << 1 | z << 2: bit order, not the reference's local numbering). The
+// outputs of component c are handed to sink(c, y_c[8]) as soon as they are formed, which keeps few of them live.
 template <class Sink>
-__device__ __forceinline__ void hex_apply2(const HexOpF& op, float2 E, float2 (&u)[3][8], Sink&& sink) {
+__device__ __forceinline__ void hex_apply2(const HexOpF& op, float2 E, const float2 (&lo)[3][4],
+                                           const float2 (&hi)[3][4], Sink&& sink) {
+  float2 u[3][8];
 #pragma unroll
-  for (int c = 0; c < 3; ++c) wht8x2(u[c]);
+  for (int c = 0; c < 3; ++c)
+#pragma unroll
+    for (int a = 0; a < 4; ++a) {
+      u[c][a] = f2add(hi[c][a], lo[c][a]);
+      u[c][a + 4] = f2sub(hi[c][a], lo[c][a]);
+    }
   float2 d[2][3], lam[2], mu[2];
 #pragma unroll
   for (int a = 0; a < 2; ++a) {
@@ -634,8 +656,18 @@ __device__ __forceinline__ int mv32f_body(const GridDims& g, const A& a, int zse
   };
 
   wait_rel(0);
-  float ub[4][3];
-  gather4(0, ub);
+  float tb[3][4], nb3[3];  // the plane below the step's: its wht4, and its node (1, 1)
+  {
+    float ub[4][3];
+    gather4(0, ub);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+#pragma unroll
+      for (int b = 0; b < 4; ++b) tb[c][b] = ub[b][c];
+      wht4s(tb[c]);
+      nb3[c] = ub[3][c];
+    }
+  }
   __syncthreads();  // stage of rel 0 is refilled in the first step
   float carry[3] = {0.f, 0.f, 0.f};
   double pap = 0.0;
@@ -670,17 +702,21 @@ __device__ __forceinline__ int mv32f_body(const GridDims& g, const A& a, int zse
         for (int c = 0; c < 3; ++c) a.pnew[fbase + fplane * (kk + 2) + c] = ut[3][c];
       }
     }
-    float2 u[3][8];
+    float2 lo[3][4], hi[3][4];  // local z = 0: planes kk, kk + 1; local z = 1: planes kk + 1, kk + 2
 #pragma unroll
-    for (int c = 0; c < 3; ++c)
+    for (int c = 0; c < 3; ++c) {
+#pragma unroll
+      for (int b = 0; b < 4; ++b) hi[c][b] = make_float2(um[b][c], ut[b][c]);
+      wht4x2(hi[c]);
 #pragma unroll
       for (int b = 0; b < 4; ++b) {
-        u[c][b] = make_float2(ub[b][c], um[b][c]);      // local z = 0: planes kk, kk + 1
-        u[c][b + 4] = make_float2(um[b][c], ut[b][c]);  // local z = 1: planes kk + 1, kk + 2
+        lo[c][b] = make_float2(tb[c][b], hi[c][b].x);
+        tb[c][b] = hi[c][b].y;
       }
+    }
     // comb[by][pl][c]: node column ex + 1, node row ey + by, node plane kk + pl, after the x-neighbour's part
     float comb[2][3][3];
-    hex_apply2(*a.op, e2, u, [&](int c, float2 (&yc)[8]) {
+    hex_apply2(*a.op, e2, lo, hi, [&](int c, float2 (&yc)[8]) {
 #pragma unroll
       for (int by = 0; by < 2; ++by) {
         const int a = 2 * by;
@@ -705,7 +741,7 @@ __device__ __forceinline__ int mv32f_body(const GridDims& g, const A& a, int zse
         const float s1 = comb[1][1][c] + ybr[(3 + c) * FX];
         const float s2 = comb[1][2][c] + ybr[(6 + c) * FX];
         if (kk >= k0) {  // node plane kk: the element plane below (carried) + plane kk's bottom faces
-          const float pv = ub[3][c];
+          const float pv = nb3[c];
           const float yo = (f0 >> c & 1) ? pv : carry[c] + s0;
           a.y[fbase + fplane * kk + c] = yo;
           if (MODE == 1) pap += (double)pv * (double)yo;
@@ -720,9 +756,7 @@ __device__ __forceinline__ int mv32f_body(const GridDims& g, const A& a, int zse
       }
     }
 #pragma unroll
-    for (int b = 0; b < 4; ++b)
-#pragma unroll
-      for (int c = 0; c < 3; ++c) ub[b][c] = ut[b][c];
+    for (int c = 0; c < 3; ++c) nb3[c] = ut[3][c];
   }
   // every copy has landed when all waits succeeded: the mbarriers are retired, so a persistent CTA can set
   // them up again for its next tile (after a failed wait a copy may still be in flight: they stay as they are)
@@ -780,19 +814,6 @@ static dim3 fac_grid(const GridDims& g, int zseg) {
 // MODE 1 fuses p_t = z + beta p_{t-1}, the write of p_t and the p.Ap partials.
 // ---------------------------------------------------------------------------------------------------------
 template <class T>
-__device__ __forceinline__ void wht8s(T (&v)[8]) {
-#pragma unroll
-  for (int bit = 1; bit < 8; bit <<= 1)
-#pragma unroll
-    for (int a = 0; a < 8; ++a)
-      if (!(a & bit)) {
-        const T lo = v[a], hi = v[a | bit];
-        v[a] = hi + lo;
-        v[a | bit] = hi - lo;
-      }
-}
-
-template <class T>
 __device__ __forceinline__ void iwht8s(T (&v)[8]) {
 #pragma unroll
   for (int bit = 1; bit < 8; bit <<= 1)
@@ -805,11 +826,18 @@ __device__ __forceinline__ void iwht8s(T (&v)[8]) {
       }
 }
 
-// y = E KE(h) u for one element in FP64 (same basis and constants as hex_apply2); sink(c, y_c[8])
+// y = E KE(h) u for one element in FP64 (same basis, planes and constants as hex_apply2); sink(c, y_c[8])
 template <class Sink>
-__device__ __forceinline__ void hex_apply64(const HexOpD& op, double E, double (&u)[3][8], Sink&& sink) {
+__device__ __forceinline__ void hex_apply64(const HexOpD& op, double E, const double (&lo)[3][4],
+                                            const double (&hi)[3][4], Sink&& sink) {
+  double u[3][8];
 #pragma unroll
-  for (int c = 0; c < 3; ++c) wht8s(u[c]);
+  for (int c = 0; c < 3; ++c)
+#pragma unroll
+    for (int a = 0; a < 4; ++a) {
+      u[c][a] = hi[c][a] + lo[c][a];
+      u[c][a + 4] = hi[c][a] - lo[c][a];
+    }
   double d[2][3], lam[2], mu[2];
 #pragma unroll
   for (int a = 0; a < 2; ++a) {
@@ -917,8 +945,18 @@ __global__ void __launch_bounds__(FX * FY, 2) k_mv64f(GridDims g, const __grid_c
 
   wait_plane(k0 - 1);
   wait_plane(k0);
-  double ub[4][3];
-  gather4(k0 - 1, ub);
+  double tb[3][4], nb3[3];  // the plane below the step's: its wht4, and its node (1, 1)
+  {
+    double ub[4][3];
+    gather4(k0 - 1, ub);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+#pragma unroll
+      for (int b = 0; b < 4; ++b) tb[c][b] = ub[b][c];
+      wht4s(tb[c]);
+      nb3[c] = ub[3][c];
+    }
+  }
   __syncthreads();  // the stage of plane k0 - 1 is refilled in the first step
   double carry[3] = {0.0, 0.0, 0.0};
   double pap = 0.0;
@@ -942,16 +980,15 @@ __global__ void __launch_bounds__(FX * FY, 2) k_mv64f(GridDims g, const __grid_c
 #pragma unroll
       for (int c = 0; c < 3; ++c) pnew[fbase + fplane * (kk + 1) + c] = ut[3][c];
     }
-    double u[3][8];
+    double tt[3][4];
 #pragma unroll
-    for (int c = 0; c < 3; ++c)
+    for (int c = 0; c < 3; ++c) {
 #pragma unroll
-      for (int b = 0; b < 4; ++b) {
-        u[c][b] = ub[b][c];
-        u[c][b + 4] = ut[b][c];
-      }
+      for (int b = 0; b < 4; ++b) tt[c][b] = ut[b][c];
+      wht4s(tt[c]);
+    }
     double comb[2][2][3];  // [y][z][c]
-    hex_apply64(op, e_cur, u, [&](int c, double (&yc)[8]) {
+    hex_apply64(op, e_cur, tb, tt, [&](int c, double (&yc)[8]) {
 #pragma unroll
       for (int by = 0; by < 2; ++by)
 #pragma unroll
@@ -974,7 +1011,7 @@ __global__ void __launch_bounds__(FX * FY, 2) k_mv64f(GridDims g, const __grid_c
         const double bot = comb[1][0][c] + ybr[c * FX];
         top[c] = comb[1][1][c] + ybr[(3 + c) * FX];
         if (outp) {
-          const double pv = ub[3][c];
+          const double pv = nb3[c];
           const double yo = (f >> c & 1) ? pv : carry[c] + bot;
           y[fbase + fplane * kk + c] = yo;
           if (MODE == 1) pap += pv * yo;
@@ -984,9 +1021,11 @@ __global__ void __launch_bounds__(FX * FY, 2) k_mv64f(GridDims g, const __grid_c
       for (int c = 0; c < 3; ++c) carry[c] = top[c];
     }
 #pragma unroll
-    for (int b = 0; b < 4; ++b)
+    for (int c = 0; c < 3; ++c) {
 #pragma unroll
-      for (int c = 0; c < 3; ++c) ub[b][c] = ut[b][c];
+      for (int b = 0; b < 4; ++b) tb[c][b] = tt[c][b];
+      nb3[c] = ut[3][c];
+    }
   }
   if (!ok && err) atomicExch(err, 1);
   if (MODE == 1)
