@@ -10,6 +10,7 @@
 #include <cstdio>
 #include <cstring>
 #include <deque>
+#include <memory>
 #include <string>
 #include <thread>
 #include <unordered_map>
@@ -427,6 +428,7 @@ extern "C" int32_t mycel_ctx_destroy(mycel_ctx* c) {
   cudaSetDevice(c->device);
   pack_release(c);  // frees on the stream: before it goes
   fan_release(c);
+  host_copy_release(c);
   if (c->stream) {
     cudaStreamSynchronize(c->stream);
     cudaStreamDestroy(c->stream);
@@ -569,11 +571,13 @@ extern "C" int32_t mycel_problem_create(mycel_ctx* c, const mycel_grid* grid, co
       }
     }
   }
-  std::vector<int32_t> active;
-  active.reserve((size_t)g.ne);
-  for (int64_t e = 0; e < g.ne; ++e)
-    if (domain[e]) active.push_back((int32_t)e);
-  p->n_active = (int64_t)active.size();
+  std::unique_ptr<int32_t[]> active(new int32_t[(size_t)g.ne + 1]);
+  int64_t n_act = 0;
+  for (int64_t e = 0; e < g.ne; ++e) {
+    active[(size_t)n_act] = (int32_t)e;
+    n_act += domain[e] != 0;
+  }
+  p->n_active = n_act;
   for (const auto& kv : facc)
     if (kv.second != 0.0) p->f_idx.push_back((int32_t)kv.first);
   std::sort(p->f_idx.begin(), p->f_idx.end());
@@ -601,8 +605,8 @@ extern "C" int32_t mycel_problem_create(mycel_ctx* c, const mycel_grid* grid, co
     return set_error(c, MYCEL_E_OOM, "out of device memory for the problem");
   }
   cudaMemsetAsync(p->d_invdf, 0, sizeof(float) * g.n32, s);  // pads of the padded FP32 layout stay zero
-  cudaMemcpyAsync(p->d_domain, domain, g.ne, cudaMemcpyHostToDevice, s);
-  if (p->n_active) cudaMemcpyAsync(p->d_active, active.data(), sizeof(int32_t) * p->n_active, cudaMemcpyHostToDevice, s);
+  cudaError_t ce = copy_in(c, p->d_domain, domain, g.ne);
+  if (ce == cudaSuccess && p->n_active) ce = copy_in(c, p->d_active, active.get(), sizeof(int32_t) * p->n_active);
   // F: zero, then its non-zero entries scattered (their values staged in tmp0)
   cudaMemsetAsync(p->d_F, 0, sizeof(double) * g.nd, s);
   if (p->n_fnz) {
@@ -613,10 +617,10 @@ extern "C" int32_t mycel_problem_create(mycel_ctx* c, const mycel_grid* grid, co
   }
   if (n_fixed) cudaMemcpyAsync(p->d_fixed, fixed, sizeof(int32_t) * n_fixed, cudaMemcpyHostToDevice, s);
   if (density) {
-    cudaMemcpyAsync(p->d_rho_box, density, sizeof(double) * g.ne, cudaMemcpyHostToDevice, s);
+    if (ce == cudaSuccess) ce = copy_in(c, p->d_rho_box, density, sizeof(double) * g.ne);
   } else {
     std::vector<double> ones((size_t)g.ne, 1.0);
-    cudaMemcpyAsync(p->d_rho_box, ones.data(), sizeof(double) * g.ne, cudaMemcpyHostToDevice, s);
+    if (ce == cudaSuccess) ce = copy_in(c, p->d_rho_box, ones.data(), sizeof(double) * g.ne);
     cudaStreamSynchronize(s);
   }
   cudaMemsetAsync(d_cnt, 0, 16, s);
@@ -638,9 +642,10 @@ extern "C" int32_t mycel_problem_create(mycel_ctx* c, const mycel_grid* grid, co
   // zero b on constrained DOFs: download flags once (set-up) to count active nodes and fixed DOFs
   std::vector<uint8_t> nf((size_t)g.nn);
   int32_t hcnt = 0;
-  cudaMemcpyAsync(nf.data(), p->d_nflags, g.nn, cudaMemcpyDeviceToHost, s);
+  if (ce == cudaSuccess) ce = copy_out(c, nf.data(), p->d_nflags, g.nn);
   cudaMemcpyAsync(&hcnt, d_cnt, sizeof(int32_t), cudaMemcpyDeviceToHost, s);
   cudaError_t e = cudaGetLastError();
+  if (e == cudaSuccess) e = ce;
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   dfree(c->stream, d_cnt);
   if (e != cudaSuccess) {
@@ -770,7 +775,7 @@ int32_t ensure_cases(mycel_problem* p) {
   const int64_t nd = p->g.nd;
   const int m = p->n_cases;
   std::vector<uint8_t> nf((size_t)p->g.nn);
-  MYCEL_CUDA(c, cudaMemcpyAsync(nf.data(), p->d_nflags, p->g.nn, cudaMemcpyDeviceToHost, s));
+  MYCEL_CUDA(c, copy_out(c, nf.data(), p->d_nflags, p->g.nn));
   MYCEL_CUDA(c, cudaStreamSynchronize(s));
   std::vector<double> f((size_t)nd), b((size_t)nd);
   std::vector<int32_t> lists;
@@ -801,8 +806,8 @@ int32_t ensure_cases(mycel_problem* p) {
       if (b[i] != 0.0) lists.push_back((int32_t)i);
     }
     p->case_nz_cnt[2 * k + 1] = (int32_t)lists.size() - p->case_nz_off[2 * k + 1];
-    MYCEL_CUDA(c, cudaMemcpyAsync(p->d_case_F + k * nd, f.data(), sizeof(double) * nd, cudaMemcpyHostToDevice, s));
-    MYCEL_CUDA(c, cudaMemcpyAsync(p->d_case_b + k * nd, b.data(), sizeof(double) * nd, cudaMemcpyHostToDevice, s));
+    MYCEL_CUDA(c, copy_in(c, p->d_case_F + k * nd, f.data(), sizeof(double) * nd));
+    MYCEL_CUDA(c, copy_in(c, p->d_case_b + k * nd, b.data(), sizeof(double) * nd));
     MYCEL_CUDA(c, cudaStreamSynchronize(s));  // f and b are refilled for the next case
   }
   if (dalloc(p, &p->d_case_nz, std::max<size_t>(lists.size(), 1))) {
@@ -836,7 +841,7 @@ extern "C" int32_t mycel_update_densities(mycel_problem* p, const double* dens, 
   if (!p || !dens) return set_error(p ? p->ctx : nullptr, MYCEL_E_ARG, "NULL argument");
   cudaSetDevice(p->ctx->device);
   cudaStream_t s = p->ctx->stream;
-  MYCEL_CUDA(p->ctx, cudaMemcpyAsync(p->d_rho_box, dens, sizeof(double) * p->g.ne, cudaMemcpyHostToDevice, s));
+  MYCEL_CUDA(p->ctx, copy_in(p->ctx, p->d_rho_box, dens, sizeof(double) * p->g.ne));
   p->penal = penal;
   launch_update_E(p, p->d_rho_box, penal);
   launch_diag(p);
@@ -847,7 +852,7 @@ extern "C" int32_t mycel_update_densities(mycel_problem* p, const double* dens, 
 extern "C" int32_t mycel_diagonal(mycel_problem* p, double* out) {
   if (!p || !out) return set_error(p ? p->ctx : nullptr, MYCEL_E_ARG, "NULL argument");
   cudaSetDevice(p->ctx->device);
-  MYCEL_CUDA(p->ctx, cudaMemcpyAsync(out, p->d_diag, sizeof(double) * p->g.nd, cudaMemcpyDeviceToHost, p->ctx->stream));
+  MYCEL_CUDA(p->ctx, copy_out(p->ctx, out, p->d_diag, sizeof(double) * p->g.nd));
   MYCEL_CUDA(p->ctx, cudaStreamSynchronize(p->ctx->stream));
   return MYCEL_OK;
 }
@@ -856,7 +861,7 @@ extern "C" int32_t mycel_apply_k(mycel_problem* p, const double* x, double* y, i
   if (!p || !x || !y) return set_error(p ? p->ctx : nullptr, MYCEL_E_ARG, "NULL argument");
   cudaSetDevice(p->ctx->device);
   cudaStream_t s = p->ctx->stream;
-  MYCEL_CUDA(p->ctx, cudaMemcpyAsync(p->d_tmp0, x, sizeof(double) * p->g.nd, cudaMemcpyHostToDevice, s));
+  MYCEL_CUDA(p->ctx, copy_in(p->ctx, p->d_tmp0, x, sizeof(double) * p->g.nd));
   if (precision == MYCEL_PRECISION_MIXED || precision == MYCEL_PRECISION_MIXED_MG) {
     int32_t st = ensure_pcg_workspace(p);
     if (st) return st;
@@ -869,7 +874,7 @@ extern "C" int32_t mycel_apply_k(mycel_problem* p, const double* x, double* y, i
   } else {
     launch_matvec64(p, p->d_tmp0, p->d_tmp1, projected);
   }
-  MYCEL_CUDA(p->ctx, cudaMemcpyAsync(y, p->d_tmp1, sizeof(double) * p->g.nd, cudaMemcpyDeviceToHost, s));
+  MYCEL_CUDA(p->ctx, copy_out(p->ctx, y, p->d_tmp1, sizeof(double) * p->g.nd));
   MYCEL_CUDA(p->ctx, cudaStreamSynchronize(s));
   return MYCEL_OK;
 }
@@ -881,8 +886,8 @@ extern "C" int32_t mycel_pcg_solve(mycel_problem* p, const double* b, double* x,
   cudaStream_t s = p->ctx->stream;
   int32_t st = ensure_pcg_workspace(p);
   if (st) return st;
-  MYCEL_CUDA(p->ctx, cudaMemcpyAsync(p->d_tmp1, b, sizeof(double) * p->g.nd, cudaMemcpyHostToDevice, s));
-  MYCEL_CUDA(p->ctx, cudaMemcpyAsync(p->d_x, x, sizeof(double) * p->g.nd, cudaMemcpyHostToDevice, s));
+  MYCEL_CUDA(p->ctx, copy_in(p->ctx, p->d_tmp1, b, sizeof(double) * p->g.nd));
+  MYCEL_CUDA(p->ctx, copy_in(p->ctx, p->d_x, x, sizeof(double) * p->g.nd));
   int32_t* nz = (int32_t*)p->d_tmp0;
   int32_t cnt = 0;
   if ((st = build_nz_list(p, p->d_tmp1, nz, &cnt))) return st;
@@ -893,7 +898,7 @@ extern "C" int32_t mycel_pcg_solve(mycel_problem* p, const double* b, double* x,
     st = pcg_solve_fp64(p, p->d_tmp1, nz, cnt, p->d_x, tol, max_iter, nullptr, res);
   }
   if (st) return st;
-  MYCEL_CUDA(p->ctx, cudaMemcpyAsync(x, p->d_x, sizeof(double) * p->g.nd, cudaMemcpyDeviceToHost, s));
+  MYCEL_CUDA(p->ctx, copy_out(p->ctx, x, p->d_x, sizeof(double) * p->g.nd));
   MYCEL_CUDA(p->ctx, cudaStreamSynchronize(s));
   return MYCEL_OK;
 }
@@ -1003,9 +1008,9 @@ extern "C" int32_t mycel_average_element_to_node(mycel_problem* p, const double*
   if (len != p->g.ne) return set_error(p->ctx, MYCEL_E_ARG, "elementScalar length must equal TotalElements.");
   cudaSetDevice(p->ctx->device);
   cudaStream_t s = p->ctx->stream;
-  MYCEL_CUDA(p->ctx, cudaMemcpyAsync(p->d_tmp0, element_scalar, sizeof(double) * p->g.ne, cudaMemcpyHostToDevice, s));
+  MYCEL_CUDA(p->ctx, copy_in(p->ctx, p->d_tmp0, element_scalar, sizeof(double) * p->g.ne));
   launch_average_e2n(p, p->d_tmp0, p->d_tmp1);
-  MYCEL_CUDA(p->ctx, cudaMemcpyAsync(nodal_out, p->d_tmp1, sizeof(double) * p->g.nn, cudaMemcpyDeviceToHost, s));
+  MYCEL_CUDA(p->ctx, copy_out(p->ctx, nodal_out, p->d_tmp1, sizeof(double) * p->g.nn));
   MYCEL_CUDA(p->ctx, cudaStreamSynchronize(s));
   return MYCEL_OK;
 }
@@ -1028,7 +1033,7 @@ extern "C" int32_t mycel_static_solve(mycel_problem* p, const mycel_static_optio
   // new FemOperator(model): E from ElementDensity and Penal
   launch_update_E(p, p->d_rho_box, p->penal);
   launch_diag(p);
-  if (warm) MYCEL_CUDA(c, cudaMemcpyAsync(p->d_x, warm, sizeof(double) * p->g.nd, cudaMemcpyHostToDevice, s));
+  if (warm) MYCEL_CUDA(c, copy_in(c, p->d_x, warm, sizeof(double) * p->g.nd));
   else MYCEL_CUDA(c, cudaMemsetAsync(p->d_x, 0, sizeof(double) * p->g.nd, s));
   mycel_pcg_result local;
   mycel_pcg_result* r = res ? res : &local;
@@ -1044,15 +1049,15 @@ extern "C" int32_t mycel_static_solve(mycel_problem* p, const mycel_static_optio
   if (reactions_out) {
     launch_matvec64(p, p->d_x, p->d_ap, 0);  // ApplyK(u) (StaticAnalysis.cs:103-110)
     launch_reactions(p, p->d_ap, p->d_tmp1, p->d_fixed, (int32_t)p->fixed_host.size());
-    MYCEL_CUDA(c, cudaMemcpyAsync(reactions_out, p->d_tmp1, sizeof(double) * p->g.nd, cudaMemcpyDeviceToHost, s));
+    MYCEL_CUDA(c, copy_out(c, reactions_out, p->d_tmp1, sizeof(double) * p->g.nd));
   }
   if (vm_out) {
     launch_von_mises(p, p->d_x, p->d_tmp0);
-    MYCEL_CUDA(c, cudaMemcpyAsync(vm_out, p->d_tmp0, sizeof(double) * p->g.ne, cudaMemcpyDeviceToHost, s));
+    MYCEL_CUDA(c, copy_out(c, vm_out, p->d_tmp0, sizeof(double) * p->g.ne));
   }
   double* hsc = (double*)c->pinned;
   MYCEL_CUDA(c, cudaMemcpyAsync(hsc, d_sc, 2 * sizeof(double), cudaMemcpyDeviceToHost, s));
-  MYCEL_CUDA(c, cudaMemcpyAsync(u_out, p->d_x, sizeof(double) * p->g.nd, cudaMemcpyDeviceToHost, s));
+  MYCEL_CUDA(c, copy_out(c, u_out, p->d_x, sizeof(double) * p->g.nd));
   MYCEL_CUDA(c, cudaStreamSynchronize(s));
   if (compliance_out) *compliance_out = hsc[0];
   if (maxdisp_out) *maxdisp_out = hsc[1];
@@ -1110,7 +1115,7 @@ extern "C" int32_t mycel_static_solve_cases(mycel_problem* p, const mycel_static
                       d_sc);
     launch_max_disp(p, p->d_x, d_sc + 1);
     MYCEL_CUDA(c, cudaMemcpyAsync(hsc, d_sc, 2 * sizeof(double), cudaMemcpyDeviceToHost, s));
-    MYCEL_CUDA(c, cudaMemcpyAsync(u_out + k * nd, p->d_x, sizeof(double) * nd, cudaMemcpyDeviceToHost, s));
+    MYCEL_CUDA(c, copy_out(c, u_out + k * nd, p->d_x, sizeof(double) * nd));
     MYCEL_CUDA(c, cudaStreamSynchronize(s));
     if (compliance_out) compliance_out[k] = hsc[0];
     if (maxdisp_out) maxdisp_out[k] = hsc[1];
@@ -1157,12 +1162,12 @@ static int32_t filter_io(mycel_filter* f, const double* in, double* out, int adj
   int32_t st = ensure_pcg_workspace(p);
   if (st) return st;
   double* d_outbox = p->d_z;
-  MYCEL_CUDA(p->ctx, cudaMemcpyAsync(d_in, in, sizeof(double) * p->n_active, cudaMemcpyHostToDevice, s));
+  MYCEL_CUDA(p->ctx, copy_in(p->ctx, d_in, in, sizeof(double) * p->n_active));
   launch_scatter_active(p, d_in, d_box, 0.0);
   if (adj) launch_filter_adj(f, d_box, d_outbox);
   else launch_filter_fwd(f, d_box, d_outbox);
   launch_gather_active(p, d_outbox, d_in);
-  MYCEL_CUDA(p->ctx, cudaMemcpyAsync(out, d_in, sizeof(double) * p->n_active, cudaMemcpyDeviceToHost, s));
+  MYCEL_CUDA(p->ctx, copy_out(p->ctx, out, d_in, sizeof(double) * p->n_active));
   MYCEL_CUDA(p->ctx, cudaStreamSynchronize(s));
   return MYCEL_OK;
 }
@@ -1175,7 +1180,7 @@ extern "C" int32_t mycel_filter_s(mycel_filter* f, double* out) {
   mycel_problem* p = f->p;
   cudaSetDevice(p->ctx->device);
   launch_gather_active(p, f->d_s, p->d_tmp0);
-  MYCEL_CUDA(p->ctx, cudaMemcpyAsync(out, p->d_tmp0, sizeof(double) * p->n_active, cudaMemcpyDeviceToHost, p->ctx->stream));
+  MYCEL_CUDA(p->ctx, copy_out(p->ctx, out, p->d_tmp0, sizeof(double) * p->n_active));
   MYCEL_CUDA(p->ctx, cudaStreamSynchronize(p->ctx->stream));
   return MYCEL_OK;
 }
@@ -1187,12 +1192,12 @@ extern "C" int32_t mycel_sensitivities(mycel_problem* p, const double* u, const 
   cudaStream_t s = p->ctx->stream;
   int32_t st = ensure_pcg_workspace(p);
   if (st) return st;
-  MYCEL_CUDA(p->ctx, cudaMemcpyAsync(p->d_r, u, sizeof(double) * p->g.nd, cudaMemcpyHostToDevice, s));
-  MYCEL_CUDA(p->ctx, cudaMemcpyAsync(p->d_tmp0, rho_active, sizeof(double) * p->n_active, cudaMemcpyHostToDevice, s));
+  MYCEL_CUDA(p->ctx, copy_in(p->ctx, p->d_r, u, sizeof(double) * p->g.nd));
+  MYCEL_CUDA(p->ctx, copy_in(p->ctx, p->d_tmp0, rho_active, sizeof(double) * p->n_active));
   launch_scatter_active(p, p->d_tmp0, p->d_tmp1, 0.0);
   launch_sens(p, p->d_r, p->d_tmp1, penal, p->d_z);
   launch_gather_active(p, p->d_z, p->d_tmp0);
-  MYCEL_CUDA(p->ctx, cudaMemcpyAsync(dc_active, p->d_tmp0, sizeof(double) * p->n_active, cudaMemcpyDeviceToHost, s));
+  MYCEL_CUDA(p->ctx, copy_out(p->ctx, dc_active, p->d_tmp0, sizeof(double) * p->n_active));
   MYCEL_CUDA(p->ctx, cudaStreamSynchronize(s));
   return MYCEL_OK;
 }
@@ -1217,10 +1222,11 @@ extern "C" int32_t mycel_oc_update(mycel_ctx* c, int32_t n, const double* rho, c
   MYCEL_CUDA(c, cudaMallocAsync((void**)&d_out, sizeof(OcOut), s));
   if (passive) MYCEL_CUDA(c, cudaMallocAsync((void**)&d_pas, nn, s));
   MYCEL_CUDA(c, cudaMemsetAsync(d_out, 0, sizeof(OcOut), s));
+  cudaError_t ce = cudaSuccess;
   if (n) {
-    cudaMemcpyAsync(d_rho, rho, n * 8, cudaMemcpyHostToDevice, s);
-    cudaMemcpyAsync(d_dc, dc, n * 8, cudaMemcpyHostToDevice, s);
-    cudaMemcpyAsync(d_s, sv, n * 8, cudaMemcpyHostToDevice, s);
+    ce = copy_in(c, d_rho, rho, n * 8);
+    if (ce == cudaSuccess) ce = copy_in(c, d_dc, dc, n * 8);
+    if (ce == cudaSuccess) ce = copy_in(c, d_s, sv, n * 8);
     if (passive) cudaMemcpyAsync(d_pas, passive, n, cudaMemcpyHostToDevice, s);
   }
   OcParams prm{f, move, rho_min, lambda_guess, vol_tol, max_bisect, 0};
@@ -1229,9 +1235,10 @@ extern "C" int32_t mycel_oc_update(mycel_ctx* c, int32_t n, const double* rho, c
   std::memset(ho, 0, sizeof(OcOut));
   if (!st) {
     cudaMemcpyAsync(ho, d_out, sizeof(OcOut), cudaMemcpyDeviceToHost, s);
-    if (n) cudaMemcpyAsync(rho_new, d_new, n * 8, cudaMemcpyDeviceToHost, s);
+    if (n && ce == cudaSuccess) ce = copy_out(c, rho_new, d_new, n * 8);
   }
   cudaError_t e = cudaStreamSynchronize(s);
+  if (e == cudaSuccess) e = ce;
   OcOut h = *ho;
   cudaFreeAsync(d_rho, s); cudaFreeAsync(d_dc, s); cudaFreeAsync(d_s, s); cudaFreeAsync(d_new, s);
   cudaFreeAsync(d_scr, s); cudaFreeAsync(d_out, s);

@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -93,6 +94,7 @@ struct DevBuf {
 };
 
 struct MgHier;  // multigrid hierarchy of a problem (fp32_kernels.cu)
+struct HostCopy;  // hostcopy.cpp
 }  // namespace mycel
 
 // ---- opaque handles of the C ABI ----
@@ -118,6 +120,9 @@ struct mycel_ctx {
   void* fan = nullptr;     // side streams for independent per-problem work of a batch step (mycel::fan_*)
   cudaStream_t main_stream = nullptr, main_side = nullptr;  // the context's own streams while a fan slot is in use
   int64_t packed_rhs = 0;  // right-hand sides whose solves ran through packed launches (a statistic)
+  mycel::HostCopy* copier = nullptr;  // threads and pinned slots of large host copies, made on first use
+  bool copier_failed = false;
+  std::mutex copier_mu;
 };
 
 struct mycel_problem {
@@ -333,6 +338,11 @@ struct PackJob {
 // together by packed launches; jobs the packed form cannot take are solved alone. Each result equals the
 // problem's solve alone in the mixed multigrid form.
 int32_t mg_solve_packed(mycel_ctx* c, int njobs, PackJob* jobs, const volatile int32_t* cancel);
+// Copies of a caller's array to and from the device on the context's stream (hostcopy.cpp); copy_out may return before
+// the bytes are there (pinned memory): synchronise the stream before they are read.
+cudaError_t copy_in(mycel_ctx* c, void* d, const void* h, size_t n);
+cudaError_t copy_out(mycel_ctx* c, void* h, const void* d, size_t n);
+void host_copy_release(mycel_ctx* c);
 void pack_release(mycel_ctx* c);
 // Asynchronous packed run (mycel_simp_run_many): the right-hand sides of the jobs share one packed plan for a
 // whole optimisation and each job's solves start and end on their own. pkr_open leaves out the jobs the

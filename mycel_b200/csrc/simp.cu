@@ -130,8 +130,12 @@ extern "C" int32_t mycel_simp_begin(mycel_problem* p, const mycel_simp_options* 
   // passive mask (TopologyOptimizer.cs:45-84): option mask and hinge shell PassiveRegion.Build(r = 1)
   std::vector<uint8_t> pas((size_t)g.ne, 0);
   std::vector<uint8_t> dom((size_t)g.ne);
-  cudaMemcpyAsync(dom.data(), p->d_domain, g.ne, cudaMemcpyDeviceToHost, st);
-  cudaStreamSynchronize(st);
+  cudaError_t de = copy_out(c, dom.data(), p->d_domain, g.ne);
+  if (de == cudaSuccess) de = cudaStreamSynchronize(st);
+  if (de != cudaSuccess) {
+    delete s;
+    return set_error(c, MYCEL_E_DEVICE, std::string("SIMP set-up: ") + cudaGetErrorString(de));
+  }
   if (o.passive_mask)
     for (int64_t e = 0; e < g.ne; ++e)
       if (dom[e] && e < o.passive_mask_len && o.passive_mask[e] != 0) pas[e] = 1;
@@ -202,20 +206,21 @@ extern "C" int32_t mycel_simp_begin(mycel_problem* p, const mycel_simp_options* 
     return set_error(c, MYCEL_E_OOM, "out of device memory for the SIMP state");
   }
   if (!o.enable_heaviside) s->d_rb = s->d_rt;
-  cudaMemcpyAsync(s->d_rho, rho.data(), sizeof(double) * g.ne, cudaMemcpyHostToDevice, st);
-  cudaMemcpyAsync(s->d_rho_new, rho.data(), sizeof(double) * g.ne, cudaMemcpyHostToDevice, st);
-  cudaMemcpyAsync(s->d_pas, pas.data(), g.ne, cudaMemcpyHostToDevice, st);
+  cudaError_t ce = copy_in(c, s->d_rho, rho.data(), sizeof(double) * g.ne);
+  cudaMemcpyAsync(s->d_rho_new, s->d_rho, sizeof(double) * g.ne, cudaMemcpyDeviceToDevice, st);
+  if (ce == cudaSuccess) ce = copy_in(c, s->d_pas, pas.data(), g.ne);
   cudaMemsetAsync(s->d_rt, 0, sizeof(double) * g.ne, st);
   cudaMemsetAsync(s->d_dcb, 0, sizeof(double) * g.ne, st);
   cudaMemsetAsync(s->d_dc, 0, sizeof(double) * g.ne, st);
   if (o.warm_start_displacements && o.warm_start_len == g.nd && s->ncase == 1)
-    cudaMemcpyAsync(s->d_u, o.warm_start_displacements, sizeof(double) * g.nd, cudaMemcpyHostToDevice, st);
+    ce = ce == cudaSuccess ? copy_in(c, s->d_u, o.warm_start_displacements, sizeof(double) * g.nd) : ce;
   else
     cudaMemsetAsync(s->d_u, 0, sizeof(double) * g.nd, st);
   if (s->d_uc) cudaMemsetAsync(s->d_uc, 0, sizeof(double) * s->ncase * g.nd, st);
   for (auto& e : s->ev) cudaEventCreate(&e);
   if (cudaMallocHost(&s->h_pin, 256) != cudaSuccess) s->h_pin = nullptr;
   cudaError_t pe = cudaGetLastError();
+  if (pe == cudaSuccess) pe = ce;
   if (pe == cudaSuccess && !s->h_pin) pe = cudaErrorMemoryAllocation;
   if (pe != cudaSuccess) {
     mycel_simp_end(s);
@@ -581,18 +586,18 @@ extern "C" int32_t mycel_simp_read(mycel_simp_session* s, double* u, float* phys
   cudaStream_t st = c->stream;
   if (phys || des) {
     snapshot(s);
-    if (phys) MYCEL_CUDA(c, cudaMemcpyAsync(phys, s->d_phys_f, sizeof(float) * p->g.ne, cudaMemcpyDeviceToHost, st));
-    if (des) MYCEL_CUDA(c, cudaMemcpyAsync(des, s->d_des_f, sizeof(float) * p->g.ne, cudaMemcpyDeviceToHost, st));
+    if (phys) MYCEL_CUDA(c, copy_out(c, phys, s->d_phys_f, sizeof(float) * p->g.ne));
+    if (des) MYCEL_CUDA(c, copy_out(c, des, s->d_des_f, sizeof(float) * p->g.ne));
   }
-  if (u) MYCEL_CUDA(c, cudaMemcpyAsync(u, s->d_u, sizeof(double) * p->g.nd, cudaMemcpyDeviceToHost, st));
+  if (u) MYCEL_CUDA(c, copy_out(c, u, s->d_u, sizeof(double) * p->g.nd));
   if (rpa) {
     launch_gather_active(p, s->d_rb, p->d_tmp0);
-    MYCEL_CUDA(c, cudaMemcpyAsync(rpa, p->d_tmp0, sizeof(double) * p->n_active, cudaMemcpyDeviceToHost, st));
+    MYCEL_CUDA(c, copy_out(c, rpa, p->d_tmp0, sizeof(double) * p->n_active));
     MYCEL_CUDA(c, cudaStreamSynchronize(st));
   }
   if (rda) {
     launch_gather_active(p, s->d_rho, p->d_tmp1);
-    MYCEL_CUDA(c, cudaMemcpyAsync(rda, p->d_tmp1, sizeof(double) * p->n_active, cudaMemcpyDeviceToHost, st));
+    MYCEL_CUDA(c, copy_out(c, rda, p->d_tmp1, sizeof(double) * p->n_active));
   }
   MYCEL_CUDA(c, cudaStreamSynchronize(st));
   if (lambda) *lambda = s->lambda;
@@ -734,9 +739,13 @@ extern "C" int32_t mycel_simp_run(mycel_problem* p, const mycel_simp_options* op
     if (history && s->count - 1 < cap) history[s->count - 1] = r;
     if (progress) {
       snapshot(s);
-      cudaMemcpyAsync(s->h_phys.data(), s->d_phys_f, sizeof(float) * p->g.ne, cudaMemcpyDeviceToHost, c->stream);
-      cudaMemcpyAsync(s->h_des.data(), s->d_des_f, sizeof(float) * p->g.ne, cudaMemcpyDeviceToHost, c->stream);
-      cudaStreamSynchronize(c->stream);
+      cudaError_t ce = copy_out(c, s->h_phys.data(), s->d_phys_f, sizeof(float) * p->g.ne);
+      if (ce == cudaSuccess) ce = copy_out(c, s->h_des.data(), s->d_des_f, sizeof(float) * p->g.ne);
+      if (ce == cudaSuccess) ce = cudaStreamSynchronize(c->stream);
+      if (ce != cudaSuccess) {
+        err = set_error(c, MYCEL_E_DEVICE, std::string("density snapshot: ") + cudaGetErrorString(ce));
+        break;
+      }
       progress(user, &r, s->h_phys.data(), s->h_des.data());
     }
   }
