@@ -2445,20 +2445,38 @@ struct MgAxis {
   }
 };
 
-// restriction r_c = W^T res of a level's residual, component cc at coarse node n (box layout)
-__device__ __forceinline__ void mg_restrict_comp(const MgDims& f, const float* __restrict__ tf, const MgDims& c,
-                                                 const float* __restrict__ invdc, float* __restrict__ rc, int64_t n,
-                                                 int cc, float* __restrict__ xc, float omega) {
+// restriction r_c = W^T res of a level's residual, component cc at coarse node n. PAD: the voxel grid in the padded FP32
+// layout (row pitch pitch), res = r - t; otherwise box layout, res = t. Coarse DOFs with a zero diagonal get 0. With xc
+// also the coarse level's first Jacobi sweep from x = 0: x = omega invd r. All loads go out before the first use, and
+// before the solver's state (st, or null) is looked at.
+// A thread per DOF: latency bounds the small levels, and a thread per node with three chains had a third of the
+// threads for the same loads. B200, us (coarse nodes): 512 4.8 -> 2.7, 18,490 voxel-level 6.3 -> 3.9, 233,000 voxel-level
+// 19.6 -> 18.9.
+template <bool PAD>
+__device__ __forceinline__ void mg_restrict_row(const MgDims& f, int pitch, const float* __restrict__ rf,
+                                                const float* __restrict__ tf, const MgDims& c,
+                                                const float* __restrict__ invdc, float* __restrict__ rc, int64_t n,
+                                                int cc, float* __restrict__ xc, float omega, const MixState* st) {
   int I, J, K;
   mg_ijk(n, c.nx + 1, c.ny + 1, &I, &J, &K);
-  const MgAxis ax(I, f.nx, 3), ay(J, f.ny, 3 * (f.nx + 1)), az(K, f.nz, 3 * (f.nx + 1) * (f.ny + 1));
+  const int rowp = PAD ? pitch : 3 * (f.nx + 1);
+  const MgAxis ax(I, f.nx, 3), ay(J, f.ny, rowp), az(K, f.nz, rowp * (f.ny + 1));
+  float t[27], r[PAD ? 27 : 1];
+#pragma unroll
+  for (int q = 0; q < 27; ++q) {
+    const int b = az.o[q / 9] + ay.o[q / 3 % 3] + ax.o[q % 3] + cc;
+    t[q] = tf[b];
+    if (PAD) r[q] = rf[b];
+  }
+  const float d = invdc[3 * n + cc];
+  if (!mg_running(st)) return;
   float a = 0.f;
 #pragma unroll
   for (int q = 0; q < 27; ++q)
-    a = fmaf(az.w[q / 9] * ay.w[q / 3 % 3] * ax.w[q % 3], tf[az.o[q / 9] + ay.o[q / 3 % 3] + ax.o[q % 3] + cc], a);
-  const float d = invdc[3 * n + cc], rv = d != 0.f ? a : 0.f;
+    a = fmaf(az.w[q / 9] * ay.w[q / 3 % 3] * ax.w[q % 3], PAD ? r[q] - t[q] : t[q], a);
+  const float rv = d != 0.f ? a : 0.f;
   rc[3 * n + cc] = rv;
-  if (xc) xc[3 * n + cc] = omega * d * rv;  // the coarse level's first Jacobi sweep from x = 0
+  if (xc) xc[3 * n + cc] = omega * d * rv;
 }
 
 // prolongation x_f += W x_c, component cc at fine node n, on the finer level's free DOFs. PAD: the voxel grid
@@ -2498,56 +2516,19 @@ __device__ __forceinline__ void mg_prolong_comp(const MgDims& f, int pitch, cons
   if (fr) xf[(PAD ? (int64_t)pitch * (j + (int64_t)fy1 * k) + 3 * i : 3 * n) + cc] += a;
 }
 
-// the same transfers for all three components of a node in one pass (the per-level kernels):
-// restriction r_c = W^T res of a level's residual at coarse node n. PAD: the voxel grid in the padded FP32
-// layout (row pitch pitch), res = r - t; otherwise box layout, res = t. Coarse DOFs with a zero diagonal get 0.
-template <bool PAD>
-__device__ __forceinline__ void mg_restrict_node(const MgDims& f, int pitch, const float* __restrict__ rf,
-                                                 const float* __restrict__ tf, const MgDims& c,
-                                                 const float* __restrict__ invdc, float* __restrict__ rc, int64_t n,
-                                                 float* __restrict__ xc, float omega) {
-  int I, J, K;
-  mg_ijk(n, c.nx + 1, c.ny + 1, &I, &J, &K);
-  const int rowp = PAD ? pitch : 3 * (f.nx + 1);
-  const MgAxis ax(I, f.nx, 3), ay(J, f.ny, rowp), az(K, f.nz, rowp * (f.ny + 1));
-  float a0 = 0.f, a1 = 0.f, a2 = 0.f;
-#pragma unroll
-  for (int q = 0; q < 27; ++q) {
-    const float w = az.w[q / 9] * ay.w[q / 3 % 3] * ax.w[q % 3];
-    const int b = az.o[q / 9] + ay.o[q / 3 % 3] + ax.o[q % 3];
-    if (PAD) {
-      a0 = fmaf(w, rf[b] - tf[b], a0);
-      a1 = fmaf(w, rf[b + 1] - tf[b + 1], a1);
-      a2 = fmaf(w, rf[b + 2] - tf[b + 2], a2);
-    } else {
-      a0 = fmaf(w, tf[b], a0);
-      a1 = fmaf(w, tf[b + 1], a1);
-      a2 = fmaf(w, tf[b + 2], a2);
-    }
-  }
-  const float d0 = invdc[3 * n], d1 = invdc[3 * n + 1], d2 = invdc[3 * n + 2];
-  const float r0 = d0 != 0.f ? a0 : 0.f, r1 = d1 != 0.f ? a1 : 0.f, r2 = d2 != 0.f ? a2 : 0.f;
-  rc[3 * n] = r0;
-  rc[3 * n + 1] = r1;
-  rc[3 * n + 2] = r2;
-  if (xc) {  // the coarse level's first Jacobi sweep from x = 0: x = omega invd r
-    xc[3 * n] = omega * d0 * r0;
-    xc[3 * n + 1] = omega * d1 * r1;
-    xc[3 * n + 2] = omega * d2 * r2;
-  }
-}
-
 template <bool PAD, bool MULTI>
-__global__ void k_mg_restrict(MgDims f, int pitch, const __grid_constant__ MgPtrs rf, const __grid_constant__ MgPtrs tf,
-                              MgDims c, const float* __restrict__ invdc, const __grid_constant__ MgPtrs rc,
-                              const MixState* st, const __grid_constant__ MgPtrs xc, int first_sweep,
-                              const float* __restrict__ om, int ncase) {
+__global__ void __launch_bounds__(kMgDofThreads) k_mg_restrict(MgDims f, int pitch, const __grid_constant__ MgPtrs rf,
+                                                               const __grid_constant__ MgPtrs tf, MgDims c,
+                                                               const float* __restrict__ invdc,
+                                                               const __grid_constant__ MgPtrs rc, const MixState* st,
+                                                               const __grid_constant__ MgPtrs xc, int first_sweep,
+                                                               const float* __restrict__ om, int ncase) {
   int64_t n;
   int k;
-  mg_item_case<MULTI>(blockIdx.x * (int64_t)blockDim.x + threadIdx.x, ncase, &n, &k);
-  if (n >= mg_nn(c) || !mg_running(st ? st + k : nullptr)) return;
-  const float omega = first_sweep ? *om : 0.f;
-  mg_restrict_node<PAD>(f, pitch, rf.p[k], tf.p[k], c, invdc, rc.p[k], n, first_sweep ? xc.p[k] : nullptr, omega);
+  mg_item_case<MULTI>(mg_dof_node(), ncase, &n, &k);
+  if (n >= mg_nn(c)) return;
+  mg_restrict_row<PAD>(f, pitch, rf.p[k], tf.p[k], c, invdc, rc.p[k], n, mg_dof_comp(), first_sweep ? xc.p[k] : nullptr,
+                       first_sweep ? *om : 0.f, st ? st + k : nullptr);
 }
 
 // prolongation x_f += W x_c on the finer level's free DOFs, for the pair of fine nodes (2 c, 2 c + 1) of a node row
@@ -2794,8 +2775,8 @@ __device__ __forceinline__ void mg_tail_body(const MgTail& tl, const float* __re
       int k;
       mg_item_case<MULTI>(q, ncase, &it, &k);
       if (live(k))
-        mg_restrict_comp(v.d, v.t + k * nd, cv.d, cv.invd, cv.r + k * cnd, it / 3, (int)(it % 3),
-                                smoothed ? cv.xa + k * cnd : nullptr, wc);
+        mg_restrict_row<false>(v.d, 0, nullptr, v.t + k * nd, cv.d, cv.invd, cv.r + k * cnd, it / 3, (int)(it % 3),
+                               smoothed ? cv.xa + k * cnd : nullptr, wc, nullptr);
     }
     mg_cluster_sync();
     xc[l] = x;
@@ -4097,7 +4078,7 @@ static int mg_vcycle(mycel_problem* p, cudaStream_t s, const MgRun& R) {
     }
   nl += launch_mv32_cases<0>(p, s, nc, R.xf, nullptr, nullptr, R.tf, st, R.pitch);
   // restriction to level 1, with level 1's first sweep (unless level 1 is the coarsest)
-  (nc == 1 ? k_mg_restrict<true, false> : k_mg_restrict<true, true>)<<<mg_blocks(lv[1].nn * nc), 256, 0, s>>>(lv[0].d, g.rp, mg_ptrs(R.rf, nc), mg_ptrs(R.tf, nc),
+  (nc == 1 ? k_mg_restrict<true, false> : k_mg_restrict<true, true>)<<<mg_dof_blocks(lv[1].nn * nc), kMgDofThreads, 0, s>>>(lv[0].d, g.rp, mg_ptrs(R.rf, nc), mg_ptrs(R.tf, nc),
                                                                lv[1].d, lv[1].invd, lv_ptrs(lv[1].r, lv[1].nd, nc), st,
                                                                lv_ptrs(lv[1].xa, lv[1].nd, nc), 1 < mg->L - 1 ? 1 : 0,
                                                                om + 1, nc);
@@ -4115,7 +4096,7 @@ static int mg_vcycle(mycel_problem* p, cudaStream_t s, const MgRun& R) {
     launch_mg_apply(s, v, lv_ptrs(x, v.nd, nc), r, v.invd, lv_ptrs(v.t, v.nd, nc), 2, om + l, st, nc);
     if (l == 1 && mg->l1_timing) cudaEventRecordWithFlags(mg->l1_timing[1], s, cudaEventRecordExternal);
     MgLevel& cv = lv[l + 1];
-    (nc == 1 ? k_mg_restrict<false, false> : k_mg_restrict<false, true>)<<<mg_blocks(cv.nn * nc), 256, 0, s>>>(v.d, 0, lv_ptrs(nullptr, 0, nc),
+    (nc == 1 ? k_mg_restrict<false, false> : k_mg_restrict<false, true>)<<<mg_dof_blocks(cv.nn * nc), kMgDofThreads, 0, s>>>(v.d, 0, lv_ptrs(nullptr, 0, nc),
                                                                lv_ptrs(v.t, v.nd, nc), cv.d, cv.invd,
                                                                lv_ptrs(cv.r, cv.nd, nc), st,
                                                                lv_ptrs(cv.xa, cv.nd, nc), l + 1 < mg->L - 1 ? 1 : 0,
@@ -5305,20 +5286,19 @@ struct PkRestrict {  // restriction of a problem's level to the next coarser one
 };
 
 template <bool PAD, bool MULTI>
-__global__ void k_mg_restrict_pk(const PkRestrict* __restrict__ tab,
-                                                        const unsigned* __restrict__ items,
-                                                        const unsigned* __restrict__ count) {
+__global__ void __launch_bounds__(kMgDofThreads) k_mg_restrict_pk(const PkRestrict* __restrict__ tab,
+                                                                  const unsigned* __restrict__ items,
+                                                                  const unsigned* __restrict__ count) {
   const unsigned cnt = *count;
   for (unsigned w = blockIdx.x; w < cnt; w += gridDim.x) {
     const unsigned code = items[w];
     const PkRestrict& a = tab[code >> kPkLbBits];
     int64_t q;
     int k;
-    mg_item_case<MULTI>((int64_t)(code & kPkLbMask) * blockDim.x + threadIdx.x, a.ncase, &q, &k);
-    if (q >= mg_nn(a.c) || !mg_running(a.st ? a.st + k : nullptr)) continue;
-    const float omega = a.first_sweep ? *a.om : 0.f;
-    mg_restrict_node<PAD>(a.f, a.pitch, a.rf.p[k], a.tf.p[k], a.c, a.invdc, a.rc.p[k], q,
-                          a.first_sweep ? a.xc.p[k] : nullptr, omega);
+    mg_item_case<MULTI>((int64_t)(code & kPkLbMask) * 64 + (threadIdx.x & 63), a.ncase, &q, &k);
+    if (q >= mg_nn(a.c)) continue;
+    mg_restrict_row<PAD>(a.f, a.pitch, a.rf.p[k], a.tf.p[k], a.c, a.invdc, a.rc.p[k], q, mg_dof_comp(),
+                         a.first_sweep ? a.xc.p[k] : nullptr, a.first_sweep ? *a.om : 0.f, a.st ? a.st + k : nullptr);
   }
 }
 
@@ -5557,7 +5537,7 @@ static int pk_resident(int kind, bool pad, bool multi) {
     case PK_RESTRICT:
       e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(
           &o, pad ? (multi ? k_mg_restrict_pk<true, true> : k_mg_restrict_pk<true, false>)
-                  : (multi ? k_mg_restrict_pk<false, true> : k_mg_restrict_pk<false, false>), 256, 0);
+                  : (multi ? k_mg_restrict_pk<false, true> : k_mg_restrict_pk<false, false>), kMgDofThreads, 0);
       break;
     case PK_PROLONG:
       e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(
@@ -5605,7 +5585,7 @@ static void pk_issue(const PackPlan& P, const PkLaunch& L, cudaStream_t s, int s
     case PK_RESTRICT: {
       auto k = L.pad ? (L.multi ? k_mg_restrict_pk<true, true> : k_mg_restrict_pk<true, false>)
                      : (L.multi ? k_mg_restrict_pk<false, true> : k_mg_restrict_pk<false, false>);
-      k<<<g, 256, 0, s>>>((const PkRestrict*)tab, it, cn);
+      k<<<g, kMgDofThreads, 0, s>>>((const PkRestrict*)tab, it, cn);
       break;
     }
     case PK_PROLONG: {
@@ -5803,7 +5783,7 @@ static int32_t pk_build(mycel_ctx* c, PackWork* w, std::vector<PkUnit>& units, c
       a.om = mg->sc->omega + 1;
       a.ncase = q.nc;
       e.push_back(a);
-      nb.push_back(mg_blocks(v1.nn * q.nc));
+      nb.push_back(mg_dof_blocks(v1.nn * q.nc));
       es.push_back({const_cast<MixState*>(q.st), q.nc});
     }
     B.add(P.vcycle, PK_RESTRICT, true, multi == 1, 0, e, nb, es);
@@ -5864,7 +5844,7 @@ static int32_t pk_build(mycel_ctx* c, PackWork* w, std::vector<PkUnit>& units, c
         a.om = mg->sc->omega + l + 1;
         a.ncase = q.nc;
         e.push_back(a);
-        nb.push_back(mg_blocks(cv.nn * q.nc));
+        nb.push_back(mg_dof_blocks(cv.nn * q.nc));
         es.push_back({const_cast<MixState*>(q.st), q.nc});
         xc[qi][l] = v.xa;
       }
