@@ -2532,16 +2532,22 @@ __global__ void __launch_bounds__(kMgDofThreads) k_mg_restrict(MgDims f, int pit
 }
 
 // prolongation x_f += W x_c on the finer level's free DOFs, for the pair of fine nodes (2 c, 2 c + 1) of a node row
-// that share their coarse columns, which are read once for both. PAD: the voxel grid (padded FP32 layout, free = node flag bit clear); otherwise box layout, free =
-// nonzero diagonal. Items of a level: (nx + 2) / 2 pairs a row. (192x96x96 elements: 32.7 us with a thread per node
-// and its eight coarse nodes one after another, 17.3 now; the small levels keep their 3.5 us.)
+// that share their coarse columns, which are read once for both. PAD: the voxel grid (padded FP32 layout, free = node
+// flag bit clear); otherwise box layout, free = nonzero diagonal. Items of a level: (nx + 2) / 2 pairs a row.
+// (192x96x96 elements: 32.7 us with a thread per node and its eight coarse nodes one after another.)
 __host__ __device__ __forceinline__ int64_t mg_pairs(const MgDims& d) {
   return (int64_t)((d.nx + 2) >> 1) * (d.ny + 1) * (d.nz + 1);
 }
-template <bool PAD>
+// N = 1: component cc of a pair; N = 3: all of them (cc 0). The loads go out before the solver's state (st, or null) is
+// looked at. A thread per component on small levels, which latency bounds (85x53x27, us: 5.1 -> 3.6, 3.9 -> 3.1, 3.3 ->
+// 2.9), up to kMgPairMax pairs; a thread per pair above, where the index work shared by the components counts
+// (192x96x96: 15.5 against 21.6 with a thread per component; its next level, 118 thousand pairs, 5.4 against 5.1).
+constexpr int64_t kMgPairMax = 262144;
+template <bool PAD, int N>
 __device__ __forceinline__ void mg_prolong_pair(const MgDims& f, int pitch, const uint8_t* __restrict__ nf,
                                                 const float* __restrict__ invdf, float* __restrict__ xf,
-                                                const MgDims& c, const float* __restrict__ xc, int64_t item) {
+                                                const MgDims& c, const float* __restrict__ xc, int64_t item, int cc,
+                                                const MixState* st) {
   int ci, j, k;
   mg_ijk(item, (f.nx + 2) >> 1, f.ny + 1, &ci, &j, &k);
   const int i = 2 * ci;
@@ -2558,53 +2564,69 @@ __device__ __forceinline__ void mg_prolong_pair(const MgDims& f, int pitch, cons
   axis(j, f.ny, c.ny, &cj, &wj[0], &wj[1]);
   axis(k, f.nz, c.nz, &ck, &wk[0], &wk[1]);
   const int row = 3 * (c.nx + 1), plane = row * (c.ny + 1);
-  const float* base = xc + 3 * ci + row * cj + plane * ck;
+  const float* base = xc + 3 * ci + row * cj + plane * ck + cc;
   const int64_t n = i + (int64_t)(f.nx + 1) * (j + (int64_t)(f.ny + 1) * k);
-  const int64_t b = PAD ? (int64_t)pitch * (j + (int64_t)(f.ny + 1) * k) + 3 * i : 3 * n;
+  float* x = xf + (PAD ? (int64_t)pitch * (j + (int64_t)(f.ny + 1) * k) + 3 * i : 3 * n) + cc;
   // every load first (an absent coarse row is read at its neighbour, an absent column or node at the first)
   const int oy = wj[1] != 0.f ? row : 0, oz = wk[1] != 0.f ? plane : 0, ox = odd ? 3 : 0;
-  float v[4][6], x[6], d[6];
-  uint8_t fl[2];
-#pragma unroll
-  for (int q = 0; q < 4; ++q)
-#pragma unroll
-    for (int cc = 0; cc < 3; ++cc) {
-      v[q][cc] = base[(q & 1 ? oy : 0) + (q >> 1 ? oz : 0) + cc];
-      v[q][3 + cc] = base[(q & 1 ? oy : 0) + (q >> 1 ? oz : 0) + ox + cc];
-    }
-#pragma unroll
-  for (int cc = 0; cc < 3; ++cc) {
-    x[cc] = xf[b + cc];
-    x[3 + cc] = xf[b + ox + cc];
-    if (!PAD) d[cc] = invdf[3 * n + cc], d[3 + cc] = invdf[3 * n + ox + cc];
-  }
-  if (PAD) fl[0] = nf[n], fl[1] = nf[n + (odd ? 1 : 0)];
-  float e[3] = {0.f, 0.f, 0.f}, o[3] = {0.f, 0.f, 0.f};  // the even and the odd node's sums
+  float v[4][2][N], x0[N], x1[N];
+  bool f0[N], f1[N];  // free
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
-    const float w = wj[q & 1] * wk[q >> 1];  // x weight 1 (even node, or the last of an odd count) or 1/2
+    const float* p = base + (q & 1 ? oy : 0) + (q >> 1 ? oz : 0);
 #pragma unroll
-    for (int cc = 0; cc < 3; ++cc) {
-      e[cc] = fmaf(w, v[q][cc], e[cc]);
-      o[cc] = last ? fmaf(w, v[q][3 + cc], o[cc]) : fmaf(0.5f * w, v[q][3 + cc], fmaf(0.5f * w, v[q][cc], o[cc]));
+    for (int m = 0; m < N; ++m) {
+      v[q][0][m] = p[m];
+      v[q][1][m] = p[ox + m];
     }
   }
+  const uint8_t n0 = PAD ? nf[n] : (uint8_t)0, n1 = PAD ? nf[n + (odd ? 1 : 0)] : (uint8_t)0;
 #pragma unroll
-  for (int q = 0; q < 6; ++q) {
-    const bool fr = PAD ? !(fl[q / 3] & (1 << q % 3)) : d[q] != 0.0f;
-    if (fr && (q < 3 || odd)) xf[b + q] = x[q] + (q < 3 ? e[q] : o[q - 3]);
+  for (int m = 0; m < N; ++m) {
+    x0[m] = x[m];
+    x1[m] = x[ox + m];
+    f0[m] = PAD ? !(n0 & (1 << (cc + m))) : invdf[3 * n + cc + m] != 0.0f;
+    f1[m] = PAD ? !(n1 & (1 << (cc + m))) : invdf[3 * n + ox + cc + m] != 0.0f;
+  }
+  if (!mg_running(st)) return;
+#pragma unroll
+  for (int m = 0; m < N; ++m) {
+    float e = 0.f, o = 0.f;  // the even and the odd node's sums
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const float w = wj[q & 1] * wk[q >> 1];  // x weight 1 (even node, or the last of an odd count) or 1/2
+      e = fmaf(w, v[q][0][m], e);
+      o = last ? fmaf(w, v[q][1][m], o) : fmaf(0.5f * w, v[q][1][m], fmaf(0.5f * w, v[q][0][m], o));
+    }
+    if (f0[m]) x[m] = x0[m] + e;
+    if (f1[m] && odd) x[3 + m] = x1[m] + o;
   }
 }
 
-template <bool PAD, bool MULTI>
-__global__ void k_mg_prolong(MgDims f, int pitch, const uint8_t* __restrict__ nf, const float* __restrict__ invdf,
-                             const __grid_constant__ MgPtrs xf, MgDims c, const __grid_constant__ MgPtrs xc,
-                             const MixState* st, int ncase) {
+template <bool PAD, bool MULTI, bool PAIRS>
+__global__ void __launch_bounds__(kMgDofThreads) k_mg_prolong(MgDims f, int pitch, const uint8_t* __restrict__ nf,
+                                                              const float* __restrict__ invdf,
+                                                              const __grid_constant__ MgPtrs xf, MgDims c,
+                                                              const __grid_constant__ MgPtrs xc, const MixState* st,
+                                                              int ncase) {
   int64_t n;
   int k;
-  mg_item_case<MULTI>(blockIdx.x * (int64_t)blockDim.x + threadIdx.x, ncase, &n, &k);
-  if (n >= mg_pairs(f) || !mg_running(st ? st + k : nullptr)) return;
-  mg_prolong_pair<PAD>(f, pitch, nf, invdf, xf.p[k], c, xc.p[k], n);
+  mg_item_case<MULTI>(PAIRS ? blockIdx.x * (int64_t)blockDim.x + threadIdx.x : mg_dof_node(), ncase, &n, &k);
+  if (n >= mg_pairs(f)) return;
+  mg_prolong_pair<PAD, PAIRS ? 3 : 1>(f, pitch, nf, invdf, xf.p[k], c, xc.p[k], n, PAIRS ? 0 : mg_dof_comp(),
+                                      st ? st + k : nullptr);
+}
+static bool mg_by_pairs(const MgDims& f, int nc) { return mg_pairs(f) * nc > kMgPairMax; }
+static unsigned mg_prolong_blocks(const MgDims& f, int nc) {
+  const int64_t n = mg_pairs(f) * nc;
+  return mg_by_pairs(f, nc) ? (unsigned)((n + kMgDofThreads - 1) / kMgDofThreads) : mg_dof_blocks(n);
+}
+template <bool PAD>
+static void launch_mg_prolong(cudaStream_t s, const MgDims& f, int pitch, const uint8_t* nf, const float* invdf,
+                              const MgPtrs& xf, const MgDims& c, const MgPtrs& xc, const MixState* st, int nc) {
+  (mg_by_pairs(f, nc) ? (nc == 1 ? k_mg_prolong<PAD, false, true> : k_mg_prolong<PAD, true, true>)
+                      : (nc == 1 ? k_mg_prolong<PAD, false, false> : k_mg_prolong<PAD, true, false>))
+      <<<mg_prolong_blocks(f, nc), kMgDofThreads, 0, s>>>(f, pitch, nf, invdf, xf, c, xc, st, nc);
 }
 
 
@@ -4111,8 +4133,8 @@ static int mg_vcycle(mycel_problem* p, cudaStream_t s, const MgRun& R) {
     MgLevel& v = lv[l];
     float* x = xc[l];
     float* o = x == v.xa ? v.xb : v.xa;
-    (nc == 1 ? k_mg_prolong<false, false> : k_mg_prolong<false, true>)<<<mg_blocks(mg_pairs(v.d) * nc), 256, 0, s>>>(v.d, 0, nullptr, v.invd, lv_ptrs(x, v.nd, nc), lv[l + 1].d,
-                                                              lv_ptrs(xc[l + 1], lv[l + 1].nd, nc), st, nc);
+    launch_mg_prolong<false>(s, v.d, 0, nullptr, v.invd, lv_ptrs(x, v.nd, nc), lv[l + 1].d,
+                             lv_ptrs(xc[l + 1], lv[l + 1].nd, nc), st, nc);
     const MgPtrs r = lv_ptrs(v.r, v.nd, nc);
     for (int k = 0; k < mg->sweeps; ++k) {
       launch_mg_apply(s, v, lv_ptrs(x, v.nd, nc), r, v.invd, lv_ptrs(o, v.nd, nc), 1, om + l, st, nc);
@@ -4121,8 +4143,8 @@ static int mg_vcycle(mycel_problem* p, cudaStream_t s, const MgRun& R) {
     xc[l] = x;
     nl += 1 + mg->sweeps;
   }
-  (nc == 1 ? k_mg_prolong<true, false> : k_mg_prolong<true, true>)<<<mg_blocks(mg_pairs(lv[0].d) * nc), 256, 0, s>>>(lv[0].d, g.rp, p->d_nflags, nullptr, mg_ptrs(R.xf, nc),
-                                                              lv[1].d, lv_ptrs(xc[1], lv[1].nd, nc), st, nc);
+  launch_mg_prolong<true>(s, lv[0].d, g.rp, p->d_nflags, nullptr, mg_ptrs(R.xf, nc), lv[1].d,
+                          lv_ptrs(xc[1], lv[1].nd, nc), st, nc);
   nl++;
   for (int q = 1; q < mg->sweeps; ++q)
     for (int k = 0; k < nc; ++k) {
@@ -5309,21 +5331,25 @@ struct PkProlong {  // prolongation of a problem's level to the next finer one (
   const float* invdf;
   MgPtrs xf, xc;
   const MixState* st;
+  bool pairs;  // a thread per pair (mg_by_pairs)
 };
 
 template <bool PAD, bool MULTI>
-__global__ void k_mg_prolong_pk(const PkProlong* __restrict__ tab,
-                                                       const unsigned* __restrict__ items,
-                                                       const unsigned* __restrict__ count) {
+__global__ void __launch_bounds__(kMgDofThreads) k_mg_prolong_pk(const PkProlong* __restrict__ tab,
+                                                                 const unsigned* __restrict__ items,
+                                                                 const unsigned* __restrict__ count) {
   const unsigned cnt = *count;
   for (unsigned w = blockIdx.x; w < cnt; w += gridDim.x) {
     const unsigned code = items[w];
     const PkProlong& a = tab[code >> kPkLbBits];
     int64_t q;
     int k;
-    mg_item_case<MULTI>((int64_t)(code & kPkLbMask) * blockDim.x + threadIdx.x, a.ncase, &q, &k);
-    if (q >= mg_pairs(a.f) || !mg_running(a.st ? a.st + k : nullptr)) continue;
-    mg_prolong_pair<PAD>(a.f, a.pitch, a.nf, a.invdf, a.xf.p[k], a.c, a.xc.p[k], q);
+    const int64_t cta = code & kPkLbMask;
+    mg_item_case<MULTI>(a.pairs ? cta * kMgDofThreads + threadIdx.x : cta * 64 + (threadIdx.x & 63), a.ncase, &q, &k);
+    if (q >= mg_pairs(a.f)) continue;
+    const MixState* st = a.st ? a.st + k : nullptr;
+    if (a.pairs) mg_prolong_pair<PAD, 3>(a.f, a.pitch, a.nf, a.invdf, a.xf.p[k], a.c, a.xc.p[k], q, 0, st);
+    else mg_prolong_pair<PAD, 1>(a.f, a.pitch, a.nf, a.invdf, a.xf.p[k], a.c, a.xc.p[k], q, mg_dof_comp(), st);
   }
 }
 
@@ -5542,7 +5568,7 @@ static int pk_resident(int kind, bool pad, bool multi) {
     case PK_PROLONG:
       e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(
           &o, pad ? (multi ? k_mg_prolong_pk<true, true> : k_mg_prolong_pk<true, false>)
-                  : (multi ? k_mg_prolong_pk<false, true> : k_mg_prolong_pk<false, false>), 256, 0);
+                  : (multi ? k_mg_prolong_pk<false, true> : k_mg_prolong_pk<false, false>), kMgDofThreads, 0);
       break;
     default: o = 1;
   }
@@ -5591,7 +5617,7 @@ static void pk_issue(const PackPlan& P, const PkLaunch& L, cudaStream_t s, int s
     case PK_PROLONG: {
       auto k = L.pad ? (L.multi ? k_mg_prolong_pk<true, true> : k_mg_prolong_pk<true, false>)
                      : (L.multi ? k_mg_prolong_pk<false, true> : k_mg_prolong_pk<false, false>);
-      k<<<g, 256, 0, s>>>((const PkProlong*)tab, it, cn);
+      k<<<g, kMgDofThreads, 0, s>>>((const PkProlong*)tab, it, cn);
       break;
     }
     case PK_TAIL: {  // one cluster per problem (not listed: a done problem's cluster returns at once)
@@ -5895,7 +5921,8 @@ static int32_t pk_build(mycel_ctx* c, PackWork* w, std::vector<PkUnit>& units, c
         a.st = q.st;
         a.ncase = q.nc;
         e.push_back(a);
-        nb.push_back(mg_blocks(mg_pairs(v.d) * q.nc));
+        e.back().pairs = mg_by_pairs(v.d, q.nc);
+        nb.push_back(mg_prolong_blocks(v.d, q.nc));
         es.push_back({const_cast<MixState*>(q.st), q.nc});
       }
       B.add(P.vcycle, PK_PROLONG, false, multi == 1, 0, e, nb, es);
@@ -5923,7 +5950,8 @@ static int32_t pk_build(mycel_ctx* c, PackWork* w, std::vector<PkUnit>& units, c
       a.st = q.st;
       a.ncase = q.nc;
       e.push_back(a);
-      nb.push_back(mg_blocks(mg_pairs(mg->lv[0].d) * q.nc));
+      e.back().pairs = mg_by_pairs(mg->lv[0].d, q.nc);
+      nb.push_back(mg_prolong_blocks(mg->lv[0].d, q.nc));
       es.push_back({const_cast<MixState*>(q.st), q.nc});
     }
     B.add(P.vcycle, PK_PROLONG, true, multi == 1, 0, e, nb, es);
