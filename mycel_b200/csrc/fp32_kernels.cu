@@ -29,6 +29,7 @@
 #include <cstring>
 #include <map>
 #include <mutex>
+#include <numeric>
 #include <string>
 #include <tuple>
 #include <type_traits>
@@ -775,6 +776,7 @@ __global__ void __launch_bounds__(FX * FY, 2) k_mv32f(GridDims g, const __grid_c
                                                       float* __restrict__ pnew, float* __restrict__ y,
                                                       const float* __restrict__ E, const uint8_t* __restrict__ nf,
                                                       int projected, MixState* st, double* part, int zseg, int* err) {
+  dep_begin();
   const MvArgs a{&op, &tm_a, &tm_b, pnew, y, E, nf, st, part, err, projected};
   mv32f_body<MODE>(g, a, zseg, blockIdx.x, blockIdx.y,
                    blockIdx.z, gridDim.x * gridDim.y * gridDim.z,
@@ -885,6 +887,7 @@ __global__ void __launch_bounds__(FX * FY, 2) k_mv64f(GridDims g, const __grid_c
                                                       double* __restrict__ pnew, double* __restrict__ y,
                                                       const double* __restrict__ E, const uint8_t* __restrict__ nf,
                                                       int projected, MixState* st, double* part, int zseg, int* err) {
+  dep_begin();
   extern __shared__ __align__(128) unsigned char fac_smem[];
   double* yb = reinterpret_cast<double*>(fac_smem + (size_t)FNST * kFac64StagePitch * (MODE == 1 ? 2 : 1));
   __shared__ __align__(8) unsigned long long full[FNST];
@@ -1405,7 +1408,8 @@ static void launch_mv64f(mycel_problem* p, cudaStream_t s, const double* xin, co
   }
   const dim3 grid((unsigned)((g.nx1 + FOX - 1) / FOX), (unsigned)((g.ny1 + FOY - 1) / FOY),
                   (unsigned)((g.nz1 + zs - 1) / zs));
-  k_mv64f<MODE><<<grid, dim3(FX, FY), fac64_smem_bytes(MODE), s>>>(g, p->hexop64, *ta, *tb, pnew, y, p->d_E,
+  launch_dep(dep_early(p), k_mv64f<MODE>, grid, dim3(FX, FY), fac64_smem_bytes(MODE), s,
+               g, p->hexop64, *ta, *tb, pnew, y, p->d_E,
                                                                      p->d_nflags, projected, st, part, zs, p->d_err);
 }
 
@@ -1446,8 +1450,8 @@ static void launch_mv32_variant(mycel_problem* p, cudaStream_t s, const float* x
       std::fprintf(stderr, "mycel: FP32 matvec input is not a mapped work vector\n");
       std::abort();
     }
-    k_mv32f<MODE><<<fac_grid(g, zs), dim3(FX, FY), fac_smem_bytes(MODE), s>>>(
-        g, p->hexop, *ta, *tb, pnew, y, p->d_Ef, p->d_nflags, projected, st, part, zs, p->d_err);
+    launch_dep(dep_early(p), k_mv32f<MODE>, fac_grid(g, zs), dim3(FX, FY), fac_smem_bytes(MODE), s,
+               g, p->hexop, *ta, *tb, pnew, y, p->d_Ef, p->d_nflags, projected, st, part, zs, p->d_err);
   }
 }
 
@@ -1580,6 +1584,7 @@ __global__ void __launch_bounds__(kT) k_xr64(int64_t n, double* __restrict__ x, 
                                              double* __restrict__ z, const double* __restrict__ p,
                                              const double* __restrict__ ap, const double* __restrict__ invd,
                                              MixState* st, double* part, int mode) {
+  dep_begin();
   constexpr int U = 4;
   double rr = 0.0, rz = 0.0;
   const int64_t n2 = n >> 1;
@@ -1632,6 +1637,7 @@ __global__ void __launch_bounds__(kT) k_xr32(int64_t n, float* __restrict__ x, f
                                              float* __restrict__ z, const float* __restrict__ p,
                                              const float* __restrict__ ap, const float* __restrict__ invd,
                                              MixState* st, double* part, int mode) {
+  dep_begin();
   if (mode == 0 && st->status != MIX_RUNNING) return;
   const float alpha = mode ? 0.f : (float)st->alpha;
   double rr = 0.0, rz = 0.0;
@@ -1844,6 +1850,7 @@ __global__ void __launch_bounds__(FX * FY, 2) k_mv32f_cases(GridDims g, const __
                                                             const __grid_constant__ CasesMv<MODE> v,
                                                             const float* __restrict__ E,
                                                             const uint8_t* __restrict__ nf, int zseg, int* err) {
+  dep_begin();
   const int c = blockIdx.z / v.tiles_z, bz = blockIdx.z % v.tiles_z;
   const MvArgs a{&op, &v.tm_a[c], &v.tm_b[MODE == 1 ? c : 0], v.pnew[c], v.y[c], E, nf,
                  v.st ? v.st + c : nullptr, v.part + (size_t)c * v.pitch, err, 1};
@@ -2192,6 +2199,7 @@ __global__ void __launch_bounds__(256) k_mg_apply_nodes(MgDims d, const float* _
                                                         const float* __restrict__ invd,
                                                         const __grid_constant__ MgPtrs y, int mode,
                                                         const float* __restrict__ om, const MixState* st, int ncase) {
+  dep_begin();
   const int64_t nn = mg_nn(d);
   int64_t n;
   int c;
@@ -2213,7 +2221,7 @@ template <bool MULTI>
 __device__ __forceinline__ void mg_apply_rows(const MgDims& d, int64_t t0, int ncase, const float* __restrict__ S,
                                               const MgPtrs& x, const MgPtrs& r, const float* __restrict__ invd,
                                               const MgPtrs& y, int mode, const float* __restrict__ om,
-                                              const MixState* st, float* xs) {
+                                              const MixState* st, float* xs, bool begin) {
   const int64_t nn = mg_nn(d), ns = mg_ns(d);
   const int nx1 = d.nx + 1, sxy = nx1 * (d.ny + 1);
   int64_t n, lo;
@@ -2224,6 +2232,21 @@ __device__ __forceinline__ void mg_apply_rows(const MgDims& d, int64_t t0, int n
   const bool valid = n < nn;
   const int R3 = MULTI ? 3 * (63 / ncase + 4) : 198;  // floats of a run: the items' nodes and one on either side
   const int64_t n3 = 3 * nn;
+  float sv[27][3];
+  const MgNode g(d, (int)n);
+  const int64_t q = 3 * n + ci;
+  if (valid) {
+    const float* own = S + 3 * ci * ns + n;
+    const float* tr = S + ci * ns;
+#pragma unroll
+    for (int nb = 0; nb < 27; ++nb) {
+      const float* s =
+          nb >= 13 ? own + (int64_t)(nb - 13) * 9 * ns : tr + (int64_t)(13 - nb) * 9 * ns + max(g.at(nb), 0);
+#pragma unroll
+      for (int k = 0; k < 3; ++k) sv[nb][k] = s[(nb >= 13 ? k : 3 * k) * ns];
+    }
+  }
+  if (begin) dep_begin();
   auto stage = [&](const float* src, int run, int row, int o) {
     const int64_t q = 3 * (lo - 1 + nx1 * (run % 3 - 1) + sxy * (run / 3 - 1)) + o;
     const bool in = q >= 0 && q < n3;
@@ -2240,23 +2263,10 @@ __device__ __forceinline__ void mg_apply_rows(const MgDims& d, int64_t t0, int n
     }
   }
   __pipeline_commit();
-  float sv[27][3];
   float rq = 0.f, iq = 0.f;
-  const MgNode g(d, (int)n);
-  const int64_t q = 3 * n + ci;
-  if (valid) {
-    const float* own = S + 3 * ci * ns + n;
-    const float* tr = S + ci * ns;
-#pragma unroll
-    for (int nb = 0; nb < 27; ++nb) {
-      const float* s = nb >= 13 ? own + (int64_t)(nb - 13) * 9 * ns : tr + (int64_t)(13 - nb) * 9 * ns + max(g.at(nb), 0);
-#pragma unroll
-      for (int k = 0; k < 3; ++k) sv[nb][k] = s[(nb >= 13 ? k : 3 * k) * ns];
-    }
-    if (mode != 0) {
-      rq = r.p[c][q];
-      iq = invd[q];
-    }
+  if (valid && mode != 0) {
+    rq = r.p[c][q];
+    iq = invd[q];
   }
   const float omega = mode == 1 ? *om : 0.0f;
   const bool run = valid && mg_running(st ? st + c : nullptr);
@@ -2289,8 +2299,9 @@ __global__ void __launch_bounds__(kMgDofThreads) k_mg_apply(MgDims d, const floa
                                                             int ncase) {
   if constexpr (SHARED) {
     __shared__ float xs[kRowStage];
-    mg_apply_rows<MULTI>(d, (int64_t)blockIdx.x * 64, ncase, S, x, r, invd, y, mode, om, st, xs);
+    mg_apply_rows<MULTI>(d, (int64_t)blockIdx.x * 64, ncase, S, x, r, invd, y, mode, om, st, xs, true);
   } else {
+    dep_begin();
     const int64_t nn = mg_nn(d);
     int64_t n;  // (node, case) pair, the case fastest
     int c;
@@ -2326,6 +2337,7 @@ __global__ void __launch_bounds__(256) k_mg_apply_nodes_tma(MgDims d, const __gr
                                                             const float* __restrict__ invd, float* __restrict__ y,
                                                             int mode, const float* __restrict__ om,
                                                             const MixState* st, int* err) {
+  dep_begin();
   extern __shared__ __align__(128) unsigned char s1_smem[];
   __shared__ __align__(8) unsigned long long full[kS1Stages];
   if (!mg_running(st)) return;  // one case: the same for every CTA
@@ -2523,6 +2535,7 @@ __global__ void __launch_bounds__(kMgDofThreads) k_mg_restrict(MgDims f, int pit
                                                                const __grid_constant__ MgPtrs rc, const MixState* st,
                                                                const __grid_constant__ MgPtrs xc, int first_sweep,
                                                                const float* __restrict__ om, int ncase) {
+  dep_begin();
   int64_t n;
   int k;
   mg_item_case<MULTI>(mg_dof_node(), ncase, &n, &k);
@@ -2609,6 +2622,7 @@ __global__ void __launch_bounds__(kMgDofThreads) k_mg_prolong(MgDims f, int pitc
                                                               const __grid_constant__ MgPtrs xf, MgDims c,
                                                               const __grid_constant__ MgPtrs xc, const MixState* st,
                                                               int ncase) {
+  dep_begin();
   int64_t n;
   int k;
   mg_item_case<MULTI>(PAIRS ? blockIdx.x * (int64_t)blockDim.x + threadIdx.x : mg_dof_node(), ncase, &n, &k);
@@ -2622,11 +2636,13 @@ static unsigned mg_prolong_blocks(const MgDims& f, int nc) {
   return mg_by_pairs(f, nc) ? (unsigned)((n + kMgDofThreads - 1) / kMgDofThreads) : mg_dof_blocks(n);
 }
 template <bool PAD>
-static void launch_mg_prolong(cudaStream_t s, const MgDims& f, int pitch, const uint8_t* nf, const float* invdf,
+static void launch_mg_prolong(bool early, cudaStream_t s, const MgDims& f, int pitch, const uint8_t* nf,
+                              const float* invdf,
                               const MgPtrs& xf, const MgDims& c, const MgPtrs& xc, const MixState* st, int nc) {
-  (mg_by_pairs(f, nc) ? (nc == 1 ? k_mg_prolong<PAD, false, true> : k_mg_prolong<PAD, true, true>)
-                      : (nc == 1 ? k_mg_prolong<PAD, false, false> : k_mg_prolong<PAD, true, false>))
-      <<<mg_prolong_blocks(f, nc), kMgDofThreads, 0, s>>>(f, pitch, nf, invdf, xf, c, xc, st, nc);
+  launch_dep(early, (mg_by_pairs(f, nc) ? (nc == 1 ? k_mg_prolong<PAD, false, true> : k_mg_prolong<PAD, true, true>)
+                      : (nc == 1 ? k_mg_prolong<PAD, false, false> : k_mg_prolong<PAD, true, false>)),
+             mg_prolong_blocks(f, nc), kMgDofThreads, 0, s,
+               f, pitch, nf, invdf, xf, c, xc, st, nc);
 }
 
 
@@ -2887,9 +2903,6 @@ __device__ __forceinline__ void mg_put_all(float* p, float v) {
 __device__ __forceinline__ void mg_tail_smem(const MgTail& tl, const float* __restrict__ om, const MixState* st,
                                              int ncase, int rank, float* sm) {
   const int tid = threadIdx.x, nth = blockDim.x, warp = tid >> 5, lane = tid & 31, nwarp = nth >> 5;
-  unsigned live = 0;
-  for (int k = 0; k < ncase; ++k) live |= mg_running(st ? st + k : nullptr) ? 1u << k : 0u;
-  if (!live) return;  // the same for every CTA of the cluster
   mg_cluster_arrive();  // remote stores wait until every CTA has started
   int* smi = reinterpret_cast<int*>(sm);
   const int T = tl.T, L = tl.L, nc = tl.nc;
@@ -2949,6 +2962,15 @@ __device__ __forceinline__ void mg_tail_smem(const MgTail& tl, const float* __re
       reinterpret_cast<float4*>(sm + v.ox)[q] = make_float4(0.f, 0.f, 0.f, 0.f);
       reinterpret_cast<float4*>(sm + v.ot)[q] = make_float4(0.f, 0.f, 0.f, 0.f);
     }
+  }
+  dep_begin();  // so far: stencils and places, which a solve leaves as they are
+  unsigned live = 0;
+  for (int k = 0; k < ncase; ++k) live |= mg_running(st ? st + k : nullptr) ? 1u << k : 0u;
+  if (!live) {  // the same for every CTA of the cluster
+    __pipeline_commit();
+    __pipeline_wait_prior(0);
+    mg_cluster_wait();
+    return;
   }
   bool started = false;
   for (int c0 = 0; c0 < ncase; c0 += tl.group) {
@@ -3131,10 +3153,13 @@ template <bool MULTI>
 __global__ void __launch_bounds__(kMgTailThreads)
     k_mg_tail(const __grid_constant__ MgTail tl, const float* __restrict__ om, const MixState* st, int ncase) {
   extern __shared__ __align__(16) float tail_smem[];
-  if (tl.group) mg_tail_smem(tl, om, st, ncase, (int)blockIdx.x, tail_smem);
-  else
+  if (tl.group) {
+    mg_tail_smem(tl, om, st, ncase, (int)blockIdx.x, tail_smem);
+  } else {
+    dep_begin();
     mg_tail_body<MULTI>(tl, om, st, ncase, blockIdx.x * (int64_t)blockDim.x + threadIdx.x,
                         (int64_t)gridDim.x * blockDim.x);
+  }
 }
 
 // Shared-memory layout of mg_tail_smem for the levels from T and up to ncase load cases: every level's stencil rows
@@ -3234,6 +3259,7 @@ __global__ void __launch_bounds__(kT) k_mg_enter(GridDims g, double* __restrict_
                                                  const float* __restrict__ invdf, float* __restrict__ rf,
                                                  float* __restrict__ xf, const float* __restrict__ om, MixState* st,
                                                  double* part, int mode) {
+  dep_begin();
   if (!mg_running(st)) return;
   const double alpha = st->alpha;
   const float omega = *om;
@@ -3318,6 +3344,7 @@ __global__ void __launch_bounds__(kT) k_mg_exit(GridDims g, const float* __restr
                                                 const double* __restrict__ r, const double* __restrict__ q,
                                                 double* __restrict__ z, const float* __restrict__ om, MixState* st,
                                                 double* part, int mode) {
+  dep_begin();
   if (!mg_running(st)) return;
   const float omega = *om;
   double zr = 0.0, zq = 0.0, rr = 0.0;
@@ -3419,6 +3446,7 @@ __global__ void __launch_bounds__(kT) k_mg_enter32(int64_t n, float* __restrict_
                                                    const float* __restrict__ p, const float* __restrict__ q,
                                                    const float* __restrict__ invd, float* __restrict__ xf,
                                                    const float* __restrict__ om, MixState* st, double* part, int mode) {
+  dep_begin();
   mg_enter32_body<U>(n, x, r, p, q, invd, xf, om, st, part, mode, blockIdx.x, gridDim.x);
 }
 
@@ -3472,6 +3500,7 @@ __global__ void __launch_bounds__(kT) k_mg_exit32(int64_t n, const float* __rest
                                                   float* __restrict__ z, const float* __restrict__ invd,
                                                   const float* __restrict__ q, const float* __restrict__ om,
                                                   MixState* st, double* part, int mode) {
+  dep_begin();
   mg_exit32_body<U>(n, r, tf, z, invd, q, om, st, part, mode, blockIdx.x, gridDim.x);
 }
 static bool outer_wide(const mycel_problem* p, int sb) { return sb <= 3 * p->ctx->num_sms; }
@@ -3640,6 +3669,7 @@ struct MgLevel {
   int64_t nn = 0, nd = 0;
   float *S = nullptr, *invd = nullptr, *xa = nullptr, *xb = nullptr, *r = nullptr, *t = nullptr;
   bool staged = false;  // products of one case by k_mg_apply_nodes_tma through tm_s
+  bool early = false;  // its kernels as early dependents (launch_dep)
   int64_t max_shared = 0;  // products of up to this many nodes x cases by CTAs that share x (mg_apply_rows)
   int* err = nullptr;   // the problem's bounded-wait error word
   CUtensorMap tm_s{};   // the stencil as a 2-D tensor [126 rows][ns nodes], boxes of [9][kS1Box]
@@ -3801,11 +3831,12 @@ static int32_t mg_ensure(mycel_problem* p, bool* available) {
     v.d = dims[l];
     v.nn = mg_nn(v.d);
     v.nd = 3 * v.nn;
+    v.max_shared = (int64_t)3 * p->ctx->num_sms * 64;
+    v.early = dep_early(p);
     if (l == 0) continue;
     v.S = (float*)alloc(sizeof(float) * 9 * kMgHalf * mg_ns(v.d));  // zeroed: the row padding stays 0
     v.invd = (float*)alloc(sizeof(float) * v.nd);
     v.err = p->d_err;
-    v.max_shared = (int64_t)3 * p->ctx->num_sms * 64;
     if (v.S && v.nn > kMgDofMaxNodes) {  // the levels whose products run a thread per node
       const PFN_cuTensorMapEncodeTiled encode = tensor_map_encoder();
       cuuint64_t dims[2] = {(cuuint64_t)mg_ns(v.d), (cuuint64_t)(9 * kMgHalf)};
@@ -3922,13 +3953,15 @@ static void launch_mg_tail(cudaStream_t s, MgHier* mg, const float* om, const Mi
   const MgTail& tl = mg->tail(nc);
   cfg.dynamicSmemBytes = (size_t)tl.smem;
   cfg.stream = s;
-  cudaLaunchAttribute at{};
-  at.id = cudaLaunchAttributeClusterDimension;
-  at.val.clusterDim.x = kMgTailCtas;
-  at.val.clusterDim.y = 1;
-  at.val.clusterDim.z = 1;
-  cfg.attrs = &at;
-  cfg.numAttrs = 1;
+  cudaLaunchAttribute at[2] = {};
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = kMgTailCtas;
+  at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = 1;
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // see dep_begin
+  at[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = mg->lv[0].early ? 2 : 1;
   if (nc == 1) cudaLaunchKernelEx(&cfg, k_mg_tail<false>, tl, om, st, nc);
   else cudaLaunchKernelEx(&cfg, k_mg_tail<true>, tl, om, st, nc);
 }
@@ -3943,15 +3976,16 @@ static MgPtrs lv_ptrs(float* base, int64_t nd, int n) {
 static void launch_mg_apply(cudaStream_t s, const MgLevel& v, const MgPtrs& x, const MgPtrs& r, const float* invd,
                             const MgPtrs& y, int mode, const float* om, const MixState* st, int nc) {
   if (v.nn * nc <= kMgDofMaxNodes)
-    (v.nn * nc <= v.max_shared ? (nc == 1 ? k_mg_apply<false, true> : k_mg_apply<true, true>)
-                               : (nc == 1 ? k_mg_apply<false, false> : k_mg_apply<true, false>))
-        <<<mg_dof_blocks(v.nn * nc), kMgDofThreads, 0, s>>>(v.d, v.S, x, r, invd, y, mode, om, st, nc);
+    launch_dep(v.early, (v.nn * nc <= v.max_shared ? (nc == 1 ? k_mg_apply<false, true> : k_mg_apply<true, true>)
+                               : (nc == 1 ? k_mg_apply<false, false> : k_mg_apply<true, false>)),
+               mg_dof_blocks(v.nn * nc), kMgDofThreads, 0, s,
+               v.d, v.S, x, r, invd, y, mode, om, st, nc);
   else if (nc == 1 && v.staged)
-    k_mg_apply_nodes_tma<<<(unsigned)((v.nn + kS1Nodes - 1) / kS1Nodes), 256, kS1Smem, s>>>(
-        v.d, v.tm_s, x.p[0], r.p[0], invd, y.p[0], mode, om, st, v.err);
+    launch_dep(v.early, k_mg_apply_nodes_tma, (unsigned)((v.nn + kS1Nodes - 1) / kS1Nodes), 256, kS1Smem, s,
+               v.d, v.tm_s, x.p[0], r.p[0], invd, y.p[0], mode, om, st, v.err);
   else
-    (nc == 1 ? k_mg_apply_nodes<false> : k_mg_apply_nodes<true>)<<<mg_blocks(v.nn * nc), 256, 0, s>>>(
-        v.d, v.S, x, r, invd, y, mode, om, st, nc);
+    launch_dep(v.early, (nc == 1 ? k_mg_apply_nodes<false> : k_mg_apply_nodes<true>), mg_blocks(v.nn * nc), 256, 0, s,
+               v.d, v.S, x, r, invd, y, mode, om, st, nc);
 }
 
 // Per case the input (MODE 0: x; 1: z, with the old direction), pnew and y of launch_mv32_variant, which runs them one
@@ -3983,7 +4017,8 @@ static int launch_mv32_cases(mycel_problem* p, cudaStream_t s, int n, float* con
       v.pitch = pitch;
       v.tiles_z = (int)grid.z;
       grid.z *= (unsigned)n;
-      k_mv32f_cases<MODE><<<grid, dim3(FX, FY), fac_smem_bytes(MODE), s>>>(p->g, p->hexop, v, p->d_Ef, p->d_nflags, zs,
+      launch_dep(dep_early(p), k_mv32f_cases<MODE>, grid, dim3(FX, FY), fac_smem_bytes(MODE), s,
+               p->g, p->hexop, v, p->d_Ef, p->d_nflags, zs,
                                                                            p->d_err);
       return 1;
     }
@@ -4100,7 +4135,9 @@ static int mg_vcycle(mycel_problem* p, cudaStream_t s, const MgRun& R) {
     }
   nl += launch_mv32_cases<0>(p, s, nc, R.xf, nullptr, nullptr, R.tf, st, R.pitch);
   // restriction to level 1, with level 1's first sweep (unless level 1 is the coarsest)
-  (nc == 1 ? k_mg_restrict<true, false> : k_mg_restrict<true, true>)<<<mg_dof_blocks(lv[1].nn * nc), kMgDofThreads, 0, s>>>(lv[0].d, g.rp, mg_ptrs(R.rf, nc), mg_ptrs(R.tf, nc),
+  launch_dep(lv[1].early, (nc == 1 ? k_mg_restrict<true, false> : k_mg_restrict<true, true>),
+             mg_dof_blocks(lv[1].nn * nc), kMgDofThreads, 0, s,
+               lv[0].d, g.rp, mg_ptrs(R.rf, nc), mg_ptrs(R.tf, nc),
                                                                lv[1].d, lv[1].invd, lv_ptrs(lv[1].r, lv[1].nd, nc), st,
                                                                lv_ptrs(lv[1].xa, lv[1].nd, nc), 1 < mg->L - 1 ? 1 : 0,
                                                                om + 1, nc);
@@ -4118,7 +4155,9 @@ static int mg_vcycle(mycel_problem* p, cudaStream_t s, const MgRun& R) {
     launch_mg_apply(s, v, lv_ptrs(x, v.nd, nc), r, v.invd, lv_ptrs(v.t, v.nd, nc), 2, om + l, st, nc);
     if (l == 1 && mg->l1_timing) cudaEventRecordWithFlags(mg->l1_timing[1], s, cudaEventRecordExternal);
     MgLevel& cv = lv[l + 1];
-    (nc == 1 ? k_mg_restrict<false, false> : k_mg_restrict<false, true>)<<<mg_dof_blocks(cv.nn * nc), kMgDofThreads, 0, s>>>(v.d, 0, lv_ptrs(nullptr, 0, nc),
+    launch_dep(cv.early, (nc == 1 ? k_mg_restrict<false, false> : k_mg_restrict<false, true>),
+               mg_dof_blocks(cv.nn * nc), kMgDofThreads, 0, s,
+               v.d, 0, lv_ptrs(nullptr, 0, nc),
                                                                lv_ptrs(v.t, v.nd, nc), cv.d, cv.invd,
                                                                lv_ptrs(cv.r, cv.nd, nc), st,
                                                                lv_ptrs(cv.xa, cv.nd, nc), l + 1 < mg->L - 1 ? 1 : 0,
@@ -4133,7 +4172,7 @@ static int mg_vcycle(mycel_problem* p, cudaStream_t s, const MgRun& R) {
     MgLevel& v = lv[l];
     float* x = xc[l];
     float* o = x == v.xa ? v.xb : v.xa;
-    launch_mg_prolong<false>(s, v.d, 0, nullptr, v.invd, lv_ptrs(x, v.nd, nc), lv[l + 1].d,
+    launch_mg_prolong<false>(v.early, s, v.d, 0, nullptr, v.invd, lv_ptrs(x, v.nd, nc), lv[l + 1].d,
                              lv_ptrs(xc[l + 1], lv[l + 1].nd, nc), st, nc);
     const MgPtrs r = lv_ptrs(v.r, v.nd, nc);
     for (int k = 0; k < mg->sweeps; ++k) {
@@ -4143,7 +4182,7 @@ static int mg_vcycle(mycel_problem* p, cudaStream_t s, const MgRun& R) {
     xc[l] = x;
     nl += 1 + mg->sweeps;
   }
-  launch_mg_prolong<true>(s, lv[0].d, g.rp, p->d_nflags, nullptr, mg_ptrs(R.xf, nc), lv[1].d,
+  launch_mg_prolong<true>(lv[0].early, s, lv[0].d, g.rp, p->d_nflags, nullptr, mg_ptrs(R.xf, nc), lv[1].d,
                           lv_ptrs(xc[1], lv[1].nd, nc), st, nc);
   nl++;
   for (int q = 1; q < mg->sweeps; ++q)
@@ -4171,23 +4210,24 @@ static int launch_mg_step(mycel_problem* p, cudaStream_t s, const void* pcur, in
   MgRun R;
   R.st = st;
   if (f64) {
-    (outer_wide(p, sb) ? k_mg_enter<8> : k_mg_enter<2>)<<<sb, kT, 0, s>>>(
-        p->g, p->g_x, p->g_r, (const double*)pcur, p->g_ap, p->d_invdf, p->f_r, p->f_p0, om, st, p->d_part2, mode);
+    launch_dep(dep_early(p), (outer_wide(p, sb) ? k_mg_enter<8> : k_mg_enter<2>), sb, kT, 0, s,
+               p->g, p->g_x, p->g_r, (const double*)pcur, p->g_ap, p->d_invdf, p->f_r, p->f_p0, om, st, p->d_part2,
+               mode);
     R.rf[0] = p->f_r;
     R.xf[0] = p->f_p0;
     R.tf[0] = p->f_ap;
     nl += 1 + mg_vcycle(p, s, R);
-    (outer_wide(p, sb) ? k_mg_exit<8> : k_mg_exit<2>)<<<sb, kT, 0, s>>>(
-        p->g, p->f_r, p->f_ap, p->f_p0, p->d_invdf, p->g_r, p->g_ap, p->g_z, om, st, p->d_part2, mode);
+    launch_dep(dep_early(p), (outer_wide(p, sb) ? k_mg_exit<8> : k_mg_exit<2>), sb, kT, 0, s,
+               p->g, p->f_r, p->f_ap, p->f_p0, p->d_invdf, p->g_r, p->g_ap, p->g_z, om, st, p->d_part2, mode);
   } else {
-    (outer_wide(p, sb) ? k_mg_enter32<4> : k_mg_enter32<1>)<<<sb, kT, 0, s>>>(
-        p->g.n32, p->f_x, p->f_r, (const float*)pcur, p->f_ap, p->d_invdf, p->f_z, om, st, p->d_part2, mode);
+    launch_dep(dep_early(p), (outer_wide(p, sb) ? k_mg_enter32<4> : k_mg_enter32<1>), sb, kT, 0, s,
+               p->g.n32, p->f_x, p->f_r, (const float*)pcur, p->f_ap, p->d_invdf, p->f_z, om, st, p->d_part2, mode);
     R.rf[0] = p->f_r;
     R.xf[0] = p->f_z;
     R.tf[0] = mg->f_t;
     nl += 1 + mg_vcycle(p, s, R);
-    (outer_wide(p, sb) ? k_mg_exit32<4> : k_mg_exit32<1>)<<<sb, kT, 0, s>>>(
-        p->g.n32, p->f_r, mg->f_t, p->f_z, p->d_invdf, p->f_ap, om, st, p->d_part2, mode);
+    launch_dep(dep_early(p), (outer_wide(p, sb) ? k_mg_exit32<4> : k_mg_exit32<1>), sb, kT, 0, s,
+               p->g.n32, p->f_r, mg->f_t, p->f_z, p->d_invdf, p->f_ap, om, st, p->d_part2, mode);
   }
   return nl + 1;
 }
@@ -4245,10 +4285,12 @@ static int launch_inner_xr(mycel_problem* p, const InnerForm& F, cudaStream_t s,
   const int sb = stream_blocks(p);
   if (F.mg) return launch_mg_step(p, s, pcur, mode, F.f64);
   if (F.f64)
-    k_xr64<<<sb, kT, 0, s>>>(F.n, (double*)F.x, (double*)F.r, (double*)F.z, (const double*)pcur, (const double*)F.ap,
+    launch_dep(dep_early(p), k_xr64, sb, kT, 0, s,
+               F.n, (double*)F.x, (double*)F.r, (double*)F.z, (const double*)pcur, (const double*)F.ap,
                              (const double*)F.invd, mix_state(p), p->d_part2, mode);
   else
-    k_xr32<<<sb, kT, 0, s>>>(F.n, (float*)F.x, (float*)F.r, (float*)F.z, (const float*)pcur, (const float*)F.ap,
+    launch_dep(dep_early(p), k_xr32, sb, kT, 0, s,
+               F.n, (float*)F.x, (float*)F.r, (float*)F.z, (const float*)pcur, (const float*)F.ap,
                              (const float*)F.invd, mix_state(p), p->d_part2, mode);
   return 1;
 }
@@ -4699,6 +4741,7 @@ template <int U>
 __global__ void __launch_bounds__(kT) k_mg_enter32_cases(int64_t n, const __grid_constant__ CasesVec v,
                                                          const float* __restrict__ invd, const float* __restrict__ om,
                                                          MixState* st, double* part, int pitch, int mode) {
+  dep_begin();
   const int c = blockIdx.y;
   mg_enter32_body<U>(n, v.x[c], v.r[c], v.p[c], v.q[c], invd, v.z[c], om, st + c, part + (size_t)c * pitch, mode,
                      blockIdx.x, gridDim.x);
@@ -4707,6 +4750,7 @@ template <int U>
 __global__ void __launch_bounds__(kT) k_mg_exit32_cases(int64_t n, const __grid_constant__ CasesVec v,
                                                         const float* __restrict__ invd, const float* __restrict__ om,
                                                         MixState* st, double* part, int pitch, int mode) {
+  dep_begin();
   const int c = blockIdx.y;
   mg_exit32_body<U>(n, v.r[c], v.t[c], v.z[c], invd, v.q[c], om, st + c, part + (size_t)c * pitch, mode, blockIdx.x,
                     gridDim.x);
@@ -4746,12 +4790,12 @@ static int launch_mg_step_cases(mycel_problem* p, cudaStream_t s, int n, const i
     return w;
   };
   for (int k = 0; k < n; k += m, ++nl)
-    (wide ? k_mg_enter32_cases<4> : k_mg_enter32_cases<1>)<<<dim3(sb, m), kT, 0, s>>>(
-        p->g.n32, from(k), p->d_invdf, om, R.st + k, p->d_part2, pitch, mode);
+    launch_dep(dep_early(p), (wide ? k_mg_enter32_cases<4> : k_mg_enter32_cases<1>), dim3(sb, m), kT, 0, s,
+               p->g.n32, from(k), p->d_invdf, om, R.st + k, p->d_part2, pitch, mode);
   nl += mg_vcycle(p, s, R);
   for (int k = 0; k < n; k += m, ++nl)
-    (wide ? k_mg_exit32_cases<4> : k_mg_exit32_cases<1>)<<<dim3(sb, m), kT, 0, s>>>(
-        p->g.n32, from(k), p->d_invdf, om, R.st + k, p->d_part2, pitch, mode);
+    launch_dep(dep_early(p), (wide ? k_mg_exit32_cases<4> : k_mg_exit32_cases<1>), dim3(sb, m), kT, 0, s,
+               p->g.n32, from(k), p->d_invdf, om, R.st + k, p->d_part2, pitch, mode);
   return nl;
 }
 
@@ -5198,6 +5242,7 @@ struct alignas(64) PkMv {  // one FP32 matvec (k_mv32f) of a right-hand side
 template <int MODE>
 __global__ void __launch_bounds__(FX * FY, 2) k_mv32f_pk(const PkMv* __restrict__ tab, const unsigned* __restrict__ items,
                                                          const unsigned* __restrict__ count) {
+  dep_begin();
   const unsigned cnt = *count;
   for (unsigned w = blockIdx.x; w < cnt; w += gridDim.x) {
     __syncthreads();  // the previous tile is done with the shared memory
@@ -5234,6 +5279,7 @@ struct PkVec {  // k_mg_enter32 / k_mg_exit32 of a right-hand side
 
 __global__ void __launch_bounds__(kT, 2) k_mg_enter32_pk(const PkVec* __restrict__ tab, const unsigned* __restrict__ items,
                                                       const unsigned* __restrict__ count, int mode) {
+  dep_begin();
   const unsigned cnt = *count;
   for (unsigned w = blockIdx.x; w < cnt; w += gridDim.x) {
     __syncthreads();
@@ -5246,6 +5292,7 @@ __global__ void __launch_bounds__(kT, 2) k_mg_enter32_pk(const PkVec* __restrict
 
 __global__ void __launch_bounds__(kT, 2) k_mg_exit32_pk(const PkVec* __restrict__ tab, const unsigned* __restrict__ items,
                                                      const unsigned* __restrict__ count, int mode) {
+  dep_begin();
   const unsigned cnt = *count;
   for (unsigned w = blockIdx.x; w < cnt; w += gridDim.x) {
     __syncthreads();
@@ -5270,6 +5317,7 @@ template <bool MULTI>
 __global__ void __launch_bounds__(256) k_mg_apply_nodes_pk(const PkApply* __restrict__ tab,
                                                            const unsigned* __restrict__ items,
                                                            const unsigned* __restrict__ count, int mode) {
+  dep_begin();
   const unsigned cnt = *count;
   for (unsigned w = blockIdx.x; w < cnt; w += gridDim.x) {
     const unsigned code = items[w];
@@ -5287,13 +5335,14 @@ template <bool MULTI>
 __global__ void __launch_bounds__(kMgDofThreads) k_mg_apply_pk(const PkApply* __restrict__ tab,
                                                                const unsigned* __restrict__ items,
                                                                const unsigned* __restrict__ count, int mode) {
+  dep_begin();
   __shared__ float xs[kRowStage];
   const unsigned cnt = *count;
   for (unsigned w = blockIdx.x; w < cnt; w += gridDim.x) {
     const unsigned code = items[w];
     const PkApply& a = tab[code >> kPkLbBits];
     mg_apply_rows<MULTI>(a.d, (int64_t)(code & kPkLbMask) * 64, a.ncase, a.S, a.x, a.r, a.invd, a.y, mode, a.om, a.st,
-                         xs);
+                         xs, false);
     __syncthreads();  // xs is the next item's
   }
 }
@@ -5311,6 +5360,7 @@ template <bool PAD, bool MULTI>
 __global__ void __launch_bounds__(kMgDofThreads) k_mg_restrict_pk(const PkRestrict* __restrict__ tab,
                                                                   const unsigned* __restrict__ items,
                                                                   const unsigned* __restrict__ count) {
+  dep_begin();
   const unsigned cnt = *count;
   for (unsigned w = blockIdx.x; w < cnt; w += gridDim.x) {
     const unsigned code = items[w];
@@ -5338,6 +5388,7 @@ template <bool PAD, bool MULTI>
 __global__ void __launch_bounds__(kMgDofThreads) k_mg_prolong_pk(const PkProlong* __restrict__ tab,
                                                                  const unsigned* __restrict__ items,
                                                                  const unsigned* __restrict__ count) {
+  dep_begin();
   const unsigned cnt = *count;
   for (unsigned w = blockIdx.x; w < cnt; w += gridDim.x) {
     const unsigned code = items[w];
@@ -5364,10 +5415,13 @@ template <bool MULTI>
 __global__ void __launch_bounds__(kMgTailThreads) k_mg_tail_pk(const PkTail* __restrict__ tab) {
   extern __shared__ __align__(16) float tail_smem[];
   const PkTail& t = tab[blockIdx.x / kMgTailCtas];
-  if (t.tl.group) mg_tail_smem(t.tl, t.om, t.st, t.ncase, (int)(blockIdx.x % kMgTailCtas), tail_smem);
-  else
+  if (t.tl.group) {
+    mg_tail_smem(t.tl, t.om, t.st, t.ncase, (int)(blockIdx.x % kMgTailCtas), tail_smem);
+  } else {
+    dep_begin();
     mg_tail_body<MULTI>(t.tl, t.om, t.st, t.ncase, (int64_t)(blockIdx.x % kMgTailCtas) * blockDim.x + threadIdx.x,
-                      (int64_t)kMgTailCtas * blockDim.x);
+                        (int64_t)kMgTailCtas * blockDim.x);
+  }
 }
 static const void* mg_tail_pk_kernel(bool multi) {
   return multi ? (const void*)k_mg_tail_pk<true> : (const void*)k_mg_tail_pk<false>;
@@ -5462,6 +5516,7 @@ struct PackPlan {
   int n_iter[2] = {0, 0}, n_step = 0;
   cudaGraphExec_t chunk = nullptr;
   int per_chunk = 0;
+  bool early = false;           // its kernels as early dependents (launch_dep): the units together are small
 };
 
 // packed-solve workspace of a context: the plan of the latest set of right-hand sides and pinned host slots
@@ -5589,35 +5644,43 @@ static void pk_issue(const PackPlan& P, const PkLaunch& L, cudaStream_t s, int s
   const unsigned g = L.grid;
   switch (L.kind) {
     case PK_MV0:
-      k_mv32f_pk<0><<<g, dim3(FX, FY), fac_smem_bytes(0), s>>>((const PkMv*)tab, it, cn);
+      launch_dep(P.early, k_mv32f_pk<0>, g, dim3(FX, FY), fac_smem_bytes(0), s,
+               (const PkMv*)tab, it, cn);
       break;
     case PK_MV1:
-      k_mv32f_pk<1><<<g, dim3(FX, FY), fac_smem_bytes(1), s>>>((const PkMv*)tab, it, cn);
+      launch_dep(P.early, k_mv32f_pk<1>, g, dim3(FX, FY), fac_smem_bytes(1), s,
+               (const PkMv*)tab, it, cn);
       break;
     case PK_ENTER:
-      k_mg_enter32_pk<<<g, kT, 0, s>>>((const PkVec*)tab, it, cn, step_mode);
+      launch_dep(P.early, k_mg_enter32_pk, g, kT, 0, s,
+               (const PkVec*)tab, it, cn, step_mode);
       break;
     case PK_EXIT:
-      k_mg_exit32_pk<<<g, kT, 0, s>>>((const PkVec*)tab, it, cn, step_mode);
+      launch_dep(P.early, k_mg_exit32_pk, g, kT, 0, s,
+               (const PkVec*)tab, it, cn, step_mode);
       break;
     case PK_APPLY_DOF:
-      (L.multi ? k_mg_apply_pk<true> : k_mg_apply_pk<false>)<<<g, kMgDofThreads, 0, s>>>((const PkApply*)tab, it, cn,
+      launch_dep(P.early, (L.multi ? k_mg_apply_pk<true> : k_mg_apply_pk<false>), g, kMgDofThreads, 0, s,
+               (const PkApply*)tab, it, cn,
                                                                                          L.mode);
       break;
     case PK_APPLY_NODE:
-      (L.multi ? k_mg_apply_nodes_pk<true> : k_mg_apply_nodes_pk<false>)<<<g, 256, 0, s>>>((const PkApply*)tab, it,
+      launch_dep(P.early, (L.multi ? k_mg_apply_nodes_pk<true> : k_mg_apply_nodes_pk<false>), g, 256, 0, s,
+               (const PkApply*)tab, it,
                                                                                            cn, L.mode);
       break;
     case PK_RESTRICT: {
       auto k = L.pad ? (L.multi ? k_mg_restrict_pk<true, true> : k_mg_restrict_pk<true, false>)
                      : (L.multi ? k_mg_restrict_pk<false, true> : k_mg_restrict_pk<false, false>);
-      k<<<g, kMgDofThreads, 0, s>>>((const PkRestrict*)tab, it, cn);
+      launch_dep(P.early, k, g, kMgDofThreads, 0, s,
+               (const PkRestrict*)tab, it, cn);
       break;
     }
     case PK_PROLONG: {
       auto k = L.pad ? (L.multi ? k_mg_prolong_pk<true, true> : k_mg_prolong_pk<true, false>)
                      : (L.multi ? k_mg_prolong_pk<false, true> : k_mg_prolong_pk<false, false>);
-      k<<<g, kMgDofThreads, 0, s>>>((const PkProlong*)tab, it, cn);
+      launch_dep(P.early, k, g, kMgDofThreads, 0, s,
+               (const PkProlong*)tab, it, cn);
       break;
     }
     case PK_TAIL: {  // one cluster per problem (not listed: a done problem's cluster returns at once)
@@ -5626,13 +5689,15 @@ static void pk_issue(const PackPlan& P, const PkLaunch& L, cudaStream_t s, int s
       cfg.blockDim = dim3(kMgTailThreads);
       cfg.dynamicSmemBytes = L.smem;
       cfg.stream = s;
-      cudaLaunchAttribute at{};
-      at.id = cudaLaunchAttributeClusterDimension;
-      at.val.clusterDim.x = kMgTailCtas;
-      at.val.clusterDim.y = 1;
-      at.val.clusterDim.z = 1;
-      cfg.attrs = &at;
-      cfg.numAttrs = 1;
+      cudaLaunchAttribute at[2] = {};
+      at[0].id = cudaLaunchAttributeClusterDimension;
+      at[0].val.clusterDim.x = kMgTailCtas;
+      at[0].val.clusterDim.y = 1;
+      at[0].val.clusterDim.z = 1;
+      at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // see dep_begin
+      at[1].val.programmaticStreamSerializationAllowed = 1;
+      cfg.attrs = at;
+      cfg.numAttrs = P.early ? 2 : 1;
       if (L.multi) cudaLaunchKernelEx(&cfg, k_mg_tail_pk<true>, (const PkTail*)tab);
       else cudaLaunchKernelEx(&cfg, k_mg_tail_pk<false>, (const PkTail*)tab);
       break;
@@ -5748,6 +5813,8 @@ static int32_t pk_build(mycel_ctx* c, PackWork* w, std::vector<PkUnit>& units, c
       nb.push_back(v.nb);
       es.push_back({u.st, 1});
     }
+    const int64_t all = std::accumulate(nb.begin(), nb.end(), int64_t{0});
+    P.early = !units.empty() && all <= units[0].p->ctx->num_sms;
     B.add(P.enter[sel], PK_ENTER, false, false, 0, e, nb, es);
     if (sel == 0) B.add(P.exitl, PK_EXIT, false, false, 0, e, nb, es);
   }

@@ -274,6 +274,21 @@ __global__ void __launch_bounds__(kMvNodes, 4) k_matvec64(GridDims g, const __gr
   const int n0 = (int)(blockIdx.x - (unsigned)k * chunks) * kMvNodes;
   const MvStage m = mv_stage(g.nx1);
   const int half = 3 * m.nseg * m.segstep;
+  const int nl = n0 + tid, n = nl < np ? nl : np - 1;
+  const int j = n / g.nx1, i = n - j * g.nx1;
+  const bool mine = nl < np;
+  // the node's elements (i-1+sx, j-1+sy, k-1+sz): E and whether they contribute
+  double ee[8];
+  unsigned act = 0;
+#pragma unroll
+  for (int v = 0; v < 8; ++v) {
+    const int ex = i - 1 + (v & 1), ey = j - 1 + ((v >> 1) & 1), ez = k - 1 + (v >> 2);
+    const bool in = mine && ex >= 0 && ex < g.nx && ey >= 0 && ey < g.ny && ez >= 0 && ez < g.nz;
+    const int64_t e = ex + (int64_t)g.nx * (ey + (int64_t)g.ny * ez);
+    if (in && dom[e]) act |= 1u << v;
+    ee[v] = in ? E[e] : 0.0;
+  }
+  dep_begin();
   const int status = st ? st->status : PCG_RUNNING;
   const double beta = FUSE ? st->beta : 0.0;
   const bool first = FUSE ? st->first != 0 : false;
@@ -305,20 +320,6 @@ __global__ void __launch_bounds__(kMvNodes, 4) k_matvec64(GridDims g, const __gr
     }
   }
   __pipeline_commit();
-  const int nl = n0 + tid, n = nl < np ? nl : np - 1;
-  const int j = n / g.nx1, i = n - j * g.nx1;
-  const bool mine = nl < np;
-  // the node's elements (i-1+sx, j-1+sy, k-1+sz): E and whether they contribute
-  double ee[8];
-  unsigned act = 0;
-#pragma unroll
-  for (int v = 0; v < 8; ++v) {
-    const int ex = i - 1 + (v & 1), ey = j - 1 + ((v >> 1) & 1), ez = k - 1 + (v >> 2);
-    const bool in = mine && ex >= 0 && ex < g.nx && ey >= 0 && ey < g.ny && ez >= 0 && ez < g.nz;
-    const int64_t e = ex + (int64_t)g.nx * (ey + (int64_t)g.ny * ez);
-    if (in && dom[e]) act |= 1u << v;
-    ee[v] = in ? E[e] : 0.0;
-  }
   __pipeline_wait_prior(0);
   __syncthreads();
   if (status != PCG_RUNNING) return;
@@ -426,8 +427,10 @@ static void launch_mv(mycel_problem* p, const double* x, const double* pold, dou
   const GridDims& g = p->g;
   const unsigned chunks = (unsigned)(((int64_t)g.nx1 * g.ny1 + kMvNodes - 1) / kMvNodes);
   allow_smem<k_matvec64<FUSE>>(p->ctx->device, std::max(mv_smem(kMvNodes + 2, FUSE != 0), mv_smem(kMvNodes + 3, FUSE != 0)));
-  k_matvec64<FUSE><<<chunks * (unsigned)g.nz1, kMvNodes, mv_smem(g.nx1, FUSE != 0), p->ctx->stream>>>(
-      g, p->ke, x, pold, pnew, y, p->d_E, p->d_domain, p->d_nflags, projected, st, chunks);
+  // in the iteration an early dependent; E and the domain, which its first loads read, are older than the solve
+  launch_dep(FUSE != 0 && dep_early(p), k_matvec64<FUSE>, chunks * (unsigned)g.nz1, kMvNodes,
+             mv_smem(g.nx1, FUSE != 0), p->ctx->stream, g, p->ke, x, pold, pnew, y, p->d_E, p->d_domain, p->d_nflags,
+             projected, st, chunks);
   p->ctx->launches++;
 }
 
@@ -582,6 +585,7 @@ enum DotPhase : int { PH_PAP = 0, PH_INIT_RR = 1 };
 __global__ void __launch_bounds__(chain_threads(1), 4) k_dot_exact(const double* __restrict__ a, const double* __restrict__ b,
                                                              int64_t n, double* part, PcgState* st, int phase) {
   __shared__ __align__(16) double buf[kRing][1][4][kRow];
+  dep_begin();
   const int64_t start = (int64_t)blockIdx.x * kBlock;
   const int cnt = (int)min((int64_t)kBlock, n - start);
   const int vc4 = cnt & ~3;
@@ -647,6 +651,7 @@ __global__ void __launch_bounds__(chain_threads(2), 3) k_xr_exact(double* __rest
   extern __shared__ __align__(16) double xr_buf[];
   auto buf = reinterpret_cast<double (*)[2][4][kRow]>(xr_buf);  // sets: r.r (not used at a start), r.z
   __shared__ double rz_sum;
+  dep_begin();
   const int64_t start = (int64_t)blockIdx.x * kBlock;
   const int cnt = (int)min((int64_t)kBlock, n - start);
   const int vc4 = cnt & ~3;
@@ -756,8 +761,8 @@ __global__ void __launch_bounds__(chain_threads(2), 3) k_xr_exact(double* __rest
 }
 
 static void launch_dot(mycel_problem* p, const double* a, const double* b, int phase) {
-  k_dot_exact<<<(unsigned)num_blocks8192(p->g.nd), chain_threads(1), 0, p->ctx->stream>>>(a, b, p->g.nd, p->d_part,
-                                                                                          p->d_state, phase);
+  launch_dep(dep_early(p), k_dot_exact, (unsigned)num_blocks8192(p->g.nd), chain_threads(1), 0, p->ctx->stream, a, b,
+             p->g.nd, p->d_part, p->d_state, phase);
   p->ctx->launches++;
 }
 
@@ -765,8 +770,8 @@ template <int INIT>
 static void launch_xr(mycel_problem* p, const double* dir) {
   constexpr size_t smem = sizeof(double) * kRing * 2 * 4 * kRow;
   allow_smem<k_xr_exact<INIT>>(p->ctx->device, smem);
-  k_xr_exact<INIT><<<(unsigned)num_blocks8192(p->g.nd), chain_threads(2), smem, p->ctx->stream>>>(
-      p->d_x, p->d_r, p->d_z, dir, p->d_ap, p->d_invd, p->g.nd, p->d_part, p->d_state);
+  launch_dep(dep_early(p), k_xr_exact<INIT>, (unsigned)num_blocks8192(p->g.nd), chain_threads(2), smem,
+             p->ctx->stream, p->d_x, p->d_r, p->d_z, dir, p->d_ap, p->d_invd, p->g.nd, p->d_part, p->d_state);
   p->ctx->launches++;
 }
 
