@@ -1581,8 +1581,8 @@ __device__ __forceinline__ void xr_tail(double rr, double rz, MixState* st, doub
 // few hundred thousand nodes (a thread takes 8 pairs, whatever the size, up to 8 CTAs an SM): the loads of 4 pairs
 // go out together, the first before the state is looked at. 58 thousand nodes: 11.5 us -> 8.1 us.
 __global__ void __launch_bounds__(kT) k_xr64(int64_t n, double* __restrict__ x, double* __restrict__ r,
-                                             double* __restrict__ z, const double* __restrict__ p,
-                                             const double* __restrict__ ap, const double* __restrict__ invd,
+                                             double* __restrict__ z, const double* p,
+                                             const double* ap, const double* __restrict__ invd,
                                              MixState* st, double* part, int mode) {
   dep_begin();
   constexpr int U = 4;
@@ -1634,8 +1634,8 @@ __global__ void __launch_bounds__(kT) k_xr64(int64_t n, double* __restrict__ x, 
 // x += alpha p, r -= alpha Ap, z = r invD; partials of r.r and r.z (FP64). mode 0: CG step; 1: residual
 // replacement (z, rho from the new r; beta = rho_new / rho_old); 2: start (z, rho; next step starts p = z).
 __global__ void __launch_bounds__(kT) k_xr32(int64_t n, float* __restrict__ x, float* __restrict__ r,
-                                             float* __restrict__ z, const float* __restrict__ p,
-                                             const float* __restrict__ ap, const float* __restrict__ invd,
+                                             float* __restrict__ z, const float* p,
+                                             const float* ap, const float* __restrict__ invd,
                                              MixState* st, double* part, int mode) {
   dep_begin();
   if (mode == 0 && st->status != MIX_RUNNING) return;
@@ -2119,7 +2119,7 @@ struct MgNode {
 // Later neighbours' blocks are n's own (row ci at entries 3 ci + cj), earlier ones the transposed blocks stored at
 // the neighbour (row ci at entries 3 cj + ci).
 __device__ __forceinline__ void mg_apply_node(const MgDims& d, int64_t ns, int n, const float* __restrict__ S,
-                                              const float* __restrict__ x, const float* __restrict__ r,
+                                              const float* x, const float* r,
                                               const float* __restrict__ invd, float* __restrict__ y, int mode,
                                               float omega) {
   const MgNode g(d, n);
@@ -2158,8 +2158,8 @@ __device__ __forceinline__ void mg_apply_node(const MgDims& d, int64_t ns, int n
 
 // the same for one row (DOF ci of node n): a third of the loads of a node
 __device__ __forceinline__ void mg_apply_row(const MgDims& d, int64_t ns, int n, int ci,
-                                             const float* __restrict__ S, const float* __restrict__ x,
-                                             const float* __restrict__ r, const float* __restrict__ invd,
+                                             const float* __restrict__ S, const float* x,
+                                             const float* r, const float* __restrict__ invd,
                                              float* __restrict__ y, int mode, float omega) {
   const MgNode g(d, n);
   const float* own = S + 3 * ci * ns + n;
@@ -2465,8 +2465,8 @@ struct MgAxis {
 // threads for the same loads. B200, us (coarse nodes): 512 4.8 -> 2.7, 18,490 voxel-level 6.3 -> 3.9, 233,000 voxel-level
 // 19.6 -> 18.9.
 template <bool PAD>
-__device__ __forceinline__ void mg_restrict_row(const MgDims& f, int pitch, const float* __restrict__ rf,
-                                                const float* __restrict__ tf, const MgDims& c,
+__device__ __forceinline__ void mg_restrict_row(const MgDims& f, int pitch, const float* rf,
+                                                const float* tf, const MgDims& c,
                                                 const float* __restrict__ invdc, float* __restrict__ rc, int64_t n,
                                                 int cc, float* __restrict__ xc, float omega, const MixState* st) {
   int I, J, K;
@@ -2559,7 +2559,7 @@ constexpr int64_t kMgPairMax = 262144;
 template <bool PAD, int N>
 __device__ __forceinline__ void mg_prolong_pair(const MgDims& f, int pitch, const uint8_t* __restrict__ nf,
                                                 const float* __restrict__ invdf, float* __restrict__ xf,
-                                                const MgDims& c, const float* __restrict__ xc, int64_t item, int cc,
+                                                const MgDims& c, const float* xc, int64_t item, int cc,
                                                 const MixState* st) {
   int ci, j, k;
   mg_ijk(item, (f.nx + 2) >> 1, f.ny + 1, &ci, &j, &k);
@@ -3255,7 +3255,7 @@ struct RowWalk {
 // 110x22x22: k_mg_enter 14.5 us -> 8.3 us, k_mg_exit 15.0 us -> 7.2 us.
 template <int U>
 __global__ void __launch_bounds__(kT) k_mg_enter(GridDims g, double* __restrict__ x, double* __restrict__ r,
-                                                 const double* __restrict__ p, const double* __restrict__ q,
+                                                 const double* p, const double* q,
                                                  const float* __restrict__ invdf, float* __restrict__ rf,
                                                  float* __restrict__ xf, const float* __restrict__ om, MixState* st,
                                                  double* part, int mode) {
@@ -3339,9 +3339,9 @@ __device__ __forceinline__ void mg_exit_tail(double zr, double zq, double rr, Mi
 // Outer step, part 2: the voxel level's last Jacobi sweep written as the FP64 preconditioned residual
 // z = xf + omega invd (rf - tf) (tf = A xf), then (z, r), (z, A p) and (r, r) (mg_exit_tail).
 template <int U>
-__global__ void __launch_bounds__(kT) k_mg_exit(GridDims g, const float* __restrict__ rf, const float* __restrict__ tf,
-                                                const float* __restrict__ xf, const float* __restrict__ invdf,
-                                                const double* __restrict__ r, const double* __restrict__ q,
+__global__ void __launch_bounds__(kT) k_mg_exit(GridDims g, const float* rf, const float* tf,
+                                                const float* xf, const float* __restrict__ invdf,
+                                                const double* r, const double* q,
                                                 double* __restrict__ z, const float* __restrict__ om, MixState* st,
                                                 double* part, int mode) {
   dep_begin();
@@ -3390,7 +3390,7 @@ __global__ void __launch_bounds__(kT) k_mg_exit(GridDims g, const float* __restr
 // 30.9 us, 29.4 us -> 25.0 us.
 template <int U>
 __device__ __forceinline__ void mg_enter32_body(int64_t n, float* __restrict__ x, float* __restrict__ r,
-                                                const float* __restrict__ p, const float* __restrict__ q,
+                                                const float* p, const float* q,
                                                 const float* __restrict__ invd, float* __restrict__ xf,
                                                 const float* __restrict__ om, MixState* st, double* part, int mode,
                                                 unsigned bx, unsigned nb) {
@@ -3443,7 +3443,7 @@ __device__ __forceinline__ void mg_enter32_body(int64_t n, float* __restrict__ x
 
 template <int U>
 __global__ void __launch_bounds__(kT) k_mg_enter32(int64_t n, float* __restrict__ x, float* __restrict__ r,
-                                                   const float* __restrict__ p, const float* __restrict__ q,
+                                                   const float* p, const float* q,
                                                    const float* __restrict__ invd, float* __restrict__ xf,
                                                    const float* __restrict__ om, MixState* st, double* part, int mode) {
   dep_begin();
@@ -3451,9 +3451,9 @@ __global__ void __launch_bounds__(kT) k_mg_enter32(int64_t n, float* __restrict_
 }
 
 template <int U>
-__device__ __forceinline__ void mg_exit32_body(int64_t n, const float* __restrict__ r, const float* __restrict__ tf,
+__device__ __forceinline__ void mg_exit32_body(int64_t n, const float* r, const float* tf,
                                                float* __restrict__ z, const float* __restrict__ invd,
-                                               const float* __restrict__ q, const float* __restrict__ om,
+                                               const float* q, const float* __restrict__ om,
                                                MixState* st, double* part, int mode, unsigned bx, unsigned nb) {
   double zr = 0.0, zq = 0.0, rr = 0.0;
   const int64_t n4 = n >> 2;
@@ -3496,9 +3496,9 @@ __device__ __forceinline__ void mg_exit32_body(int64_t n, const float* __restric
 }
 
 template <int U>
-__global__ void __launch_bounds__(kT) k_mg_exit32(int64_t n, const float* __restrict__ r, const float* __restrict__ tf,
+__global__ void __launch_bounds__(kT) k_mg_exit32(int64_t n, const float* r, const float* tf,
                                                   float* __restrict__ z, const float* __restrict__ invd,
-                                                  const float* __restrict__ q, const float* __restrict__ om,
+                                                  const float* q, const float* __restrict__ om,
                                                   MixState* st, double* part, int mode) {
   dep_begin();
   mg_exit32_body<U>(n, r, tf, z, invd, q, om, st, part, mode, blockIdx.x, gridDim.x);

@@ -262,11 +262,11 @@ inline size_t mv_smem(int nx1, bool fuse) {
 
 template <int FUSE>
 __global__ void __launch_bounds__(kMvNodes, 4) k_matvec64(GridDims g, const __grid_constant__ KeD ke,
-                                                          const double* __restrict__ x, const double* __restrict__ pold,
+                                                          const double* x, const double* pold,
                                                           double* __restrict__ pnew, double* __restrict__ y,
                                                           const double* __restrict__ E, const uint8_t* __restrict__ dom,
                                                           const uint8_t* __restrict__ nf, int projected,
-                                                          const PcgState* __restrict__ st, unsigned chunks) {
+                                                          const PcgState* st, unsigned chunks) {
   extern __shared__ __align__(16) double xs[];  // [plane k-1, k, k+1][range][position][component]; FUSE: then p_old's
   const int tid = threadIdx.x;
   const int k = (int)(blockIdx.x / chunks);
@@ -582,7 +582,7 @@ __device__ __forceinline__ bool sum_blocks(double* part, unsigned* counter, doub
 // Phases of the single-chain dot kernel.
 enum DotPhase : int { PH_PAP = 0, PH_INIT_RR = 1 };
 
-__global__ void __launch_bounds__(chain_threads(1), 4) k_dot_exact(const double* __restrict__ a, const double* __restrict__ b,
+__global__ void __launch_bounds__(chain_threads(1), 4) k_dot_exact(const double* a, const double* b,
                                                              int64_t n, double* part, PcgState* st, int phase) {
   __shared__ __align__(16) double buf[kRing][1][4][kRow];
   dep_begin();
@@ -644,8 +644,8 @@ __global__ void __launch_bounds__(chain_threads(1), 4) k_dot_exact(const double*
 // Fused x/r update with ||r||^2 and z = r*invD with r.z. INIT: only the z part (rho0; the first direction is z).
 template <int INIT>
 __global__ void __launch_bounds__(chain_threads(2), 3) k_xr_exact(double* __restrict__ x, double* __restrict__ r,
-                                                            double* __restrict__ z, const double* __restrict__ p,
-                                                            const double* __restrict__ ap,
+                                                            double* __restrict__ z, const double* p,
+                                                            const double* ap,
                                                             const double* __restrict__ invd, int64_t n, double* part,
                                                             PcgState* st) {
   extern __shared__ __align__(16) double xr_buf[];

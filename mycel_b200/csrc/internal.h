@@ -343,8 +343,9 @@ int32_t mg_solve_packed(mycel_ctx* c, int njobs, PackJob* jobs, const volatile i
 // launched as programmatic dependents (launch_dep with early): the next kernel's CTAs are placed while this one's run,
 // instead of after its last. dep_begin is where a kernel waits until all before it have completed and their writes are
 // visible; nothing another kernel of the chain writes is touched before. It then lets its own successor be placed, so
-// that at most one kernel waits. Work on data that the solve does not change (stencils, moduli, coordinates) may come
-// before it. Launched the ordinary way, a kernel finds nothing to wait for.
+// that at most one kernel waits. Vectors that the kernel before writes are not declared const __restrict__: that would
+// promise that nobody writes them while this kernel is there. Work on data that the solve does not change (stencils,
+// moduli, coordinates) may come before the wait. Launched the ordinary way, a kernel finds nothing to wait for.
 // Whole solves, ms without / with: 110x22x22 (multigrid, 59 thousand nodes) 6.5 / 5.9, 64x48x48 4.8 / 4.4; SIMP loop
 // 85x53x27 (130 thousand nodes) 51.9 / 49.2; the plain FP64 form at 30x10x4 15.6 / 15.4, 96x48x24 117.5 / 116.3. At
 // 90x70x70 nothing is gained, at 192x96x96 1% is lost (waiting CTAs take places), so early is for problems up to about
