@@ -2903,7 +2903,6 @@ __device__ __forceinline__ void mg_put_all(float* p, float v) {
 __device__ __forceinline__ void mg_tail_smem(const MgTail& tl, const float* __restrict__ om, const MixState* st,
                                              int ncase, int rank, float* sm) {
   const int tid = threadIdx.x, nth = blockDim.x, warp = tid >> 5, lane = tid & 31, nwarp = nth >> 5;
-  mg_cluster_arrive();  // remote stores wait until every CTA has started
   int* smi = reinterpret_cast<int*>(sm);
   const int T = tl.T, L = tl.L, nc = tl.nc;
   // What comes from global memory is copied asynchronously, all of it on its way at once (a load and a store a
@@ -2963,6 +2962,7 @@ __device__ __forceinline__ void mg_tail_smem(const MgTail& tl, const float* __re
       reinterpret_cast<float4*>(sm + v.ot)[q] = make_float4(0.f, 0.f, 0.f, 0.f);
     }
   }
+  mg_cluster_arrive();  // remote stores wait until every CTA has started and zeroed its vectors
   dep_begin();  // so far: stencils and places, which a solve leaves as they are
   unsigned live = 0;
   for (int k = 0; k < ncase; ++k) live |= mg_running(st ? st + k : nullptr) ? 1u << k : 0u;

@@ -1,0 +1,24 @@
+"""Orders of memory accesses that only timing would hide if they were wrong, read from the kernels' source."""
+import pathlib
+import re
+
+SRC = (pathlib.Path(__file__).parent.parent / "mycel_b200/csrc/fp32_kernels.cu").read_text()
+
+
+def _body(name):
+    """The function's body, comments taken out."""
+    at = re.search(r"__device__ __forceinline__ \w+ " + name + r"\(", SRC).start()
+    open_, depth = SRC.index("{", at), 0
+    for i in range(open_, len(SRC)):
+        depth += {"{": 1, "}": -1}.get(SRC[i], 0)
+        if depth == 0:
+            return re.sub(r"//[^\n]*", "", SRC[open_:i])
+
+
+def test_cluster_waits_for_every_cta_zeros():
+    """The CTAs of the cluster kernel write into one another's vectors: each has to count itself in at the cluster
+    barrier after its own zeros are stored, or a slow CTA's zeros overwrite what a fast one has put there."""
+    body = _body("mg_tail_smem")
+    zeros = [m.start() for m in re.finditer(r"make_float4\(0\.f, 0\.f, 0\.f, 0\.f\)", body)]
+    arrive, wait, put = (body.index(s) for s in ("mg_cluster_arrive()", "mg_cluster_wait()", "mg_put_all("))
+    assert zeros and max(zeros) < arrive < wait < put
