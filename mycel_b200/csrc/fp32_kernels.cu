@@ -121,6 +121,7 @@ __device__ __forceinline__ bool grid_sums(double (&v)[N], double* part, unsigned
   if (tid == 0)
     asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(before) : "l"(counter) : "memory");
   before = __shfl_sync(0xffffffffu, before, 0);
+  __syncwarp();  // what lane 0 acquired is there for the other lanes too (a shuffle orders no memory)
   if (before != nblk - 1) return false;
   constexpr int B = N == 1 ? 16 : N == 2 ? 8 : 6;
 #pragma unroll

@@ -22,3 +22,12 @@ def test_cluster_waits_for_every_cta_zeros():
     zeros = [m.start() for m in re.finditer(r"make_float4\(0\.f, 0\.f, 0\.f, 0\.f\)", body)]
     arrive, wait, put = (body.index(s) for s in ("mg_cluster_arrive()", "mg_cluster_wait()", "mg_put_all("))
     assert zeros and max(zeros) < arrive < wait < put
+
+
+def test_sums_read_other_ctas_parts_after_a_warp_barrier():
+    """Lane 0 alone acquires the other CTAs' partial sums; a warp barrier has to stand between that and the other
+    lanes' loads of them."""
+    body = _body("grid_sums")
+    acquired = body.index("atom.add.acq_rel")
+    read = body.index("const volatile double*", acquired)
+    assert "__syncwarp()" in body[acquired:read]
