@@ -2334,7 +2334,7 @@ static_assert(kS1Stages % kS1Group == 0 && 27 % kS1Group == 0, "stage groups");
 static_assert(kS1Nodes % 4 == 0 && kS1Nodes + 3 < kS1Box, "TMA boxes: 16-byte aligned starts cover the CTA");
 
 __global__ void __launch_bounds__(256) k_mg_apply_nodes_tma(MgDims d, const __grid_constant__ CUtensorMap tm,
-                                                            const float* __restrict__ x, const float* __restrict__ r,
+                                                            const float* x, const float* r,
                                                             const float* __restrict__ invd, float* __restrict__ y,
                                                             int mode, const float* __restrict__ om,
                                                             const MixState* st, int* err) {
@@ -2497,7 +2497,7 @@ __device__ __forceinline__ void mg_restrict_row(const MgDims& f, int pitch, cons
 template <bool PAD>
 __device__ __forceinline__ void mg_prolong_comp(const MgDims& f, int pitch, const uint8_t* __restrict__ nf,
                                                 const float* __restrict__ invdf, float* __restrict__ xf,
-                                                const MgDims& c, const float* __restrict__ xc, int64_t n, int cc) {
+                                                const MgDims& c, const float* xc, int64_t n, int cc) {
   const int fx1 = f.nx + 1, fy1 = f.ny + 1;
   int i, j, k;
   mg_ijk(n, fx1, fy1, &i, &j, &k);
@@ -5241,8 +5241,8 @@ struct alignas(64) PkMv {  // one FP32 matvec (k_mv32f) of a right-hand side
 };
 
 template <int MODE>
-__global__ void __launch_bounds__(FX * FY, 2) k_mv32f_pk(const PkMv* __restrict__ tab, const unsigned* __restrict__ items,
-                                                         const unsigned* __restrict__ count) {
+__global__ void __launch_bounds__(FX * FY, 2) k_mv32f_pk(const PkMv* __restrict__ tab, const unsigned* items,
+                                                         const unsigned* count) {
   dep_begin();
   const unsigned cnt = *count;
   for (unsigned w = blockIdx.x; w < cnt; w += gridDim.x) {
@@ -5278,8 +5278,8 @@ struct PkVec {  // k_mg_enter32 / k_mg_exit32 of a right-hand side
   unsigned nb;
 };
 
-__global__ void __launch_bounds__(kT, 2) k_mg_enter32_pk(const PkVec* __restrict__ tab, const unsigned* __restrict__ items,
-                                                      const unsigned* __restrict__ count, int mode) {
+__global__ void __launch_bounds__(kT, 2) k_mg_enter32_pk(const PkVec* __restrict__ tab, const unsigned* items,
+                                                      const unsigned* count, int mode) {
   dep_begin();
   const unsigned cnt = *count;
   for (unsigned w = blockIdx.x; w < cnt; w += gridDim.x) {
@@ -5291,8 +5291,8 @@ __global__ void __launch_bounds__(kT, 2) k_mg_enter32_pk(const PkVec* __restrict
   }
 }
 
-__global__ void __launch_bounds__(kT, 2) k_mg_exit32_pk(const PkVec* __restrict__ tab, const unsigned* __restrict__ items,
-                                                     const unsigned* __restrict__ count, int mode) {
+__global__ void __launch_bounds__(kT, 2) k_mg_exit32_pk(const PkVec* __restrict__ tab, const unsigned* items,
+                                                     const unsigned* count, int mode) {
   dep_begin();
   const unsigned cnt = *count;
   for (unsigned w = blockIdx.x; w < cnt; w += gridDim.x) {
@@ -5316,8 +5316,8 @@ struct PkApply {  // a coarse-level product of a problem (all its cases)
 
 template <bool MULTI>
 __global__ void __launch_bounds__(256) k_mg_apply_nodes_pk(const PkApply* __restrict__ tab,
-                                                           const unsigned* __restrict__ items,
-                                                           const unsigned* __restrict__ count, int mode) {
+                                                           const unsigned* items,
+                                                           const unsigned* count, int mode) {
   dep_begin();
   const unsigned cnt = *count;
   for (unsigned w = blockIdx.x; w < cnt; w += gridDim.x) {
@@ -5334,8 +5334,8 @@ __global__ void __launch_bounds__(256) k_mg_apply_nodes_pk(const PkApply* __rest
 
 template <bool MULTI>
 __global__ void __launch_bounds__(kMgDofThreads) k_mg_apply_pk(const PkApply* __restrict__ tab,
-                                                               const unsigned* __restrict__ items,
-                                                               const unsigned* __restrict__ count, int mode) {
+                                                               const unsigned* items,
+                                                               const unsigned* count, int mode) {
   dep_begin();
   __shared__ float xs[kRowStage];
   const unsigned cnt = *count;
@@ -5359,8 +5359,8 @@ struct PkRestrict {  // restriction of a problem's level to the next coarser one
 
 template <bool PAD, bool MULTI>
 __global__ void __launch_bounds__(kMgDofThreads) k_mg_restrict_pk(const PkRestrict* __restrict__ tab,
-                                                                  const unsigned* __restrict__ items,
-                                                                  const unsigned* __restrict__ count) {
+                                                                  const unsigned* items,
+                                                                  const unsigned* count) {
   dep_begin();
   const unsigned cnt = *count;
   for (unsigned w = blockIdx.x; w < cnt; w += gridDim.x) {
@@ -5387,8 +5387,8 @@ struct PkProlong {  // prolongation of a problem's level to the next finer one (
 
 template <bool PAD, bool MULTI>
 __global__ void __launch_bounds__(kMgDofThreads) k_mg_prolong_pk(const PkProlong* __restrict__ tab,
-                                                                 const unsigned* __restrict__ items,
-                                                                 const unsigned* __restrict__ count) {
+                                                                 const unsigned* items,
+                                                                 const unsigned* count) {
   dep_begin();
   const unsigned cnt = *count;
   for (unsigned w = blockIdx.x; w < cnt; w += gridDim.x) {

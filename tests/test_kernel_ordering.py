@@ -2,7 +2,8 @@
 import pathlib
 import re
 
-SRC = (pathlib.Path(__file__).parent.parent / "mycel_b200/csrc/fp32_kernels.cu").read_text()
+CSRC = pathlib.Path(__file__).parent.parent / "mycel_b200/csrc"
+SRC = (CSRC / "fp32_kernels.cu").read_text()
 
 
 def _body(name):
@@ -31,3 +32,24 @@ def test_sums_read_other_ctas_parts_after_a_warp_barrier():
     acquired = body.index("atom.add.acq_rel")
     read = body.index("const volatile double*", acquired)
     assert "__syncwarp()" in body[acquired:read]
+
+
+def test_dependent_kernels_promise_read_only_for_fixed_data_only():
+    """A kernel that waits for the one before it (dep_begin) may not declare read-only what that one writes: the
+    compiler could load it before the wait. Read-only are what a solve leaves as it is (moduli, stencils, inverse
+    diagonals, flags, dampings) and the descriptor tables."""
+    fixed = {"E", "S", "dom", "nf", "invd", "invdf", "invdc", "om", "tab"}
+    seen = 0
+    for name in ("fp32_kernels.cu", "fp64_kernels.cu"):
+        src = (CSRC / name).read_text()
+        for m in re.finditer(r"__global__[^;{]*?\b(k_\w+)\(([^{;]*)\)\s*\{", src):
+            depth, i = 1, m.end()
+            while depth:
+                depth += {"{": 1, "}": -1}.get(src[i], 0)
+                i += 1
+            if not re.search(r"dep_begin|mg_tail_smem|mg_apply_rows", src[m.end():i]):
+                continue
+            seen += 1
+            named = set(re.findall(r"const \w+\* __restrict__ (\w+)", m.group(2)))
+            assert named <= fixed, (m.group(1), named - fixed)
+    assert seen >= 20
