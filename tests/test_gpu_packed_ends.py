@@ -1,0 +1,47 @@
+"""Packs in which some problems have ended, or wait for their next solve, while others still run, on both sides of the
+line up to which a pack's kernels are launched as early dependents (its vector steps' CTAs against the SMs). Each
+problem must come out with the bits of its run alone (tolerance 0)."""
+import pytest
+import torch
+
+from mycel_b200 import api
+from mycel_b200 import workloads as W
+from mycel_b200.model import OptimizerOptions
+from test_gpu_packed import _alone, _same, _session
+
+pytestmark = pytest.mark.gpu
+
+BASE = OptimizerOptions(volume_fraction=0.3, filter_radius_mm=1.5, precision="mixed-mg", solver_tolerance_initial=1e-6,
+                        solver_tolerance_final=1e-6, solver_max_iterations=20000)
+
+
+def _jobs(early):
+    """(model, options, runs): one iteration, five and three; a looser tolerance ends solves early as well."""
+    grids = [(20, 10, 8), (26, 13, 9), (33, 17, 11)] if early else [(64, 32, 30), (44, 22, 40), (71, 35, 33)]
+    jobs = []
+    for (nx, ny, nz), iters, tol in zip(grids, (1, 5, 3), (1e-3, 1e-7, 1e-5)):
+        jobs.append((W.cantilever(nx, ny, nz, e0=1.0, emin_ratio=1e-9, force=-1.0),
+                     BASE.replace(max_iterations=iters, solver_tolerance_initial=tol, solver_tolerance_final=tol)))
+    bp = next(b for b in W.batched_instances(count=16, seed=7, scale=0.25 if early else 0.6) if len(b.load_cases) >= 3)
+    jobs.append((bp.model, bp.options.replace(max_iterations=2, precision="mixed-mg", separate_load_cases=True)))
+    return jobs
+
+
+@pytest.mark.parametrize("early", [True, False])
+def test_problems_that_end_at_different_times(ctx, early):
+    jobs = _jobs(early)
+    ctas = sum(-(-(m.total_dofs // 4) // 1024) * (len(m.loads) if o.separate_load_cases else 1) for m, o in jobs)
+    assert (ctas <= torch.cuda.get_device_properties(0).multi_processor_count) == early
+    alone = [_alone(ctx, m, o, o.max_iterations) for m, o in jobs]
+    made = [_session(ctx, m, o) for m, o in jobs]
+    try:
+        before = ctx.packed_count
+        out = api.SimpSession.run_many([s for _, s in made])
+        reads = [s.read() for _, s in made]
+        assert ctx.packed_count > before
+    finally:
+        for p, s in made:
+            s.close()
+            p.close()
+    for k, (ra, da) in enumerate(alone):
+        _same(ra, da, out[k], reads[k])
