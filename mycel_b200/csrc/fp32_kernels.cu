@@ -5344,19 +5344,27 @@ __global__ void __launch_bounds__(256) k_mg_apply_nodes_pk(const PkApply* __rest
   }
 }
 
-template <bool MULTI>
-__global__ void __launch_bounds__(kMgDofThreads) k_mg_apply_pk(const PkApply* __restrict__ tab,
-                                                               const unsigned* items,
+template <bool MULTI, bool SHARED>
+__global__ void __launch_bounds__(kMgDofThreads) k_mg_apply_pk(const PkApply* __restrict__ tab, const unsigned* items,
                                                                const unsigned* count, int mode) {
   dep_begin();
-  __shared__ float xs[kRowStage];
+  __shared__ float xs[SHARED ? kRowStage : 1];
   const unsigned cnt = *count;
   for (unsigned w = blockIdx.x; w < cnt; w += gridDim.x) {
     const unsigned code = items[w];
     const PkApply& a = tab[code >> kPkLbBits];
-    mg_apply_rows<MULTI>(a.d, (int64_t)(code & kPkLbMask) * 64, a.ncase, a.S, a.x, a.r, a.invd, a.y, mode, a.om, a.st,
-                         xs, false);
-    __syncthreads();  // xs is the next item's
+    const int64_t t0 = (int64_t)(code & kPkLbMask) * 64;
+    if constexpr (SHARED) {
+      mg_apply_rows<MULTI>(a.d, t0, a.ncase, a.S, a.x, a.r, a.invd, a.y, mode, a.om, a.st, xs, false);
+      __syncthreads();  // xs is the next item's
+    } else {
+      int64_t q;
+      int c;
+      mg_item_case<MULTI>(t0 + (threadIdx.x & 63), a.ncase, &q, &c);
+      if (q >= mg_nn(a.d) || !mg_running(a.st ? a.st + c : nullptr)) continue;
+      mg_apply_row(a.d, mg_ns(a.d), (int)q, mg_dof_comp(), a.S, a.x.p[c], a.r.p[c], a.invd, a.y.p[c], mode,
+                   mode == 1 ? *a.om : 0.0f);
+    }
   }
 }
 
@@ -5497,6 +5505,7 @@ struct PkLaunch {
   int n;
   unsigned blocks;  // work items when every entry runs (its launches alone's CTAs)
   unsigned grid;    // persistent CTAs of the launch
+  bool few;         // at most three items an SM
   size_t smem = 0;  // cluster kernel: the largest shared memory of its entries
 };
 
@@ -5605,11 +5614,22 @@ struct PkBuilder {
   }
 };
 
+// The coarse products' form by the items of the whole launch, with the line that MgLevel::max_shared draws for a problem
+// alone. 48 problems of 7 thousand to 470 thousand elements (16 to 105 items an SM in one pack), SIMP iterations a second
+// with shared rows whatever the items / direct rows: loads apart, four packs 136.7 / 145.7, one pack 125.8 / 132.5; loads
+// summed 333 / 355 and 317 / 328.
+static auto pk_apply_kernel(bool multi, bool few) {
+  return few ? (multi ? k_mg_apply_pk<true, true> : k_mg_apply_pk<false, true>)
+             : (multi ? k_mg_apply_pk<true, false> : k_mg_apply_pk<false, false>);
+}
+
 // resident CTAs per SM of a packed kernel (its persistent grid: this times the SMs, at most its work items)
-static int pk_resident(int kind, bool pad, bool multi) {
+static int pk_resident(const PkLaunch& L) {
+  const int kind = L.kind;
+  const bool pad = L.pad, multi = L.multi, few = L.few;
   static std::mutex mu;
   static std::map<int, int> memo;
-  const int key = kind * 4 + (pad ? 2 : 0) + (multi ? 1 : 0);
+  const int key = kind * 8 + (few ? 4 : 0) + (pad ? 2 : 0) + (multi ? 1 : 0);
   std::lock_guard<std::mutex> lk(mu);
   auto it = memo.find(key);
   if (it != memo.end()) return it->second;
@@ -5621,8 +5641,7 @@ static int pk_resident(int kind, bool pad, bool multi) {
     case PK_ENTER: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, k_mg_enter32_pk, kT, 0); break;
     case PK_EXIT: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, k_mg_exit32_pk, kT, 0); break;
     case PK_APPLY_DOF:
-      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, multi ? k_mg_apply_pk<true> : k_mg_apply_pk<false>,
-                                                        kMgDofThreads, 0);
+      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, pk_apply_kernel(multi, few), kMgDofThreads, 0);
       break;
     case PK_APPLY_NODE:
       e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(
@@ -5665,17 +5684,13 @@ static void pk_issue(const PackPlan& P, const PkLaunch& L, cudaStream_t s, int s
                (const PkMv*)tab, it, cn);
       break;
     case PK_ENTER:
-      launch_dep(P.early, k_mg_enter32_pk, g, kT, 0, s,
-               (const PkVec*)tab, it, cn, step_mode);
+      launch_dep(P.early, k_mg_enter32_pk, g, kT, 0, s, (const PkVec*)tab, it, cn, step_mode);
       break;
     case PK_EXIT:
-      launch_dep(P.early, k_mg_exit32_pk, g, kT, 0, s,
-               (const PkVec*)tab, it, cn, step_mode);
+      launch_dep(P.early, k_mg_exit32_pk, g, kT, 0, s, (const PkVec*)tab, it, cn, step_mode);
       break;
     case PK_APPLY_DOF:
-      launch_dep(P.early, (L.multi ? k_mg_apply_pk<true> : k_mg_apply_pk<false>), g, kMgDofThreads, 0, s,
-               (const PkApply*)tab, it, cn,
-                                                                                         L.mode);
+      launch_dep(P.early, pk_apply_kernel(L.multi, L.few), g, kMgDofThreads, 0, s, (const PkApply*)tab, it, cn, L.mode);
       break;
     case PK_APPLY_NODE:
       launch_dep(P.early, (L.multi ? k_mg_apply_nodes_pk<true> : k_mg_apply_nodes_pk<false>), g, 256, 0, s,
@@ -6041,8 +6056,10 @@ static int32_t pk_build(mycel_ctx* c, PackWork* w, std::vector<PkUnit>& units, c
   // persistent grids: the resident CTAs, at most the work items (the cluster kernels are not persistent)
   for (std::vector<PkLaunch>* v : {&P.mv1[0], &P.mv1[1], &P.enter[0], &P.enter[1], &P.exitl, &P.vcycle})
     for (PkLaunch& L : *v)
-      if (L.kind != PK_TAIL)
-        L.grid = std::max(1u, std::min<unsigned>(L.blocks, (unsigned)(pk_resident(L.kind, L.pad, L.multi) * c->num_sms)));
+      if (L.kind != PK_TAIL) {
+        L.few = L.blocks <= 3u * (unsigned)c->num_sms;
+        L.grid = std::max(1u, std::min<unsigned>(L.blocks, (unsigned)(pk_resident(L) * c->num_sms)));
+      }
   // work-list groups, written once the arena's address is known
   std::vector<const PkLaunch*> gi[2], gs;
   auto listed = [](std::vector<const PkLaunch*>& g, const std::vector<PkLaunch>& v) {
