@@ -5290,7 +5290,8 @@ struct PkVec {  // k_mg_enter32 / k_mg_exit32 of a right-hand side
   unsigned nb;
 };
 
-__global__ void __launch_bounds__(kT, 2) k_mg_enter32_pk(const PkVec* __restrict__ tab, const unsigned* items,
+template <int U>
+__global__ void __launch_bounds__(kT, U == 1 ? 0 : 2) k_mg_enter32_pk(const PkVec* __restrict__ tab, const unsigned* items,
                                                       const unsigned* count, int mode) {
   dep_begin();
   const unsigned cnt = *count;
@@ -5299,11 +5300,12 @@ __global__ void __launch_bounds__(kT, 2) k_mg_enter32_pk(const PkVec* __restrict
     const unsigned code = items[w];
     const PkVec& a = tab[code >> kPkLbBits];
     const int md = mode >= 0 ? mode : *(const volatile int*)&a.st->pmode;
-    mg_enter32_body<4>(a.n, a.x, a.r, a.p, a.q, a.invd, a.z, a.om, a.st, a.part, md, code & kPkLbMask, a.nb);
+    mg_enter32_body<U>(a.n, a.x, a.r, a.p, a.q, a.invd, a.z, a.om, a.st, a.part, md, code & kPkLbMask, a.nb);
   }
 }
 
-__global__ void __launch_bounds__(kT, 2) k_mg_exit32_pk(const PkVec* __restrict__ tab, const unsigned* items,
+template <int U>
+__global__ void __launch_bounds__(kT, U == 1 ? 0 : 2) k_mg_exit32_pk(const PkVec* __restrict__ tab, const unsigned* items,
                                                      const unsigned* count, int mode) {
   dep_begin();
   const unsigned cnt = *count;
@@ -5312,7 +5314,7 @@ __global__ void __launch_bounds__(kT, 2) k_mg_exit32_pk(const PkVec* __restrict_
     const unsigned code = items[w];
     const PkVec& a = tab[code >> kPkLbBits];
     const int md = mode >= 0 ? mode : *(const volatile int*)&a.st->pmode;
-    mg_exit32_body<4>(a.n, a.r, a.t, a.z, a.invd, a.q, a.om, a.st, a.part, md, code & kPkLbMask, a.nb);
+    mg_exit32_body<U>(a.n, a.r, a.t, a.z, a.invd, a.q, a.om, a.st, a.part, md, code & kPkLbMask, a.nb);
   }
 }
 
@@ -5614,10 +5616,13 @@ struct PkBuilder {
   }
 };
 
-// The coarse products' form by the items of the whole launch, with the line that MgLevel::max_shared draws for a problem
-// alone. 48 problems of 7 thousand to 470 thousand elements (16 to 105 items an SM in one pack), SIMP iterations a second
-// with shared rows whatever the items / direct rows: loads apart, four packs 136.7 / 145.7, one pack 125.8 / 132.5; loads
-// summed 333 / 355 and 317 / 328.
+// The coarse products' form and the vector steps' loads in flight (U), by the items of the whole launch with the lines
+// that MgLevel::max_shared and outer_wide draw for a problem alone. 48 problems of 7 thousand to 470 thousand elements
+// (16 to 105 products' and 36 to 111 steps' items an SM in one pack), SIMP iterations a second with shared rows and U = 4
+// whatever the items / direct rows / also U = 1: loads apart, four packs 136.7 / 145.7 / 150.4, one pack 125.8 / 132.5 /
+// 136.6; loads summed 333 / 355 / 363 and 317 / 328 / 335.
+static auto pk_enter_kernel(bool few) { return few ? k_mg_enter32_pk<4> : k_mg_enter32_pk<1>; }
+static auto pk_exit_kernel(bool few) { return few ? k_mg_exit32_pk<4> : k_mg_exit32_pk<1>; }
 static auto pk_apply_kernel(bool multi, bool few) {
   return few ? (multi ? k_mg_apply_pk<true, true> : k_mg_apply_pk<false, true>)
              : (multi ? k_mg_apply_pk<true, false> : k_mg_apply_pk<false, false>);
@@ -5638,8 +5643,8 @@ static int pk_resident(const PkLaunch& L) {
   switch (kind) {
     case PK_MV0: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, k_mv32f_pk<0>, FX * FY, fac_smem_bytes(0)); break;
     case PK_MV1: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, k_mv32f_pk<1>, FX * FY, fac_smem_bytes(1)); break;
-    case PK_ENTER: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, k_mg_enter32_pk, kT, 0); break;
-    case PK_EXIT: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, k_mg_exit32_pk, kT, 0); break;
+    case PK_ENTER: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, pk_enter_kernel(few), kT, 0); break;
+    case PK_EXIT: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, pk_exit_kernel(few), kT, 0); break;
     case PK_APPLY_DOF:
       e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, pk_apply_kernel(multi, few), kMgDofThreads, 0);
       break;
@@ -5684,10 +5689,10 @@ static void pk_issue(const PackPlan& P, const PkLaunch& L, cudaStream_t s, int s
                (const PkMv*)tab, it, cn);
       break;
     case PK_ENTER:
-      launch_dep(P.early, k_mg_enter32_pk, g, kT, 0, s, (const PkVec*)tab, it, cn, step_mode);
+      launch_dep(P.early, pk_enter_kernel(L.few), g, kT, 0, s, (const PkVec*)tab, it, cn, step_mode);
       break;
     case PK_EXIT:
-      launch_dep(P.early, k_mg_exit32_pk, g, kT, 0, s, (const PkVec*)tab, it, cn, step_mode);
+      launch_dep(P.early, pk_exit_kernel(L.few), g, kT, 0, s, (const PkVec*)tab, it, cn, step_mode);
       break;
     case PK_APPLY_DOF:
       launch_dep(P.early, pk_apply_kernel(L.multi, L.few), g, kMgDofThreads, 0, s, (const PkApply*)tab, it, cn, L.mode);
