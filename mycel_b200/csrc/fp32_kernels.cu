@@ -2492,15 +2492,13 @@ __device__ __forceinline__ void mg_restrict_row(const MgDims& f, int pitch, cons
   if (xc) xc[3 * n + cc] = omega * d * rv;
 }
 
-// prolongation x_f += W x_c, component cc at fine node n, on the finer level's free DOFs. PAD: the voxel grid
-// (padded FP32 layout, free = node flag bit clear); otherwise box layout, free = nonzero diagonal.
-template <bool PAD>
-__device__ __forceinline__ void mg_prolong_comp(const MgDims& f, int pitch, const uint8_t* __restrict__ nf,
-                                                const float* __restrict__ invdf, float* __restrict__ xf,
-                                                const MgDims& c, const float* xc, int64_t n, int cc) {
-  const int fx1 = f.nx + 1, fy1 = f.ny + 1;
+// prolongation x_f += W x_c between box-ordered levels, component cc at fine node n, on the finer level's free DOFs
+// (nonzero diagonal)
+__device__ __forceinline__ void mg_prolong_comp(const MgDims& f, const float* __restrict__ invdf,
+                                                float* __restrict__ xf, const MgDims& c, const float* xc, int64_t n,
+                                                int cc) {
   int i, j, k;
-  mg_ijk(n, fx1, fy1, &i, &j, &k);
+  mg_ijk(n, f.nx + 1, f.ny + 1, &i, &j, &k);
   // per axis: two coarse nodes with their weights (the second with weight 0 unless the fine node lies midway)
   int ci[2], cj[2], ck[2];
   float wi[2], wj[2], wk[2];
@@ -2525,8 +2523,7 @@ __device__ __forceinline__ void mg_prolong_comp(const MgDims& f, int pitch, cons
         const int64_t m = ci[qx] + (int64_t)cx1 * (cj[qy] + (int64_t)cy1 * ck[qz]);
         a = fmaf(wi[qx] * wj[qy] * wk[qz], xc[3 * m + cc], a);
       }
-  const bool fr = PAD ? !(nf[n] & (1 << cc)) : (invdf[3 * n + cc] != 0.0f);
-  if (fr) xf[(PAD ? (int64_t)pitch * (j + (int64_t)fy1 * k) + 3 * i : 3 * n) + cc] += a;
+  if (invdf[3 * n + cc] != 0.0f) xf[3 * n + cc] += a;
 }
 
 template <bool PAD, bool MULTI>
@@ -2724,8 +2721,9 @@ __global__ void __launch_bounds__(1024) k_mg_coarse_setup(MgDims d, const float*
 // The coarse levels from T down to the coarsest and back in one launch of one thread-block cluster: levels
 // this small cost more in separate launches than in work. The cluster's CTAs are co-scheduled, so a cluster
 // barrier separates the phases.
-// Sixteen CTAs (the opt-in size): a level of up to about 1,700 nodes fits in their shared memory with its stencil,
-// and the copies at the start take half as long as with eight (16.8 against 20.9 us for 480 + 105 + 24 nodes).
+// Sixteen CTAs (the opt-in size): a level of up to about 1,400 nodes fits in their shared memory for one case with its
+// stencil and the levels below it (33x17x16 -> 17x9x9 nodes; mg_tail_layout), and the copies at the start take half as
+// long as with eight (16.8 against 20.9 us for 480 + 105 + 24 nodes).
 constexpr int kMgTailCtas = 16, kMgTailThreads = 512;
 // levels of at most this many nodes go to the cluster kernel, as far as they fit (mg_tail_plan)
 constexpr int64_t kMgTailMaxNodes = 2048;
@@ -2737,16 +2735,15 @@ struct MgTailLevel {
   const float* invd;
   float *xa, *xb, *r, *t;  // case 0's vectors; case k's at + k * 3 nn
   // the level in the shared-memory form (mg_tail_smem): padded node grid's row and plane strides and size (nodes),
-  // rows (DOFs) and rows per CTA, and the shared-memory offsets (4-byte words) of the CTA's stencil rows (-1: read
-  // from global memory), x, t (4 psize a case), 1/diag (all rows), r (the CTA's rows, a case) and the nodes'
-  // coordinates
+  // rows (DOFs) and rows per CTA, and the shared-memory offsets (4-byte words) of the CTA's stencil rows, x, t (4 psize
+  // a case), 1/diag (all rows), r (the CTA's rows, a case) and the nodes' coordinates
   int psy, psz, psize, rows, rpc;
   int oS, ox, ot, oi, orr, oc;
 };
 struct MgTail {
   int T, L, sweeps, nc;
   const double* ainv;
-  int group;     // load cases the shared-memory form takes at once (0: it does not fit, vectors stay in global memory)
+  bool in_smem;  // levels and vectors in shared memory (mg_tail_smem), else vectors in global memory (mg_tail_body)
   int ocr, ocx;  // shared-memory offsets of the coarsest level's r and x (nc a case)
   int smem;      // its bytes
   MgTailLevel lv[kMgMaxLevels];
@@ -2761,8 +2758,8 @@ __device__ __forceinline__ void mg_cluster_sync() {
 // Levels T .. L-1 of the V-cycle for ncase load cases: from r of level T (restricted by the caller) to the
 // smoothed correction of level T, left in its xa. Work items are numbered with the case fastest; a case whose
 // state is not running is skipped, and the kernel returns at once (every thread alike) when none is.
-// Body for the threads gt (of gs) of the cluster that runs this V-cycle's tail, with the vectors in global memory: used
-// where the levels do not fit in shared memory (mg_tail_plan) and for several sweeps.
+// Body for the threads gt (of gs) of the cluster that runs this V-cycle's tail, with the vectors in global memory: for
+// several sweeps (mg_tail_plan).
 template <bool MULTI>
 __device__ __forceinline__ void mg_tail_body(const MgTail& tl, const float* __restrict__ om, const MixState* st,
                                              int ncase, int64_t gt, int64_t gs) {
@@ -2850,8 +2847,7 @@ __device__ __forceinline__ void mg_tail_body(const MgTail& tl, const float* __re
       int k;
       mg_item_case<MULTI>(q, ncase, &it, &k);
       if (live(k))
-        mg_prolong_comp<false>(v.d, 0, nullptr, v.invd, x + k * nd, tl.lv[l + 1].d, xc[l + 1] + k * cnd, it / 3,
-                               (int)(it % 3));
+        mg_prolong_comp(v.d, v.invd, x + k * nd, tl.lv[l + 1].d, xc[l + 1] + k * cnd, it / 3, (int)(it % 3));
     }
     mg_cluster_sync();
     for (int k = 0; k < tl.sweeps; ++k) {
@@ -2881,7 +2877,7 @@ __device__ __forceinline__ void mg_tail_body(const MgTail& tl, const float* __re
 // (copied once at the start), the whole of every level's x and t (four floats a node, padded by a zero node on each
 // side, so that a neighbour is a constant step away and needs no test), 1/diag and the nodes' coordinates, and a row
 // is 129 instructions. Only the products and the coarsest solve are split over the cluster: a thread per row writes
-// its result to all eight CTAs' copies, and one cluster barrier follows; restriction and prolongation are done by
+// its result to all sixteen CTAs' copies, and one cluster barrier follows; restriction and prolongation are done by
 // every CTA for itself. Each row's chain of products, each restriction and prolongation sum and the coarsest rows are
 // formed in the order of mg_tail_body, so the results are its bits (an absent neighbour's zero product leaves a sum
 // as it is). 480 + 105 + 24 nodes: 42 -> 16.8 us; four cases on 1,683 nodes and below: 125 -> 21 us and the four
@@ -2926,7 +2922,6 @@ __device__ __forceinline__ void mg_tail_smem(const MgTail& tl, const float* __re
   for (int l = T; l < L - 1; ++l) {
     const MgTailLevel& v = tl.lv[l];
     const int lo = rank * v.rpc, nr = max(0, min(v.rpc, v.rows - lo)), nch = (nr + 31) >> 5;
-    if (v.oS < 0) continue;
     const int64_t ns = mg_ns(v.d);
     const int nx1 = v.d.nx + 1, sxy = nx1 * (v.d.ny + 1);
     for (int q = warp; q < nch * 9; q += nwarp) {
@@ -2972,7 +2967,7 @@ __device__ __forceinline__ void mg_tail_smem(const MgTail& tl, const float* __re
       smi[v.oc + n] = i | j << 10 | k << 20;
     }
     if (l == L - 1) break;
-    for (int q = tid; q < v.psize * tl.group; q += nth) {
+    for (int q = tid; q < v.psize * ncase; q += nth) {
       reinterpret_cast<float4*>(sm + v.ox)[q] = make_float4(0.f, 0.f, 0.f, 0.f);
       reinterpret_cast<float4*>(sm + v.ot)[q] = make_float4(0.f, 0.f, 0.f, 0.f);
     }
@@ -2985,188 +2980,169 @@ __device__ __forceinline__ void mg_tail_smem(const MgTail& tl, const float* __re
     return;
   }
   mg_cluster_arrive();  // remote stores wait until every CTA has started and zeroed its vectors
-  bool started = false;
-  for (int c0 = 0; c0 < ncase; c0 += tl.group) {
-    const int g = min(tl.group, ncase - c0);
-    if (!(live >> c0 & ((1u << g) - 1))) continue;
-    // item of a loop over `items` items x cases -> item, case (items x cases is far below 2^20)
-    auto split = [&](int it, int items, int* c) {
-      *c = g == 1 ? 0 : __float2int_rz(((float)it + 0.5f) * (1.0f / (float)items));
-      return it - *c * items;
-    };
-    auto pad = [&](const MgTailLevel& v, int n) {  // padded position of a node
-      const int q = smi[v.oc + n];
-      return ((q & 1023) + 1) + v.psy * ((q >> 10 & 1023) + 1) + v.psz * ((q >> 20) + 1);
-    };
-    __syncthreads();  // coordinates and zeros; an earlier group is done with its vectors
-    {  // level T: x = omega invd r (written with r by the restriction into it) and the CTA's rows of r
-      const MgTailLevel& v = tl.lv[T];
-      const int lo = rank * v.rpc, nr = max(0, min(v.rpc, v.rows - lo));
-      if (T < L - 1) {
-        for (int it = tid; it < v.rows * g; it += nth) {
-          int c;
-          const int row = split(it, v.rows, &c), n = row / 3;
-          __pipeline_memcpy_async(sm + v.ox + 4 * (c * v.psize + pad(v, n)) + row - 3 * n,
-                                  v.xa + ((int64_t)(c0 + c) * v.rows + row), 4);
-        }
-        for (int it = tid; it < nr * g; it += nth) {
-          int c;
-          const int lr = split(it, nr, &c);
-          __pipeline_memcpy_async(sm + v.orr + c * v.rpc + lr, v.r + ((int64_t)(c0 + c) * v.rows + lo + lr), 4);
-        }
-      } else {
-        for (int it = tid; it < nc * g; it += nth) __pipeline_memcpy_async(sm + tl.ocr + it, v.r + ((int64_t)c0 * nc + it), 4);
-      }
-    }
-    __pipeline_commit();
-    __pipeline_wait_prior(0);
-    __syncthreads();
-    if (!started) mg_cluster_wait();
-    started = true;
-    // rows of A x on level l, x in shared memory; the result handed to put(case, row, its word, value)
-    auto apply = [&](const MgTailLevel& v, int mode, float w, auto&& put) {
-      const int lo = rank * v.rpc, nr = max(0, min(v.rpc, v.rows - lo));
-      const int sy = 4 * v.psy, sz = 4 * v.psz;
-      for (int it = tid; it < nr * g; it += nth) {
+  // item of a loop over `items` items x cases -> item, case (items x cases is far below 2^20)
+  auto split = [&](int it, int items, int* c) {
+    *c = ncase == 1 ? 0 : __float2int_rz(((float)it + 0.5f) * (1.0f / (float)items));
+    return it - *c * items;
+  };
+  auto pad = [&](const MgTailLevel& v, int n) {  // padded position of a node
+    const int q = smi[v.oc + n];
+    return ((q & 1023) + 1) + v.psy * ((q >> 10 & 1023) + 1) + v.psz * ((q >> 20) + 1);
+  };
+  __syncthreads();  // coordinates and zeros
+  {  // level T: x = omega invd r (written with r by the restriction into it) and the CTA's rows of r
+    const MgTailLevel& v = tl.lv[T];
+    const int lo = rank * v.rpc, nr = max(0, min(v.rpc, v.rows - lo));
+    if (T < L - 1) {
+      for (int it = tid; it < v.rows * ncase; it += nth) {
         int c;
-        const int lr = split(it, nr, &c), row = lo + lr, n = row / 3, ci = row - 3 * n;
-        const int at = 4 * (c * v.psize + pad(v, n));
-        const float* x = sm + v.ox + at;
-        float a = 0.f;
-        if (v.oS >= 0) {
-          const float4* s4 = reinterpret_cast<const float4*>(sm + v.oS + lr * kTailEnt);
-          float s[kTailEnt];
-#pragma unroll
-          for (int q = 0; q < kTailEnt / 4; ++q) {
-            const float4 t = s4[q];
-            s[4 * q] = t.x; s[4 * q + 1] = t.y; s[4 * q + 2] = t.z; s[4 * q + 3] = t.w;
-          }
-#pragma unroll
-          for (int nb = 0; nb < 27; ++nb) {
-            const float4 xm = *reinterpret_cast<const float4*>(x + 4 * (nb % 3 - 1) + sy * ((nb / 3) % 3 - 1) + sz * (nb / 9 - 1));
-            a = fmaf(s[3 * nb], xm.x, fmaf(s[3 * nb + 1], xm.y, fmaf(s[3 * nb + 2], xm.z, a)));
-          }
-        } else {
-          const int64_t ns = mg_ns(v.d);
-          const MgNode gn(v.d, n);
-#pragma unroll
-          for (int nb = 0; nb < 27; ++nb) {
-            const float4 xm = *reinterpret_cast<const float4*>(x + 4 * (nb % 3 - 1) + sy * ((nb / 3) % 3 - 1) + sz * (nb / 9 - 1));
-            const float* q = nb >= 13 ? v.S + ((int64_t)(nb - 13) * 9 + 3 * ci) * ns + n
-                                      : v.S + ((int64_t)(13 - nb) * 9 + ci) * ns + max(gn.at(nb), 0);
-            const int64_t step = nb >= 13 ? ns : 3 * ns;
-            a = fmaf(q[0], xm.x, fmaf(q[step], xm.y, fmaf(q[2 * step], xm.z, a)));
-          }
-        }
-        const float id = sm[v.oi + row], rv = sm[v.orr + c * v.rpc + lr];
-        put(c, row, at + ci, mode == 1 ? fmaf(w * id, rv - a, x[ci]) : (id != 0.0f ? rv - a : 0.0f));
+        const int row = split(it, v.rows, &c), n = row / 3;
+        __pipeline_memcpy_async(sm + v.ox + 4 * (c * v.psize + pad(v, n)) + row - 3 * n,
+                                v.xa + ((int64_t)c * v.rows + row), 4);
       }
-    };
-    for (int l = T; l < L - 1; ++l) {
-      const MgTailLevel& v = tl.lv[l];
-      const MgTailLevel& cv = tl.lv[l + 1];
-      apply(v, 2, 0.0f, [&](int, int, int at, float val) { mg_put_all(sm + v.ot + at, val); });
-      mg_cluster_arrive();
-      mg_cluster_wait();
-      const bool smoothed = l + 1 < L - 1;
-      const float wc = smoothed ? om[l + 1] : 0.0f;
-      const int clo = rank * cv.rpc;
-      for (int it = tid; it < cv.rows * g; it += nth) {  // restriction, every CTA for itself
+      for (int it = tid; it < nr * ncase; it += nth) {
         int c;
-        const int row = split(it, cv.rows, &c), n = row / 3, ci = row - 3 * n, q = smi[cv.oc + n];
-        const int I = q & 1023, J = q >> 10 & 1023, K = q >> 20;
-        const MgAxis ax(I, v.d.nx, 4), ay(J, v.d.ny, 4 * v.psy), az(K, v.d.nz, 4 * v.psz);
-        const float* t = sm + v.ot + 4 * (c * v.psize + 1 + v.psy + v.psz) + ci;
-        float a = 0.f;
-#pragma unroll
-        for (int u = 0; u < 27; ++u)
-          a = fmaf(az.w[u / 9] * ay.w[u / 3 % 3] * ax.w[u % 3], t[az.o[u / 9] + ay.o[u / 3 % 3] + ax.o[u % 3]], a);
-        const float d = sm[cv.oi + row], rv = d != 0.f ? a : 0.f;
-        if (smoothed) {
-          if (row >= clo && row < clo + cv.rpc) sm[cv.orr + c * cv.rpc + row - clo] = rv;
-          sm[cv.ox + 4 * (c * cv.psize + (I + 1) + cv.psy * (J + 1) + cv.psz * (K + 1)) + ci] = wc * d * rv;
-        } else {
-          sm[tl.ocr + c * nc + row] = rv;
-        }
+        const int lr = split(it, nr, &c);
+        __pipeline_memcpy_async(sm + v.orr + c * v.rpc + lr, v.r + ((int64_t)c * v.rows + lo + lr), 4);
       }
-      __syncthreads();
+    } else {
+      for (int it = tid; it < nc * ncase; it += nth) __pipeline_memcpy_async(sm + tl.ocr + it, v.r + it, 4);
     }
-    for (int it = rank * nwarp + warp; it < nc * g; it += kMgTailCtas * nwarp) {  // coarsest: x = A^-1 r, a warp a row
+  }
+  __pipeline_commit();
+  __pipeline_wait_prior(0);
+  __syncthreads();
+  mg_cluster_wait();
+  // rows of A x on level l, x in shared memory; the result handed to put(case, row, its word, value)
+  auto apply = [&](const MgTailLevel& v, int mode, float w, auto&& put) {
+    const int lo = rank * v.rpc, nr = max(0, min(v.rpc, v.rows - lo));
+    const int sy = 4 * v.psy, sz = 4 * v.psz;
+    for (int it = tid; it < nr * ncase; it += nth) {
       int c;
-      const int row = split(it, nc, &c);
-      const float* r = sm + tl.ocr + c * nc;
-      double acc = 0.0;
-      for (int col = lane; col < nc; col += 32) acc = fma(tl.ainv[(int64_t)row * nc + col], (double)r[col], acc);
+      const int lr = split(it, nr, &c), row = lo + lr, n = row / 3, ci = row - 3 * n;
+      const int at = 4 * (c * v.psize + pad(v, n));
+      const float* x = sm + v.ox + at;
+      float a = 0.f;
+      const float4* s4 = reinterpret_cast<const float4*>(sm + v.oS + lr * kTailEnt);
+      float s[kTailEnt];
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-      if (lane < kMgTailCtas) {
-        uint32_t ra;
-        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(smem_u32(sm + tl.ocx + c * nc + row)), "r"(lane));
-        asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(ra), "f"((float)acc) : "memory");
+      for (int q = 0; q < kTailEnt / 4; ++q) {
+        const float4 t = s4[q];
+        s[4 * q] = t.x; s[4 * q + 1] = t.y; s[4 * q + 2] = t.z; s[4 * q + 3] = t.w;
       }
+#pragma unroll
+      for (int nb = 0; nb < 27; ++nb) {
+        const float4 xm = *reinterpret_cast<const float4*>(x + 4 * (nb % 3 - 1) + sy * ((nb / 3) % 3 - 1) + sz * (nb / 9 - 1));
+        a = fmaf(s[3 * nb], xm.x, fmaf(s[3 * nb + 1], xm.y, fmaf(s[3 * nb + 2], xm.z, a)));
+      }
+      const float id = sm[v.oi + row], rv = sm[v.orr + c * v.rpc + lr];
+      put(c, row, at + ci, mode == 1 ? fmaf(w * id, rv - a, x[ci]) : (id != 0.0f ? rv - a : 0.0f));
     }
+  };
+  for (int l = T; l < L - 1; ++l) {
+    const MgTailLevel& v = tl.lv[l];
+    const MgTailLevel& cv = tl.lv[l + 1];
+    apply(v, 2, 0.0f, [&](int, int, int at, float val) { mg_put_all(sm + v.ot + at, val); });
     mg_cluster_arrive();
     mg_cluster_wait();
-    for (int l = L - 2; l >= T; --l) {
-      const MgTailLevel& v = tl.lv[l];
-      const MgTailLevel& cv = tl.lv[l + 1];
-      // the coarse x: three floats a node on the coarsest level, else padded (a smoothed level's is where t was)
-      const bool coarsest = l + 1 == L - 1;
-      const int cs = coarsest ? 3 : 4, csy = coarsest ? cs * (cv.d.nx + 1) : cs * cv.psy,
-                csz = coarsest ? csy * (cv.d.ny + 1) : cs * cv.psz;
-      for (int it = tid; it < (int)v.nn * g; it += nth) {  // prolongation, every CTA for itself
-        int c;
-        const int n = split(it, (int)v.nn, &c), q = smi[v.oc + n], i = q & 1023, j = q >> 10 & 1023, k = q >> 20;
-        // per axis: two coarse nodes and their weights (an absent second one has weight 0 and is not read)
-        int o[3][2];
-        float w[3][2];
-        auto axis = [&](int a, int f_, int n_, int nc_, int stride) {
-          const bool mid = (f_ & 1) && f_ != n_;
-          const int c_ = ((f_ & 1) && f_ == n_) ? nc_ : (f_ >> 1);
-          o[a][0] = c_ * stride;
-          o[a][1] = mid ? o[a][0] + stride : o[a][0];
-          w[a][0] = mid ? 0.5f : 1.0f;
-          w[a][1] = mid ? 0.5f : 0.0f;
-        };
-        axis(0, i, v.d.nx, cv.d.nx, cs);
-        axis(1, j, v.d.ny, cv.d.ny, csy);
-        axis(2, k, v.d.nz, cv.d.nz, csz);
-        const float* xc = coarsest ? sm + tl.ocx + c * nc : sm + cv.ot + 4 * (c * cv.psize + 1 + cv.psy + cv.psz);
-        float a[3] = {0.f, 0.f, 0.f};
+    const bool smoothed = l + 1 < L - 1;
+    const float wc = smoothed ? om[l + 1] : 0.0f;
+    const int clo = rank * cv.rpc;
+    for (int it = tid; it < cv.rows * ncase; it += nth) {  // restriction, every CTA for itself
+      int c;
+      const int row = split(it, cv.rows, &c), n = row / 3, ci = row - 3 * n, q = smi[cv.oc + n];
+      const int I = q & 1023, J = q >> 10 & 1023, K = q >> 20;
+      const MgAxis ax(I, v.d.nx, 4), ay(J, v.d.ny, 4 * v.psy), az(K, v.d.nz, 4 * v.psz);
+      const float* t = sm + v.ot + 4 * (c * v.psize + 1 + v.psy + v.psz) + ci;
+      float a = 0.f;
 #pragma unroll
-        for (int u = 0; u < 8; ++u) {
-          const float wt = w[0][u & 1] * w[1][u >> 1 & 1] * w[2][u >> 2];
-          const float* p = xc + o[0][u & 1] + o[1][u >> 1 & 1] + o[2][u >> 2];
-#pragma unroll
-          for (int ci = 0; ci < 3; ++ci) a[ci] = fmaf(wt, p[ci], a[ci]);
-        }
-        float* x = sm + v.ox + 4 * (c * v.psize + (i + 1) + v.psy * (j + 1) + v.psz * (k + 1));
-#pragma unroll
-        for (int ci = 0; ci < 3; ++ci)
-          if (sm[v.oi + 3 * n + ci] != 0.0f) x[ci] += a[ci];
-      }
-      __syncthreads();
-      if (l > T) {  // the smoothed x goes where t was
-        apply(v, 1, om[l], [&](int, int, int at, float val) { mg_put_all(sm + v.ot + at, val); });
-        mg_cluster_arrive();
-        mg_cluster_wait();
+      for (int u = 0; u < 27; ++u)
+        a = fmaf(az.w[u / 9] * ay.w[u / 3 % 3] * ax.w[u % 3], t[az.o[u / 9] + ay.o[u / 3 % 3] + ax.o[u % 3]], a);
+      const float d = sm[cv.oi + row], rv = d != 0.f ? a : 0.f;
+      if (smoothed) {
+        if (row >= clo && row < clo + cv.rpc) sm[cv.orr + c * cv.rpc + row - clo] = rv;
+        sm[cv.ox + 4 * (c * cv.psize + (I + 1) + cv.psy * (J + 1) + cv.psz * (K + 1)) + ci] = wc * d * rv;
       } else {
-        apply(v, 1, om[l], [&](int c, int row, int, float val) {
-          if (live >> (c0 + c) & 1) v.xa[(int64_t)(c0 + c) * v.rows + row] = val;
-        });
+        sm[tl.ocr + c * nc + row] = rv;
       }
     }
-    if (T == L - 1 && rank == 0)
-      for (int it = tid; it < nc * g; it += nth)
-        if (live >> (c0 + it / nc) & 1) tl.lv[T].xa[(int64_t)c0 * nc + it] = sm[tl.ocx + it];
+    __syncthreads();
   }
+  for (int it = rank * nwarp + warp; it < nc * ncase; it += kMgTailCtas * nwarp) {  // coarsest: x = A^-1 r, a warp a row
+    int c;
+    const int row = split(it, nc, &c);
+    const float* r = sm + tl.ocr + c * nc;
+    double acc = 0.0;
+    for (int col = lane; col < nc; col += 32) acc = fma(tl.ainv[(int64_t)row * nc + col], (double)r[col], acc);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    if (lane < kMgTailCtas) {
+      uint32_t ra;
+      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(smem_u32(sm + tl.ocx + c * nc + row)), "r"(lane));
+      asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(ra), "f"((float)acc) : "memory");
+    }
+  }
+  mg_cluster_arrive();
+  mg_cluster_wait();
+  for (int l = L - 2; l >= T; --l) {
+    const MgTailLevel& v = tl.lv[l];
+    const MgTailLevel& cv = tl.lv[l + 1];
+    // the coarse x: three floats a node on the coarsest level, else padded (a smoothed level's is where t was)
+    const bool coarsest = l + 1 == L - 1;
+    const int cs = coarsest ? 3 : 4, csy = coarsest ? cs * (cv.d.nx + 1) : cs * cv.psy,
+              csz = coarsest ? csy * (cv.d.ny + 1) : cs * cv.psz;
+    for (int it = tid; it < (int)v.nn * ncase; it += nth) {  // prolongation, every CTA for itself
+      int c;
+      const int n = split(it, (int)v.nn, &c), q = smi[v.oc + n], i = q & 1023, j = q >> 10 & 1023, k = q >> 20;
+      // per axis: two coarse nodes and their weights (an absent second one has weight 0 and is not read)
+      int o[3][2];
+      float w[3][2];
+      auto axis = [&](int a, int f_, int n_, int nc_, int stride) {
+        const bool mid = (f_ & 1) && f_ != n_;
+        const int c_ = ((f_ & 1) && f_ == n_) ? nc_ : (f_ >> 1);
+        o[a][0] = c_ * stride;
+        o[a][1] = mid ? o[a][0] + stride : o[a][0];
+        w[a][0] = mid ? 0.5f : 1.0f;
+        w[a][1] = mid ? 0.5f : 0.0f;
+      };
+      axis(0, i, v.d.nx, cv.d.nx, cs);
+      axis(1, j, v.d.ny, cv.d.ny, csy);
+      axis(2, k, v.d.nz, cv.d.nz, csz);
+      const float* xc = coarsest ? sm + tl.ocx + c * nc : sm + cv.ot + 4 * (c * cv.psize + 1 + cv.psy + cv.psz);
+      float a[3] = {0.f, 0.f, 0.f};
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        const float wt = w[0][u & 1] * w[1][u >> 1 & 1] * w[2][u >> 2];
+        const float* p = xc + o[0][u & 1] + o[1][u >> 1 & 1] + o[2][u >> 2];
+#pragma unroll
+        for (int ci = 0; ci < 3; ++ci) a[ci] = fmaf(wt, p[ci], a[ci]);
+      }
+      float* x = sm + v.ox + 4 * (c * v.psize + (i + 1) + v.psy * (j + 1) + v.psz * (k + 1));
+#pragma unroll
+      for (int ci = 0; ci < 3; ++ci)
+        if (sm[v.oi + 3 * n + ci] != 0.0f) x[ci] += a[ci];
+    }
+    __syncthreads();
+    if (l > T) {  // the smoothed x goes where t was
+      apply(v, 1, om[l], [&](int, int, int at, float val) { mg_put_all(sm + v.ot + at, val); });
+      mg_cluster_arrive();
+      mg_cluster_wait();
+    } else {
+      apply(v, 1, om[l], [&](int c, int row, int, float val) {
+        if (live >> c & 1) v.xa[(int64_t)c * v.rows + row] = val;
+      });
+    }
+  }
+  if (T == L - 1 && rank == 0)
+    for (int it = tid; it < nc * ncase; it += nth)
+      if (live >> (it / nc) & 1) tl.lv[T].xa[it] = sm[tl.ocx + it];
 }
 
 template <bool MULTI>
 __global__ void __launch_bounds__(kMgTailThreads)
     k_mg_tail(const __grid_constant__ MgTail tl, const float* __restrict__ om, const MixState* st, int ncase) {
   extern __shared__ __align__(16) float tail_smem[];
-  if (tl.group) {
+  if (tl.in_smem) {
     mg_tail_smem(tl, om, st, ncase, (int)blockIdx.x, false, tail_smem);
   } else {
     dep_begin();
@@ -3175,11 +3151,10 @@ __global__ void __launch_bounds__(kMgTailThreads)
   }
 }
 
-// Shared-memory layout of mg_tail_smem for the levels from T and up to ncase load cases: every level's stencil rows
-// resident if that leaves room for a case, else the finest level's read from global memory; as many cases at once
-// as fit. group 0: not even one does (or several sweeps are asked for), the vectors stay in global memory.
+// Shared-memory layout of mg_tail_smem for the levels from T on, their stencil rows resident, and ncase load cases;
+// whether it fits.
 constexpr int kMgTailSmemMax = 220 * 1024;
-static bool mg_tail_layout(MgTail& tl, int g, bool resident) {
+static bool mg_tail_layout(MgTail& tl, int ncase) {
   int64_t o = 0;
   auto take = [&](int64_t n) {
     const int64_t at = o;
@@ -3196,34 +3171,26 @@ static bool mg_tail_layout(MgTail& tl, int g, bool resident) {
     v.psy = v.d.nx + 3;
     v.psz = v.psy * (v.d.ny + 3);
     v.psize = v.psz * (v.d.nz + 3);
-    v.ox = take((int64_t)g * 4 * v.psize);
-    v.ot = take((int64_t)g * 4 * v.psize);
-    v.orr = take((int64_t)g * v.rpc);
-    v.oS = resident || l > tl.T ? take((int64_t)kTailEnt * v.rpc) : -1;
+    v.ox = take((int64_t)ncase * 4 * v.psize);
+    v.ot = take((int64_t)ncase * 4 * v.psize);
+    v.orr = take((int64_t)ncase * v.rpc);
+    v.oS = take((int64_t)kTailEnt * v.rpc);
   }
-  tl.ocr = take((int64_t)g * tl.nc);
-  tl.ocx = take((int64_t)g * tl.nc);
-  tl.group = g;
+  tl.ocr = take((int64_t)ncase * tl.nc);
+  tl.ocx = take((int64_t)ncase * tl.nc);
   tl.smem = (int)std::min<int64_t>(o * (int64_t)sizeof(float), INT_MAX);
   return o * (int64_t)sizeof(float) <= kMgTailSmemMax;
 }
-// The tail of ncase load cases: from the first level of at most kMgTailMaxNodes nodes whose cases all fit with its
-// stencil (a level that took its cases in several passes, or its stencil from L2, is cheaper as separate kernels:
-// 125 us against about 50 for four cases on 1,683 nodes); none fits or several sweeps: from the first level of at
-// most kMgTailMaxNodes nodes, as few cases at a time as must be.
+// The tail of ncase load cases: from the first level of at most kMgTailMaxNodes nodes that fits for all of them with its
+// stencil and the levels below it (the coarsest always does: 10 KB). A level that took its cases in several passes, or
+// its stencil from L2, was dearer than separate kernels: 125 us against about 50 for four cases on 1,683 nodes. Several
+// sweeps: vectors in global memory (mg_tail_body), from the first level of at most kMgTailMaxNodes nodes.
 static void mg_tail_plan(MgTail& tl, int ncase) {
-  const int T0 = tl.T, gmax = std::min(ncase, kMgMaxCases);
-  if (tl.sweeps == 1) {
-    for (tl.T = T0; tl.T < tl.L; ++tl.T)
-      if (mg_tail_layout(tl, gmax, true)) return;
-    tl.T = T0;
-    for (int resident = 1; resident >= 0; --resident)
-      for (int g = gmax; g >= 1; --g)
-        if (mg_tail_layout(tl, g, resident != 0)) return;
-  }
-  tl.T = T0;
-  tl.group = 0;
-  tl.smem = 0;
+  tl.in_smem = tl.sweeps == 1;
+  if (tl.in_smem)
+    while (!mg_tail_layout(tl, ncase) && tl.T < tl.L - 1) ++tl.T;
+  else
+    tl.smem = 0;
 }
 
 // End of an outer step's first part: ||r|| against the stop and replacement thresholds.
@@ -5438,7 +5405,7 @@ template <bool MULTI>
 __global__ void __launch_bounds__(kMgTailThreads) k_mg_tail_pk(const PkTail* __restrict__ tab) {
   extern __shared__ __align__(16) float tail_smem[];
   const PkTail& t = tab[blockIdx.x / kMgTailCtas];
-  if (t.tl.group) {
+  if (t.tl.in_smem) {
     mg_tail_smem(t.tl, t.om, t.st, t.ncase, (int)(blockIdx.x % kMgTailCtas), true, tail_smem);
   } else {
     dep_begin();
