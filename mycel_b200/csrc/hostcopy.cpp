@@ -40,7 +40,6 @@ struct HostCopy {
   std::vector<cudaEvent_t> ev;     // per slot: its latest copy
   std::vector<char> used;
   std::vector<std::thread> threads;
-  std::mutex call;                 // one copy at a time
 
   std::mutex mu;
   std::condition_variable wake;
@@ -127,22 +126,23 @@ struct HostCopy {
       pinned = nullptr;
       return false;
     }
-    used.assign(2 * (size_t)want, 0);
-    for (int k = 0; k < 2 * want; ++k) {
-      cudaEvent_t e;
-      if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) {
-        cudaGetLastError();
-        return false;
-      }
-      ev.push_back(e);
-    }
     parts = 1;
     try {
+      used.assign(2 * (size_t)want, 0);
+      ev.reserve(2 * (size_t)want);
+      for (int k = 0; k < 2 * want; ++k) {
+        cudaEvent_t e;
+        if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) {
+          cudaGetLastError();
+          return false;
+        }
+        ev.push_back(e);
+      }
       for (int w = 1; w < want; ++w) {
         threads.emplace_back([this, w] { loop(w); });
         ++parts;
       }
-    } catch (...) {  // no more threads to be had: the ones there are
+    } catch (...) {  // no more memory or threads to be had: the threads there are
     }
     return parts >= 2;
   }
