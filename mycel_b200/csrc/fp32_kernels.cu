@@ -2725,6 +2725,7 @@ __global__ void __launch_bounds__(1024) k_mg_coarse_setup(MgDims d, const float*
 // stencil and the levels below it (33x17x16 -> 17x9x9 nodes; mg_tail_layout), and the copies at the start take half as
 // long as with eight (16.8 against 20.9 us for 480 + 105 + 24 nodes).
 constexpr int kMgTailCtas = 16, kMgTailThreads = 512;
+constexpr int kMgTailPortable = 8;  // CTAs of the form without shared memory where the opt-in size cannot be scheduled
 // levels of at most this many nodes go to the cluster kernel, as far as they fit (mg_tail_plan)
 constexpr int64_t kMgTailMaxNodes = 2048;
 
@@ -2743,6 +2744,7 @@ struct MgTailLevel {
 struct MgTail {
   int T, L, sweeps, nc;
   const double* ainv;
+  int ctas;      // of the cluster: kMgTailCtas, or kMgTailPortable
   bool in_smem;  // levels and vectors in shared memory (mg_tail_smem), else vectors in global memory (mg_tail_body)
   int ocr, ocx;  // shared-memory offsets of the coarsest level's r and x (nc a case)
   int smem;      // its bytes
@@ -2759,7 +2761,7 @@ __device__ __forceinline__ void mg_cluster_sync() {
 // smoothed correction of level T, left in its xa. Work items are numbered with the case fastest; a case whose
 // state is not running is skipped, and the kernel returns at once (every thread alike) when none is.
 // Body for the threads gt (of gs) of the cluster that runs this V-cycle's tail, with the vectors in global memory: for
-// several sweeps (mg_tail_plan).
+// several sweeps, and where the shared-memory form cannot be scheduled (mg_tail_plan, mg_tail_fit).
 template <bool MULTI>
 __device__ __forceinline__ void mg_tail_body(const MgTail& tl, const float* __restrict__ om, const MixState* st,
                                              int ncase, int64_t gt, int64_t gs) {
@@ -3186,6 +3188,7 @@ static bool mg_tail_layout(MgTail& tl, int ncase) {
 // its stencil from L2, was dearer than separate kernels: 125 us against about 50 for four cases on 1,683 nodes. Several
 // sweeps: vectors in global memory (mg_tail_body), from the first level of at most kMgTailMaxNodes nodes.
 static void mg_tail_plan(MgTail& tl, int ncase) {
+  tl.ctas = kMgTailCtas;
   tl.in_smem = tl.sweeps == 1;
   if (tl.in_smem)
     while (!mg_tail_layout(tl, ncase) && tl.T < tl.L - 1) ++tl.T;
@@ -3761,6 +3764,42 @@ void mg_release(mycel_problem* p) {
 
 static const void* mg_tail_pk_kernel(bool multi);  // the packed launches' cluster kernel
 
+// whether a cluster of the plan's size and shared memory can be resident, of the single and the packed kernel
+static bool mg_tail_schedulable(const MgTail& tl, bool multi) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)tl.ctas);
+  cfg.blockDim = dim3(kMgTailThreads);
+  cfg.dynamicSmemBytes = (size_t)tl.smem;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = (unsigned)tl.ctas;
+  at.val.clusterDim.y = 1;
+  at.val.clusterDim.z = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  const void* single = multi ? (const void*)k_mg_tail<true> : (const void*)k_mg_tail<false>;
+  for (const void* k : {single, mg_tail_pk_kernel(multi)}) {
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, k, &cfg) != cudaSuccess || n < 1) {
+      cudaGetLastError();
+      return false;
+    }
+  }
+  return true;
+}
+// The plan for ncase cases from tl's levels that this device can run: sixteen CTAs with the shared memory it needs, else
+// (a part of a GPU, say) eight with the vectors in global memory; false if neither. MYCEL_MG_TAIL=global takes the
+// second at once (for comparisons).
+static bool mg_tail_fit(MgTail& out, const MgTail& tl, int ncase, bool multi) {
+  const char* e = std::getenv("MYCEL_MG_TAIL");
+  out = tl;
+  mg_tail_plan(out, ncase);
+  if (!(e && !std::strcmp(e, "global")) && mg_tail_schedulable(out, multi)) return true;
+  out = tl;
+  out.ctas = kMgTailPortable;
+  return mg_tail_schedulable(out, multi);
+}
+
 static int32_t mg_ensure(mycel_problem* p, bool* available) {
   static std::once_flag smem_once;
   static cudaError_t smem_err = cudaSuccess;
@@ -3774,10 +3813,9 @@ static int32_t mg_ensure(mycel_problem* p, bool* available) {
                           mg_tail_pk_kernel(true)})
       if (smem_err == cudaSuccess)
         smem_err = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kMgTailSmemMax);
-    if (kMgTailCtas > 8)
-      for (const void* k : {(const void*)k_mg_tail<false>, (const void*)k_mg_tail<true>, mg_tail_pk_kernel(false),
-                            mg_tail_pk_kernel(true)})
-        if (smem_err == cudaSuccess) smem_err = cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    for (const void* k : {(const void*)k_mg_tail<false>, (const void*)k_mg_tail<true>, mg_tail_pk_kernel(false),
+                          mg_tail_pk_kernel(true)})
+      if (smem_err == cudaSuccess) smem_err = cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
   });
   if (smem_err != cudaSuccess)
     return set_error(p->ctx, MYCEL_E_DEVICE, std::string("multigrid shared memory: ") + cudaGetErrorString(smem_err));
@@ -3871,26 +3909,7 @@ static int32_t mg_ensure(mycel_problem* p, bool* available) {
     cudaMemcpyAsync(mg->G, G.data(), sizeof(float) * G.size(), cudaMemcpyHostToDevice, s);
     cudaStreamSynchronize(s);
   }
-  {  // the cluster kernel must fit: kMgTailCtas CTAs of kMgTailThreads threads co-resident
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(kMgTailCtas);
-    cfg.blockDim = dim3(kMgTailThreads);
-    cfg.dynamicSmemBytes = kMgTailSmemMax;
-    cudaLaunchAttribute at{};
-    at.id = cudaLaunchAttributeClusterDimension;
-    at.val.clusterDim.x = kMgTailCtas;
-    at.val.clusterDim.y = 1;
-    at.val.clusterDim.z = 1;
-    cfg.attrs = &at;
-    cfg.numAttrs = 1;
-    int nclusters = 0;
-    int ncl2 = 0;
-    if (cudaOccupancyMaxActiveClusters(&nclusters, k_mg_tail<false>, &cfg) != cudaSuccess || nclusters < 1 ||
-        cudaOccupancyMaxActiveClusters(&ncl2, k_mg_tail<true>, &cfg) != cudaSuccess || ncl2 < 1) {
-      cudaGetLastError();
-      return set_error(p->ctx, MYCEL_E_DEVICE, "multigrid: the coarse-level cluster kernel cannot be scheduled");
-    }
-  }
+  bool fits = true;
   // levels T .. L-1 in one cluster launch: T is the first coarse level of at most kMgTailMaxNodes nodes
   MgTail tl{};
   tl.T = L - 1;
@@ -3907,15 +3926,18 @@ static int32_t mg_ensure(mycel_problem* p, bool* available) {
     const MgLevel& v = mg->lv[l];
     tl.lv[l] = {v.d, v.nn, v.S, v.invd, v.xa, v.xb, v.r, v.t};
   }
-  mg->tails[0] = mg->tails[1] = tl;
-  mg_tail_plan(mg->tails[0], 1);
-  mg_tail_plan(mg->tails[1], mg->ncap);
+  for (int multi = 0; multi < 2; ++multi)
+    if (!mg_tail_fit(mg->tails[multi], tl, multi ? mg->ncap : 1, multi != 0)) fits = false;
   // launches per outer iteration: matvec, k_mg_enter*, the V-cycle (as issued by mg_vcycle), k_mg_exit*
   const int sw = mg->sweeps, T = mg->tails[0].T;
   const int cycle = 4 * (sw - 1) + 2 + (T - 1) * (1 + sw) + 1 + (T - 1) * (1 + sw) + 1 + 1;
   mg->per_iter = 3 + cycle;
   p->mg = mg;
   if (oom) return set_error(p->ctx, MYCEL_E_OOM, "out of device memory for the multigrid hierarchy");
+  if (!fits) {
+    mg_release(p);
+    return set_error(p->ctx, MYCEL_E_DEVICE, "multigrid: the coarse-level cluster kernel cannot be scheduled");
+  }
   *available = true;
   return MYCEL_OK;
 }
@@ -3927,15 +3949,15 @@ static unsigned mg_blocks(int64_t n) { return (unsigned)((n + 255) / 256); }
 // the small levels' kernel: one cluster of kMgTailCtas with cluster barriers between phases (a single CTA with CTA
 // barriers was measured slower: 51.9 against 56.6 SIMP iter/s on the bridge)
 static void launch_mg_tail(cudaStream_t s, MgHier* mg, const float* om, const MixState* st, int nc) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(kMgTailCtas);
-  cfg.blockDim = dim3(kMgTailThreads);
   const MgTail& tl = mg->tail(nc);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)tl.ctas);
+  cfg.blockDim = dim3(kMgTailThreads);
   cfg.dynamicSmemBytes = (size_t)tl.smem;
   cfg.stream = s;
   cudaLaunchAttribute at[2] = {};
   at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = kMgTailCtas;
+  at[0].val.clusterDim.x = (unsigned)tl.ctas;
   at[0].val.clusterDim.y = 1;
   at[0].val.clusterDim.z = 1;
   at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // see dep_begin
@@ -5402,15 +5424,15 @@ struct PkTail {  // the cluster kernel of a problem's V-cycle (all its cases); o
 };
 
 template <bool MULTI>
-__global__ void __launch_bounds__(kMgTailThreads) k_mg_tail_pk(const PkTail* __restrict__ tab) {
+__global__ void __launch_bounds__(kMgTailThreads) k_mg_tail_pk(const PkTail* __restrict__ tab, unsigned ctas) {
   extern __shared__ __align__(16) float tail_smem[];
-  const PkTail& t = tab[blockIdx.x / kMgTailCtas];
+  const PkTail& t = tab[blockIdx.x / ctas];
+  const unsigned rank = blockIdx.x % ctas;
   if (t.tl.in_smem) {
-    mg_tail_smem(t.tl, t.om, t.st, t.ncase, (int)(blockIdx.x % kMgTailCtas), true, tail_smem);
+    mg_tail_smem(t.tl, t.om, t.st, t.ncase, (int)rank, true, tail_smem);
   } else {
     dep_begin();
-    mg_tail_body<MULTI>(t.tl, t.om, t.st, t.ncase, (int64_t)(blockIdx.x % kMgTailCtas) * blockDim.x + threadIdx.x,
-                        (int64_t)kMgTailCtas * blockDim.x);
+    mg_tail_body<MULTI>(t.tl, t.om, t.st, t.ncase, (int64_t)rank * blockDim.x + threadIdx.x, (int64_t)ctas * blockDim.x);
   }
 }
 static const void* mg_tail_pk_kernel(bool multi) {
@@ -5476,6 +5498,7 @@ struct PkLaunch {
   unsigned grid;    // persistent CTAs of the launch
   bool few;         // at most three items an SM
   size_t smem = 0;  // cluster kernel: the largest shared memory of its entries
+  unsigned ctas = 0;  // cluster kernel: CTAs of a cluster, the same for its entries
 };
 
 // A right-hand side of a packed solve: its voxel-level FP32 vectors, state, RHS and solution.
@@ -5685,21 +5708,21 @@ static void pk_issue(const PackPlan& P, const PkLaunch& L, cudaStream_t s, int s
     }
     case PK_TAIL: {  // one cluster per problem (not listed: a done problem's cluster returns at once)
       cudaLaunchConfig_t cfg = {};
-      cfg.gridDim = dim3((unsigned)(kMgTailCtas * L.n));
+      cfg.gridDim = dim3(L.ctas * (unsigned)L.n);
       cfg.blockDim = dim3(kMgTailThreads);
       cfg.dynamicSmemBytes = L.smem;
       cfg.stream = s;
       cudaLaunchAttribute at[2] = {};
       at[0].id = cudaLaunchAttributeClusterDimension;
-      at[0].val.clusterDim.x = kMgTailCtas;
+      at[0].val.clusterDim.x = L.ctas;
       at[0].val.clusterDim.y = 1;
       at[0].val.clusterDim.z = 1;
       at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // see dep_begin
       at[1].val.programmaticStreamSerializationAllowed = 1;
       cfg.attrs = at;
       cfg.numAttrs = P.early ? 2 : 1;
-      if (L.multi) cudaLaunchKernelEx(&cfg, k_mg_tail_pk<true>, (const PkTail*)tab);
-      else cudaLaunchKernelEx(&cfg, k_mg_tail_pk<false>, (const PkTail*)tab);
+      if (L.multi) cudaLaunchKernelEx(&cfg, k_mg_tail_pk<true>, (const PkTail*)tab, L.ctas);
+      else cudaLaunchKernelEx(&cfg, k_mg_tail_pk<false>, (const PkTail*)tab, L.ctas);
       break;
     }
   }
@@ -5944,28 +5967,28 @@ static int32_t pk_build(mycel_ctx* c, PackWork* w, std::vector<PkUnit>& units, c
       B.add(P.vcycle, PK_RESTRICT, false, multi == 1, 0, e, nb, es);
     }
   }
-  for (int multi = 0; multi < 2; ++multi) {  // the cluster kernels
+  for (int form = 0; form < 4; ++form) {  // the cluster kernels: one case or several, by the clusters' size
+    const bool multi = (form & 1) != 0;
+    const int ctas = form & 2 ? kMgTailPortable : kMgTailCtas;
     std::vector<PkTail> e;
     std::vector<unsigned> nb;
     std::vector<std::pair<MixState*, int>> es;
+    size_t smem = 0;
     for (size_t qi = 0; qi < probs.size(); ++qi) {
       const Prob& q = probs[qi];
-      if ((q.nc > 1) != (multi == 1)) continue;
       MgHier* mg = q.p->mg;
-      PkTail t{};
-      t.tl = mg->tail(q.nc);
-      t.om = mg->sc->omega;
-      t.st = q.st;
-      t.ncase = q.nc;
-      e.push_back(t);
-      nb.push_back(kMgTailCtas);
+      const MgTail& tl = mg->tail(q.nc);
+      if ((q.nc > 1) != multi || tl.ctas != ctas) continue;
+      e.push_back({tl, mg->sc->omega, q.st, q.nc});
+      nb.push_back((unsigned)ctas);
       es.push_back({const_cast<MixState*>(q.st), q.nc});
-      xc[qi][t.tl.T] = mg->lv[t.tl.T].xa;
+      xc[qi][tl.T] = mg->lv[tl.T].xa;
+      smem = std::max(smem, (size_t)tl.smem);
     }
-    size_t smem = 0;
-    for (const PkTail& t : e) smem = std::max(smem, (size_t)t.tl.smem);
-    B.add(P.vcycle, PK_TAIL, false, multi == 1, 0, e, nb, es);
-    if (!e.empty()) P.vcycle.back().smem = smem;
+    B.add(P.vcycle, PK_TAIL, false, multi, 0, e, nb, es);
+    if (e.empty()) continue;
+    P.vcycle.back().smem = smem;
+    P.vcycle.back().ctas = (unsigned)ctas;
   }
   for (int l = maxT - 1; l >= 1; --l) {
     for (int multi = 0; multi < 2; ++multi) {  // level l + 1 -> l, into xa (the downward sweep's vector)
