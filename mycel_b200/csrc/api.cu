@@ -43,6 +43,7 @@ cudaError_t dalloc(mycel_problem* p, T** ptr, size_t count) {
   // work of others running on other streams (the serving loop)
   cudaError_t e = cudaMallocAsync((void**)ptr, bytes, p->ctx->stream);
   if (e == cudaSuccess) p->device_bytes += (int64_t)bytes;
+  else (void)cudaGetLastError();  // the caller reports it
   return e;
 }
 
@@ -107,11 +108,12 @@ void fill_result(const PcgState& st, mycel_pcg_result* res) {
 }  // namespace
 namespace mycel {
 int32_t ensure_pcg_workspace(mycel_problem* p) {
-  if (p->d_x) return MYCEL_OK;
+  if (p->d_state) return MYCEL_OK;  // the last one: after a failure a later call takes what is missing
   int64_t nd = p->g.nd;
   int64_t nb = num_blocks8192(nd);
-  if (dalloc(p, &p->d_x, nd) || dalloc(p, &p->d_r, nd) || dalloc(p, &p->d_z, nd) || dalloc(p, &p->d_p, nd) ||
-      dalloc(p, &p->d_ap, nd) || dalloc(p, &p->d_part, 2 * nb + 64) || dalloc(p, &p->d_state, 1))
+  for (double** v : {&p->d_x, &p->d_r, &p->d_z, &p->d_p, &p->d_ap})
+    if (!*v && dalloc(p, v, nd)) return set_error(p->ctx, MYCEL_E_OOM, "out of device memory for the PCG workspace");
+  if ((!p->d_part && dalloc(p, &p->d_part, 2 * nb + 64)) || dalloc(p, &p->d_state, 1))
     return set_error(p->ctx, MYCEL_E_OOM, "out of device memory for the PCG workspace");
   cudaMemsetAsync(p->d_state, 0, sizeof(PcgState), p->ctx->stream);
   return MYCEL_OK;

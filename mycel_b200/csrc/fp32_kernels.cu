@@ -3558,12 +3558,16 @@ static int32_t ensure_mixed(mycel_problem* p) {
   });
   if (smem_err != cudaSuccess)
     return set_error(p->ctx, MYCEL_E_DEVICE, std::string("matvec shared memory: ") + cudaGetErrorString(smem_err));
-  if (p->f_x) return MYCEL_OK;
+  if (p->f_ready) return MYCEL_OK;
   const size_t fb = sizeof(float) * (size_t)p->g.n32 + 64;
   cudaError_t e = cudaSuccess;
   float** bufs[] = {&p->f_x, &p->f_r, &p->f_z, &p->f_p0, &p->f_p1, &p->f_ap};
   for (float** b : bufs) {
-    if ((e = cudaMallocAsync((void**)b, fb, p->ctx->stream)) != cudaSuccess) break;
+    if (*b) continue;  // of an earlier call that ran out of memory
+    if ((e = cudaMallocAsync((void**)b, fb, p->ctx->stream)) != cudaSuccess) {
+      (void)cudaGetLastError();
+      break;
+    }
     p->device_bytes += (int64_t)fb;
     cudaMemsetAsync(*b, 0, fb, p->ctx->stream);
   }
@@ -3573,6 +3577,7 @@ static int32_t ensure_mixed(mycel_problem* p) {
     int32_t st = encode_plane_map(p, mapped[q], false, &p->f_tmap[q]);
     if (st) return st;
   }
+  p->f_ready = true;
   return MYCEL_OK;
 }
 
@@ -3600,12 +3605,16 @@ static int32_t ensure_f64f(mycel_problem* p) {
   });
   if (smem_err != cudaSuccess)
     return set_error(p->ctx, MYCEL_E_DEVICE, std::string("FP64 matvec shared memory: ") + cudaGetErrorString(smem_err));
-  if (p->g_x) return MYCEL_OK;
+  if (p->g_ready) return MYCEL_OK;
   const size_t fb = sizeof(double) * (size_t)p->g.n64 + 64;
   cudaError_t e = cudaSuccess;
   double** bufs[] = {&p->g_x, &p->g_r, &p->g_z, &p->g_p0, &p->g_p1, &p->g_ap, &p->g_invd};
   for (double** b : bufs) {
-    if ((e = cudaMallocAsync((void**)b, fb, p->ctx->stream)) != cudaSuccess) break;
+    if (*b) continue;  // of an earlier call that ran out of memory
+    if ((e = cudaMallocAsync((void**)b, fb, p->ctx->stream)) != cudaSuccess) {
+      (void)cudaGetLastError();
+      break;
+    }
     p->device_bytes += (int64_t)fb;
     cudaMemsetAsync(*b, 0, fb, p->ctx->stream);
   }
@@ -3615,6 +3624,7 @@ static int32_t ensure_f64f(mycel_problem* p) {
     int32_t st = encode_plane_map(p, mapped[q], true, &p->g_tmap[q]);
     if (st) return st;
   }
+  p->g_ready = true;
   return MYCEL_OK;
 }
 
@@ -3833,14 +3843,16 @@ static int32_t mg_ensure(mycel_problem* p, bool* available) {
   if (const char* e = std::getenv("MYCEL_MG_SWEEPS")) mg->sweeps = std::max(1, std::atoi(e));
   cudaStream_t s = p->ctx->stream;
   bool oom = false;
+  int64_t taken = 0;
   auto alloc = [&](size_t bytes) -> void* {
     void* ptr = nullptr;
     if (oom || cudaMallocAsync(&ptr, bytes + 64, s) != cudaSuccess) {
+      (void)cudaGetLastError();
       oom = true;
       return nullptr;
     }
     cudaMemsetAsync(ptr, 0, bytes + 64, s);
-    p->device_bytes += (int64_t)bytes + 64;
+    taken += (int64_t)bytes + 64;
     mg->bufs.push_back(ptr);
     return ptr;
   };
@@ -3933,11 +3945,12 @@ static int32_t mg_ensure(mycel_problem* p, bool* available) {
   const int cycle = 4 * (sw - 1) + 2 + (T - 1) * (1 + sw) + 1 + (T - 1) * (1 + sw) + 1 + 1;
   mg->per_iter = 3 + cycle;
   p->mg = mg;
-  if (oom) return set_error(p->ctx, MYCEL_E_OOM, "out of device memory for the multigrid hierarchy");
-  if (!fits) {
+  if (oom || !fits) {  // nothing is kept: a later call starts over
     mg_release(p);
-    return set_error(p->ctx, MYCEL_E_DEVICE, "multigrid: the coarse-level cluster kernel cannot be scheduled");
+    return oom ? set_error(p->ctx, MYCEL_E_OOM, "out of device memory for the multigrid hierarchy")
+               : set_error(p->ctx, MYCEL_E_DEVICE, "multigrid: the coarse-level cluster kernel cannot be scheduled");
   }
+  p->device_bytes += taken;
   *available = true;
   return MYCEL_OK;
 }
@@ -4694,19 +4707,21 @@ static int32_t mg_ensure_cases(mycel_problem* p, int n) {
   if (cw.n > 0 || n > mg->ncap) return set_error(p->ctx, MYCEL_E_ARG, "multigrid case workspace: too many cases");
   cudaStream_t s = p->ctx->stream;
   const size_t fb = sizeof(float) * (size_t)p->g.n32 + 64;
+  auto oom = [&] {
+    (void)cudaGetLastError();
+    return set_error(p->ctx, MYCEL_E_OOM, "out of device memory for the load cases' multigrid workspace");
+  };
   for (int k = 0; k < n; ++k)
     for (int q = 0; q < 7; ++q) {
       void* b = nullptr;
-      if (cudaMallocAsync(&b, fb, s) != cudaSuccess)
-        return set_error(p->ctx, MYCEL_E_OOM, "out of device memory for the load cases' multigrid workspace");
+      if (cudaMallocAsync(&b, fb, s) != cudaSuccess) return oom();
       cudaMemsetAsync(b, 0, fb, s);
       p->device_bytes += (int64_t)fb;
       mg->bufs.push_back(b);
       cw.v[k][q] = (float*)b;
     }
   void* st = nullptr;
-  if (cudaMallocAsync(&st, sizeof(MixState) * n, s) != cudaSuccess)
-    return set_error(p->ctx, MYCEL_E_OOM, "out of device memory for the load cases' multigrid workspace");
+  if (cudaMallocAsync(&st, sizeof(MixState) * n, s) != cudaSuccess) return oom();
   cudaMemsetAsync(st, 0, sizeof(MixState) * n, s);
   p->device_bytes += (int64_t)(sizeof(MixState) * n);
   mg->bufs.push_back(st);

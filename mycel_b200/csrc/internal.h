@@ -186,6 +186,7 @@ struct mycel_problem {
   mycel::PcgState* d_state = nullptr;
   // mixed-form workspace
   float *f_x = nullptr, *f_r = nullptr, *f_z = nullptr, *f_p0 = nullptr, *f_p1 = nullptr, *f_ap = nullptr;
+  bool f_ready = false, g_ready = false;  // all of it is there, its TMA descriptors too (g: the fast FP64 form's)
   CUtensorMap f_tmap[4];          // TMA descriptors of f_r, f_z, f_p0, f_p1 (node-plane boxes of the FP32 matvec)
   // fast FP64 form (factorised operator, FP64 recurrences): padded FP64 work vectors, TMA maps, graphs
   double *g_x = nullptr, *g_r = nullptr, *g_z = nullptr, *g_p0 = nullptr, *g_p1 = nullptr, *g_ap = nullptr,
