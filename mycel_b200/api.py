@@ -51,9 +51,23 @@ class Context:
         _check(lib.mycel_ctx_create(device, C.byref(h)))
         self.handle = h.value
         self.device = device
+        # live problems' handles and their live filters': the members of a reference cycle, and the globals of an
+        # ending program, are finalised in no particular order, so each closes what belongs to it first
+        self._problems = {}
+
+    def _end_problem(self, handle):
+        filters = self._problems.pop(handle, None)
+        if filters is None:  # ended with the context
+            return
+        for f in filters:
+            L.load().mycel_filter_destroy(f)
+        filters.clear()
+        L.load().mycel_problem_destroy(handle)  # ends its sessions
 
     def close(self):
         if getattr(self, "handle", None):
+            for h in list(self._problems):
+                self._end_problem(h)
             L.load().mycel_ctx_destroy(self.handle)
             self.handle = None
 
@@ -136,13 +150,14 @@ class Problem:
                                         fixed.ctypes.data if fixed.size else None, fixed.size, loads, len(model.loads),
                                         dens.ctypes.data, model.penal, C.byref(h)), self.ctx)
         self.handle = h.value
+        self._filters = self.ctx._problems[self.handle] = set()
         self._keep = []
 
     def close(self):
         if getattr(self, "handle", None):
             for sess in list(getattr(self, "_sessions", ())):
                 sess.close()
-            L.load().mycel_problem_destroy(self.handle)
+            self.ctx._end_problem(self.handle)
             self.handle = None
 
     def __del__(self):
@@ -244,10 +259,13 @@ class DensityFilter:
         _check(L.load().mycel_filter_create(problem.handle, float(rmin), C.byref(h)), problem.ctx)
         self.handle = h.value
         self.n = problem.model.active_element_count
+        problem._filters.add(self.handle)
 
     def close(self):
         if getattr(self, "handle", None):
-            L.load().mycel_filter_destroy(self.handle)
+            if self.handle in self.problem._filters:  # an ended problem has ended its filters already
+                self.problem._filters.discard(self.handle)
+                L.load().mycel_filter_destroy(self.handle)
             self.handle = None
 
     def __del__(self):
@@ -672,7 +690,7 @@ class SimpSession:
 
     def close(self):
         if getattr(self, "handle", None):
-            if getattr(self.problem, "handle", None):  # a destroyed problem has ended its sessions already
+            if self.problem.handle in self.problem.ctx._problems:  # an ended problem has ended its sessions already
                 L.load().mycel_simp_end(self.handle)
             self.handle = None
 
