@@ -4,13 +4,20 @@
 // GB/s out of it into freshly allocated arrays, whose pages the same thread faults in one by one. Here large copies go
 // in chunks through pinned slots of the context, and a few threads fill or empty the slots (and touch the caller's
 // pages) while the copy engine runs. 16-core host, 192x96x96: a static solve that returns 58 MB in fresh arrays 37.3 ->
-// 23.6 ms, creating its problem (25 MB in) 5.9 -> 3.3 ms; a product K x of 5.6 MB either way 0.91 -> 0.56 ms.
+// 23.6 ms, creating its problem (25 MB in) 5.3 -> 2.8 ms; a product K x of 44 MB either way 13.0 -> 3.3 ms, of 5.6 MB
+// 1.12 -> 1.00 ms.
+// What the threads touch costs more to unmap afterwards (every core that ran one is interrupted): a caller that makes
+// and drops an array for each call loses what the copy gains, up to 0.2 ms at 2 MB and 0.9 ms at 14 MB. So the mesh
+// entry points, which get arrays made for the call, take their inputs by the driver's copy.
 //
 // The threads and slots belong to the context: made at its first large copy, given back with it. One copy at a time
 // per context; contexts are independent. Memory the driver already knows (pinned, managed, device) and short copies
 // take cudaMemcpyAsync, as does everything where the threads or slots cannot be had.
 #include <cuda_runtime.h>
 #include <string.h>
+#if defined(__SSE2__)
+#include <emmintrin.h>
+#endif
 
 #include <algorithm>
 #include <atomic>
@@ -30,6 +37,27 @@ constexpr size_t kStagedMin = 1 << 20;   // shorter copies: waking the threads c
 constexpr size_t kSlot = 1 << 20;        // bytes of a pinned slot, the largest chunk
 constexpr size_t kMinChunk = 128 << 10;
 constexpr int kMaxThreads = 6;           // the caller's thread and up to five more
+
+// Into a slot (16-byte aligned), past the caches: from lines that six cores' caches hold the copy engine read at a third
+// of the speed, and copies of 3 to 16 MB took longer than the driver's (us, driver / cached stores / these: 2 MB 143 /
+// 145 / 110, 8 MB 485 / 693 / 288, 16 MB 870 / 1,100 / 490, 32 MB 1,800 / 1,550 / 960).
+void fill_slot(char* slot, const char* src, size_t n) {
+#if defined(__SSE2__)
+  size_t i = 0;
+  for (; i + 64 <= n; i += 64) {
+    const __m128i a = _mm_loadu_si128((const __m128i*)(src + i)), b = _mm_loadu_si128((const __m128i*)(src + i + 16));
+    const __m128i c = _mm_loadu_si128((const __m128i*)(src + i + 32)), d = _mm_loadu_si128((const __m128i*)(src + i + 48));
+    _mm_stream_si128((__m128i*)(slot + i), a);
+    _mm_stream_si128((__m128i*)(slot + i + 16), b);
+    _mm_stream_si128((__m128i*)(slot + i + 32), c);
+    _mm_stream_si128((__m128i*)(slot + i + 48), d);
+  }
+  memcpy(slot + i, src + i, n - i);
+  _mm_sfence();
+#else
+  memcpy(slot, src, n);
+#endif
+}
 
 }  // namespace
 
@@ -84,7 +112,7 @@ struct HostCopy {
     if (!to_host) {
       for (size_t c; (c = next.fetch_add(1)) < chunks; s ^= 1) {
         if (!slot_ready(s)) return;
-        memcpy(pinned + (size_t)s * kSlot, host + c * chunk, len(c));
+        fill_slot(pinned + (size_t)s * kSlot, host + c * chunk, len(c));
         if (!issue(c, s)) return;
       }
       return;

@@ -743,7 +743,8 @@ int32_t surface_nets_core(mycel_ctx* ctx, int32_t nx, int32_t ny, int32_t nz, fl
   int* d_flags = (int*)alloc(sizeof(int) * 8);
   if (oom) return set_error(ctx, MYCEL_E_OOM, "out of device memory for the iso-surface");
   long long* h_scal = (long long*)ctx->pinned;  // at least 64 bytes of pinned scratch
-  if (h_density) MYCEL_CUDA(ctx, copy_in(ctx, d_in, h_density, sizeof(float) * n));
+  // the driver's copy: the array is often made for this call, see hostcopy.cpp
+  if (h_density) MYCEL_CUDA(ctx, cudaMemcpyAsync(d_in, h_density, sizeof(float) * n, cudaMemcpyHostToDevice, s));
   MYCEL_CUDA(ctx, cudaMemsetAsync(d_scal, 0, sizeof(long long) * 8, s));
   MYCEL_CUDA(ctx, cudaMemsetAsync(d_flags, 0, sizeof(int) * 8, s));
   const int nsm = ctx->num_sms;
@@ -891,8 +892,10 @@ extern "C" int32_t mycel_taubin_smooth(mycel_ctx* ctx, float* positions, int64_t
   if (oom) return set_error(ctx, MYCEL_E_OOM, "out of device memory for the mesh smoother");
   int* h_bad = (int*)ctx->pinned;
   const int nsm = ctx->num_sms;
-  MYCEL_CUDA(ctx, copy_in(ctx, d_idx, indices, sizeof(int32_t) * ni));
-  MYCEL_CUDA(ctx, copy_in(ctx, d_a, positions, sizeof(float) * 3 * nv));
+  // the driver's copies: mesh arrays are often made for this call, see hostcopy.cpp (75 thousand vertices, us: 613, through
+  // the slots 831)
+  MYCEL_CUDA(ctx, cudaMemcpyAsync(d_idx, indices, sizeof(int32_t) * ni, cudaMemcpyHostToDevice, s));
+  MYCEL_CUDA(ctx, cudaMemcpyAsync(d_a, positions, sizeof(float) * 3 * nv, cudaMemcpyHostToDevice, s));
   MYCEL_CUDA(ctx, cudaMemsetAsync(d_bad, 0, sizeof(int), s));
   MYCEL_CUDA(ctx, cudaMemsetAsync(d_deg, 0, sizeof(int32_t) * nv, s));
   k_tb_check<<<sn_grid_blocks(ni, nsm), 256, 0, s>>>(ni, d_idx, nv, d_bad);
