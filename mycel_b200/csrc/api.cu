@@ -421,6 +421,7 @@ extern "C" int32_t mycel_ctx_create(int32_t device, mycel_ctx** out) {
     cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
   }
   cudaGetLastError();
+  host_copy_attach(c);
   *out = c;
   return MYCEL_OK;
 }

@@ -8,11 +8,14 @@
 // 1.12 -> 1.00 ms.
 // What the threads touch costs more to unmap afterwards (every core that ran one is interrupted): a caller that makes
 // and drops an array for each call loses what the copy gains, up to 0.2 ms at 2 MB and 0.9 ms at 14 MB. So the mesh
-// entry points, which get arrays made for the call, take their inputs by the driver's copy.
+// entry points, whose arrays are often made for the call, leave their copies to the driver.
 //
-// The threads and slots belong to the context: made at its first large copy, given back with it. One copy at a time
-// per context; contexts are independent. Memory the driver already knows (pinned, managed, device) and short copies
-// take cudaMemcpyAsync, as does everything where the threads or slots cannot be had.
+// The threads and slots belong to the device, at most kMaxCopiers sets of them: made at the first large copies, borrowed by
+// one copy at a time, given back with the device's last context. (A set for each context made contexts that come and go
+// expensive: making and freeing 12 MB of pinned memory each, and a free waits for the device and holds up the other
+// contexts' launches. Four contexts of 12 problems each took 58 ms to set up instead of 35 to 42 (22 without any), and where one ended
+// before the others these stood still for up to 0.7 s.) Memory the driver already knows (pinned, managed, device) and short
+// copies take cudaMemcpyAsync, as does everything where the threads or slots cannot be had.
 #include <cuda_runtime.h>
 #include <string.h>
 #if defined(__SSE2__)
@@ -37,6 +40,7 @@ constexpr size_t kStagedMin = 1 << 20;   // shorter copies: waking the threads c
 constexpr size_t kSlot = 1 << 20;        // bytes of a pinned slot, the largest chunk
 constexpr size_t kMinChunk = 128 << 10;
 constexpr int kMaxThreads = 6;           // the caller's thread and up to five more
+constexpr int kMaxCopiers = 2;           // of a device: copies that find none idle are the driver's
 
 // Into a slot (16-byte aligned), past the caches: from lines that six cores' caches hold the copy engine read at a third
 // of the speed, and copies of 3 to 16 MB took longer than the driver's (us, driver / cached stores / these: 2 MB 143 /
@@ -210,9 +214,57 @@ struct HostCopy {
   }
 };
 
+// The copiers of a device: contexts borrow one for the length of a copy. All are given back with the device's last
+// context.
+struct Pool {
+  std::mutex mu;
+  HostCopy* idle[kMaxCopiers] = {};
+  int n_idle = 0, made = 0;
+  int contexts = 0;
+  bool failed = false;  // threads or slots could not be had: not tried again before the next first context
+};
+static Pool* pool_of(int device) {
+  static Pool pools[64];
+  return device >= 0 && device < 64 ? &pools[device] : nullptr;
+}
+
+void host_copy_attach(mycel_ctx* c) {
+  if (Pool* p = pool_of(c->device)) {
+    std::lock_guard<std::mutex> l(p->mu);
+    ++p->contexts;
+  }
+}
+
 void host_copy_release(mycel_ctx* c) {
-  delete c->copier;
-  c->copier = nullptr;
+  Pool* p = pool_of(c->device);
+  if (!p) return;
+  HostCopy* old[kMaxCopiers];
+  int n = 0;
+  {
+    std::lock_guard<std::mutex> l(p->mu);
+    if (--p->contexts > 0) return;
+    while (p->n_idle > 0) old[n++] = p->idle[--p->n_idle];
+    p->made = 0;
+    p->failed = false;
+  }
+  while (n > 0) delete old[--n];
+}
+
+// one that is idle, a new one up to the bound, or none
+static HostCopy* borrow(Pool* p, int device) {
+  {
+    std::lock_guard<std::mutex> l(p->mu);
+    if (p->n_idle > 0) return p->idle[--p->n_idle];
+    if (p->failed || p->made == kMaxCopiers || p->contexts == 0) return nullptr;
+    ++p->made;
+  }
+  HostCopy* h = new (std::nothrow) HostCopy();
+  if (h && h->start(device)) return h;
+  delete h;
+  std::lock_guard<std::mutex> l(p->mu);
+  --p->made;
+  p->failed = true;
+  return nullptr;
 }
 
 static cudaError_t host_copy(mycel_ctx* c, bool out, void* h, void* d, size_t n) {
@@ -225,22 +277,17 @@ static cudaError_t host_copy(mycel_ctx* c, bool out, void* h, void* d, size_t n)
     return plain();
   }
   if (a.type != cudaMemoryTypeUnregistered) return plain();
-  std::lock_guard<std::mutex> one(c->copier_mu);
-  if (!c->copier && !c->copier_failed) {
-    HostCopy* p = new (std::nothrow) HostCopy();
-    if (p && !p->start(c->device)) {
-      delete p;
-      p = nullptr;
-    }
-    c->copier = p;
-    c->copier_failed = !p;
-  }
-  if (!c->copier) return plain();
+  Pool* p = pool_of(c->device);
   if (out) {  // wait for the producers here, not in every thread
     const cudaError_t e = cudaStreamSynchronize(c->stream);
     if (e != cudaSuccess) return e;
   }
-  return c->copier->run(out, (char*)h, (char*)d, n, c->stream);
+  HostCopy* k = p ? borrow(p, c->device) : nullptr;
+  if (!k) return plain();
+  const cudaError_t e = k->run(out, (char*)h, (char*)d, n, c->stream);
+  std::lock_guard<std::mutex> l(p->mu);
+  p->idle[p->n_idle++] = k;
+  return e;
 }
 
 cudaError_t copy_in(mycel_ctx* c, void* d, const void* h, size_t n) {

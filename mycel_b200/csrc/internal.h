@@ -4,7 +4,6 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
-#include <mutex>
 #include <string>
 #include <vector>
 
@@ -94,7 +93,6 @@ struct DevBuf {
 };
 
 struct MgHier;  // multigrid hierarchy of a problem (fp32_kernels.cu)
-struct HostCopy;  // hostcopy.cpp
 }  // namespace mycel
 
 // ---- opaque handles of the C ABI ----
@@ -120,9 +118,6 @@ struct mycel_ctx {
   void* fan = nullptr;     // side streams for independent per-problem work of a batch step (mycel::fan_*)
   cudaStream_t main_stream = nullptr, main_side = nullptr;  // the context's own streams while a fan slot is in use
   int64_t packed_rhs = 0;  // right-hand sides whose solves ran through packed launches (a statistic)
-  mycel::HostCopy* copier = nullptr;  // threads and pinned slots of large host copies, made on first use
-  bool copier_failed = false;
-  std::mutex copier_mu;
 };
 
 struct mycel_problem {
@@ -378,7 +373,8 @@ inline bool dep_early(const mycel_problem* p) { return p->g.nd <= (int64_t)4096 
 // the bytes are there (pinned memory): synchronise the stream before they are read.
 cudaError_t copy_in(mycel_ctx* c, void* d, const void* h, size_t n);
 cudaError_t copy_out(mycel_ctx* c, void* h, const void* d, size_t n);
-void host_copy_release(mycel_ctx* c);
+void host_copy_attach(mycel_ctx* c);   // once at a context's creation
+void host_copy_release(mycel_ctx* c);  // once at its end
 void pack_release(mycel_ctx* c);
 // Asynchronous packed run (mycel_simp_run_many): the right-hand sides of the jobs share one packed plan for a
 // whole optimisation and each job's solves start and end on their own. pkr_open leaves out the jobs the

@@ -917,7 +917,7 @@ extern "C" int32_t mycel_taubin_smooth(mycel_ctx* ctx, float* positions, int64_t
     ctx->launches += 2;
   }
   MYCEL_CUDA(ctx, cudaGetLastError());
-  MYCEL_CUDA(ctx, copy_out(ctx, positions, d_a, sizeof(float) * 3 * nv));
+  MYCEL_CUDA(ctx, cudaMemcpyAsync(positions, d_a, sizeof(float) * 3 * nv, cudaMemcpyDeviceToHost, s));
   MYCEL_CUDA(ctx, cudaStreamSynchronize(s));
   return MYCEL_OK;
 }
