@@ -1409,9 +1409,8 @@ static void launch_mv64f(mycel_problem* p, cudaStream_t s, const double* xin, co
   }
   const dim3 grid((unsigned)((g.nx1 + FOX - 1) / FOX), (unsigned)((g.ny1 + FOY - 1) / FOY),
                   (unsigned)((g.nz1 + zs - 1) / zs));
-  launch_dep(dep_early(p), k_mv64f<MODE>, grid, dim3(FX, FY), fac64_smem_bytes(MODE), s,
-               g, p->hexop64, *ta, *tb, pnew, y, p->d_E,
-                                                                     p->d_nflags, projected, st, part, zs, p->d_err);
+  launch_dep(dep_early(p), k_mv64f<MODE>, grid, dim3(FX, FY), fac64_smem_bytes(MODE), s, g, p->hexop64, *ta, *tb, pnew,
+             y, p->d_E, p->d_nflags, projected, st, part, zs, p->d_err);
 }
 
 // resident CTAs per SM of the factorised FP32 matvec (same for both modes: same block, registers within bounds);
@@ -1451,8 +1450,8 @@ static void launch_mv32_variant(mycel_problem* p, cudaStream_t s, const float* x
       std::fprintf(stderr, "mycel: FP32 matvec input is not a mapped work vector\n");
       std::abort();
     }
-    launch_dep(dep_early(p), k_mv32f<MODE>, fac_grid(g, zs), dim3(FX, FY), fac_smem_bytes(MODE), s,
-               g, p->hexop, *ta, *tb, pnew, y, p->d_Ef, p->d_nflags, projected, st, part, zs, p->d_err);
+    launch_dep(dep_early(p), k_mv32f<MODE>, fac_grid(g, zs), dim3(FX, FY), fac_smem_bytes(MODE), s, g, p->hexop, *ta,
+               *tb, pnew, y, p->d_Ef, p->d_nflags, projected, st, part, zs, p->d_err);
   }
 }
 
@@ -2637,10 +2636,9 @@ template <bool PAD>
 static void launch_mg_prolong(bool early, cudaStream_t s, const MgDims& f, int pitch, const uint8_t* nf,
                               const float* invdf,
                               const MgPtrs& xf, const MgDims& c, const MgPtrs& xc, const MixState* st, int nc) {
-  launch_dep(early, (mg_by_pairs(f, nc) ? (nc == 1 ? k_mg_prolong<PAD, false, true> : k_mg_prolong<PAD, true, true>)
-                      : (nc == 1 ? k_mg_prolong<PAD, false, false> : k_mg_prolong<PAD, true, false>)),
-             mg_prolong_blocks(f, nc), kMgDofThreads, 0, s,
-               f, pitch, nf, invdf, xf, c, xc, st, nc);
+  auto k = mg_by_pairs(f, nc) ? (nc == 1 ? k_mg_prolong<PAD, false, true> : k_mg_prolong<PAD, true, true>)
+                              : (nc == 1 ? k_mg_prolong<PAD, false, false> : k_mg_prolong<PAD, true, false>);
+  launch_dep(early, k, mg_prolong_blocks(f, nc), kMgDofThreads, 0, s, f, pitch, nf, invdf, xf, c, xc, st, nc);
 }
 
 
@@ -3957,8 +3955,6 @@ static int32_t mg_ensure(mycel_problem* p, bool* available) {
 
 static unsigned mg_blocks(int64_t n) { return (unsigned)((n + 255) / 256); }
 
-// coarse-level product on the stream: a thread per DOF up to 64k nodes, a thread per node above (measured on
-// the bridge: level 2, 31k nodes, 9.6 vs 14.5 us; level 1, 233k nodes, 43 vs 51 us)
 // the small levels' kernel: one cluster of kMgTailCtas with cluster barriers between phases (a single CTA with CTA
 // barriers was measured slower: 51.9 against 56.6 SIMP iter/s on the bridge)
 static void launch_mg_tail(cudaStream_t s, MgHier* mg, const float* om, const MixState* st, int nc) {
@@ -3988,19 +3984,21 @@ static MgPtrs lv_ptrs(float* base, int64_t nd, int n) {
   return r;
 }
 
+// coarse-level product on the stream: a thread per DOF up to 64k nodes, a thread per node above (measured on
+// the bridge: level 2, 31k nodes, 9.6 vs 14.5 us; level 1, 233k nodes, 43 vs 51 us)
 static void launch_mg_apply(cudaStream_t s, const MgLevel& v, const MgPtrs& x, const MgPtrs& r, const float* invd,
                             const MgPtrs& y, int mode, const float* om, const MixState* st, int nc) {
-  if (v.nn * nc <= kMgDofMaxNodes)
-    launch_dep(v.early, (v.nn * nc <= v.max_shared ? (nc == 1 ? k_mg_apply<false, true> : k_mg_apply<true, true>)
-                               : (nc == 1 ? k_mg_apply<false, false> : k_mg_apply<true, false>)),
-               mg_dof_blocks(v.nn * nc), kMgDofThreads, 0, s,
-               v.d, v.S, x, r, invd, y, mode, om, st, nc);
-  else if (nc == 1 && v.staged)
-    launch_dep(v.early, k_mg_apply_nodes_tma, (unsigned)((v.nn + kS1Nodes - 1) / kS1Nodes), 256, kS1Smem, s,
-               v.d, v.tm_s, x.p[0], r.p[0], invd, y.p[0], mode, om, st, v.err);
-  else
+  if (v.nn * nc <= kMgDofMaxNodes) {
+    auto k = v.nn * nc <= v.max_shared ? (nc == 1 ? k_mg_apply<false, true> : k_mg_apply<true, true>)
+                                       : (nc == 1 ? k_mg_apply<false, false> : k_mg_apply<true, false>);
+    launch_dep(v.early, k, mg_dof_blocks(v.nn * nc), kMgDofThreads, 0, s, v.d, v.S, x, r, invd, y, mode, om, st, nc);
+  } else if (nc == 1 && v.staged) {
+    launch_dep(v.early, k_mg_apply_nodes_tma, (unsigned)((v.nn + kS1Nodes - 1) / kS1Nodes), 256, kS1Smem, s, v.d,
+               v.tm_s, x.p[0], r.p[0], invd, y.p[0], mode, om, st, v.err);
+  } else {
     launch_dep(v.early, (nc == 1 ? k_mg_apply_nodes<false> : k_mg_apply_nodes<true>), mg_blocks(v.nn * nc), 256, 0, s,
                v.d, v.S, x, r, invd, y, mode, om, st, nc);
+  }
 }
 
 // Per case the input (MODE 0: x; 1: z, with the old direction), pnew and y of launch_mv32_variant, which runs them one
@@ -4032,9 +4030,8 @@ static int launch_mv32_cases(mycel_problem* p, cudaStream_t s, int n, float* con
       v.pitch = pitch;
       v.tiles_z = (int)grid.z;
       grid.z *= (unsigned)n;
-      launch_dep(dep_early(p), k_mv32f_cases<MODE>, grid, dim3(FX, FY), fac_smem_bytes(MODE), s,
-               p->g, p->hexop, v, p->d_Ef, p->d_nflags, zs,
-                                                                           p->d_err);
+      launch_dep(dep_early(p), k_mv32f_cases<MODE>, grid, dim3(FX, FY), fac_smem_bytes(MODE), s, p->g, p->hexop, v,
+                 p->d_Ef, p->d_nflags, zs, p->d_err);
       return 1;
     }
   }
@@ -4151,11 +4148,9 @@ static int mg_vcycle(mycel_problem* p, cudaStream_t s, const MgRun& R) {
   nl += launch_mv32_cases<0>(p, s, nc, R.xf, nullptr, nullptr, R.tf, st, R.pitch);
   // restriction to level 1, with level 1's first sweep (unless level 1 is the coarsest)
   launch_dep(lv[1].early, (nc == 1 ? k_mg_restrict<true, false> : k_mg_restrict<true, true>),
-             mg_dof_blocks(lv[1].nn * nc), kMgDofThreads, 0, s,
-               lv[0].d, g.rp, mg_ptrs(R.rf, nc), mg_ptrs(R.tf, nc),
-                                                               lv[1].d, lv[1].invd, lv_ptrs(lv[1].r, lv[1].nd, nc), st,
-                                                               lv_ptrs(lv[1].xa, lv[1].nd, nc), 1 < mg->L - 1 ? 1 : 0,
-                                                               om + 1, nc);
+             mg_dof_blocks(lv[1].nn * nc), kMgDofThreads, 0, s, lv[0].d, g.rp, mg_ptrs(R.rf, nc), mg_ptrs(R.tf, nc),
+             lv[1].d, lv[1].invd, lv_ptrs(lv[1].r, lv[1].nd, nc), st, lv_ptrs(lv[1].xa, lv[1].nd, nc),
+             1 < mg->L - 1 ? 1 : 0, om + 1, nc);
   nl++;
   float* xc[kMgMaxLevels] = {};
   for (int l = 1; l < T; ++l) {
@@ -4171,12 +4166,9 @@ static int mg_vcycle(mycel_problem* p, cudaStream_t s, const MgRun& R) {
     if (l == 1 && mg->l1_timing) cudaEventRecordWithFlags(mg->l1_timing[1], s, cudaEventRecordExternal);
     MgLevel& cv = lv[l + 1];
     launch_dep(cv.early, (nc == 1 ? k_mg_restrict<false, false> : k_mg_restrict<false, true>),
-               mg_dof_blocks(cv.nn * nc), kMgDofThreads, 0, s,
-               v.d, 0, lv_ptrs(nullptr, 0, nc),
-                                                               lv_ptrs(v.t, v.nd, nc), cv.d, cv.invd,
-                                                               lv_ptrs(cv.r, cv.nd, nc), st,
-                                                               lv_ptrs(cv.xa, cv.nd, nc), l + 1 < mg->L - 1 ? 1 : 0,
-                                                               om + l + 1, nc);
+               mg_dof_blocks(cv.nn * nc), kMgDofThreads, 0, s, v.d, 0, lv_ptrs(nullptr, 0, nc), lv_ptrs(v.t, v.nd, nc),
+               cv.d, cv.invd, lv_ptrs(cv.r, cv.nd, nc), st, lv_ptrs(cv.xa, cv.nd, nc), l + 1 < mg->L - 1 ? 1 : 0,
+               om + l + 1, nc);
     xc[l] = x;
     nl += 1 + mg->sweeps;
   }
@@ -4225,24 +4217,23 @@ static int launch_mg_step(mycel_problem* p, cudaStream_t s, const void* pcur, in
   MgRun R;
   R.st = st;
   if (f64) {
-    launch_dep(dep_early(p), (outer_wide(p, sb) ? k_mg_enter<8> : k_mg_enter<2>), sb, kT, 0, s,
-               p->g, p->g_x, p->g_r, (const double*)pcur, p->g_ap, p->d_invdf, p->f_r, p->f_p0, om, st, p->d_part2,
-               mode);
+    launch_dep(dep_early(p), (outer_wide(p, sb) ? k_mg_enter<8> : k_mg_enter<2>), sb, kT, 0, s, p->g, p->g_x, p->g_r,
+               (const double*)pcur, p->g_ap, p->d_invdf, p->f_r, p->f_p0, om, st, p->d_part2, mode);
     R.rf[0] = p->f_r;
     R.xf[0] = p->f_p0;
     R.tf[0] = p->f_ap;
     nl += 1 + mg_vcycle(p, s, R);
-    launch_dep(dep_early(p), (outer_wide(p, sb) ? k_mg_exit<8> : k_mg_exit<2>), sb, kT, 0, s,
-               p->g, p->f_r, p->f_ap, p->f_p0, p->d_invdf, p->g_r, p->g_ap, p->g_z, om, st, p->d_part2, mode);
+    launch_dep(dep_early(p), (outer_wide(p, sb) ? k_mg_exit<8> : k_mg_exit<2>), sb, kT, 0, s, p->g, p->f_r, p->f_ap,
+               p->f_p0, p->d_invdf, p->g_r, p->g_ap, p->g_z, om, st, p->d_part2, mode);
   } else {
-    launch_dep(dep_early(p), (outer_wide(p, sb) ? k_mg_enter32<4> : k_mg_enter32<1>), sb, kT, 0, s,
-               p->g.n32, p->f_x, p->f_r, (const float*)pcur, p->f_ap, p->d_invdf, p->f_z, om, st, p->d_part2, mode);
+    launch_dep(dep_early(p), (outer_wide(p, sb) ? k_mg_enter32<4> : k_mg_enter32<1>), sb, kT, 0, s, p->g.n32, p->f_x,
+               p->f_r, (const float*)pcur, p->f_ap, p->d_invdf, p->f_z, om, st, p->d_part2, mode);
     R.rf[0] = p->f_r;
     R.xf[0] = p->f_z;
     R.tf[0] = mg->f_t;
     nl += 1 + mg_vcycle(p, s, R);
-    launch_dep(dep_early(p), (outer_wide(p, sb) ? k_mg_exit32<4> : k_mg_exit32<1>), sb, kT, 0, s,
-               p->g.n32, p->f_r, mg->f_t, p->f_z, p->d_invdf, p->f_ap, om, st, p->d_part2, mode);
+    launch_dep(dep_early(p), (outer_wide(p, sb) ? k_mg_exit32<4> : k_mg_exit32<1>), sb, kT, 0, s, p->g.n32, p->f_r,
+               mg->f_t, p->f_z, p->d_invdf, p->f_ap, om, st, p->d_part2, mode);
   }
   return nl + 1;
 }
@@ -4300,13 +4291,11 @@ static int launch_inner_xr(mycel_problem* p, const InnerForm& F, cudaStream_t s,
   const int sb = stream_blocks(p);
   if (F.mg) return launch_mg_step(p, s, pcur, mode, F.f64);
   if (F.f64)
-    launch_dep(dep_early(p), k_xr64, sb, kT, 0, s,
-               F.n, (double*)F.x, (double*)F.r, (double*)F.z, (const double*)pcur, (const double*)F.ap,
-                             (const double*)F.invd, mix_state(p), p->d_part2, mode);
+    launch_dep(dep_early(p), k_xr64, sb, kT, 0, s, F.n, (double*)F.x, (double*)F.r, (double*)F.z, (const double*)pcur,
+               (const double*)F.ap, (const double*)F.invd, mix_state(p), p->d_part2, mode);
   else
-    launch_dep(dep_early(p), k_xr32, sb, kT, 0, s,
-               F.n, (float*)F.x, (float*)F.r, (float*)F.z, (const float*)pcur, (const float*)F.ap,
-                             (const float*)F.invd, mix_state(p), p->d_part2, mode);
+    launch_dep(dep_early(p), k_xr32, sb, kT, 0, s, F.n, (float*)F.x, (float*)F.r, (float*)F.z, (const float*)pcur,
+               (const float*)F.ap, (const float*)F.invd, mix_state(p), p->d_part2, mode);
   return 1;
 }
 
@@ -4807,12 +4796,12 @@ static int launch_mg_step_cases(mycel_problem* p, cudaStream_t s, int n, const i
     return w;
   };
   for (int k = 0; k < n; k += m, ++nl)
-    launch_dep(dep_early(p), (wide ? k_mg_enter32_cases<4> : k_mg_enter32_cases<1>), dim3(sb, m), kT, 0, s,
-               p->g.n32, from(k), p->d_invdf, om, R.st + k, p->d_part2, pitch, mode);
+    launch_dep(dep_early(p), (wide ? k_mg_enter32_cases<4> : k_mg_enter32_cases<1>), dim3(sb, m), kT, 0, s, p->g.n32,
+               from(k), p->d_invdf, om, R.st + k, p->d_part2, pitch, mode);
   nl += mg_vcycle(p, s, R);
   for (int k = 0; k < n; k += m, ++nl)
-    launch_dep(dep_early(p), (wide ? k_mg_exit32_cases<4> : k_mg_exit32_cases<1>), dim3(sb, m), kT, 0, s,
-               p->g.n32, from(k), p->d_invdf, om, R.st + k, p->d_part2, pitch, mode);
+    launch_dep(dep_early(p), (wide ? k_mg_exit32_cases<4> : k_mg_exit32_cases<1>), dim3(sb, m), kT, 0, s, p->g.n32,
+               from(k), p->d_invdf, om, R.st + k, p->d_part2, pitch, mode);
   return nl;
 }
 
@@ -5686,12 +5675,10 @@ static void pk_issue(const PackPlan& P, const PkLaunch& L, cudaStream_t s, int s
   const unsigned g = L.grid;
   switch (L.kind) {
     case PK_MV0:
-      launch_dep(P.early, k_mv32f_pk<0>, g, dim3(FX, FY), fac_smem_bytes(0), s,
-               (const PkMv*)tab, it, cn);
+      launch_dep(P.early, k_mv32f_pk<0>, g, dim3(FX, FY), fac_smem_bytes(0), s, (const PkMv*)tab, it, cn);
       break;
     case PK_MV1:
-      launch_dep(P.early, k_mv32f_pk<1>, g, dim3(FX, FY), fac_smem_bytes(1), s,
-               (const PkMv*)tab, it, cn);
+      launch_dep(P.early, k_mv32f_pk<1>, g, dim3(FX, FY), fac_smem_bytes(1), s, (const PkMv*)tab, it, cn);
       break;
     case PK_ENTER:
       launch_dep(P.early, pk_enter_kernel(L.few), g, kT, 0, s, (const PkVec*)tab, it, cn, step_mode);
@@ -5704,21 +5691,18 @@ static void pk_issue(const PackPlan& P, const PkLaunch& L, cudaStream_t s, int s
       break;
     case PK_APPLY_NODE:
       launch_dep(P.early, (L.multi ? k_mg_apply_nodes_pk<true> : k_mg_apply_nodes_pk<false>), g, 256, 0, s,
-               (const PkApply*)tab, it,
-                                                                                           cn, L.mode);
+                 (const PkApply*)tab, it, cn, L.mode);
       break;
     case PK_RESTRICT: {
       auto k = L.pad ? (L.multi ? k_mg_restrict_pk<true, true> : k_mg_restrict_pk<true, false>)
                      : (L.multi ? k_mg_restrict_pk<false, true> : k_mg_restrict_pk<false, false>);
-      launch_dep(P.early, k, g, kMgDofThreads, 0, s,
-               (const PkRestrict*)tab, it, cn);
+      launch_dep(P.early, k, g, kMgDofThreads, 0, s, (const PkRestrict*)tab, it, cn);
       break;
     }
     case PK_PROLONG: {
       auto k = L.pad ? (L.multi ? k_mg_prolong_pk<true, true> : k_mg_prolong_pk<true, false>)
                      : (L.multi ? k_mg_prolong_pk<false, true> : k_mg_prolong_pk<false, false>);
-      launch_dep(P.early, k, g, kMgDofThreads, 0, s,
-               (const PkProlong*)tab, it, cn);
+      launch_dep(P.early, k, g, kMgDofThreads, 0, s, (const PkProlong*)tab, it, cn);
       break;
     }
     case PK_TAIL: {  // one cluster per problem (not listed: a done problem's cluster returns at once)

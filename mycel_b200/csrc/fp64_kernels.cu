@@ -232,7 +232,7 @@ void launch_diag(mycel_problem* p) {
 // FUSE: x = z + beta p_old (or z at a start), formed in shared memory; the owned nodes' values go to p_new, so the
 // iteration needs no pass of its own for p.
 // Against the z-marching 64 x 4 tiles this replaces (per-node runtime KE rows), p update included: 30x10x4 elements
-// 29.9 -> 6.7 us, 96x48x24 51.3 -> 20.6 us, 192x96x96 446 (without p) -> 256 us. What is left over the FP64 pipe's
+// 29.9 -> 7.6 us, 96x48x24 51.3 -> 22.6 us, 192x96x96 446 (without p) -> 263 us. What is left over the FP64 pipe's
 // 10 and 133 us are issue slots: a constant load for each KE entry and the selects of the colour order.
 // ---------------------------------------------------------------------------------------------------------
 constexpr int kMvNodes = 128;
@@ -334,7 +334,7 @@ __global__ void __launch_bounds__(kMvNodes, 4) k_matvec64(GridDims g, const __gr
   double wl[4][3], wu[4][3];  // the elements below and above the node plane: [colour order][component]
   const bool io = i & 1, jo = j & 1;
   const double* xt = xs + 3 * (tid + 1);
-#pragma unroll 1  // half the code: the unrolled body waits for instructions (256 against 267 us on 192x96x96)
+#pragma unroll 1  // half the code: the unrolled body waits for instructions (4 % slower on 192x96x96)
   for (int sz = 0; sz < 2; ++sz) {
     const double* kz = ke.v + (1 - sz) * (4 * 3 * 24);  // KE rows of the node's local position in these elements
     const unsigned on4 = act >> (4 * sz);
@@ -452,8 +452,8 @@ void launch_pcg_matvec(mycel_problem* p, int it) {
 // for a producer's loads), the producers' accesses are contiguous over a warp (their traffic delays the chain's
 // loads: at a 32-byte stride the fused update's chain took 13.8 cycles an addition, now 11.7), and one group of
 // producers keeps ahead of the chain (two, or all chunks resident, were slower). 96x48x24 elements (44 blocks):
-// the direction's dot 22.0 -> 14.9 us, the fused update 30.8 -> 18.8 us; one block (30x10x4): 15.1 -> 9.3 and
-// 22.5 -> 10.8 us; 192x96x96 (666 blocks, bound by memory): 39 and 71 us.
+// the direction's dot 22.0 -> 15.0 us, the fused update 30.8 -> 16.5 us; one block (30x10x4): 15.1 -> 9.2 and
+// 22.5 -> 10.1 us; 192x96x96 (666 blocks, bound by memory): 39 and 74 us.
 constexpr int kCh = 768;                         // elements per chunk
 constexpr int kRing = 4;                         // chunks in shared memory
 constexpr int kRow = kCh / 4 + 4;                // doubles per staged lane row (no bank conflicts)
