@@ -165,6 +165,7 @@ typedef void (*mycel_progress_fn)(void* user, const mycel_iter_record* rec, cons
 /* ---- context ---- */
 int32_t mycel_version(void);
 int32_t mycel_ctx_create(int32_t device, mycel_ctx** out);
+/* After the context's problems, their filters and sessions: those free their memory on its stream. */
 int32_t mycel_ctx_destroy(mycel_ctx* ctx);
 /* The CUDA stream (cudaStream_t) all work of this context is issued on. */
 void* mycel_ctx_stream(mycel_ctx* ctx);
@@ -283,7 +284,7 @@ int32_t mycel_oc_update(mycel_ctx* ctx, int32_t n, const double* rho, const doub
    allocate device memory when they run this step (a host whose device memory is all reserved by another
    allocator in the process, or a loop that must not take the synchronisation of a cudaMalloc/cudaFree).
    rho, dc, s, passive (may be NULL) and rho_new are device pointers owned by the caller; lambda_out is a host
-   pointer. The kernel's scratch is a fixed 65.6 KB array inside the library, held by every GPU that loads it
+   pointer. The kernel's scratch is a fixed 98.4 KB array inside the library, held by every GPU that loads it
    until the process exits, sized for 1024 persistent blocks (devices that need more return MYCEL_E_ARG).
    The first call on a device looks up that array's device address, so make it before any stream capture.
    The work runs on the context's stream, which is not ordered after the caller's streams: the caller's writes
